@@ -105,6 +105,11 @@ int dr_destroy(dr_ctx *c) {
         c->band_cam_head.release();
         c->band_cam_pool.release();
         c->cam_used.release();
+        c->path_ctl.release();
+        c->path_active.release();
+        c->band_path_active.release();
+        c->path_rec_async.release();
+        c->path_rec_band.release();
         for (int k = 0; k < 2; ++k)
             if (c->band_stream[k]) cudaStreamSynchronize(c->band_stream[k]), cudaStreamDestroy(c->band_stream[k]);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream), cudaStreamDestroy(c->copy_stream);
@@ -189,6 +194,35 @@ int dr_set_occluders(dr_ctx *c, const dr_surface *surfaces, uint32_t n_surfaces,
     return DR_OK;
 }
 
+// Records of collided samples kept for a render of up to `pixels` pixels (slot
+// 0: asynchronous, else one of the blocking render's two band streams, which
+// render an eighth of a large tile's rows at a time): 16 MB to 512 MB (128 MB a
+// band stream), in proportion to the pixels in between.  A render whose paths
+// may exceed it runs in rounds, and a round without work costs about 8 us.
+static uint32_t rec_capacity(size_t pixels, uint32_t slot) {
+    const size_t most = slot ? (size_t)1 << 23 : (size_t)1 << 25, want = pixels * (slot ? 4 : 16);
+    return (uint32_t)std::min(most, std::max((size_t)1 << 20, want));
+}
+
+// Leaf list entries of one pool: as dr_set_camera_lists says, else 32 a pixel (8 a
+// band stream) up to kCamPool.
+static uint32_t pool_capacity(const dr_ctx *c, size_t pixels, uint32_t slot) {
+    if (c->cam_cap_set) return c->cam_cap;
+    return (uint32_t)std::min((size_t)dr_ctx::kCamPool, std::max((size_t)1 << 18, pixels * (slot ? 8 : 32)));
+}
+
+// Storage of a persistent launch's camera leaf lists and path pipeline: slot 0
+// for the asynchronous render, 1 and 2 (one allocation) for the band streams.
+static bool reserve_lists(dr_ctx *c, uint32_t slot, size_t pixels, uint32_t rec_cap) {
+    const uint32_t pool = pool_capacity(c, pixels, slot);
+    const size_t two = slot ? 2 : 1;
+    return c->cam_used.reserve(3) == cudaSuccess && c->path_ctl.reserve(3) == cudaSuccess &&
+           (slot ? c->band_cam_head : c->cam_head).reserve(2 * pixels) == cudaSuccess &&
+           (slot ? c->band_path_active : c->path_active).reserve(pixels) == cudaSuccess &&
+           (slot ? c->path_rec_band : c->path_rec_async).reserve(two * rec_cap) == cudaSuccess &&
+           (slot ? c->band_cam_pool : c->cam_pool).reserve((size_t)two * pool) == cudaSuccess;
+}
+
 int dr_set_params(dr_ctx *c, const dr_render_params *p) {
     if (!c || !p) return need(false, DR_ERR_INVALID, "dr_set_params: null argument");
     DevParams d;
@@ -216,16 +250,12 @@ int dr_set_params(dr_ctx *c, const dr_render_params *p) {
     d.step_budget = c->step_budget;
     c->params = d;
     c->has_params = true;
-    // camera leaf list storage for tiles up to the whole frame, so that renders
-    // allocate nothing (without it their camera segments traverse)
+    // list and path pipeline storage for tiles up to the whole frame, so that
+    // renders allocate nothing (without it they traverse per sample)
     const size_t frame = (size_t)p->w * p->h;
-    if (c->cam_used.reserve(3) != cudaSuccess || c->cam_head.reserve(2 * frame) != cudaSuccess ||
-        c->band_cam_head.reserve(2 * frame) != cudaSuccess || c->cam_pool.reserve(c->cam_cap) != cudaSuccess ||
-        c->band_cam_pool.reserve(2 * (size_t)c->cam_cap) != cudaSuccess) {
-        c->cam_head.release();
-        c->band_cam_head.release();
-        cudaGetLastError();  // not an error of the parameters
-    }
+    (void)reserve_lists(c, 0, frame, rec_capacity(frame, 0));
+    (void)reserve_lists(c, 1, frame, rec_capacity(frame, 1));
+    cudaGetLastError();  // a failure is not an error of the parameters
     return DR_OK;
 }
 
@@ -234,7 +264,8 @@ int dr_set_camera_lists(dr_ctx *c, uint32_t pool_entries) {
     if (pool_entries != DR_NONE && pool_entries > (1u << 28))
         return need(false, DR_ERR_INVALID, "dr_set_camera_lists: at most 2^28 entries per pool");
     std::lock_guard<std::mutex> lk(c->mu);
-    c->cam_cap = pool_entries == DR_NONE ? 0u : pool_entries ? pool_entries : dr_ctx::kCamPool;
+    c->cam_cap = pool_entries == DR_NONE ? 0u : pool_entries;
+    c->cam_cap_set = pool_entries != 0u;
     return DR_OK;
 }
 
@@ -288,25 +319,29 @@ static int tile_args(const dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uin
     return make_tile_args(x0, y0, tw, th, spp, seed, base, tile, A);
 }
 
-// Camera leaf list storage of a persistent launch: slot 0 for the asynchronous
+// The lists and pipeline storage of a launch: slot 0 for the asynchronous
 // render, 1 + (band & 1) for the blocking render's band streams (head_off: the
 // band's first pixel among the tile's headers).  A failed allocation leaves
-// the launch without lists (its camera segments traverse).
+// the launch without (its camera segments traverse per sample).
 static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t head_off) {
     CamLists L;
-    if (c->cam_cap == 0) return L;
-    DevBuf<uint4> &head = slot ? c->band_cam_head : c->cam_head;
-    DevBuf<uint4> &pool = slot ? c->band_cam_pool : c->cam_pool;
-    const size_t pool_n = (slot ? 2u : 1u) * (size_t)c->cam_cap;
-    if (c->cam_used.reserve(3) != cudaSuccess || head.reserve(2 * head_pixels) != cudaSuccess ||
-        pool.reserve(pool_n) != cudaSuccess) {
+    // the storage follows the frame, or the tile when that is larger
+    const size_t pixels = std::max(head_pixels, (size_t)c->params.w * c->params.h);
+    const uint32_t rec_cap = rec_capacity(pixels, slot);
+    if (!reserve_lists(c, slot, pixels, rec_cap)) {
         cudaGetLastError();  // not an error of the render
         return L;
     }
-    L.head = head.p + 2 * head_off;
-    L.pool = pool.p + (slot == 2 ? (size_t)c->cam_cap : 0u);
-    L.cap = c->cam_cap;
+    const size_t second = slot == 2 ? 1 : 0;
+    const uint32_t pool = pool_capacity(c, pixels, slot);
+    L.head = (slot ? c->band_cam_head : c->cam_head).p + 2 * head_off;
+    L.pool = (slot ? c->band_cam_pool : c->cam_pool).p + second * pool;
+    L.cap = pool;
     L.used = c->cam_used.p + slot;
+    L.ctl = c->path_ctl.p + slot;
+    L.active = (slot ? c->band_path_active : c->path_active).p + head_off;
+    L.records = (slot ? c->path_rec_band : c->path_rec_async).p + second * rec_cap;
+    L.rec_cap = rec_cap;
     return L;
 }
 
@@ -725,8 +760,9 @@ int dr_set_bricks_dev(dr_ctx *c, const float *bricks_dev, uint32_t n_leaves, flo
     if (!(majorant_scale == 0.0f || majorant_scale >= 1.0f) || !std::isfinite(majorant_scale))
         return need(false, DR_ERR_INVALID, "dr_set_bricks_dev: majorant_scale must be 0 or >= 1");
     if (majorant_scale > 0.0f)
-        DR_CUDA(launch_leaf_majorants(c->bufs.leaf.p, c->leaf_nodes.p, c->n_leaf_nodes, c->bufs.bricks.p,
-                                      majorant_scale, st),
+        DR_CUDA(launch_leaf_majorants(c->bufs.leaf.p, c->scene.glevels ? c->bufs.gleaf.p : nullptr,
+                                      c->scene.glevels ? c->bufs.gmaj.p : nullptr, c->leaf_nodes.p, c->n_leaf_nodes,
+                                      c->bufs.bricks.p, majorant_scale, st),
                 "dr_set_bricks_dev: majorants");
     return DR_OK;
 }

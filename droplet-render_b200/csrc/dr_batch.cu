@@ -55,6 +55,12 @@ struct dr_batch {
     DevBuf<unsigned int> cam_used;
     DevBuf<uint32_t> pix_begins;
     uint32_t n_pix = 0;
+    // path pipeline (dr_paths.cu): control words, active pixels, per-view counts of
+    // the views rendered together, and a buffer of collided samples for them and each branch
+    DevBuf<PathCtl> path_ctl;
+    DevBuf<uint32_t> path_active, view_active, view_tickets, rest_pix, rest_blocks;
+    DevBuf<uint4> path_rec;
+    uint32_t rec_cap = 0;
     std::vector<BatchView> host_views;
     std::vector<size_t> out_off;  // float4 offset of view v's sun tile; its sky tile follows
     size_t out_n = 0;             // float4 count of all outputs
@@ -62,7 +68,7 @@ struct dr_batch {
     Tuning tuning{0u, 128u, 0u, 8u, 0u, 0u, 0u, 0u};
     uint64_t n_paths = 0, launches = 0;
     bool any_sdf = false;  // a scene with surface (SDF) leaves
-    uint32_t stack_levels = 0;  // deepest traversal stack of the scenes (0: some scene's depth is unknown)
+    uint32_t glevels = 0;  // deepest block grid of the scenes (0: some scene has none)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -154,7 +160,39 @@ int build_graph(dr_batch *b) {
             rest_paths += V.A.n_paths;
         }
     }
+    const bool paths = paths_serve(b->tuning, b->glevels) && b->path_rec.p;
     BatchArgs R = B;  // the batched kernel's views
+    PathWork W{};     // and their pipeline
+    uint32_t list_blocks = 0;
+    uint64_t list_paths = 0;
+    if (paths) {
+        W.ctl = b->path_ctl.p;
+        W.pool_used = b->cam_used.p;
+        W.pool = b->cam_pool.p;
+        W.pool_cap = (uint32_t)b->cam_pool.n;
+        W.active = b->path_active.p;
+        W.records = b->path_rec.p;
+        W.cap = b->rec_cap;
+        W.view_active = b->view_active.p;
+        W.view_tickets = b->view_tickets.p;
+        W.pix_begins = b->rest_pix.p;
+        W.block_begins = b->rest_blocks.p;
+        std::vector<uint32_t> pixs, blks;
+        for (size_t v = 0; v < b->host_views.size(); ++v) {
+            if (std::find(own.begin(), own.end(), (uint32_t)v) != own.end()) continue;
+            const TileArgs &A = b->host_views[v].A;
+            pixs.push_back(pix_begins[v]);
+            blks.push_back(list_blocks);
+            list_blocks += path_list_blocks(A.cols, A.rows);
+            list_paths += (uint64_t)A.cols * A.rows * A.spp;
+        }
+        if (!pixs.empty()) {
+            DR_CUDA(cudaMemcpy(b->rest_pix.p, pixs.data(), sizeof(uint32_t) * pixs.size(), cudaMemcpyHostToDevice),
+                    "dr_batch: copy views");
+            DR_CUDA(cudaMemcpy(b->rest_blocks.p, blks.data(), sizeof(uint32_t) * blks.size(), cudaMemcpyHostToDevice),
+                    "dr_batch: copy views");
+        }
+    }
     if (!own.empty()) {
         if (!rest.empty()) {
             DR_CUDA(cudaMemcpy(b->rest_views.p, rest.data(), sizeof(BatchView) * rest.size(), cudaMemcpyHostToDevice),
@@ -179,17 +217,33 @@ int build_graph(dr_batch *b) {
     DR_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "dr_batch: begin capture");
     cudaError_t e = cudaMemsetAsync(b->out.p, 0, sizeof(float4) * b->out_n, b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->work.p, 0, sizeof(WorkQueue) * b->work.n, b->stream);
-    if (e == cudaSuccess) e = launch_batch_lists(B, bl, b->stream);
+    if (e == cudaSuccess && paths) e = cudaMemsetAsync(b->cam_used.p, 0, sizeof(unsigned int), b->stream);
+    if (e == cudaSuccess && !paths) e = launch_batch_lists(B, bl, b->stream);
     if (e == cudaSuccess && nbr) e = cudaEventRecord(b->fork, b->stream);
     for (uint32_t k = 0; k < nbr && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(b->branch[k], b->fork, 0);
     for (size_t k = 0; k < own.size() && e == cudaSuccess; ++k) {
         const BatchView &V = b->host_views[own[k]];
+        if (paths) {
+            PathWork Wv = W;
+            Wv.ctl = b->path_ctl.p + 1 + k % nbr;
+            Wv.n_active = &Wv.ctl->n_active;
+            Wv.head = b->cam_head.p + 2 * (size_t)pix_begins[own[k]];
+            Wv.active = W.active + pix_begins[own[k]];
+            Wv.records = W.records + (size_t)(1 + k % nbr) * W.cap;
+            const DevScene &S = b->host_scenes[V.scene];
+            e = launch_paths(S, V.P, V.A, b->mie_pack.p, V.sun, V.sky, b->ctx->counters.p, Wv,
+                             frame_features(S, V.P) != 0, b->ctx->device, b->branch[k % nbr], b->step.p);
+            continue;
+        }
         e = launch_batch_view(b->host_scenes[V.scene], V.P, V.A, b->mie_pack.p, V.sun, V.sky, b->ctx->counters.p,
                               b->work.p + 1 + own[k], b->step.p, b->tuning, b->ctx->device, b->branch[k % nbr]);
     }
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && paths)
+        e = launch_paths_batch(R, b->p0, b->mie_pack.p, b->ctx->counters.p, W, list_paths, list_blocks, ext,
+                               b->glevels, b->ctx->device, b->stream);
+    if (e == cudaSuccess && !paths)
         e = launch_batch_kernel(R, b->p0, b->mie_pack.p, b->ctx->counters.p, b->work.p, b->tuning, ext,
-                                b->stack_levels, b->ctx->device, b->stream);
+                                b->ctx->device, b->stream);
     // every branch joins the capture stream (also after an error, so that the capture can end)
     for (uint32_t k = 0; k < nbr; ++k) {
         const cudaError_t j = cudaEventRecord(b->join[k], b->branch[k]);
@@ -227,6 +281,13 @@ void release(dr_batch *b) {
     b->pix_begins.release();
     b->rest_views.release();
     b->rest_begins.release();
+    b->path_ctl.release();
+    b->path_active.release();
+    b->view_active.release();
+    b->view_tickets.release();
+    b->rest_pix.release();
+    b->rest_blocks.release();
+    b->path_rec.release();
     for (uint32_t k = 0; k < kBranches; ++k) {
         if (b->branch[k]) cudaStreamDestroy(b->branch[k]);
         if (b->join[k]) cudaEventDestroy(b->join[k]);
@@ -287,16 +348,16 @@ int dr_batch_create(dr_ctx *c, const dr_scene_desc *scenes, uint32_t n_scenes, c
         return code;
     };
     std::vector<DevScene> ds(n_scenes);
-    bool depth_known = true;
+    bool grids = true;
     for (uint32_t i = 0; i < n_scenes; ++i) {
         b->scene_bufs.emplace_back(new SceneBufs());
         rc = upload_scene(hs[i], *b->scene_bufs.back(), c->use_grid, b->stream, ds[i]);
         b->any_sdf = b->any_sdf || ds[i].sdf_bricks != nullptr;
         if (rc != DR_OK) return fail(rc);
-        depth_known = depth_known && ds[i].stack_levels > 0;
-        b->stack_levels = std::max(b->stack_levels, ds[i].stack_levels);
+        grids = grids && ds[i].glevels > 0;
+        b->glevels = std::max(b->glevels, ds[i].glevels);
     }
-    if (!depth_known) b->stack_levels = 0;
+    if (!grids) b->glevels = 0;
     size_t total = 0;
     b->out_off.resize(n_views);
     for (uint32_t v = 0; v < n_views; ++v) {
@@ -350,6 +411,19 @@ int dr_batch_create(dr_ctx *c, const dr_scene_desc *scenes, uint32_t n_scenes, c
             b->cam_pool.release();
             b->cam_used.release();
             cudaGetLastError();  // not an error of the batch
+        } else if (b->glevels) {
+            // the pipeline's storage: up to 2^23 records for the views rendered
+            // together and for each branch
+            uint64_t all = 0;
+            for (uint32_t v = 0; v < n_views; ++v) all += (uint64_t)hv[v].A.cols * hv[v].A.rows * hv[v].A.spp;
+            b->rec_cap = (uint32_t)std::min<uint64_t>(all, 1ull << 23);
+            if (b->path_ctl.reserve(1 + kBranches) != cudaSuccess || b->path_active.reserve(n_pix) != cudaSuccess ||
+                b->view_active.reserve(n_views) != cudaSuccess || b->view_tickets.reserve(n_views + 1) != cudaSuccess ||
+                b->rest_pix.reserve(n_views) != cudaSuccess || b->rest_blocks.reserve(n_views) != cudaSuccess ||
+                b->path_rec.reserve((size_t)(1 + kBranches) * b->rec_cap) != cudaSuccess) {
+                b->path_rec.release();
+                cudaGetLastError();  // not an error of the batch: the persistent kernels run
+            }
         }
     }
     BATCH_CUDA(b->mie_pack.reserve(pack0.size()), "dr_batch_create: alloc tables");

@@ -173,6 +173,12 @@ __device__ __forceinline__ Rng rng_seed(uint64_t seed, uint64_t pixel, uint64_t 
     return g;
 }
 
+// The stream constant rng_seed() gives the same arguments.
+__device__ __forceinline__ uint64_t rng_inc(uint64_t seed, uint64_t pixel, uint64_t sample) {
+    const uint64_t a = mix64(seed ^ mix64(pixel * 0x9e3779b97f4a7c15ull + sample));
+    return (mix64(a + 0x632be59bd9b4e019ull) << 1) | 1u;
+}
+
 // ---- per-thread counters ----------------------------------------------------
 struct Count {
     uint32_t vertices, node_visits, density_lookups, mie_evals, gave_up;
@@ -183,7 +189,7 @@ struct Count {
 // The reference's step traverser (src/KernelOctree.cpp:230-349) keeps t0, t1,
 // tm for all 16 levels.  Here only the current internal node's (t0, t1) stay
 // in registers; ancestor node ids and the ancestors' (t0, t1) live in a stack
-// (per-thread arrays in local memory, or a per-lane column of shared memory),
+// (per-thread arrays in local memory),
 // written on each descent and read back on a pop.  Without the intervals (the
 // probes) a pop
 // rebuilds the interval from the root by replaying the child slots (3 bits per
@@ -272,7 +278,7 @@ __device__ __forceinline__ void trav_init(Trav &T, const DevScene &S, const floa
 // returns kTravLeaf with (leaf, tra, trb), kTravDone when the ray has no further
 // leaf, or kTravMore when the budget ran out first (call again: the state is
 // complete after every iteration).
-// The stack (see LocalStack / SharedStack) saves the ancestors' node ids and,
+// The stack (see LocalStack) saves the ancestors' node ids and,
 // when it has room for them, their intervals at each descent, read back on a
 // pop; without intervals a pop rebuilds the interval from the root by replaying
 // the 3-bit child slots (the same floats).
@@ -285,19 +291,6 @@ enum : uint32_t { kTravMore = 0, kTravLeaf = 1, kTravDone = 2 };
 // LocalStack: node ids and intervals in the lane's own arrays (local memory),
 // the next child at each level in 4-bit fields of T.tns; without `iv` a pop
 // replays the interval from the root (returns false).
-// SharedStack: level l of this lane at col[(kShWords l + k) * STRIDE], one
-// column per lane of the block, so the lanes of a warp touch 32 consecutive
-// words whatever their levels (no bank conflicts).  k = 0..2: per axis, the
-// parent's bound the child does not share (t0 where the child lies in the upper
-// half, else t1); k = 3: the node id (below 2^25), the child's slot bits at 25-27
-// and the next child at 28-31.  A pop happens when the child's subtree is done,
-// with the child's interval still in T: the child shares the parent's t1 on
-// the axes where its bit is set and the parent's t0 elsewhere, so the saved
-// bound completes the parent's interval with the same floats.  `levels` entries
-// fit, and a descent that would need more gives up like the reference's depth
-// limit (the host sizes the stack from the octree's depth, so that never happens).
-constexpr int kShWords = 4;
-
 struct LocalStack {
     uint32_t *nodes;
     float (*iv)[6];
@@ -325,33 +318,6 @@ struct LocalStack {
     }
     __device__ __forceinline__ bool has_iv() const { return iv != nullptr; }
     __device__ __forceinline__ bool full(int l) const { return l + 1 >= kMaxDepth - 1; }
-};
-
-template <int STRIDE>
-struct SharedStack {
-    float *col;
-    int levels;
-    __device__ __forceinline__ void push(Trav &T, int l, uint32_t cb) const {
-        col[(kShWords * l + 0) * STRIDE] = (cb & 1u) ? T.t0[0] : T.t1[0];
-        col[(kShWords * l + 1) * STRIDE] = (cb & 2u) ? T.t0[1] : T.t1[1];
-        col[(kShWords * l + 2) * STRIDE] = (cb & 4u) ? T.t0[2] : T.t1[2];
-        col[(kShWords * l + 3) * STRIDE] = __uint_as_float(T.node | (cb << 25) | (T.tn << 28));
-    }
-    __device__ __forceinline__ bool pop(Trav &T, int l) const {
-        const uint32_t w = __float_as_uint(col[(kShWords * l + 3) * STRIDE]);
-        T.node = w & 0x01ffffffu;
-        T.tn = w >> 28;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float o = col[(kShWords * l + k) * STRIDE];
-            if ((w >> (25 + k)) & 1u) T.t0[k] = o;
-            else T.t1[k] = o;
-        }
-        return true;
-    }
-    __device__ __forceinline__ bool has_iv() const { return true; }
-    // levels <= 13 (the host allows at most 7), so the reference's depth limit is implied
-    __device__ __forceinline__ bool full(int l) const { return l >= levels; }
 };
 
 template <class ST>
@@ -653,6 +619,329 @@ __device__ __forceinline__ uint32_t walk_step(Walk &W, const DevScene &S, uint32
     }
     W.check = true;
     return 0u;
+}
+
+// ---- grid traversal: the same leaf sequence from a grid of 4^3-cell blocks ------
+// When every leaf sits at one depth L, the octree visits cells of a 2^L grid in
+// the order the cell walk above spells out: cross the nearest exit plane (ties
+// to z, then y, then x), and when the crossing enters an aligned 2^t block (t =
+// trailing zeros of the new index) an axis whose entry plane ties with the
+// crossed one descends again.  This version keeps what a step needs at hand:
+//  * entry planes are not kept: crossing axis k, the new cell's entry plane is
+//    the crossed plane itself, and its exit plane follows from the exit planes
+//    of the enclosing nodes by the tree's own midpoints 0.5f*(lo + hi).  Exit
+//    planes of the cell and of its 2^3 block sit in registers, those of the
+//    4^3 block and of the larger nodes in the lane's column of shared memory
+//    (words 3j + k: axis k, level 2 + j), so a step costs one or two midpoints on
+//    one axis instead of the six of an octree examination;
+//  * a 4^3 block's occupancy is one 64-bit mask in registers, so steps inside a
+//    block load nothing; a leaf's slot is its rank in the mask;
+//  * a tie is seen as the crossed plane not lying behind the previous crossing
+//    (every entry plane is at most that crossing, and one equals it): rare, and
+//    handled out of line.
+// Node visits are the octree's: entering a 2^t block visits one node per level
+// from t down, as far as the octree has one (gblock's w, the bits of the
+// present 2^3 nodes and the cells' occupancy).
+// Not for rays with a zero direction component (non-finite planes).
+constexpr uint32_t kGridEmpty = 64u;   // loc: nothing below the block, planes are the block's
+constexpr uint32_t kGridCheck = 128u;  // loc: the first cell is a leaf not yet reported
+
+struct GridTrav {
+    float x[3];         // exit planes of the current cell (of the block when it is empty)
+    float h[3];         // exit planes of the 2^3 block holding it
+    float tc;           // the plane the current cell was entered through
+    uint32_t mlo, mhi;  // occupancy of the current block
+    uint32_t base;      // its first leaf slot, and its present 2^3 nodes << 24
+    uint32_t c;         // block coordinates in the mirrored frame, packed as gblock's index
+    uint32_t am;        // mirror mask of c
+    uint32_t loc;       // bits 0-5 the cell in the block (Morton, mirrored), 6-7 kGrid*, 8-13 mirror mask of the
+                        // cell, 16-31 ties resolved
+};
+
+// Words of a lane's column: 3 per level from 2 to L, then the current block's entry planes.
+__host__ __device__ constexpr uint32_t grid_words(uint32_t levels) { return 3u * levels; }
+
+// One axis of the grid descended anew from the root: the levels below t choose
+// the half holding te (as first_node does), the others keep the cell's bits.
+// Rewrites the axis's column and returns its planes and cell.
+struct GridAxis {
+    float x, h;
+    uint32_t cell;
+};
+template <int STRIDE>
+__device__ __noinline__ GridAxis grid_axis(float *col, uint32_t k, float ro, float rd, float root_c, float root_e,
+                                           uint32_t levels, uint32_t cell, uint32_t t, float te) {
+    float ros = (ro - root_c) + root_e, rds = rd;
+    const float mx = 2.0f * root_e;
+    if (rds < 0.0f) {
+        ros = mx - ros;
+        rds = -rds;
+    }
+    float lo = (0.0f - ros) / rds, hi = (mx - ros) / rds;
+    GridAxis g;
+    g.cell = 0;
+    g.h = hi;
+    for (int j = (int)levels - 1; j >= 0; --j) {
+        const float mid = 0.5f * (lo + hi);
+        const bool up = (uint32_t)j >= t ? ((cell >> j) & 1u) != 0u : mid < te;
+        if (up) lo = mid;
+        else hi = mid;
+        g.cell = 2u * g.cell + (up ? 1u : 0u);
+        if (j >= 2) col[(3 * (j - 2) + (int)k) * STRIDE] = hi;
+        if (j == 2) col[(3 * ((int)levels - 1) + (int)k) * STRIDE] = lo;
+        if (j == 1) g.h = hi;
+    }
+    g.x = hi;
+    return g;
+}
+
+// Puts axis k's cell into the block coordinates and the local index.
+__device__ __forceinline__ void grid_put(GridTrav &G, uint32_t k, uint32_t lb, uint32_t nbm, uint32_t cell) {
+    const uint32_t s = k * lb, b = 9u << k;
+    G.c = (G.c & ~(nbm << s)) | ((cell >> 2) << s);
+    G.loc = (G.loc & ~b) | ((cell & 1u) << k) | (((cell >> 1) & 1u) << (k + 3u));
+}
+
+// Resolves a tie: the other two axes descend again inside the 2^t block entered
+// at te.  Between two of these the coordinates only grow, so the count in loc's
+// upper bits bounds the segment: false when it runs out (65,535; a ray through
+// a few plane intersections needs as many).
+template <int STRIDE>
+__device__ __forceinline__ bool grid_resync(GridTrav &G, const DevScene &S, float *col, const float ro[3],
+                                            const float rd[3], uint32_t axis_bit, uint32_t t, float te) {
+    const uint32_t lb = S.glevels - 2u, nbm = (1u << lb) - 1u;
+#pragma unroll
+    for (uint32_t k = 0; k < 3; ++k) {
+        if (axis_bit == (1u << k)) continue;
+        const uint32_t cell =
+            (((G.c >> (k * lb)) & nbm) << 2) | (((G.loc >> (k + 3u)) & 1u) << 1) | ((G.loc >> k) & 1u);
+        const GridAxis g = grid_axis<STRIDE>(col, k, ro[k], rd[k], S.root_ce[k], S.root_ce[3], S.glevels, cell, t, te);
+        G.x[k] = g.x;
+        G.h[k] = g.h;
+        grid_put(G, k, lb, nbm, g.cell);
+    }
+    G.loc += 0x10000u;
+    return G.loc >= 0x10000u;
+}
+
+// The cell's index in gblock's order and the occupancy word holding its bit.
+__device__ __forceinline__ uint32_t grid_cell_word(const GridTrav &G, uint32_t &idx) {
+    idx = (G.loc ^ (G.loc >> 8)) & 63u;
+    return (idx & 32u) ? G.mhi : G.mlo;
+}
+
+// Returns 0: no leaf on this ray, 1: ready, 2: use the stack traversal.
+template <int STRIDE>
+__device__ __forceinline__ uint32_t grid_init(GridTrav &G, const DevScene &S, float *col, const float ro[3],
+                                              const float rd[3], Count &cnt) {
+    const int L = (int)S.glevels;
+    const float mx = 2.0f * S.root_ce[3];
+    float lo[3], hi[3];
+    uint32_t a = 0;
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float ros = (ro[k] - S.root_ce[k]) + S.root_ce[3], rds = rd[k];
+        if (rds < 0.0f) {
+            ros = mx - ros;
+            rds = -rds;
+            a |= 1u << k;
+        }
+        lo[k] = (0.0f - ros) / rds;
+        hi[k] = (mx - ros) / rds;
+        finite = finite && fabsf(lo[k]) < 1e30f && fabsf(hi[k]) < 1e30f;  // sums of planes stay finite
+    }
+    if (!finite) return 2u;
+    const float te = std_max(std_max(lo[0], lo[1]), lo[2]);
+    if (!(te < std_min(std_min(hi[0], hi[1]), hi[2])) || hi[0] < 0.0f || hi[1] < 0.0f || hi[2] < 0.0f) return 0u;
+    ++cnt.node_visits;  // the root
+    // the first cell holds the entry point, or the origin when that lies inside
+    // (the octree skips, uncounted, every node behind the origin)
+    const float ts = te > 0.0f ? te : 0.0f;
+    uint32_t c[3] = {0u, 0u, 0u};
+    G.loc = (a * 9u) << 8;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) col[(3 * (L - 2) + k) * STRIDE] = hi[k];
+#pragma unroll 1
+    for (int j = L - 1; j >= 2; --j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float mid = 0.5f * (lo[k] + hi[k]);
+            const bool up = mid < ts;
+            lo[k] = up ? mid : lo[k];
+            hi[k] = up ? hi[k] : mid;
+            c[k] = 2u * c[k] + (up ? 1u : 0u);
+            col[(3 * (j - 2) + k) * STRIDE] = hi[k];
+        }
+    }
+    const uint32_t lb = (uint32_t)L - 2u, nbm = (1u << lb) - 1u;
+    G.c = c[0] | (c[1] << lb) | (c[2] << (2u * lb));
+    G.am = ((a & 1u) ? nbm : 0u) | ((a & 2u) ? nbm << lb : 0u) | ((a & 4u) ? nbm << (2u * lb) : 0u);
+    const uint4 e = __ldg(&S.gblock[G.c ^ G.am]);
+    G.mlo = e.x;
+    G.mhi = e.y;
+    G.base = e.z;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        col[(3 * (L - 1) + k) * STRIDE] = lo[k];
+        G.x[k] = hi[k];
+    }
+    cnt.node_visits += (uint32_t)max(0, L - 1 - (int)e.w);
+    if (!(e.z >> 24)) {
+        G.tc = std_max(std_max(lo[0], lo[1]), lo[2]);
+        G.loc |= kGridEmpty;
+        return 1u;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float mid = 0.5f * (lo[k] + hi[k]);
+        bool up = mid < ts;
+        lo[k] = up ? mid : lo[k];
+        hi[k] = up ? hi[k] : mid;
+        G.loc |= up ? 8u << k : 0u;
+        G.h[k] = hi[k];
+        mid = 0.5f * (lo[k] + hi[k]);
+        up = mid < ts;
+        lo[k] = up ? mid : lo[k];
+        G.x[k] = up ? hi[k] : mid;
+        G.loc |= up ? 1u << k : 0u;
+    }
+    G.tc = std_max(std_max(lo[0], lo[1]), lo[2]);
+    uint32_t idx;
+    const uint32_t w = grid_cell_word(G, idx);
+    const uint32_t occ = (w >> (idx & 31u)) & 1u;
+    cnt.node_visits += ((G.base >> (24u + (idx >> 3))) & 1u) + occ;
+    if (occ) G.loc |= kGridCheck;
+    return 1u;
+}
+
+__device__ __forceinline__ uint32_t grid_leaf(const GridTrav &G, uint32_t idx, uint32_t w, float &tra, float &trb) {
+    tra = G.tc;
+    trb = std_min(std_min(G.x[0], G.x[1]), G.x[2]);
+    return (G.base & 0xffffffu) + ((idx & 32u) ? __popc(G.mlo) : 0) + __popc(w & ((1u << (idx & 31u)) - 1u));
+}
+
+// Up to `budget` steps towards the next leaf: kTravLeaf with its slot and
+// interval, kTravDone past the last leaf, or kTravMore.
+template <int STRIDE>
+__device__ __forceinline__ uint32_t grid_next(GridTrav &G, const DevScene &S, float *col, const float ro[3],
+                                              const float rd[3], uint32_t &leaf, float &tra, float &trb, Count &cnt,
+                                              uint32_t budget) {
+    uint32_t idx;
+    if (G.loc & kGridCheck) {
+        G.loc &= ~kGridCheck;
+        const uint32_t w = grid_cell_word(G, idx);
+        leaf = grid_leaf(G, idx, w, tra, trb);
+        return kTravLeaf;
+    }
+    for (uint32_t it = 0; it != budget; ++it) {
+        // OctreeNextNode's choice (src/KernelOctree.cpp:62-71) as the exit axis
+        const bool xy = G.x[0] < G.x[1];
+        const bool bx = xy && G.x[0] < G.x[2];
+        const bool by = !xy && G.x[1] < G.x[2];
+        const float Xa = bx ? G.x[0] : (by ? G.x[1] : G.x[2]);
+        const uint32_t b = bx ? 1u : (by ? 2u : 4u);
+        const int k = bx ? 0 : (by ? 1 : 2);
+        const bool tie = !(G.tc < Xa);
+        G.tc = Xa;
+        bool half = true;  // a 2^3 block is entered
+        if (!(G.loc & kGridEmpty) && (G.loc & (9u * b)) != 9u * b) {
+            float nx, nh;
+            if (!(G.loc & b)) {  // the upper cell of the same 2^3 block
+                half = false;
+                nh = bx ? G.h[0] : (by ? G.h[1] : G.h[2]);
+                nx = nh;
+                G.loc |= b;
+            } else {  // the next 2^3 block of the same 4^3 block
+                nh = col[k * STRIDE];
+                nx = 0.5f * (Xa + nh);
+                G.loc ^= 9u * b;
+            }
+            if (bx) { G.x[0] = nx; G.h[0] = nh; }
+            else if (by) { G.x[1] = nx; G.h[1] = nh; }
+            else { G.x[2] = nx; G.h[2] = nh; }
+            if (half && tie && !grid_resync<STRIDE>(G, S, col, ro, rd, b, 1u, Xa)) {
+                ++cnt.gave_up;
+                return kTravDone;
+            }
+        } else {  // the next 4^3 block
+            const uint32_t lb = S.glevels - 2u, nbm = (1u << lb) - 1u;
+            const uint32_t s = (uint32_t)k * lb, f = (G.c >> s) & nbm;
+            if (f == nbm) return kTravDone;
+            G.c += 1u << s;
+            const int tz = __ffs((int)(f + 1u)) - 1;  // levels 2 .. 2 + tz are entered
+            float hi = col[(3 * (tz + 1) + k) * STRIDE];
+#pragma unroll 1
+            for (int j = tz;; --j) {
+                col[(3 * j + k) * STRIDE] = hi;
+                if (j == 0) break;
+                hi = 0.5f * (Xa + hi);
+            }
+            col[(3 * ((int)S.glevels - 1) + k) * STRIDE] = Xa;
+            const bool was_empty = (G.loc & kGridEmpty) != 0u;
+            G.loc &= ~(9u * b);
+            if (tie && !grid_resync<STRIDE>(G, S, col, ro, rd, b, 2u + (uint32_t)tz, Xa)) {
+                ++cnt.gave_up;
+                return kTravDone;
+            }
+            const uint4 e = __ldg(&S.gblock[G.c ^ G.am]);
+            G.mlo = e.x;
+            G.mhi = e.y;
+            G.base = e.z;
+            cnt.node_visits += (uint32_t)max(0, 2 + tz - (int)e.w);
+            if (!(e.z >> 24)) {
+                G.loc |= kGridEmpty;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) G.x[q] = col[q * STRIDE];
+                continue;
+            }
+            const float nh = 0.5f * (Xa + hi), nx = 0.5f * (Xa + nh);
+            if (was_empty) {
+                // the cell of the other axes that holds the crossing
+                G.loc &= ~kGridEmpty;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    float l = col[(3 * ((int)S.glevels - 1) + q) * STRIDE], h = col[q * STRIDE];
+                    float mid = 0.5f * (l + h);
+                    bool up = mid < Xa;
+                    l = up ? mid : l;
+                    h = up ? h : mid;
+                    G.loc = (G.loc & ~(9u << q)) | (up ? 8u << q : 0u);
+                    G.h[q] = h;
+                    mid = 0.5f * (l + h);
+                    up = mid < Xa;
+                    G.x[q] = up ? h : mid;
+                    G.loc |= up ? 1u << q : 0u;
+                }
+            } else {
+                if (bx) { G.x[0] = nx; G.h[0] = nh; }
+                else if (by) { G.x[1] = nx; G.h[1] = nh; }
+                else { G.x[2] = nx; G.h[2] = nh; }
+            }
+        }
+        const uint32_t w = grid_cell_word(G, idx);
+        const uint32_t occ = (w >> (idx & 31u)) & 1u;
+        cnt.node_visits += (half ? (G.base >> (24u + (idx >> 3))) & 1u : 0u) + occ;
+        if (occ) {
+            leaf = grid_leaf(G, idx, w, tra, trb);
+            return kTravLeaf;
+        }
+    }
+    return kTravMore;
+}
+
+// ---- free flights that need no logarithm ---------------------------------------
+// Most leaves are thin: of the 8.5 leaves a segment of the 512^3 cumulus crosses,
+// 7.3 are left by the first flight.  That much is decided without the logarithm
+// and the division: -ln u >= 1 - u, so the flight -ln(u) / denom leaves the
+// leaf whenever 1 - u >= denom * (distance left).  The factor covers the roundings
+// (dlog, the products and the differences are each within a few ulp; what
+// follows, s0 + sr against tr1, rounds monotonically).  A flight that passes needs
+// no other result: the next leaf starts a flight of its own at trb.
+// 0 * denom passes like its infinite flight; a distance < 0 passes too.
+__device__ __forceinline__ bool leaves_at_once(float u, float denom, float tra, float trb, float td) {
+    const float tr1 = trb - td, s0 = tra > td ? tra - td : 0.0f;
+    return 1.0f - u >= 1.0001f * (denom * (tr1 - s0));
 }
 
 // ---- brick lookup: SampleVoxelSpace, src/kernel.cpp:96-126 ----------------
@@ -1073,7 +1362,7 @@ __device__ __forceinline__ bool occ_box(float x0, float y0, float z0, float x1, 
 // frame came out smaller (384 B) than its node and interval stacks need at once
 // (448 B), and that kernel read out of bounds; every caller's frame now holds
 // all three stacks.
-__device__ __noinline__ bool occluded_bvh(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+static __device__ __noinline__ bool occluded_bvh(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
                                           uint32_t n_nodes, float ox, float oy, float oz, float dx, float dy,
                                           float dz) {
     const float o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};

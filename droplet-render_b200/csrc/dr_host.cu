@@ -1,4 +1,5 @@
 // Host-side helpers of the C ABI: errors, scene and settings conversion.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -70,6 +71,68 @@ static void mie_exact_table(const float *pdf_rgb, uint32_t n, float *out) {
     e[1] = e[2] = e[3] = 0.0f;
 }
 
+// A node of the octree with its place in the grid of its level (2^depth nodes per axis).
+struct TreeNode {
+    uint32_t node, depth, x, y, z;
+};
+
+// Block grid of the grid traversal (layout at DevScene::gblock) of a tree whose
+// leaves all sit at depth `levels`; `inner` holds its other nodes.
+static void build_block_grid(const std::vector<TreeNode> &leaves, const std::vector<TreeNode> &inner, uint32_t levels,
+                             HostScene &out) {
+    const uint32_t b = levels - 2;
+    auto at = [](uint32_t bits, uint32_t x, uint32_t y, uint32_t z) {
+        return x | (size_t)y << bits | (size_t)z << (2 * bits);
+    };
+    auto cell_of = [](const TreeNode &c) {
+        return (c.x & 1u) | (c.y & 1u) << 1 | (c.z & 1u) << 2 | (c.x >> 1 & 1u) << 3 | (c.y >> 1 & 1u) << 4 |
+               (c.z >> 1 & 1u) << 5;
+    };
+    auto block_of = [&](const TreeNode &c) { return at(b, c.x >> 2, c.y >> 2, c.z >> 2); };
+    std::vector<uint64_t> mask((size_t)1 << (3 * b), 0ull);
+    std::vector<uint32_t> half(mask.size(), 0u);  // present 2^3 nodes of each block
+    for (const TreeNode &c : leaves) mask[block_of(c)] |= 1ull << cell_of(c);
+    // absent[i] at level j: 1 when the node exists, else the level of the largest
+    // missing node holding it (a node's children are missing with it)
+    std::vector<uint8_t> above(1, 1), absent;
+    for (uint32_t j = levels; j-- > 2;) {
+        const uint32_t bits = levels - j, n = 1u << bits;
+        absent.assign((size_t)1 << (3 * bits), 0);
+        for (const TreeNode &c : inner)
+            if (c.depth == bits) absent[at(bits, c.x, c.y, c.z)] = 1;
+        for (uint32_t z = 0; z < n; ++z)
+            for (uint32_t y = 0; y < n; ++y)
+                for (uint32_t x = 0; x < n; ++x) {
+                    uint8_t &v = absent[at(bits, x, y, z)];
+                    const uint8_t up = above[at(bits - 1, x >> 1, y >> 1, z >> 1)];
+                    if (!v) v = up == 1 ? (uint8_t)j : up;
+                }
+        above.swap(absent);
+    }
+    for (const TreeNode &c : inner)
+        if (c.depth == levels - 1)
+            half[at(b, c.x >> 1, c.y >> 1, c.z >> 1)] |= 1u << ((c.x & 1u) | (c.y & 1u) << 1 | (c.z & 1u) << 2);
+    out.gblock.resize(mask.size());
+    uint32_t slot = 0;
+    for (size_t i = 0; i < mask.size(); ++i) {
+        out.gblock[i] = make_uint4((uint32_t)mask[i], (uint32_t)(mask[i] >> 32), slot | half[i] << 24, above[i]);
+        slot += (uint32_t)__builtin_popcountll(mask[i]);
+    }
+    out.gleaf.resize(2 * (size_t)slot);
+    out.gmaj.resize(slot);
+    for (const TreeNode &c : leaves) {
+        const uint64_t i = block_of(c);
+        const uint32_t k =
+            (out.gblock[i].z & 0xffffffu) + (uint32_t)__builtin_popcountll(mask[i] & ((1ull << cell_of(c)) - 1));
+        float4 &meta = out.leaf[2 * (size_t)c.node + 1];
+        std::memcpy(&meta.w, &k, 4);
+        out.gleaf[2 * (size_t)k] = out.leaf[2 * (size_t)c.node];
+        out.gleaf[2 * (size_t)k + 1] = meta;
+        out.gmaj[k] = meta.x;
+    }
+    out.glevels = levels;
+}
+
 int prepare_scene(const dr_scene_desc *s, HostScene &out) {
     if (!s || !s->nodes || !s->bricks) return need(false, DR_ERR_INVALID, "dr_upload_scene: null argument");
     if (s->lvoxc != kLvox) return need(false, DR_ERR_INVALID, "dr_upload_scene: bricks must be 8^3");
@@ -121,10 +184,10 @@ int prepare_scene(const dr_scene_desc *s, HostScene &out) {
     cells.clear();
     uint32_t levels = 0, n = 0, mdim = 0;
     {
-        struct Item { uint32_t node, depth, x, y, z; };
+        using Item = TreeNode;
         std::vector<Item> stack{{0u, 0u, 0u, 0u, 0u}};
         std::vector<uint8_t> seen(s->n_nodes, 0);
-        std::vector<Item> leaves;
+        std::vector<Item> leaves, inner;
         bool ok = true;
         int leaf_depth = -1;
         while (!stack.empty() && ok) {
@@ -138,6 +201,7 @@ int prepare_scene(const dr_scene_desc *s, HostScene &out) {
                 leaves.push_back(it);
                 continue;
             }
+            inner.push_back(it);
             for (uint32_t k = 0; k < 8; ++k) {
                 const uint32_t ch = N[it.node].chn[k];
                 if (ch) stack.push_back({ch, it.depth + 1, 2 * it.x + (k & 1), 2 * it.y + ((k >> 1) & 1), 2 * it.z + (k >> 2)});
@@ -156,15 +220,17 @@ int prepare_scene(const dr_scene_desc *s, HostScene &out) {
                 }
                 cells[(size_t)macro[m] * 512 + (lf.z & 7) * 64 + (lf.y & 7) * 8 + (lf.x & 7)] = lf.node;
             }
+            // (an internal node at the leaves' depth has no place in the grid)
+            const bool deep = std::any_of(inner.begin(), inner.end(),
+                                          [&](const Item &i) { return i.depth >= (uint32_t)leaf_depth; });
+            if (levels >= 2 && levels <= kGridMaxLevels && !deep && leaves.size() < (1u << 24))
+                build_block_grid(leaves, inner, levels, out);
         } else {
             macro.assign(1, kNone);
         }
         if (cells.empty()) cells.assign(512, kNone);
     }
     out.levels = levels;
-    // a tree with every leaf at depth d pushes at most d - 1 ancestors; the
-    // shared-memory stack packs node ids into 25 bits
-    out.stack_levels = (levels >= 2 && s->n_nodes < (1u << 25)) ? levels - 1 : 0u;
     out.n = n;
     out.mdim = mdim;
     out.n_nodes = s->n_nodes;
@@ -196,6 +262,19 @@ int upload_scene(const HostScene &h, SceneBufs &b, bool use_grid, cudaStream_t s
             "dr_upload_scene: copy nodes");
     DR_CUDA(cudaMemcpyAsync(b.leaf.p, h.leaf.data(), h.leaf.size() * sizeof(float4), cudaMemcpyHostToDevice, st),
             "dr_upload_scene: copy leaves");
+    if (h.glevels) {
+        DR_CUDA(b.gblock.reserve(h.gblock.size()), "dr_upload_scene: alloc grid");
+        DR_CUDA(b.gleaf.reserve(h.gleaf.size()), "dr_upload_scene: alloc grid");
+        DR_CUDA(b.gmaj.reserve(h.gmaj.size()), "dr_upload_scene: alloc grid");
+        DR_CUDA(cudaMemcpyAsync(b.gmaj.p, h.gmaj.data(), h.gmaj.size() * sizeof(float), cudaMemcpyHostToDevice, st),
+                "dr_upload_scene: copy grid");
+        DR_CUDA(cudaMemcpyAsync(b.gblock.p, h.gblock.data(), h.gblock.size() * sizeof(uint4), cudaMemcpyHostToDevice,
+                                st),
+                "dr_upload_scene: copy grid");
+        DR_CUDA(cudaMemcpyAsync(b.gleaf.p, h.gleaf.data(), h.gleaf.size() * sizeof(float4), cudaMemcpyHostToDevice,
+                                st),
+                "dr_upload_scene: copy grid");
+    }
     if (nb)
         DR_CUDA(cudaMemcpyAsync(b.bricks.p, h.bricks, nb * 4, cudaMemcpyHostToDevice, st),
                 "dr_upload_scene: copy bricks");
@@ -217,7 +296,10 @@ int upload_scene(const HostScene &h, SceneBufs &b, bool use_grid, cudaStream_t s
     S.levels = use_grid ? h.levels : 0u;
     S.n = h.n;
     S.mdim = h.mdim;
-    S.stack_levels = h.stack_levels;
+    S.gblock = h.glevels ? b.gblock.p : nullptr;
+    S.gleaf = h.glevels ? b.gleaf.p : nullptr;
+    S.gmaj = h.glevels ? b.gmaj.p : nullptr;
+    S.glevels = h.glevels;
     S.occ_nodes = nullptr;
     S.occ_tris = nullptr;
     S.occ_n_nodes = 0;

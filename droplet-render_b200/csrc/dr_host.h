@@ -65,7 +65,10 @@ struct HostScene {
     std::vector<uint32_t> macro, cells;
     std::vector<uint8_t> leaf_flag;
     uint32_t levels = 0, n = 0, mdim = 0;
-    uint32_t stack_levels = 0;  // traversal stack entries a ray can need (0: unknown, local stack only)
+    std::vector<uint4> gblock;     // block grid of the grid traversal (DevScene::gblock)
+    std::vector<float4> gleaf;     // leaf records by slot (DevScene::gleaf)
+    std::vector<float> gmaj;       // majorants by slot (DevScene::gmaj)
+    uint32_t glevels = 0;
     uint32_t n_nodes = 0, n_leaves = 0;
     float root_ce[4] = {0, 0, 0, 0};
     const float *bricks = nullptr;  // the caller's brick pool (n_leaves * 512 floats)
@@ -80,6 +83,9 @@ struct SceneBufs {
     DevBuf<float> bricks;
     DevBuf<float> sdf;
     DevBuf<uint32_t> macro, cells;
+    DevBuf<uint4> gblock;
+    DevBuf<float4> gleaf;
+    DevBuf<float> gmaj;
     void release() {
         child.release();
         leaf.release();
@@ -87,6 +93,9 @@ struct SceneBufs {
         sdf.release();
         macro.release();
         cells.release();
+        gblock.release();
+        gleaf.release();
+        gmaj.release();
     }
 };
 
@@ -264,9 +273,15 @@ struct dr_ctx {
     // for the asynchronous render (slot 0) and each band stream of the blocking
     // render (slots 1, 2); allocated on first use
     static constexpr uint32_t kCamPool = 1u << 23;
-    uint32_t cam_cap = kCamPool;  // entries per pool (dr_set_camera_lists; 0: no lists)
+    uint32_t cam_cap = 0;      // entries per pool when set (dr_set_camera_lists; 0: no lists)
+    bool cam_cap_set = false;  // else in proportion to the frame, up to kCamPool
     dr::DevBuf<uint4> cam_head, cam_pool, band_cam_head, band_cam_pool;
     dr::DevBuf<unsigned int> cam_used;
+    // path pipeline (PathWork): control words and active pixels like the lists,
+    // and a buffer of collided samples
+    dr::DevBuf<dr::PathCtl> path_ctl;
+    dr::DevBuf<uint32_t> path_active, band_path_active;
+    dr::DevBuf<uint4> path_rec_async, path_rec_band;
     float *pinned = nullptr;  // 2 * pinned_n float4: sun then sky
     size_t pinned_n = 0;
     dr::CopyPool copies;      // host threads for the staging -> caller copies

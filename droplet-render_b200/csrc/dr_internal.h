@@ -24,8 +24,9 @@ constexpr uint32_t kStepBudget = 1u << 24;  // tracking steps per segment before
 //   child[2*id], child[2*id+1]: the eight child entries of node id, remapped:
 //       0 = no child, kLeafBit|c = leaf node c, c = internal node c
 //   leaf[2*id]   = (center.xyz, half extent)
-//   leaf[2*id+1] = (majorant, FOG brick index bits, SDF brick index bits, 0);
-//                  an index kNone = no such brick; SDF leaves have majorant 1
+//   leaf[2*id+1] = (majorant, FOG brick index bits, SDF brick index bits, slot
+//                  bits); an index kNone = no such brick; SDF leaves have
+//                  majorant 1; slot: the leaf's place in gleaf (0 without a block grid)
 struct DevScene {
     const uint4 *child;
     const float4 *leaf;
@@ -43,11 +44,20 @@ struct DevScene {
     uint32_t levels;     // leaf depth below the root (0 = no grid; stack traversal only)
     uint32_t n;          // leaf cells per axis
     uint32_t mdim;       // macro cells per axis
-    // Entries the stack traversal can push on any ray: internal nodes below the
-    // root on the deepest root-to-leaf path (0: unknown, e.g. leaves at mixed
-    // depths or a DAG, or 2^25 nodes or more; then only the local-memory stack
-    // is used).
-    uint32_t stack_levels;
+    // Block grid of the grid traversal (leaves all at one depth, 2 to
+    // kGridMaxLevels below the root, fewer than 2^24; glevels = that depth, else
+    // 0).  Level j = nodes of 2^j leaf cells per axis.  Blocks are the 4^3-cell
+    // nodes; block (x, y, z) has index x + (y << b) + (z << 2b), b = glevels - 2.
+    // gblock[i] = (occupancy of cells 0-31, of cells 32-63, first leaf slot | the
+    // 2^3-cell nodes present << 24, level of the largest missing octree node
+    // holding the block or 1 when it is present); cells in Morton order (x bit 0, y
+    // bit 1, z bit 2, then the next bits).  gleaf[2 * slot], [2 * slot + 1] = the
+    // leaf records of `leaf`, blocks in index order and cells in Morton order
+    // inside one.
+    const uint4 *gblock;
+    const float4 *gleaf;
+    const float *gmaj;  // majorant of each slot (gleaf[2 * slot + 1].x)
+    uint32_t glevels;
     // Occluder BVH (null: no occluders).  Node i = occ_nodes[4i .. 4i+3]: left
     // box (min xyz, max x), (max yz, right min xy), (right min z, right max
     // xyz), then (left ref, right ref, left count, right count) as uint32
@@ -59,6 +69,7 @@ struct DevScene {
     uint32_t occ_n_nodes;
 };
 
+constexpr uint32_t kGridMaxLevels = 9;  // block grid: at most 128^3 blocks (32 MB)
 constexpr uint32_t kPhaseHG = 2;     // DR_PHASE_HG
 constexpr uint32_t kEnvHosek = 0, kEnvNone = 1, kEnvMap = 2;  // DR_ENV_*
 
@@ -183,6 +194,36 @@ struct BatchArgs {
 // Work queue of the persistent kernel: next path index to hand out.
 struct WorkQueue {
     unsigned long long next;
+};
+
+// Control words of the path pipeline (dr_paths.cu), zero before a launch.
+struct PathCtl {
+    unsigned long long ticket;  // next camera ticket
+    unsigned long long base;    // the first ticket of this round
+    uint32_t records;           // collided samples recorded in this round
+    uint32_t head;              // the next record to scatter
+    uint32_t pool_used;         // leaf list entries taken
+    uint32_t n_active;          // active pixels
+};
+constexpr uint32_t kRoundTickets = 1u << 24;  // tickets of one round: 2^31 samples, so 32 bits tell them apart
+
+// Storage of the path pipeline for one launch at a time.
+struct PathWork {
+    PathCtl *ctl;
+    uint32_t *pool_used, *n_active;  // where the list kernel counts
+    uint4 *head;                     // leaf list headers, 2 per pixel (TileArgs::cam_head)
+    uint4 *pool;                     // leaf list entries: (slot, tra bits, trb bits, node visits since the previous leaf)
+    uint32_t pool_cap;
+    uint32_t *active;                // pixels (iy * cols + ix) whose camera ray meets a leaf
+    // collided camera samples: (stream state, distance bits, sample number mod 2^32)
+    uint4 *records;
+    uint32_t cap;                    // records that fit
+    uint32_t limit;                  // no new ticket above this count (set by the launcher)
+    // batches
+    uint32_t *view_tickets;          // first ticket of each view, then their number
+    uint32_t *view_active;           // active pixels of each view
+    const uint32_t *pix_begins;      // first pixel of each view
+    const uint32_t *block_begins;    // first block of each view in the list kernel
 };
 
 }  // namespace dr

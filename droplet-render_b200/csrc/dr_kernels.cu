@@ -2,83 +2,10 @@
 #include <cstdio>
 #include <mutex>
 #include <cuda_runtime.h>
-#include "dr_device.cuh"
+#include "dr_stage.cuh"
 #include "dr_kernels.h"
 
 namespace dr {
-
-// ---- shared-memory staging of the phase tables ------------------------------
-// Layout in global and shared memory: pdf as float4 (r, g, b, 0) x n, then the
-// red CDF x n (n % 4 == 0, so the block is a multiple of 16 bytes).  One thread
-// issues a bulk copy (cp.async.bulk, completion counted on an mbarrier); the
-// wait is bounded and reports a give-up instead of spinning forever.
-// Exact mode appends its sampler table: (2n + 1) float4 after the CDF.
-__device__ __forceinline__ uint32_t mie_bytes(const DevParams &P) {
-    return P.mie_n * 20u + (P.phase_mode == 1u ? (2u * P.mie_n + 1u) * 16u : 0u);
-}
-
-__device__ __forceinline__ MieSmem mie_view(const DevParams &P, unsigned char *smem) {
-    return MieSmem{reinterpret_cast<float4 *>(smem), reinterpret_cast<float *>(smem + 16u * P.mie_n), P.mie_n,
-                   P.phase_mode == 1u ? reinterpret_cast<const float4 *>(smem + 20u * P.mie_n) : nullptr};
-}
-
-__device__ __forceinline__ bool stage_mie(const void *src, uint32_t bytes, unsigned char *smem, uint64_t *mbar) {
-    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(mbar);
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-            "l"(src), "r"(bytes), "r"(bar)
-            : "memory");
-    }
-    uint32_t done = 0;
-    for (uint32_t it = 0; it < (1u << 22) && !done; ++it) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar)
-            : "memory");
-    }
-    return done != 0;
-}
-
-__device__ __forceinline__ void warp_sum_counts(Count &c, DevCounters *C, uint32_t paths) {
-    const uint32_t full = 0xffffffffu;
-    uint32_t v = __reduce_add_sync(full, c.vertices);
-    uint32_t nv = __reduce_add_sync(full, c.node_visits);
-    uint32_t dl = __reduce_add_sync(full, c.density_lookups);
-    uint32_t me = __reduce_add_sync(full, c.mie_evals);
-    uint32_t gu = __reduce_add_sync(full, c.gave_up);
-    uint32_t pa = __reduce_add_sync(full, paths);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&C->vertices, (unsigned long long)v);
-        atomicAdd(&C->node_visits, (unsigned long long)nv);
-        atomicAdd(&C->density_lookups, (unsigned long long)dl);
-        atomicAdd(&C->mie_evals, (unsigned long long)me);
-        if (gu) atomicAdd(&C->gave_up, (unsigned long long)gu);
-        atomicAdd(&C->paths, (unsigned long long)pa);
-    }
-}
-
-__device__ __forceinline__ float4 shfl_xor4(float4 v, int m) {
-    v.x = __shfl_xor_sync(0xffffffffu, v.x, m);
-    v.y = __shfl_xor_sync(0xffffffffu, v.y, m);
-    v.z = __shfl_xor_sync(0xffffffffu, v.z, m);
-    v.w = __shfl_xor_sync(0xffffffffu, v.w, m);
-    return v;
-}
-
-__device__ __forceinline__ float4 add4(float4 a, float4 b) {
-    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
 
 // One thread per (pixel, sample) path; thread g renders pixel g / spp, sample
 // g % spp, so a warp holds 32 consecutive samples of a pixel when spp % 32 == 0
@@ -287,12 +214,10 @@ __device__ __forceinline__ void finish_path(PathLane<WALK> &L, const DevParams &
 // One traversal step.  Returns 0 after moving to another cell (call again), 1
 // when a leaf was entered and its free flight prepared, 2 when the segment has
 // no further leaf (or the depth mask stops it): the segment escaped.
-// SHS: the traversal stack lives in shared memory (column shcol, shlevels
-// entries) instead of the lane's local arrays nstack / tstack.
-template <bool WALK, uint32_t FEAT, bool SHS>
+template <bool WALK, uint32_t FEAT>
 __device__ __forceinline__ uint32_t trav_step(PathLane<WALK> &L, const DevScene &S, const DevParams &P,
                                               const uint4 *cam_pool, uint32_t *nstack, Trav *slow, Count &cnt,
-                                              uint32_t visits, float (*tstack)[6], float *shcol, int shlevels) {
+                                              uint32_t visits, float (*tstack)[6]) {
     uint32_t leaf = 0;
     float tra = 0.0f, trb = 0.0f;
     uint32_t r;
@@ -316,12 +241,9 @@ __device__ __forceinline__ uint32_t trav_step(PathLane<WALK> &L, const DevScene 
                 L.st.t.tn = 0;
                 r = kTravDone;
             }
-        } else if constexpr (SHS)
-            r = L.wmode == 3u ? trav_next_s(L.st.t, S, SharedStack<kPersistentBlock>{shcol, shlevels}, leaf, tra,
-                                            trb, cnt, budget)
-                              : kTravDone;
-        else
+        } else {
             r = L.wmode == 3u ? trav_next_k(L.st.t, S, nstack, leaf, tra, trb, cnt, budget, tstack) : kTravDone;
+        }
     } else if (L.wmode == 1u) {
         r = walk_step(L.st.w, S, leaf, tra, trb, cnt);
     } else if (L.wmode == 2u) {
@@ -599,18 +521,17 @@ __device__ __forceinline__ bool start_path(PathLane<WALK> &L, uint64_t p, const 
 }
 
 // One loop iteration of a lane that holds a path (see render_persistent_kernel).
-template <bool WALK, uint32_t FEAT, bool SHS>
+template <bool WALK, uint32_t FEAT>
 __device__ __forceinline__ void lane_work(PathLane<WALK> &L, bool events, const DevScene &S, const DevParams &P,
                                           const MieSmem &M, const TileArgs &A, float4 *sun_out, float4 *sky_out,
                                           Count &cnt, uint32_t &state, uint32_t *nstack, Trav *slow, uint32_t visits,
-                                          uint32_t steps, float (*tstack)[6], float *shcol, int shlevels) {
+                                          uint32_t steps, float (*tstack)[6]) {
     if (events) {
         if (state == kEvent) path_event<WALK, FEAT>(L, S, P, M, A, sun_out, sky_out, cnt, state, slow);
         return;
     }
     if (state == kTrav) {
-        const uint32_t r =
-            trav_step<WALK, FEAT, SHS>(L, S, P, A.cam_pool, nstack, slow, cnt, visits, tstack, shcol, shlevels);
+        const uint32_t r = trav_step<WALK, FEAT>(L, S, P, A.cam_pool, nstack, slow, cnt, visits, tstack);
         if (r == 1u) {
             state = kStep;
         } else if (r == 2u) {
@@ -711,10 +632,7 @@ __device__ __forceinline__ uint32_t find_view(const BatchArgs &B, uint64_t p) {
 // BATCH: the paths of many views (each with its own scene, parameters, tile
 // and output) share one work queue; a lane looks its view up when it fetches
 // a path and reads that view's records from global memory (L1-resident).
-// SHS (stack traversal only): the traversal stack of each lane lives in
-// dynamic shared memory after the phase tables, `knobs` bits 24-31 entries
-// deep (kShWords words per entry and lane), instead of local memory.
-template <int MINB, bool WALK, bool BATCH, uint32_t FEAT, bool SHS = false>
+template <int MINB, bool WALK, bool BATCH, uint32_t FEAT>
 __global__ void __launch_bounds__(kPersistentBlock, MINB) render_persistent_kernel(DevScene S, DevParams P, TileArgs A,
                                                                             const void *mie_pack, float4 *sun_out,
                                                                             float4 *sky_out, DevCounters *C,
@@ -724,8 +642,6 @@ __global__ void __launch_bounds__(kPersistentBlock, MINB) render_persistent_kern
     // iteration (0: to the next leaf), bits 16-23 the tracking steps per iteration
     const uint32_t event_batch = knobs & 0xffu, visits = (knobs >> 8) & 0xffu;
     const uint32_t steps = ((knobs >> 16) & 0xffu) ? ((knobs >> 16) & 0xffu) : 1u;
-    const int shlevels = (int)(knobs >> 24);
-    static_assert(!(SHS && WALK), "the shared-memory stack serves the stack traversal");
     float ts[kMaxDepth][6];  // ancestors' intervals of the stack traversal (local memory)
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t mbar;
@@ -746,7 +662,6 @@ __global__ void __launch_bounds__(kPersistentBlock, MINB) render_persistent_kern
         if (B.step) shift = *B.step * A.spp;
     }
     const bool staged = stage_mie(mie_pack, mb, smem, &mbar);
-    float *const shcol = reinterpret_cast<float *>(smem + ((mb + 15u) & ~15u)) + threadIdx.x;
     Count cnt;
     cnt.zero();
     uint32_t paths = 0;
@@ -760,10 +675,9 @@ __global__ void __launch_bounds__(kPersistentBlock, MINB) render_persistent_kern
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const unsigned FULL = 0xffffffffu;
-    // this warp's sky queue, after the phase tables and the shared traversal stack
-    float *const skyq = reinterpret_cast<float *>(smem + ((mb + 15u) & ~15u) +
-                                                  (size_t)shlevels * kShWords * 4u * kPersistentBlock) +
-                        (threadIdx.x >> 5) * sky_queue_words<BATCH>();
+    // this warp's sky queue, after the phase tables
+    float *const skyq =
+        reinterpret_cast<float *>(smem + ((mb + 15u) & ~15u)) + (threadIdx.x >> 5) * sky_queue_words<BATCH>();
     uint32_t nsky = 0;
     for (;;) {
         const uint32_t want = __ballot_sync(FULL, state == kFetch);
@@ -796,15 +710,14 @@ __global__ void __launch_bounds__(kPersistentBlock, MINB) render_persistent_kern
         const bool events = ev && ((uint32_t)__popc(ev) >= event_batch || busy == 0);
         if constexpr (BATCH) {
             const BatchView &V = B.views[view];
-            lane_work<WALK, FEAT, SHS>(L, events, B.scenes[V.scene], V.P, M, V.A, V.sun, V.sky, cnt, state, nstack,
-                                      slow, visits, steps, ts, shcol, shlevels);
+            lane_work<WALK, FEAT>(L, events, B.scenes[V.scene], V.P, M, V.A, V.sun, V.sky, cnt, state, nstack, slow,
+                                  visits, steps, ts);
             // FEAT == 0: the launcher reserved the queue (views that defer set V.A.defer_sky)
             if constexpr (FEAT == 0) {
                 if (events) sky_queue_push<true>(L, V.A, view, P, sky_out, B, skyq, nsky, lane, lt_mask);
             }
         } else {
-            lane_work<WALK, FEAT, SHS>(L, events, S, P, M, A, sun_out, sky_out, cnt, state, nstack, slow, visits,
-                                      steps, ts, shcol, shlevels);
+            lane_work<WALK, FEAT>(L, events, S, P, M, A, sun_out, sky_out, cnt, state, nstack, slow, visits, steps, ts);
             if constexpr (FEAT == 0) {
                 if (events && A.defer_sky)
                     sky_queue_push<false>(L, A, 0u, P, sky_out, B, skyq, nsky, lane, lt_mask);
@@ -1505,7 +1418,8 @@ __global__ void adjoint_transmittance_kernel(DevScene S, DevParams P, const floa
 // (src/scene.cpp:889-904), times scale (>= 1: headroom that lets samples grow
 // while the majorant stays fixed); a leaf whose majorant was 0 (never
 // resampled) keeps 0.
-__global__ void leaf_majorant_kernel(float4 *leaf, const uint32_t *leaf_nodes, uint32_t n_leafnodes,
+// gleaf, gmaj: the same by slot (null without a block grid).
+__global__ void leaf_majorant_kernel(float4 *leaf, float4 *gleaf, float *gmaj, const uint32_t *leaf_nodes, uint32_t n_leafnodes,
                                      const float *bricks, float scale) {
     const uint32_t i = blockIdx.x;
     if (i >= n_leafnodes) return;
@@ -1524,6 +1438,10 @@ __global__ void leaf_majorant_kernel(float4 *leaf, const uint32_t *leaf_nodes, u
         wm[0] = fmaxf(m, wm[0]);
         if (meta.x != 0.0f) meta.x = fmaxf(wm[0], 0.01f) * scale;
         leaf[2 * (size_t)node + 1] = meta;
+        if (gleaf) {
+            gleaf[2 * (size_t)__float_as_uint(meta.w) + 1] = meta;
+            gmaj[__float_as_uint(meta.w)] = meta.x;
+        }
     }
 }
 
@@ -1591,7 +1509,7 @@ template <class F> static cudaError_t allow_smem(F fn, size_t smem) {
 }
 
 // Feature bits a frame needs.
-static uint32_t frame_features(const DevScene &S, const DevParams &P) {
+uint32_t frame_features(const DevScene &S, const DevParams &P) {
     return ((S.occ_nodes && P.embree) ? kFeatOcc : 0u) |
            ((P.phase_mode == kPhaseHG || P.env_mode != kEnvHosek) ? kFeatExt : 0u) | (S.sdf_bricks ? kFeatSdf : 0u);
 }
@@ -1631,12 +1549,6 @@ static PersistentFn persistent_variant_of(uint32_t minb, uint32_t traversal) {
                                               : render_persistent_kernel<5, true, BATCH, FEAT>;
         return minb >= 7 ? render_persistent_kernel<8, false, BATCH, FEAT> : render_persistent_kernel<5, false, BATCH, FEAT>;
     } else {
-        if (traversal == 2u) {
-            if (minb >= 8) return render_persistent_kernel<8, false, BATCH, 0, true>;
-            if (minb >= 6) return render_persistent_kernel<6, false, BATCH, 0, true>;
-            if (minb >= 5) return render_persistent_kernel<5, false, BATCH, 0, true>;
-            return render_persistent_kernel<4, false, BATCH, 0, true>;
-        }
         if (traversal == 1u) {
             if (minb >= 8) return render_persistent_kernel<8, true, BATCH, 0>;
             if (minb >= 6) return render_persistent_kernel<6, true, BATCH, 0>;
@@ -1658,15 +1570,6 @@ static PersistentFn persistent_variant(uint32_t minb, uint32_t traversal, bool b
                            : persistent_variant_of<true, 0>(minb, traversal);
     return feat ? persistent_variant_of<false, kFeatAll>(minb, traversal)
                 : persistent_variant_of<false, 0>(minb, traversal);
-}
-
-int persistent_max_blocks_per_sm(uint32_t variant, uint32_t traversal, size_t smem_bytes) {
-    int nb = 0;
-    const PersistentFn fn = persistent_variant(variant, traversal, false);
-    if (allow_smem(fn, smem_bytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kPersistentBlock, smem_bytes) != cudaSuccess)
-        return 1;
-    return nb > 0 ? nb : 1;
 }
 
 // Grid of the persistent kernel: SMs x resident blocks (the tuned count, capped
@@ -1691,32 +1594,25 @@ static cudaError_t persistent_grid(const Tuning &tune, int device, size_t smem, 
     return cudaSuccess;
 }
 
-// Largest octree depth whose traversal stack goes to shared memory: 7 entries
-// x 16 B x 128 lanes = 14 KB per block besides the phase tables.
-constexpr uint32_t kShStackMax = 7;
-
-// DR_TRAVERSAL_STACK_SHARED: only for the plain instantiation and octrees of
-// known, modest depth (and within the default 48 KB of dynamic shared memory);
-// otherwise the local-memory stack.  Returns the stack entries (0: local).
-static uint32_t shared_stack_plan(Tuning &tune, uint32_t feat, uint32_t stack_levels, size_t &smem) {
-    if (tune.traversal != 2u) return 0;
-    const size_t with = ((smem + 15) & ~(size_t)15) + (size_t)stack_levels * kShWords * 4 * kPersistentBlock;
-    if (feat == 0 && stack_levels >= 1 && stack_levels <= kShStackMax && with <= 48 * 1024) {
-        smem = with;
-        return stack_levels;
-    }
-    tune.traversal = 0;
-    return 0;
-}
-
 cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                                      float4 *sun_out, float4 *sky_out, DevCounters *C, WorkQueue *Q,
-                                     const Tuning &tune_in, int device, cudaStream_t st, const CamLists &lists) {
+                                     const Tuning &tune, int device, cudaStream_t st, const CamLists &lists) {
     if (A.n_paths == 0) return cudaSuccess;
     size_t smem = mie_smem(P);
     const uint32_t feat = frame_features(S, P);
-    Tuning tune = tune_in;
-    const uint32_t shlevels = shared_stack_plan(tune, feat, S.stack_levels, smem);
+    if (paths_serve(tune, S.glevels) && lists.ctl) {
+        PathWork W{};
+        W.ctl = lists.ctl;
+        W.pool_used = &lists.ctl->pool_used;
+        W.n_active = &lists.ctl->n_active;
+        W.head = lists.head;
+        W.pool = lists.pool;
+        W.pool_cap = lists.cap;
+        W.active = lists.active;
+        W.records = lists.records;
+        W.cap = lists.rec_cap;
+        return launch_paths(S, P, A, mie_pack, sun_out, sky_out, C, W, feat != 0, device, st);
+    }
     // sky terms evaluated by full warps (Hosek sky only; a whole-path
     // finiteness check needs the path's sky sum in place)
     TileArgs Ad = A;
@@ -1727,10 +1623,9 @@ cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, cons
     uint32_t batch;
     cudaError_t e = persistent_grid(tune, device, smem, false, feat, fn, blocks, batch);
     if (e != cudaSuccess) return e;
-    batch |= shlevels << 24;
     e = cudaMemsetAsync(Q, 0, sizeof(WorkQueue), st);
     if (e != cudaSuccess) return e;
-    if (lists.head && tune.traversal != 1u) {  // the cell walk counts grid cells: it keeps its own traversal
+    if (lists.head && lists.cap && tune.traversal != 1u) {  // the cell walk counts grid cells: it keeps its own traversal
         e = cudaMemsetAsync(lists.used, 0, sizeof(unsigned int), st);
         if (e != cudaSuccess) return e;
         const uint32_t npix = A.cols * A.rows;
@@ -1755,19 +1650,15 @@ cudaError_t launch_batch_lists(const BatchArgs &B, const BatchLists &lists, cuda
 }
 
 cudaError_t launch_batch_kernel(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                                WorkQueue *Q, const Tuning &tune_in, bool ext, uint32_t stack_levels, int device,
-                                cudaStream_t st) {
+                                WorkQueue *Q, const Tuning &tune, bool ext, int device, cudaStream_t st) {
     if (!B.n_paths) return cudaSuccess;
     size_t smem = mie_smem(P0);
-    Tuning tune = tune_in;
-    const uint32_t shlevels = shared_stack_plan(tune, ext ? kFeatAll : 0u, stack_levels, smem);
     if (!ext) smem = ((smem + 15) & ~(size_t)15) + (size_t)sky_queue_words<true>() * 4u * (kPersistentBlock / 32);
     PersistentFn fn;
     int blocks;
     uint32_t knobs;
     cudaError_t e = persistent_grid(tune, device, smem, true, ext ? kFeatAll : 0u, fn, blocks, knobs);
     if (e != cudaSuccess) return e;
-    knobs |= shlevels << 24;
     fn<<<blocks, kPersistentBlock, smem, st>>>(DevScene{}, DevParams{}, TileArgs{}, mie_pack, nullptr, nullptr, C, Q,
                                                knobs, B);
     return cudaGetLastError();
@@ -1775,12 +1666,10 @@ cudaError_t launch_batch_kernel(const BatchArgs &B, const DevParams &P0, const v
 
 cudaError_t launch_batch_view(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                               float4 *sun_out, float4 *sky_out, DevCounters *C, WorkQueue *Q,
-                              const unsigned long long *step, const Tuning &tune_in, int device, cudaStream_t st) {
+                              const unsigned long long *step, const Tuning &tune, int device, cudaStream_t st) {
     if (A.n_paths == 0) return cudaSuccess;
     size_t smem = mie_smem(P);
     const uint32_t feat = frame_features(S, P);
-    Tuning tune = tune_in;
-    const uint32_t shlevels = shared_stack_plan(tune, feat, S.stack_levels, smem);
     TileArgs Ad = A;
     Ad.defer_sky = (feat == 0 && !P.finite_paths) ? 1u : 0u;
     if (Ad.defer_sky) smem = ((smem + 15) & ~(size_t)15) + (size_t)sky_queue_words<false>() * 4u * (kPersistentBlock / 32);
@@ -1789,7 +1678,6 @@ cudaError_t launch_batch_view(const DevScene &S, const DevParams &P, const TileA
     uint32_t knobs;
     cudaError_t e = persistent_grid(tune, device, smem, false, feat, fn, blocks, knobs);
     if (e != cudaSuccess) return e;
-    knobs |= shlevels << 24;
     BatchArgs B{};
     B.step = step;
     fn<<<blocks, kPersistentBlock, smem, st>>>(S, P, Ad, mie_pack, sun_out, sky_out, C, Q, knobs, B);
@@ -1799,18 +1687,6 @@ cudaError_t launch_batch_view(const DevScene &S, const DevParams &P, const TileA
 cudaError_t launch_batch_step(unsigned long long *step, cudaStream_t st) {
     batch_step_kernel<<<1, 1, 0, st>>>(step);
     return cudaGetLastError();
-}
-
-cudaError_t launch_render_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                                WorkQueue *Q, unsigned long long *step, const Tuning &tune, bool ext,
-                                uint32_t stack_levels, int device, cudaStream_t st, const BatchLists &lists) {
-    cudaError_t e = cudaMemsetAsync(Q, 0, sizeof(WorkQueue), st);
-    if (e != cudaSuccess) return e;
-    e = launch_batch_lists(B, lists, st);  // the views' TileArgs point into these lists
-    if (e != cudaSuccess) return e;
-    e = launch_batch_kernel(B, P0, mie_pack, C, Q, tune, ext, stack_levels, device, st);
-    if (e != cudaSuccess) return e;
-    return launch_batch_step(step, st);
 }
 
 cudaError_t launch_add_counters(DevCounters *dst, const DevCounters *src, cudaStream_t st) {
@@ -1946,10 +1822,10 @@ cudaError_t launch_adjoint_transmittance(const DevScene &S, const DevParams &P, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_leaf_majorants(float4 *leaf, const uint32_t *leaf_nodes, uint32_t n_leafnodes, const float *bricks,
-                                  float scale, cudaStream_t st) {
+cudaError_t launch_leaf_majorants(float4 *leaf, float4 *gleaf, float *gmaj, const uint32_t *leaf_nodes,
+                                  uint32_t n_leafnodes, const float *bricks, float scale, cudaStream_t st) {
     if (n_leafnodes == 0) return cudaSuccess;
-    leaf_majorant_kernel<<<n_leafnodes, 128, 0, st>>>(leaf, leaf_nodes, n_leafnodes, bricks, scale);
+    leaf_majorant_kernel<<<n_leafnodes, 128, 0, st>>>(leaf, gleaf, gmaj, leaf_nodes, n_leafnodes, bricks, scale);
     return cudaGetLastError();
 }
 

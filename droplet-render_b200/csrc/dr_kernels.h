@@ -19,44 +19,58 @@ struct CamLists {
     uint4 *pool = nullptr;
     uint32_t cap = 0;
     unsigned int *used = nullptr;
+    // storage of the path pipeline (null: the persistent kernel runs)
+    PathCtl *ctl = nullptr;
+    uint32_t *active = nullptr;  // cols * rows
+    uint4 *records = nullptr;
+    uint32_t rec_cap = 0;
 };
-// Persistent path kernel; Q->next must be 0 (the launcher clears it on st).
+// Whether the path pipeline (dr_paths.cu) serves launches with this tuning:
+// scenes with a block grid, unless the cell walk is asked for.
+bool paths_serve(const Tuning &tune, uint32_t glevels);
+// The path pipeline of a tile.  feat: the frame needs the optional features.
+// step: a batch's launch counter (its view's samples start at A.sample_base + *step * spp), or null.
+cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
+                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &W, bool feat, int device,
+                         cudaStream_t st, const unsigned long long *step = nullptr);
+// The path pipeline of every view of B (their TileArgs::cam_head set); n_paths:
+// their samples, n_blocks: the sum of their path_list_blocks.
+cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
+                               const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool feat, uint32_t glevels,
+                               int device, cudaStream_t st);
+uint32_t path_list_blocks(uint32_t cols, uint32_t rows);
+// Feature bits a frame needs (0: the plain kernels).
+uint32_t frame_features(const DevScene &S, const DevParams &P);
+// Tile render: the path pipeline where the scene has a block grid (and lists.ctl
+// its storage), else the persistent path kernel; Q->next must be 0 (the launcher clears it on st).
 // With a stack traversal and lists given, the camera rays' leaf lists are built
 // on st first (camera_list_kernel).
 cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                                      float4 *sun_out, float4 *sky_out, DevCounters *C, WorkQueue *Q,
                                      const Tuning &tune, int device, cudaStream_t st, const CamLists &lists = {});
-// Batched persistent launch over all views of B (P0: the first view's parameters,
-// which fix the shared phase tables), then one increment of *step; Q->next is
-// cleared on st first.  The three launches are what a batch's graph captures.
-// stack_levels: the deepest traversal stack any of the batch's scenes needs (0: unknown)
-// lists: the views' camera leaf lists (the views' TileArgs::cam_head point at
-// lists.head + pix_begins[v]; head null when the views traverse), built first.
+// Camera leaf lists of a batch: the views' TileArgs::cam_head point at
+// lists.head + pix_begins[v]; head null when the views traverse.
 struct BatchLists {
     CamLists lists;
     const uint32_t *pix_begins = nullptr;  // first pixel of each view among the batch's pixels
     uint32_t n_pix = 0;
 };
-cudaError_t launch_render_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                                WorkQueue *Q, unsigned long long *step, const Tuning &tune, bool ext,
-                                uint32_t stack_levels, int device, cudaStream_t st, const BatchLists &lists = {});
-// The parts of launch_render_batch, for graphs that split a batch:
+// The launches of a batch's graph where the pipeline does not serve it (the
+// work queues must be 0):
 // the camera leaf lists of every view of B (nothing when lists.head is null);
 cudaError_t launch_batch_lists(const BatchArgs &B, const BatchLists &lists, cudaStream_t st);
-// one batched persistent kernel over the views of B (Q->next must be 0);
+// one batched persistent kernel over the views of B (P0: the first view's
+// parameters, which fix the shared phase tables);
 cudaError_t launch_batch_kernel(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                                WorkQueue *Q, const Tuning &tune, bool ext, uint32_t stack_levels, int device,
-                                cudaStream_t st);
+                                WorkQueue *Q, const Tuning &tune, bool ext, int device, cudaStream_t st);
 // one view of a batch as a plain persistent kernel of its own: the view's
 // parameters and tile are kernel arguments (A.cam_head: its lists, already
-// built; A.sample_base + *step * spp is its first sample; Q->next must be 0);
+// built; A.sample_base + *step * spp is its first sample);
 cudaError_t launch_batch_view(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                               float4 *sun_out, float4 *sky_out, DevCounters *C, WorkQueue *Q,
                               const unsigned long long *step, const Tuning &tune, int device, cudaStream_t st);
 // *step += 1 (the last node of a batch's graph).
 cudaError_t launch_batch_step(unsigned long long *step, cudaStream_t st);
-// Resident blocks per SM of the persistent kernel for the given dynamic shared memory.
-int persistent_max_blocks_per_sm(uint32_t variant, uint32_t traversal, size_t smem_bytes);
 cudaError_t launch_probe_leaf(const DevScene &S, const float *ro, const float *rd, uint32_t n, uint32_t maxn,
                               uint32_t *nodes, float *tr0, float *tr1, uint32_t *counts, cudaStream_t st);
 cudaError_t launch_probe_occlusion(const DevScene &S, const float *ro, const float *rd, uint32_t n, uint32_t *hit,
@@ -94,9 +108,10 @@ cudaError_t launch_reweighted_loss(const DevScene &S, const DevParams &P, const 
 cudaError_t launch_adjoint_transmittance(const DevScene &S, const DevParams &P, const float *ro, const float *rd,
                                          const float *wr, uint32_t n_rays, uint64_t nsamp, uint64_t seed, float *grad,
                                          unsigned long long *escapes, cudaStream_t st);
-// Leaf majorants of the listed leaf nodes recomputed from the brick pool.
-cudaError_t launch_leaf_majorants(float4 *leaf, const uint32_t *leaf_nodes, uint32_t n_leafnodes, const float *bricks,
-                                  float scale, cudaStream_t st);
+// Leaf majorants of the listed leaf nodes recomputed from the brick pool, in
+// the records by node id and by slot (gleaf and gmaj may be null).
+cudaError_t launch_leaf_majorants(float4 *leaf, float4 *gleaf, float *gmaj, const uint32_t *leaf_nodes,
+                                  uint32_t n_leafnodes, const float *bricks, float scale, cudaStream_t st);
 
 // dst += src, field by field (one thread; a blocking call's counters).
 cudaError_t launch_add_counters(DevCounters *dst, const DevCounters *src, cudaStream_t st);

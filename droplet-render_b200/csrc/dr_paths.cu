@@ -1,0 +1,981 @@
+// The path pipeline: three kernels that render a tile (or every view of a
+// batch) whose octree has a block grid (DevScene::gblock).
+//
+//   camera lists   one thread per pixel traverses the camera ray once and
+//                  records its leaves; pixels whose ray meets no leaf are counted
+//                  and finished here, the others go to a list of active pixels
+//   camera paths   the camera segments of the active pixels' samples, 32 samples
+//                  of a pixel side by side: a warp's lanes read the same leaf list
+//                  and run the same steps.  The samples that collide become records
+//   scatter        everything after a path's first collision, from the records
+//
+// Splitting the paths there is what the hardware asks for: a path is mostly a
+// camera segment that hits nothing (of the 512^3 cumulus frame's 133 M samples
+// 119 M meet no leaf at all and about 5 M collide), those are coherent, and the
+// rest is not.  One kernel for all three (render_persistent_kernel, which
+// serves the octrees without a block grid) was bound by instruction issue at 8
+// of 32 lanes per instruction: 38.5 ms for that frame at 64 samples, 51.9 ms for a
+// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 18.9 and 23.4 ms:
+// lists 0.26, camera 2.4, scatter 16 ms of the first, at 13 lanes per instruction.
+//
+// Per path, the operations and random draws are those of path_sample(): a
+// path's result does not depend on the kernel that computed it.
+#include <cuda_runtime.h>
+#include "dr_kernels.h"
+#include "dr_stage.cuh"
+
+namespace dr {
+
+constexpr uint32_t kFull = 0xffffffffu;
+constexpr uint32_t kChunks = 4;             // groups of 32 camera samples per ticket
+constexpr uint32_t kTicket = 32 * kChunks;  // camera samples per ticket
+constexpr int kListBlock = 128, kListTx = 16, kListTy = 8;  // camera lists: a block covers 16 x 8 pixels
+
+// ---- camera lists -------------------------------------------------------------
+// Leaf list of one camera ray: the ray's traversal run to its end, as every
+// sample of the pixel would run it.  The leaves are counted first, then a
+// contiguous range of the pool is taken and filled by a second traversal; a
+// pixel whose range does not fit gets x = ~0 and its samples traverse.
+// Rays with a zero direction component take the octree (node ids become slots).
+__device__ __noinline__ uint4 octree_list(const DevScene S, float ox, float oy, float oz, float dx, float dy, float dz,
+                                          uint4 *pool, uint32_t cap, unsigned int *used) {
+    const float ro[3] = {ox, oy, oz}, rd[3] = {dx, dy, dz};
+    uint32_t nstack[kMaxDepth];
+    float tstack[kMaxDepth][6];
+    Trav T;
+    Count c;
+    c.zero();
+    trav_init(T, S, ro, rd, c);
+    uint4 h = make_uint4(0u, 0u, c.node_visits, 0u);
+    uint32_t leaf, n = 0;
+    float tra, trb;
+    while (trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack) == kTravLeaf) ++n;
+    const unsigned int off = n ? atomicAdd(used, n) : 0u;
+    if (n && (off > cap || n > cap - off)) {
+        h.x = kNone;
+        return h;
+    }
+    h.x = off;
+    h.y = n;
+    trav_init(T, S, ro, rd, c);
+    c.zero();
+    for (uint32_t k = 0; k < n; ++k) {
+        trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack);
+        pool[off + k] = make_uint4(__float_as_uint(__ldg(&S.leaf[2 * leaf + 1]).w), __float_as_uint(tra),
+                                   __float_as_uint(trb), c.node_visits);
+        c.zero();
+    }
+    trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack);  // kTravDone
+    h.w = c.node_visits;
+    return h;
+}
+
+__device__ __forceinline__ uint4 grid_list(const DevScene &S, const float ro[3], const float rd[3], float *col,
+                                           uint4 *pool, uint32_t cap, unsigned int *used) {
+    GridTrav G;
+    Count c;
+    c.zero();
+    const uint32_t mode = grid_init<kListBlock>(G, S, col, ro, rd, c);
+    if (mode == 2u) return octree_list(S, ro[0], ro[1], ro[2], rd[0], rd[1], rd[2], pool, cap, used);
+    if (mode == 0u) return make_uint4(0u, 0u, 0u, 0u);
+    uint32_t leaf, n = 0;
+    float tra, trb;
+    while (grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
+    if (n == 0) return make_uint4(0u, 0u, 1u, c.node_visits - 1u);
+    const unsigned int off = atomicAdd(used, n);
+    if (off > cap || n > cap - off) return make_uint4(kNone, 0u, 0u, 0u);
+    c.zero();
+    grid_init<kListBlock>(G, S, col, ro, rd, c);
+    c.node_visits -= 1u;  // the root (h.z)
+    for (uint32_t k = 0; k < n; ++k) {
+        grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone);
+        pool[off + k] = make_uint4(leaf, __float_as_uint(tra), __float_as_uint(trb), c.node_visits);
+        c.zero();
+    }
+    grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone);  // kTravDone
+    return make_uint4(off, n, 1u, c.node_visits);
+}
+
+// Pixel (ix, iy) of a tile (valid lanes): its header, and its place among the
+// active pixels or, without a leaf, its samples' counters.
+__device__ __forceinline__ void list_pixel(const DevScene &S, const DevParams &P, const TileArgs &A, uint32_t ix,
+                                           uint32_t iy, bool valid, float *col, uint4 *head, const PathWork &W,
+                                           uint32_t *active, unsigned int *n_active, DevCounters *C) {
+    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+    bool ray = false;
+    const uint32_t pix = iy * A.cols + ix;
+    if (valid) {
+        float ro[3], rd[3];
+        ray = camera_ray(P, A.x0 + ix, A.y0 + iy, ro, rd);
+        if (ray) h = grid_list(S, ro, rd, col, W.pool, W.pool_cap, W.pool_used);
+        head[2 * (size_t)pix] = h;
+        head[2 * (size_t)pix + 1] =
+            make_uint4(__float_as_uint(rd[0]), __float_as_uint(rd[1]), __float_as_uint(rd[2]), ray ? 1u : 0u);
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool act = ray && (h.y > 0u || h.x == kNone);
+    const uint32_t am = __ballot_sync(kFull, act), em = __ballot_sync(kFull, ray && !act);
+    uint32_t at = 0;
+    if (lane == 0 && am) at = atomicAdd(n_active, (unsigned int)__popc(am));
+    at = __shfl_sync(kFull, at, 0);
+    if (act) active[at + __popc(am & ((1u << lane) - 1u))] = pix;
+    if (em) {
+        const uint32_t v = __reduce_add_sync(kFull, (ray && !act) ? h.z + h.w : 0u);
+        if (lane == 0) {
+            const unsigned long long n = (unsigned long long)__popc(em) * A.spp;
+            atomicAdd(&C->paths, n);
+            atomicAdd(&C->vertices, n);
+            atomicAdd(&C->node_visits, (unsigned long long)v * A.spp);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kListBlock) path_lists_kernel(DevScene S, DevParams P, TileArgs A, PathWork W,
+                                                                DevCounters *C) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float *const col = reinterpret_cast<float *>(smem) + threadIdx.x;
+    const uint32_t bx = (A.cols + kListTx - 1) / kListTx, by = blockIdx.x / bx;
+    const uint32_t ix = (blockIdx.x - by * bx) * kListTx + (threadIdx.x & (kListTx - 1));
+    const uint32_t iy = by * kListTy + threadIdx.x / kListTx;
+    list_pixel(S, P, A, ix, iy, ix < A.cols && iy < A.rows, col, W.head, W, W.active, W.n_active, C);
+}
+
+// The lists of every view of a batch: view v owns the blocks from
+// block_begins[v] on, its pixels' headers start at its TileArgs::cam_head and its
+// active pixels at active + pix_begins[v].
+__device__ __forceinline__ uint32_t find_last(const uint32_t *begins, uint32_t n, uint32_t t) {
+    uint32_t lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(&begins[mid]) <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(kListBlock) path_lists_batch_kernel(BatchArgs B, PathWork W, DevCounters *C) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float *const col = reinterpret_cast<float *>(smem) + threadIdx.x;
+    const uint32_t v = find_last(W.block_begins, B.n_views, blockIdx.x), blk = blockIdx.x - __ldg(&W.block_begins[v]);
+    const BatchView &V = B.views[v];
+    const uint32_t bx = (V.A.cols + kListTx - 1) / kListTx, by = blk / bx;
+    const uint32_t ix = (blk - by * bx) * kListTx + (threadIdx.x & (kListTx - 1));
+    const uint32_t iy = by * kListTy + threadIdx.x / kListTx;
+    list_pixel(B.scenes[V.scene], V.P, V.A, ix, iy, ix < V.A.cols && iy < V.A.rows, col,
+               const_cast<uint4 *>(V.A.cam_head), W, W.active + W.pix_begins[v], &W.view_active[v], C);
+}
+
+// First ticket of every view (and the number of tickets) from its active pixels: one warp.
+__global__ void view_tickets_kernel(BatchArgs B, PathWork W) {
+    const uint32_t lane = threadIdx.x;
+    uint32_t run = 0;
+    for (uint32_t v0 = 0; v0 < B.n_views; v0 += 32) {
+        const uint32_t v = v0 + lane;
+        uint32_t n = 0;
+        if (v < B.n_views) n = (uint32_t)(((uint64_t)W.view_active[v] * B.views[v].A.spp + kTicket - 1) / kTicket);
+        uint32_t sum = n;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(kFull, sum, d);
+            if (lane >= (uint32_t)d) sum += o;
+        }
+        if (v < B.n_views) W.view_tickets[v] = run + sum - n;
+        run += __shfl_sync(kFull, sum, 31);
+    }
+    if (lane == 0) W.view_tickets[B.n_views] = run;
+}
+
+// ---- free flight in a leaf ---------------------------------------------------------
+// A flight leaves_at_once does not decide, in full (src/kernel.cpp:241-317): a flight in leaf `slot`
+// with interval [tra, trb], entered at distance lo.  first: v is the uniform
+// draw of the first flight, else the distance flown so far in the leaf.
+// kLeft: the leaf is left; kReal: a real collision at td; kNull: a null one (v
+// is the distance flown, call again).
+enum : uint32_t { kLeft = 0, kReal = 1, kNull = 2 };
+template <uint32_t FEAT>
+__device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e, const float ro[3], const float rd[3],
+                                                uint32_t slot, float tra, float trb, float lo, bool first, float &v,
+                                                float &td, Rng &g, Count &cnt) {
+    const float4 meta = __ldg(&S.gleaf[2 * slot + 1]);
+    const float denom = sigma_e * meta.x;
+    const float tr0 = tra - lo, tr1 = trb - lo;
+    float s0 = tra > lo ? tr0 : __uint_as_float(__float_as_uint(tr0) & 1u);
+    const float *sdf = nullptr;
+    if constexpr ((FEAT & kFeatSdf) != 0) {
+        const uint32_t sdfx = __float_as_uint(meta.z);
+        if (sdfx != kNone) {
+            sdf = S.sdf_bricks + (size_t)sdfx * kBrick;
+            s0 = 0.0f;
+            if (tra > lo) {  // src/kernel.cpp:253-263
+                const float r0[3] = {ro[0] + rd[0] * tra, ro[1] + rd[1] * tra, ro[2] + rd[2] * tra};
+                if (sample_voxel_space(r0, sdf, __ldg(&S.gleaf[2 * slot])) > 0.0f) s0 = tr0;
+                if (first) ++cnt.density_lookups;
+            }
+        }
+    }
+    const float u = first ? v : g.uniform();
+    const float sr = (first ? 0.0f : v) - dlog(u) / denom;
+    v = sr;
+    const float sc = s0 + sr;
+    td = lo + sc;
+    if (!(sc < tr1)) {
+        td = trb;
+        return kLeft;
+    }
+    bool rm = sc > tr0;
+    float rho = -1.0f, dist = 1.0f;
+    if (rm) {
+        const float4 ce = __ldg(&S.gleaf[2 * slot]);
+        const float rc[3] = {ro[0] + rd[0] * td, ro[1] + rd[1] * td, ro[2] + rd[2] * td};
+        const uint32_t fog = __float_as_uint(meta.y);
+        bool look = true;
+        if constexpr ((FEAT & kFeatSdf) != 0) {
+            if (sdf) {  // src/kernel.cpp:287-300: inside the surface always collides
+                dist = sample_voxel_space(rc, sdf, ce);
+                ++cnt.density_lookups;
+                look = dist > 0.0f && fog != kNone;
+            }
+        }
+        if (look) {
+            rho = sample_voxel_space(rc, S.bricks + (size_t)fog * kBrick, ce);
+            ++cnt.density_lookups;
+        }
+    }
+    const float q = g.uniform();
+    return rm && (rho / meta.x < q) && (dist > 0.0f) ? kNull : kReal;
+}
+
+// Whether a leaf may be passed by leaves_at_once: not with a surface brick
+// (its flight starts where the distance at the entry says).
+template <uint32_t FEAT>
+__device__ __forceinline__ bool fog_only(const DevScene &S, uint32_t slot) {
+    if constexpr ((FEAT & kFeatSdf) != 0) return __float_as_uint(__ldg(&S.gleaf[2 * slot + 1]).z) == kNone;
+    else return true;
+}
+
+// ---- camera paths ---------------------------------------------------------------
+// A lane walks a sample's camera segment: it enters its next leaf and draws the
+// first flight (kWalk), or waits with a flight to be computed in full (kHard,
+// kHardAgain; these run when enough lanes wait, or all), or is done (kOut).
+enum : uint32_t { kWalk = 0, kHard = 1, kHardAgain = 2, kOut = 3 };
+constexpr uint32_t kHardBatch = 8;
+
+struct SlowSeg {
+    uint32_t res, visits, lookups, gave_up;
+    float td;
+    uint64_t state;
+};
+// A segment with a zero direction component, traced through the octree.
+template <uint32_t FEAT>
+__device__ __noinline__ SlowSeg slow_segment(const DevScene S, SegMedium med, float ox, float oy, float oz, float dx,
+                                             float dy, float dz, float depth, uint64_t state, uint64_t inc) {
+    const float ro[3] = {ox, oy, oz}, rd[3] = {dx, dy, dz};
+    uint32_t nstack[kMaxDepth];
+    const NoVisit nv;
+    Count c;
+    c.zero();
+    Rng g;
+    g.state = state;
+    g.inc = inc;
+    SlowSeg o;
+    o.res = track_v<NoVisit, (FEAT & kFeatSdf) != 0>(S, med, ro, rd, g, depth, o.td, nstack, c, nv);
+    o.visits = c.node_visits;
+    o.lookups = c.density_lookups;
+    o.gave_up = c.gave_up;
+    o.state = g.state;
+    return o;
+}
+
+struct CamSeg {
+    uint32_t res;
+    float td;
+    Rng g;
+};
+
+// Camera segments of a warp's 32 samples (alive lanes).  LISTED: along the
+// pixel's leaf list h; else by traversing.
+template <uint32_t FEAT, bool LISTED>
+__device__ __forceinline__ CamSeg camera_segments(const DevScene &S, SegMedium med, bool alive, const float ro[3],
+                                                  const float rd[3], Rng g, float depth, uint4 h, const uint4 *pool,
+                                                  float *col, Count &cnt) {
+    uint32_t k = h.x, left = h.y, budget = med.budget, slot = 0;
+    float td = 0.0f, lo = 0.0f, v = 0.0f, tra = 0.0f, trb = 0.0f;
+    CamSeg o;
+    o.res = kTrackEscaped;
+    GridTrav G;
+    uint32_t st = alive ? kWalk : kOut;
+    if (alive) {
+        if constexpr (LISTED) {
+            cnt.node_visits += h.z;
+        } else {
+            const uint32_t m = grid_init<kListBlock>(G, S, col, ro, rd, cnt);
+            if (m == 0u) st = kOut;
+            if (m == 2u) {  // a zero direction component
+                const SlowSeg q = slow_segment<FEAT>(S, med, ro[0], ro[1], ro[2], rd[0], rd[1], rd[2], depth, g.state,
+                                                     g.inc);
+                cnt.node_visits += q.visits;
+                cnt.density_lookups += q.lookups;
+                cnt.gave_up += q.gave_up;
+                o.res = q.res;
+                td = q.td;
+                g.state = q.state;
+                st = kOut;
+            }
+        }
+    }
+    for (;;) {
+        if (st == kWalk) {
+            uint32_t r;
+            if constexpr (LISTED) {
+                if (left) {
+                    const uint4 e = __ldg(&pool[k]);
+                    ++k;
+                    --left;
+                    slot = e.x;
+                    tra = __uint_as_float(e.y);
+                    trb = __uint_as_float(e.z);
+                    cnt.node_visits += e.w;
+                    r = kTravLeaf;
+                } else {
+                    cnt.node_visits += h.w;
+                    r = kTravDone;
+                }
+            } else {
+                r = grid_next<kListBlock>(G, S, col, ro, rd, slot, tra, trb, cnt, 1u);
+            }
+            if (r == kTravDone || (r == kTravLeaf && !(td < depth))) {
+                st = kOut;
+            } else if (r == kTravLeaf) {
+                const float denom = med.sigma_e * __ldg(&S.gmaj[slot]);
+                v = g.uniform();
+                if (leaves_at_once(v, denom, tra, trb, td) && fog_only<FEAT>(S, slot)) {
+                    td = trb;
+                } else {
+                    lo = td;
+                    st = kHard;
+                }
+            }
+        }
+        const bool hard = st == kHard || st == kHardAgain;
+        const uint32_t nl = __ballot_sync(kFull, hard), nb = __ballot_sync(kFull, st == kWalk);
+        if (!(nl | nb)) break;
+        if (nl && ((uint32_t)__popc(nl) >= kHardBatch || !nb) && hard) {
+            const uint32_t r = leaf_flight<FEAT>(S, med.sigma_e, ro, rd, slot, tra, trb, lo, st == kHard, v, td, g, cnt);
+            st = r == kLeft ? kWalk : kHardAgain;
+            if (r == kReal) {
+                o.res = td < depth ? kTrackCollided : kTrackCut;
+                st = kOut;
+            } else if (r == kNull && --budget == 0) {
+                ++cnt.gave_up;
+                st = kOut;
+            }
+        }
+    }
+    o.td = td;
+    o.g = g;
+    return o;
+}
+
+// Sample q of a tile's active pixels: pixel and sample number.
+__device__ __forceinline__ void active_sample(const TileArgs &A, const uint32_t *active, uint64_t q, uint32_t &pix,
+                                              uint32_t &s) {
+    uint32_t a;
+    if (q <= 0xffffffffull) {
+        a = fastdiv((uint32_t)q, A.spp_div);
+        s = (uint32_t)q - a * A.spp;
+    } else {
+        const uint64_t l = q / A.spp;
+        a = (uint32_t)l;
+        s = (uint32_t)(q - l * A.spp);
+    }
+    pix = __ldg(&active[a]);
+}
+
+// Camera samples are handed out in tickets of kTicket consecutive ones.  A warp
+// takes a ticket only while the record buffer has room for every warp's
+// (W.limit = capacity - warps * kTicket), so the buffer never overflows and the
+// tickets taken are exactly those done: the next round goes on from there.
+template <uint32_t FEAT, bool BATCH>
+__global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(DevScene S0, DevParams P0, TileArgs A0, PathWork W,
+                                                                     float4 *sun0, float4 *sky0, DevCounters *C,
+                                                                     BatchArgs B) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float *const col = reinterpret_cast<float *>(smem) + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    Count cnt;
+    cnt.zero();
+    uint32_t paths = 0;
+    uint64_t total = 0;
+    uint32_t n_tickets;
+    const uint64_t step = B.step ? *B.step : 0ull;
+    if constexpr (BATCH) {
+        n_tickets = W.view_tickets[B.n_views];
+    } else {
+        total = (uint64_t)*W.n_active * A0.spp;
+        n_tickets = (uint32_t)((total + kTicket - 1) / kTicket);
+    }
+    const unsigned long long base = W.ctl->base;
+    for (;;) {
+        unsigned long long t = ~0ull;
+        if (lane == 0) {
+            const uint32_t rec = *(volatile uint32_t *)&W.ctl->records;
+            const unsigned long long tk = *(volatile unsigned long long *)&W.ctl->ticket;
+            if (rec <= W.limit && tk < n_tickets && tk - base < kRoundTickets) t = atomicAdd(&W.ctl->ticket, 1ull);
+        }
+        t = __shfl_sync(kFull, t, 0);
+        if (t >= n_tickets) break;
+        uint32_t view = 0;
+        uint64_t q0 = t * kTicket;
+        if constexpr (BATCH) {
+            view = find_last(W.view_tickets, B.n_views, (uint32_t)t);
+            q0 = (t - W.view_tickets[view]) * kTicket;
+            total = (uint64_t)W.view_active[view] * B.views[view].A.spp;
+        }
+        const BatchView *V = BATCH ? &B.views[view] : nullptr;
+        const TileArgs &A = BATCH ? V->A : A0;
+        const DevParams &P = BATCH ? V->P : P0;
+        const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+        const uint4 *head = BATCH ? A.cam_head : W.head;
+        const uint32_t *active = BATCH ? W.active + W.pix_begins[view] : W.active;
+        for (uint32_t c = 0; c < kChunks; ++c) {
+            const uint64_t q = q0 + c * 32u + lane;
+            if (q - lane >= total) break;
+            const bool valid = q < total;
+            uint32_t pix = kNone, s = 0;
+            uint4 h = make_uint4(0u, 0u, 0u, 0u);
+            float ro[3], rd[3] = {0.0f, 0.0f, 0.0f};
+            for (int k = 0; k < 3; ++k) ro[k] = P.viewi[12 + k];
+            float depth = 3.402823466e+38f;
+            Rng g;
+            g.state = g.inc = 0;
+            if (valid) {
+                active_sample(A, active, q, pix, s);
+                h = __ldg(&head[2 * (size_t)pix]);
+                const uint4 ray = __ldg(&head[2 * (size_t)pix + 1]);
+                rd[0] = __uint_as_float(ray.x);
+                rd[1] = __uint_as_float(ray.y);
+                rd[2] = __uint_as_float(ray.z);
+                const uint32_t iy = fastdiv(pix, A.cols_div), ix = pix - iy * A.cols;
+                const uint64_t fp = (uint64_t)(A.y0 + iy) * P.w + (A.x0 + ix);
+                if (P.depth && P.depthcomp) depth = __ldg(&P.depth[fp]);
+                g = rng_seed(A.seed, fp, A.sample_base + step * A.spp + s);
+                ++paths;
+                ++cnt.vertices;
+            }
+            CamSeg o;
+            if (!__any_sync(kFull, valid && h.x == kNone))
+                o = camera_segments<FEAT, true>(S, seg_medium(P), valid, ro, rd, g, depth, h, W.pool, col, cnt);
+            else  // a pixel whose list did not fit: the whole group traverses
+                o = camera_segments<FEAT, false>(S, seg_medium(P), valid, ro, rd, g, depth, h, W.pool, col, cnt);
+            // alpha of the pixel's samples that collided (or were cut at the depth, src/kernel.cpp:370-384)
+            const bool hit = valid && first_alpha(P, o.res) != 0.0f;
+            const uint32_t hm = __ballot_sync(kFull, hit);
+            if (hit) {
+                const uint32_t same = __match_any_sync(hm, pix);
+                if (lane == (uint32_t)__ffs((int)same) - 1u) {
+                    const uint32_t iy = fastdiv(pix, A.cols_div);
+                    const size_t off = (size_t)iy * A.tw + (pix - iy * A.cols);
+                    const float a = (float)__popc(same);
+                    atomicAdd(&(BATCH ? V->sun : sun0)[off].w, a);
+                    atomicAdd(&(BATCH ? V->sky : sky0)[off].w, a);
+                }
+            }
+            const bool go = valid && o.res == kTrackCollided && P.scattevs > 0u;
+            const uint32_t gm = __ballot_sync(kFull, go);
+            if (gm) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&W.ctl->records, (uint32_t)__popc(gm));
+                at = __shfl_sync(kFull, at, 0) + __popc(gm & ((1u << lane) - 1u));
+                if (go)
+                    W.records[at] = make_uint4((uint32_t)o.g.state, (uint32_t)(o.g.state >> 32), __float_as_uint(o.td),
+                                               (uint32_t)(t * kTicket + c * 32u + lane));
+            }
+        }
+    }
+    warp_sum_counts(cnt, C, paths);
+}
+
+// Between rounds: the tickets taken so far are done, the record buffer is empty.
+__global__ void next_round_kernel(PathCtl *ctl) {
+    ctl->base = ctl->ticket;
+    ctl->records = 0;
+    ctl->head = 0;
+}
+
+// ---- scatter ------------------------------------------------------------------------
+// Each warp owns kSlots path slots in shared memory.  Its 32 lanes trace
+// segments; everything a path needs only between segments (throughput, sums,
+// the pending continuation) stays in the slot.  A path moves through
+//   event list   collided: a scattering event is due
+//   ready list   scattered: its shadow segment waits for a lane
+//   a lane       the shadow segment, then at once the continuation
+// and the warp shades its event list 32 at a time, so neither the scattering
+// code nor the tracing loop waits on lanes that hold the other kind of work.
+// Nothing is shared between warps but the record counter.
+//
+// The tracing loop's body runs a grid step, with the first flight of a leaf it
+// finds, for the lanes on their way and, when enough of them wait, the flights to
+// be computed in full; segment ends are processed when kEndBatch lanes have one.
+enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
+// Slots and residency were measured on the 512^3 frame: 64 slots at 4 blocks per
+// SM 19.7 ms, 56 at 5 20.8, 48 at 5 21.9, 48 at 6 (80 registers) 25.9; more warps
+// cost L1 (the slots are shared memory) and instruction cache.
+constexpr int kScatterBlock = 128;
+constexpr int kSlots = 64;
+constexpr uint32_t kEventBatch = kSlots - 32;  // events that make a shading pass
+constexpr uint32_t kEndBatch = 10;             // lanes at a segment end (or idle with work ready) that make an end pass
+constexpr uint32_t kWaitBatch = 10;            // lanes that make a pass of full flights
+constexpr uint32_t kFetchBatch = 16;           // free slots that make a fetch
+constexpr int kBurst = 3;                      // loop bodies between looks at the lists
+// slot words (word w of slot s at w * kSlots + s)
+enum : int { wState = 0, wInc = 2, wRo = 4, wRd = 7, wT = 10, wSun = 13, wSw = 16, wSrd = 19, wTd = 22, wOff = 23, wEv = 24,
+             wView = 25 };
+template <bool BATCH> __host__ __device__ constexpr int slot_words() { return BATCH ? 26 : 25; }
+template <bool BATCH> __host__ __device__ constexpr int skyq_words() { return (BATCH ? 8 : 7) * 32; }
+// bytes per warp: slots, three lists of slot numbers, the sky queue
+template <bool BATCH> __host__ __device__ constexpr size_t scatter_warp_bytes() {
+    return 4 * (size_t)(slot_words<BATCH>() * kSlots + skyq_words<BATCH>()) + 3 * (size_t)kSlots;
+}
+
+// The sky terms of escaped paths are evaluated by full warps: entry i of the
+// queue is (rd, T, output offset[, view]) in column i; T * sky(rd) is the value
+// the path would have added in place (its sky sum is 0 before the escape).
+template <bool BATCH>
+__device__ __noinline__ void path_sky_eval(const DevParams &P, float4 *sky_out, const BatchArgs &B, const float *q,
+                                              uint32_t i) {
+    const float rd[3] = {q[i], q[32 + i], q[64 + i]};
+    float3 sky;
+    float4 *out;
+    if constexpr (BATCH) {
+        const BatchView &V = B.views[__float_as_uint(q[224 + i])];
+        sky = escape_sky<0>(V.P, rd);
+        out = V.sky;
+    } else {
+        sky = escape_sky<0>(P, rd);
+        out = sky_out;
+    }
+    atomicAdd(&out[__float_as_uint(q[192 + i])],
+              make_float4(q[96 + i] * sky.x, q[128 + i] * sky.y, q[160 + i] * sky.z, 0.0f));
+}
+
+template <uint32_t FEAT, bool BATCH, int MINB>
+__global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __grid_constant__ DevScene S0,
+                                                                      const __grid_constant__ DevParams P0,
+                                                                      const __grid_constant__ TileArgs A0,
+                                                                      const __grid_constant__ PathWork W,
+                                                                      const void *mie_pack, float4 *sun0, float4 *sky0,
+                                                                      DevCounters *C, const __grid_constant__ BatchArgs B,
+                                                                      uint32_t colwords,
+                                                                      uint32_t defer) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint64_t mbar;
+    if (W.ctl->records == 0u) return;  // a round without records: leave before staging
+    const uint32_t mb = BATCH ? mie_bytes(B.views[0].P) : mie_bytes(P0);
+    const MieSmem M = BATCH ? mie_view(B.views[0].P, smem) : mie_view(P0, smem);
+    const bool staged = stage_mie(mie_pack, mb, smem, &mbar);
+    if (!staged) {
+        if (threadIdx.x == 0) atomicAdd(&C->gave_up, 1ull);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    unsigned char *const area = smem + ((mb + 15u) & ~15u);
+    float *const col = reinterpret_cast<float *>(area) + threadIdx.x;
+    float *const slots = reinterpret_cast<float *>(area + (size_t)colwords * 4u * kScatterBlock +
+                                                   (threadIdx.x >> 5) * scatter_warp_bytes<BATCH>());
+    float *const skyq = slots + slot_words<BATCH>() * kSlots;
+    uint8_t *const ready = reinterpret_cast<uint8_t *>(skyq + skyq_words<BATCH>());
+    uint8_t *const event = ready + kSlots, *const freed = event + kSlots;
+    uint32_t n_ready = 0, n_event = 0, n_free = kSlots, n_sky = 0;
+    for (uint32_t i = lane; i < (uint32_t)kSlots; i += 32) freed[i] = (uint8_t)i;
+    __syncwarp();
+    const uint32_t n_rec = W.ctl->records;
+    const uint64_t qbase = W.ctl->base * kTicket;
+    const uint64_t step = B.step ? *B.step : 0ull;
+    bool more = true;
+    Count cnt;
+    cnt.zero();
+    uint32_t scatters = 0;
+    // the lane's segment
+    uint32_t st = kIdle, slot = 0, res = 0, budget = 0, view = 0;
+    bool shadow = false;
+    float ro[3] = {0.f, 0.f, 0.f}, rd[3] = {0.f, 0.f, 0.f};
+    Rng g;
+    g.state = g.inc = 0;
+    GridTrav G;
+    uint32_t leaf = 0;                            // the leaf a full flight is due in,
+    float td = 0.0f, lo = 0.0f, v = 0.0f;         // the distance at its entry and leaf_flight's v
+#define SLOT(w, s) slots[(w)*kSlots + (s)]
+    for (;;) {
+        const uint32_t endm = __ballot_sync(kFull, st == kEnd), idle = __ballot_sync(kFull, st == kIdle);
+        const uint32_t busy = ~(endm | idle);
+        // ---- segment ends, and idle lanes with segments ready
+        const uint32_t due = (uint32_t)__popc(endm) + min((uint32_t)__popc(idle), n_ready);
+        if (due && (due >= kEndBatch || !busy)) {
+            bool init = false, finish = false, sky = false;
+            bool to_event = false;
+            float T[3] = {0.f, 0.f, 0.f};
+            const BatchView *V = BATCH ? &B.views[view] : nullptr;
+            const DevParams &P = BATCH ? V->P : P0;
+            const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+            if (st == kEnd) {
+                if (shadow) {
+                    if (res == kTrackEscaped && !((FEAT & kFeatOcc) && P.embree && occluded(S, ro, rd))) {
+                        const bool hit = sun_hit(P, rd);
+                        for (int k = 0; k < 3; ++k)
+                            SLOT(wSun + k, slot) = SLOT(wSun + k, slot) + SLOT(wSw + k, slot) * (hit ? P.sun_color[k] : 0.0f);
+                    }
+                    for (int k = 0; k < 3; ++k) rd[k] = SLOT(wSrd + k, slot);
+                    shadow = false;
+                    init = true;
+                } else if (res == kTrackCollided && __float_as_uint(SLOT(wEv, slot)) < P.scattevs) {
+                    SLOT(wState, slot) = __uint_as_float((uint32_t)g.state);
+                    SLOT(wState + 1, slot) = __uint_as_float((uint32_t)(g.state >> 32));
+                    SLOT(wTd, slot) = td;
+                    to_event = true;
+                } else {
+                    float4 sun = make_float4(SLOT(wSun, slot), SLOT(wSun + 1, slot), SLOT(wSun + 2, slot), 0.0f);
+                    float4 skyv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (res == kTrackEscaped && !((FEAT & kFeatOcc) && P.embree && occluded(S, ro, rd))) {
+                        const bool hit = sun_hit(P, rd);
+                        for (int k = 0; k < 3; ++k) T[k] = SLOT(wT + k, slot);
+                        sun.x = sun.x + T[0] * (hit ? P.sun_color[0] : 0.0f);
+                        sun.y = sun.y + T[1] * (hit ? P.sun_color[1] : 0.0f);
+                        sun.z = sun.z + T[2] * (hit ? P.sun_color[2] : 0.0f);
+                        const bool later = BATCH ? V->A.defer_sky != 0u : defer != 0u;
+                        if (FEAT == 0 && later) {
+                            sky = true;
+                        } else {
+                            const float3 e = escape_sky<FEAT>(P, rd);
+                            skyv.x = T[0] * e.x;
+                            skyv.y = T[1] * e.y;
+                            skyv.z = T[2] * e.z;
+                        }
+                    }
+                    drop_nonfinite(P, sun, skyv);
+                    const uint32_t off = __float_as_uint(SLOT(wOff, slot));
+                    if ((sun.x != 0.0f) | (sun.y != 0.0f) | (sun.z != 0.0f))
+                        atomicAdd(&(BATCH ? V->sun : sun0)[off], sun);
+                    if ((skyv.x != 0.0f) | (skyv.y != 0.0f) | (skyv.z != 0.0f))
+                        atomicAdd(&(BATCH ? V->sky : sky0)[off], skyv);
+                    finish = true;
+                }
+            }
+            if constexpr (FEAT == 0) {  // the sky terms go to the warp's queue, evaluated 32 at a time
+                const uint32_t sm = __ballot_sync(kFull, sky);
+                if (sm) {
+                    const uint32_t pos = n_sky + __popc(sm & lt), total = n_sky + __popc(sm);
+                    const uint32_t off = sky ? __float_as_uint(SLOT(wOff, slot)) : 0u;
+                    for (uint32_t pass = 0; pass < 2; ++pass) {
+                        const uint32_t p = pos - 32u * pass;
+                        if (sky && (pass ? pos >= 32u : pos < 32u)) {
+                            for (int k = 0; k < 3; ++k) {
+                                skyq[32 * k + p] = rd[k];
+                                skyq[96 + 32 * k + p] = T[k];
+                            }
+                            skyq[192 + p] = __uint_as_float(off);
+                            if constexpr (BATCH) skyq[224 + p] = __uint_as_float(view);
+                        }
+                        __syncwarp();
+                        if (pass == 1 || total < 32u) break;
+                        path_sky_eval<BATCH>(P0, sky0, B, skyq, lane);
+                        __syncwarp();
+                    }
+                    n_sky = total & 31u;
+                }
+            }
+            const uint32_t em = __ballot_sync(kFull, to_event), fm = __ballot_sync(kFull, finish);
+            if (to_event) event[n_event + __popc(em & lt)] = (uint8_t)slot;
+            if (finish) freed[n_free + __popc(fm & lt)] = (uint8_t)slot;
+            n_event += __popc(em);
+            n_free += __popc(fm);
+            if (to_event || finish) st = kIdle;
+            // idle lanes take ready paths: their shadow segments
+            const uint32_t im = __ballot_sync(kFull, st == kIdle);
+            const uint32_t rank = __popc(im & lt);
+            if (st == kIdle && rank < n_ready) {
+                slot = ready[n_ready - 1u - rank];
+                for (int k = 0; k < 3; ++k) {
+                    ro[k] = SLOT(wRo + k, slot);
+                    rd[k] = SLOT(wRd + k, slot);
+                }
+                g.state = (uint64_t)__float_as_uint(SLOT(wState, slot)) | (uint64_t)__float_as_uint(SLOT(wState + 1, slot)) << 32;
+                g.inc = (uint64_t)__float_as_uint(SLOT(wInc, slot)) | (uint64_t)__float_as_uint(SLOT(wInc + 1, slot)) << 32;
+                if constexpr (BATCH) view = __float_as_uint(SLOT(wView, slot));
+                shadow = true;
+                init = true;
+            }
+            n_ready -= min(n_ready, (uint32_t)__popc(im));
+            if (init) {
+                const BatchView *V2 = BATCH ? &B.views[view] : nullptr;
+                const DevScene &S2 = BATCH ? B.scenes[V2->scene] : S0;
+                const DevParams &P2 = BATCH ? V2->P : P0;
+                td = 0.0f;
+                budget = P2.step_budget;
+                const uint32_t m = grid_init<kScatterBlock>(G, S2, col, ro, rd, cnt);
+                st = kWalk;
+                if (m == 0u) {
+                    res = kTrackEscaped;
+                    st = kEnd;
+                } else if (m == 2u) {
+                    const SlowSeg o = slow_segment<FEAT>(S2, seg_medium(P2), ro[0], ro[1], ro[2], rd[0], rd[1], rd[2],
+                                                         3.402823466e+38f, g.state, g.inc);
+                    cnt.node_visits += o.visits;
+                    cnt.density_lookups += o.lookups;
+                    cnt.gave_up += o.gave_up;
+                    res = o.res;
+                    td = o.td;
+                    g.state = o.state;
+                    st = kEnd;
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        // ---- scattering events
+        if (n_event && (n_event >= kEventBatch || (!busy && !due))) {
+            const uint32_t n = min(n_event, 32u);
+            if (lane < n) {
+                const uint32_t s = event[n_event - n + lane];
+                const BatchView *V = BATCH ? &B.views[__float_as_uint(SLOT(BATCH ? wView : 0, s))] : nullptr;
+                const DevParams &P = BATCH ? V->P : P0;
+                Rng e;
+                e.state = (uint64_t)__float_as_uint(SLOT(wState, s)) | (uint64_t)__float_as_uint(SLOT(wState + 1, s)) << 32;
+                e.inc = (uint64_t)__float_as_uint(SLOT(wInc, s)) | (uint64_t)__float_as_uint(SLOT(wInc + 1, s)) << 32;
+                float d[3], srd[3], lrd[3];
+                for (int k = 0; k < 3; ++k) d[k] = SLOT(wSrd + k, s);
+                const float u1 = e.uniform(), u2 = e.uniform();
+                path_phase_sample<FEAT>(P, M, d, u1, u2, srd);
+                const float u3 = e.uniform(), u4 = e.uniform();
+                sun_sample(P, u3, u4, lrd);
+                const float3 p1 = path_phase_eval<FEAT>(P, M, dot3(srd, d));
+                const float p2 = sun_hit(P, lrd) ? P.sun_pdf : 0.0f;
+                const float3 p3 = path_phase_eval<FEAT>(P, M, dot3(lrd, d));
+                const float q1 = sun_hit(P, srd) ? P.sun_pdf : 0.0f;
+                const float f = P.albedo;
+                const float a1[3] = {p1.x, p1.y, p1.z}, a3[3] = {p3.x, p3.y, p3.z};
+                const float td = SLOT(wTd, s);
+                for (int k = 0; k < 3; ++k) {
+                    const float T = SLOT(wT + k, s);
+                    SLOT(wSw + k, s) = T * ((a3[k] / (a3[k] + p2)) * f);
+                    SLOT(wT + k, s) = T * ((a1[k] / (a1[k] + q1)) * f);
+                    SLOT(wRo + k, s) = SLOT(wRo + k, s) + d[k] * td;
+                    SLOT(wRd + k, s) = lrd[k];
+                    SLOT(wSrd + k, s) = srd[k];
+                }
+                SLOT(wState, s) = __uint_as_float((uint32_t)e.state);
+                SLOT(wState + 1, s) = __uint_as_float((uint32_t)(e.state >> 32));
+                SLOT(wEv, s) = __uint_as_float(__float_as_uint(SLOT(wEv, s)) + 1u);
+                ready[n_ready + lane] = (uint8_t)s;
+                ++scatters;
+            }
+            n_event -= n;
+            n_ready += n;
+            __syncwarp();
+            continue;
+        }
+        // ---- new paths
+        if (more && n_free && (n_free >= kFetchBatch || !busy)) {
+            const uint32_t want = min(n_free, 32u);
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&W.ctl->head, want);
+            at = __shfl_sync(kFull, at, 0);
+            const uint32_t n = at < n_rec ? min(want, n_rec - at) : 0u;
+            if (n < want) more = false;
+            if (lane < n) {
+                const uint32_t s = freed[n_free - 1u - lane];
+                const uint4 r = __ldg(&W.records[at + lane]);
+                uint64_t q = qbase + (uint32_t)(r.w - (uint32_t)qbase);
+                uint32_t v = 0;
+                if constexpr (BATCH) {
+                    v = find_last(W.view_tickets, B.n_views, (uint32_t)(q / kTicket));
+                    q -= (uint64_t)W.view_tickets[v] * kTicket;
+                    SLOT(wView, s) = __uint_as_float(v);
+                }
+                const BatchView *V = BATCH ? &B.views[v] : nullptr;
+                const TileArgs &A = BATCH ? V->A : A0;
+                const DevParams &P = BATCH ? V->P : P0;
+                uint32_t pix, sm;
+                active_sample(A, BATCH ? W.active + W.pix_begins[v] : W.active, q, pix, sm);
+                const uint4 ray = __ldg(&(BATCH ? A.cam_head : W.head)[2 * (size_t)pix + 1]);
+                const uint32_t iy = fastdiv(pix, A.cols_div), ix = pix - iy * A.cols;
+                const uint64_t inc = rng_inc(A.seed, (uint64_t)(A.y0 + iy) * P.w + (A.x0 + ix), A.sample_base + step * A.spp + sm);
+                SLOT(wState, s) = __uint_as_float(r.x);
+                SLOT(wState + 1, s) = __uint_as_float(r.y);
+                SLOT(wInc, s) = __uint_as_float((uint32_t)inc);
+                SLOT(wInc + 1, s) = __uint_as_float((uint32_t)(inc >> 32));
+                SLOT(wSrd, s) = __uint_as_float(ray.x);
+                SLOT(wSrd + 1, s) = __uint_as_float(ray.y);
+                SLOT(wSrd + 2, s) = __uint_as_float(ray.z);
+                for (int k = 0; k < 3; ++k) {
+                    SLOT(wRo + k, s) = P.viewi[12 + k];
+                    SLOT(wT + k, s) = 1.0f;
+                    SLOT(wSun + k, s) = 0.0f;
+                }
+                SLOT(wTd, s) = __uint_as_float(r.z);
+                SLOT(wOff, s) = __uint_as_float(iy * A.tw + ix);
+                SLOT(wEv, s) = __uint_as_float(0u);
+                event[n_event + lane] = (uint8_t)s;
+            }
+            n_free -= n;
+            n_event += n;
+            __syncwarp();
+            continue;
+        }
+        if (!busy && !due) break;  // nothing in flight, ready, to shade or to fetch
+        // ---- tracing
+        const BatchView *V = BATCH ? &B.views[view] : nullptr;
+        const DevParams &P = BATCH ? V->P : P0;
+        const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+#pragma unroll 1
+        for (int it = 0; it < kBurst; ++it) {
+            if (st == kWalk) {
+                float tra = 0.0f, trb = 0.0f;
+                const uint32_t r = grid_next<kScatterBlock>(G, S, col, ro, rd, leaf, tra, trb, cnt, 1u);
+                if (r == kTravDone) {
+                    res = kTrackEscaped;
+                    st = kEnd;
+                } else if (r == kTravLeaf) {
+                    const float denom = P.sigma_e * __ldg(&S.gmaj[leaf]);
+                    v = g.uniform();
+                    if (leaves_at_once(v, denom, tra, trb, td) && fog_only<FEAT>(S, leaf)) {
+                        td = trb;
+                    } else {
+                        lo = td;
+                        st = kHard;
+                    }
+                }
+            }
+            const bool hard = st == kHard || st == kHardAgain;
+            const uint32_t wait = __ballot_sync(kFull, hard);
+            if (wait && ((uint32_t)__popc(wait) >= kWaitBatch || !__any_sync(kFull, st == kWalk)) && hard) {
+                const float trb = std_min(std_min(G.x[0], G.x[1]), G.x[2]);  // the leaf is the current cell
+                const uint32_t r =
+                    leaf_flight<FEAT>(S, P.sigma_e, ro, rd, leaf, G.tc, trb, lo, st == kHard, v, td, g, cnt);
+                st = r == kLeft ? kWalk : kHardAgain;
+                if (r == kReal) {
+                    res = kTrackCollided;
+                    st = kEnd;
+                } else if (r == kNull && --budget == 0) {
+                    ++cnt.gave_up;
+                    res = kTrackEscaped;
+                    st = kEnd;
+                }
+            }
+        }
+    }
+#undef SLOT
+    if constexpr (FEAT == 0) {
+        __syncwarp();
+        if (lane < n_sky) path_sky_eval<BATCH>(P0, sky0, B, skyq, lane);
+    }
+    cnt.vertices = 2u * scatters;  // every event's shadow and continuation segments
+    cnt.mie_evals = 3u * scatters;
+    warp_sum_counts(cnt, C, 0u);
+}
+
+// ---- launches ---------------------------------------------------------------------------
+static size_t table_bytes(const DevParams &P) {
+    return (size_t)P.mie_n * 20u + (P.phase_mode == 1u ? (2u * (size_t)P.mie_n + 1u) * 16u : 0u);
+}
+
+template <class F> static cudaError_t opt_in(F fn, size_t smem) {
+    if (smem <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem);
+}
+
+static uint64_t rounds_of(uint64_t n_paths, uint64_t limit) {
+    const uint64_t span = (uint64_t)kRoundTickets * kTicket;
+    return (n_paths + limit - 1) / limit + n_paths / span;
+}
+
+using CameraFn = void (*)(DevScene, DevParams, TileArgs, PathWork, float4 *, float4 *, DevCounters *, BatchArgs);
+using ScatterFn = void (*)(DevScene, DevParams, TileArgs, PathWork, const void *, float4 *, float4 *, DevCounters *,
+                           BatchArgs, uint32_t, uint32_t);
+
+constexpr int kScatterBlocks = 4;  // resident scatter blocks per SM the kernel is compiled for
+
+// Camera and scatter rounds over the active pixels: enough of them for every path to collide.
+template <bool BATCH>
+static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const TileArgs &A, const BatchArgs &B,
+                                 PathWork W, const void *mie_pack, float4 *sun, float4 *sky, DevCounters *C,
+                                 bool feat, uint32_t glevels, uint64_t n_paths, uint32_t defer, int device,
+                                 cudaStream_t st) {
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    const CameraFn cam = feat ? camera_paths_kernel<kFeatAll, BATCH> : camera_paths_kernel<0, BATCH>;
+    const ScatterFn sca = feat ? scatter_kernel<kFeatAll, BATCH, kScatterBlocks> : scatter_kernel<0, BATCH, kScatterBlocks>;
+    const uint32_t words = grid_words(glevels);
+    const size_t cam_smem = (size_t)words * 4 * kListBlock;
+    const size_t sca_smem = ((table_bytes(P) + 15) & ~(size_t)15) + (size_t)words * 4 * kScatterBlock +
+                            scatter_warp_bytes<BATCH>() * (kScatterBlock / 32);
+    e = opt_in(sca, sca_smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sca, kScatterBlock, sca_smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const uint64_t cam_most = (n_paths + kTicket * 4 - 1) / (kTicket * 4), sca_most = (n_paths + 127) / 128;
+    unsigned cam_blocks = (unsigned)(cam_most < (uint64_t)sms * 8 ? cam_most : (uint64_t)sms * 8);
+    const unsigned sca_blocks =
+        (unsigned)(sca_most < (uint64_t)sms * per_sm ? sca_most : (uint64_t)sms * (uint64_t)per_sm);
+    // every warp of the camera kernel may add a ticket's samples after its last
+    // look at the record count: half the buffer at most is kept for that
+    const uint64_t per_block = (uint64_t)(kListBlock / 32) * kTicket;
+    if (n_paths > W.cap) {
+        if (W.cap < 2 * per_block) return cudaErrorInvalidValue;
+        if (cam_blocks * per_block > W.cap / 2) cam_blocks = (unsigned)(W.cap / 2 / per_block);
+        W.limit = (uint32_t)(W.cap - cam_blocks * per_block);
+    } else {
+        W.limit = W.cap;
+    }
+    const uint64_t rounds = rounds_of(n_paths, W.limit);
+    for (uint64_t r = 0; r < rounds; ++r) {
+        if (r) next_round_kernel<<<1, 1, 0, st>>>(W.ctl);
+        cam<<<cam_blocks, kListBlock, cam_smem, st>>>(S, P, A, W, sun, sky, C, B);
+        sca<<<sca_blocks, kScatterBlock, sca_smem, st>>>(S, P, A, W, mie_pack, sun, sky, C, B, words, defer);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+bool paths_serve(const Tuning &tune, uint32_t glevels) { return tune.traversal != 1u && glevels != 0u; }
+
+uint32_t path_list_blocks(uint32_t cols, uint32_t rows) {
+    return ((cols + kListTx - 1) / kListTx) * ((rows + kListTy - 1) / kListTy);
+}
+
+cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
+                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &W, bool feat, int device,
+                         cudaStream_t st, const unsigned long long *step) {
+    const uint64_t n_paths = (uint64_t)A.cols * A.rows * A.spp;
+    if (n_paths == 0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(W.ctl, 0, sizeof(PathCtl), st);
+    if (e != cudaSuccess) return e;
+    path_lists_kernel<<<path_list_blocks(A.cols, A.rows), kListBlock, (size_t)grid_words(S.glevels) * 4 * kListBlock,
+                        st>>>(S, P, A, W, C);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    BatchArgs B{};
+    B.step = step;
+    return launch_rounds<false>(S, P, A, B, W, mie_pack, sun, sky, C, feat, S.glevels, n_paths,
+                                (!feat && !P.finite_paths) ? 1u : 0u, device, st);
+}
+
+cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
+                               const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool feat, uint32_t glevels,
+                               int device, cudaStream_t st) {
+    if (n_paths == 0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(W.ctl, 0, sizeof(PathCtl), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(W.view_active, 0, sizeof(uint32_t) * B.n_views, st);
+    if (e != cudaSuccess) return e;
+    path_lists_batch_kernel<<<n_blocks, kListBlock, (size_t)grid_words(glevels) * 4 * kListBlock, st>>>(B, W, C);
+    view_tickets_kernel<<<1, 32, 0, st>>>(B, W);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_rounds<true>(DevScene{}, P0, TileArgs{}, B, W, mie_pack, nullptr, nullptr, C, feat, glevels, n_paths,
+                               0u, device, st);
+}
+
+}  // namespace dr

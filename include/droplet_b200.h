@@ -245,15 +245,18 @@ int dr_set_step_budget(dr_ctx *ctx, uint32_t steps);
  * camera ray is traversed once and its samples read the leaf sequence instead
  * of traversing (every sample of a pixel shares its camera ray).  Results and
  * counters are the same with or without them.  pool_entries: entries of 16
- * bytes per list pool (0 = the default 2^23; DR_NONE = no lists); the pixels
+ * bytes per list pool (0 = the default, in proportion to the frame up to 2^23; DR_NONE = no lists); the pixels
  * whose lists do not fit traverse.  Applies to later renders of the context.
  * No reference counterpart (the reference traverses per sample). */
 int dr_set_camera_lists(dr_ctx *ctx, uint32_t pool_entries);
 
 /* ---- launch shape (no reference counterpart: the reference schedules 2x2
- * pixel blocks with TBB, src/kernel.cpp:453) ------------------------------- */
-#define DR_KERNEL_PERSISTENT 0u  /* resident warps take paths from a queue (default) */
-#define DR_KERNEL_PER_PATH 1u    /* one thread per path sample */
+ * pixel blocks with TBB, src/kernel.cpp:453) --------------------------------
+ * Scenes whose octree keeps every leaf at one depth of 2 to 9 below the root
+ * (and fewer than 2^24 leaves) render through the path pipeline, whose launch
+ * shape is its own: the fields below are kept and returned, but only `kernel`
+ * and traversal DR_TRAVERSAL_WALK choose another kernel for them.  Other scenes
+ * use the persistent kernel with all fields as described. */
 typedef struct {
     uint32_t kernel;         /* DR_KERNEL_* */
     uint32_t blocks_per_sm;  /* persistent kernel: resident blocks per SM, 0 = as many as fit */
@@ -266,9 +269,7 @@ typedef struct {
 } dr_tuning;
 #define DR_TRAVERSAL_STACK 0u  /* octree descent with a node stack (the reference's order) */
 #define DR_TRAVERSAL_WALK 1u   /* cell walk over the leaf grid, same leaf order and intervals */
-#define DR_TRAVERSAL_STACK_SHARED 2u  /* the octree descent with its stack in shared memory (frames and batches
-                                         without optional features whose octrees keep every leaf at one depth
-                                         <= 8 and have fewer than 2^25 nodes; otherwise DR_TRAVERSAL_STACK) */
+#define DR_TRAVERSAL_STACK_SHARED 2u  /* accepted for the octree descent; the same as DR_TRAVERSAL_STACK */
 int dr_set_tuning(dr_ctx *ctx, const dr_tuning *tuning);
 int dr_get_tuning(dr_ctx *ctx, dr_tuning *tuning);
 

@@ -1,0 +1,156 @@
+// Host check of the grid traversal against the octree traversal, both from the
+// device headers: leaves, intervals and node visits after every leaf, one step
+// at a time, on random, lattice-aligned, tied and far-away rays.
+//   grid_check SCENE RAYS SEED    (SCENE: n_nodes, n_leaves, then the node records)
+//   grid_check flights N SEED     leaves_at_once against the flight in full
+#include "cuda_host_shim.h"
+#include "../../droplet-render_b200/csrc/dr_device.cuh"
+#include "../../include/droplet_b200.h"
+#include "../../droplet-render_b200/csrc/dr_host.h"
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <vector>
+using namespace dr;
+
+static int flights(long long n, int seed) {
+    double least = 1e9;
+    for (uint32_t k = 0; k < (1u << 23); ++k) {  // every value of Rng::uniform
+        const float u = (float)(2 * k + 1) * 5.96046448e-08f;
+        least = std::min(least, -(double)dlog(u) / (1.0 - (double)u));
+    }
+    std::mt19937_64 g(seed);
+    std::uniform_real_distribution<double> U(0, 1);
+    long long bad = 0, quick = 0, left = 0;
+    for (long long i = 0; i < n; ++i) {
+        const double len = std::pow(10, -8 + 9 * U(g));
+        const float td = (float)((g() & 1) ? 0 : std::pow(10, -3 + 6 * U(g)));
+        const float tra = (float)((g() & 3) == 0 ? td : (g() & 1) ? td + std::pow(10, -9 + 8 * U(g)) : td - len * U(g));
+        const float trb = (g() & 63) ? (float)(tra + len) : tra;
+        const float denom = (g() & 255) ? (float)(std::pow(10, -6 + 7 * U(g)) / len) : 0.0f;
+        uint32_t k = g() & 0x7fffff;
+        if (g() & 1) {  // draws around the decision
+            const double x = 1 - 1.0001 * (double)denom * ((trb - td) - (tra > td ? tra - td : 0));
+            const long kk = x > 0 && x < 1 ? (long)(x * 8388608) + (long)(g() % 9) - 4 : -1;
+            if (kk >= 0 && kk < (1 << 23)) k = (uint32_t)kk;
+        }
+        const float u = (float)(2 * k + 1) * 5.96046448e-08f;
+        const float tr0 = tra - td, tr1 = trb - td;
+        const float s0 = tra > td ? tr0 : __uint_as_float(__float_as_uint(tr0) & 1u);
+        const float sr = 0.0f - dlog(u) / denom;
+        const bool out = !(s0 + sr < tr1), q = leaves_at_once(u, denom, tra, trb, td);
+        quick += q;
+        left += out;
+        bad += q && !out;
+    }
+    std::printf("least -dlog(u) / (1 - u) %.9f quick %lld left %lld bad %lld\n", least, quick, left, bad);
+    return least < 1.0 - 1e-6 || bad || quick < left / 2;
+}
+
+int main(int argc, char **argv) {
+    if (argc != 4) return 2;
+    if (!std::strcmp(argv[1], "flights")) return flights(atoll(argv[2]), atoi(argv[3]));
+    FILE *f = std::fopen(argv[1], "rb");
+    uint32_t head[2];
+    if (!f || std::fread(head, 4, 2, f) != 2) return 2;
+    std::vector<dr_node> N(head[0]);
+    if (std::fread(N.data(), 64, head[0], f) != head[0]) return 2;
+    std::fclose(f);
+    std::vector<float> bricks((size_t)head[1] * 512, 0.f);
+    const dr_scene_desc desc{N.data(), head[0], bricks.data(), head[1], 8, nullptr, 0};
+    HostScene h;
+    if (prepare_scene(&desc, h) != DR_OK) return 2;
+    if (!h.glevels) {
+        std::printf("no block grid\n");
+        return 3;
+    }
+    DevScene S{};
+    S.child = reinterpret_cast<const uint4 *>(h.child.data());
+    S.leaf = h.leaf.data();
+    S.gblock = h.gblock.data();
+    S.gleaf = h.gleaf.data();
+    S.glevels = h.glevels;
+    for (int k = 0; k < 4; ++k) S.root_ce[k] = h.root_ce[k];
+    std::vector<uint32_t> leaves;
+    for (uint32_t i = 0; i < head[0]; ++i)
+        if (h.leaf_flag[i]) leaves.push_back(i);
+    std::mt19937_64 g(atoi(argv[3]));
+    std::uniform_real_distribution<double> U(0, 1);
+    std::normal_distribution<double> G;
+    const double c[3] = {S.root_ce[0], S.root_ce[1], S.root_ce[2]}, e = S.root_ce[3], cell = 2 * e / (1 << h.glevels);
+    static const double D[][3] = {{1, 1, 1}, {1, 1, .5}, {1, .5, .25}, {2, 1, 1e-7}, {1e-6, 1, 1}, {3, 2, 1},
+                                  {1, 0, 0}, {0, 1, 1}, {1, 1, 0}, {.5, .25, 1}, {1, .75, .5}};
+    long long bad = 0, slow = 0, ties = 0, hits = 0;
+    for (long long i = 0; i < atoll(argv[2]); ++i) {
+        double o[3], v[3] = {G(g), G(g), G(g)};
+        const int kind = (int)(i % 8);
+        const float4 L = h.leaf[2 * (size_t)leaves[g() % leaves.size()]];
+        const double lc[3] = {L.x, L.y, L.z};
+        const double n = std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+        const double far = (g() & 1) ? 2.5 : (g() & 1) ? 1e3 : 1e5;
+        const uint64_t pick = g() % 11, half = g() & 1, back = g() & 1;
+        for (int k = 0; k < 3; ++k) {
+            const double lattice = c[k] - e + cell * (double)(g() % ((1u << h.glevels) + 3)) - cell;
+            if (kind < 3) o[k] = lc[k] + (2 * U(g) - 1) * L.w;        // inside a leaf
+            else if (kind == 3) o[k] = c[k] + (2 * U(g) - 1) * e * 1.2;  // in and around the root
+            else if (kind == 4) o[k] = lattice;
+            else if (kind == 5) {
+                v[k] = D[pick][(k + i / 8) % 3] * ((g() & 1) ? 1 : -1);
+                o[k] = lattice + (half ? cell * .5 : 0);
+            } else if (kind == 6) o[k] = lc[k] - far * v[k] / n;      // aimed at a leaf from afar
+            else {
+                v[k] = (double)(g() % 9) - 4;
+                if (k == 2 && v[0] == 0 && v[1] == 0 && v[2] == 0) v[2] = 1;
+                o[k] = lattice;
+            }
+        }
+        if (kind == 7 && back)
+            for (int k = 0; k < 3; ++k) o[k] -= 1.5 * v[k];
+        const double q = std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+        float ro[3], rd[3];
+        for (int k = 0; k < 3; ++k) {
+            ro[k] = (float)o[k];
+            rd[k] = (float)(kind == 7 && half ? v[k] : v[k] / q);
+        }
+        Count ca, cb;
+        ca.zero();
+        cb.zero();
+        Trav T;
+        uint32_t nstack[kMaxDepth];
+        float iv[kMaxDepth][6];
+        trav_init(T, S, ro, rd, ca);
+        GridTrav Gt;
+        float col[3 * kGridMaxLevels];
+        const uint32_t mode = grid_init<1>(Gt, S, col, ro, rd, cb);
+        if (mode == 2) {
+            ++slow;
+            continue;
+        }
+        if ((mode == 0) != !T.active) {
+            ++bad;
+            continue;
+        }
+        if (mode == 0) continue;
+        ++hits;
+        for (;;) {
+            uint32_t la = 0, lb = 0, r2;
+            float a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+            const uint32_t r1 = trav_next_k(T, S, nstack, la, a0, a1, ca, 0xffffffffu, iv);
+            long guard = 0;
+            do {
+                r2 = grid_next<1>(Gt, S, col, ro, rd, lb, b0, b1, cb, 1);
+            } while (r2 == kTravMore && ++guard < 100000);
+            bool same = r1 == r2 && ca.node_visits == cb.node_visits;
+            if (same && r1 == kTravLeaf)
+                same = __float_as_uint(h.leaf[2 * (size_t)la + 1].w) == lb && a0 == b0 &&
+                       __float_as_uint(a1) == __float_as_uint(b1) &&
+                       !std::memcmp(&h.gleaf[2 * (size_t)lb], &h.leaf[2 * (size_t)la], 32) &&
+                       h.gmaj[lb] == h.leaf[2 * (size_t)la + 1].x;
+            bad += !same;
+            if (!same || r1 != kTravLeaf) break;
+        }
+        ties += Gt.loc >> 16;
+    }
+    std::printf("levels %u hits %lld ties %lld slow %lld bad %lld\n", h.glevels, hits, ties, slow, bad);
+    return bad || hits == 0 || ties == 0;
+}

@@ -1,0 +1,90 @@
+"""The path pipeline (csrc/dr_paths.cu) at the sizes where it can go wrong,
+against the one-thread-per-path kernel: tiles equal up to the order of the
+per-pixel float sums (the tolerance of the other tile tests) and every counter
+equal.  The per-path kernel is pinned to the CPU restatement elsewhere."""
+import numpy as np
+import pytest
+
+from conftest import c0_cfg, depth_texture, golden_octree, settings_from_cfg
+from droplet_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def renderer():
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    r = Renderer(0)
+    r.upload(Octree(*golden_octree()))
+    yield r
+    r.close()
+
+
+def _pair(r, cfg, tile, spp, seed=11):
+    """(sun, sky, counters) of the pipeline and of the per-path kernel."""
+    r.set_params(settings_from_cfg(cfg))
+    got = []
+    for kernel in (0, 1):
+        r.set_tuning(kernel)
+        r.reset_counters()
+        sun, sky = r.render_tile(*tile, spp, seed=seed, sample_base=2)
+        got.append((sun, sky, r.counters()))
+    r.set_tuning()
+    return got
+
+
+def _check(got):
+    (s0, k0, c0), (s1, k1, c1) = got
+    assert c0 == c1
+    for g, p in ((s0, s1), (k0, k1)):
+        assert np.allclose(g, p, rtol=2e-5, atol=1e-6 * np.abs(p).max() + 1e-30)
+
+
+# tile edges (list blocks of 16 x 8 pixels, odd tiles drop a row and a column), samples around the warp and the ticket
+@pytest.mark.parametrize("tile", [(30, 30, 2, 2), (20, 22, 3, 5), (9, 14, 17, 9), (5, 3, 50, 47)])
+@pytest.mark.parametrize("spp", [1, 31, 33, 130])
+def test_tile_and_sample_edges(renderer, tile, spp):
+    _check(_pair(renderer, c0_cfg(64, 64), tile, spp))
+
+
+@pytest.mark.parametrize("events", [0, 1, 40])
+def test_event_limits(renderer, events):
+    cfg = dict(c0_cfg(64, 64), scattevs=events, sigma_s=60.0, sigma_a=0.1)
+    _check(_pair(renderer, cfg, (8, 8, 48, 48), 32))
+
+
+@pytest.mark.parametrize("flags", [{"depthcomp": True}, {"finite_paths": True}, {"depthcomp": True, "embree": True}])
+def test_depth_and_flags(renderer, flags):
+    _check(_pair(renderer, dict(c0_cfg(64, 64), depth=depth_texture(64, 64), **flags), (4, 2, 56, 60), 24))
+
+
+def test_axis_parallel_rays(renderer):
+    """The middle row and column of an odd image have a zero direction component
+    (they take the octree), and the sun stands exactly on an axis."""
+    cfg = c0_cfg(33, 33)
+    viewi = np.eye(4, dtype=np.float32)
+    viewi[3, :3] = (0.5, 0.5, 3.0)
+    cfg.update(viewi=viewi, sun_dir=np.array([0.0, 1.0, 0.0], np.float32))
+    got = _pair(renderer, cfg, (0, 0, 33, 33), 48)
+    assert got[0][2]["mie_evals"] > 0
+    _check(got)
+
+
+def test_rounds(renderer):
+    """More collided samples than the record buffer holds (2^20 for this frame):
+    the launch runs in rounds."""
+    cfg = dict(c0_cfg(32, 32), sigma_s=400.0, sigma_a=4.0, scattevs=2)
+    got = _pair(renderer, cfg, (8, 8, 16, 16), 8192)
+    assert got[0][2]["mie_evals"] > 3 * (1 << 20)
+    _check(got)
+
+
+@pytest.mark.parametrize("pool", [N.DR_NONE, 1, 300])
+def test_pixels_without_lists(renderer, pool):
+    try:
+        renderer.set_camera_lists(pool)
+        _check(_pair(renderer, c0_cfg(64, 64), (4, 6, 50, 52), 37))
+    finally:
+        renderer.set_camera_lists(0)
