@@ -257,6 +257,8 @@ int dr_set_camera_lists(dr_ctx *ctx, uint32_t pool_entries);
  * shape is its own: the fields below are kept and returned, but only `kernel`
  * and traversal DR_TRAVERSAL_WALK choose another kernel for them.  Other scenes
  * use the persistent kernel with all fields as described. */
+#define DR_KERNEL_PERSISTENT 0u  /* resident warps take paths from a queue (default), or the pipeline */
+#define DR_KERNEL_PER_PATH 1u    /* one thread per path sample */
 typedef struct {
     uint32_t kernel;         /* DR_KERNEL_* */
     uint32_t blocks_per_sm;  /* persistent kernel: resident blocks per SM, 0 = as many as fit */
