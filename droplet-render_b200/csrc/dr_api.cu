@@ -379,7 +379,8 @@ int dr_shadow_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint3
     DeviceGuard g(c->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     DR_CUDA(cudaMemsetAsync(out_dev, 0, (size_t)tw * th * sizeof(float4), st), "shadow: clear");
-    DR_CUDA(launch_shadow_tile(c->scene, c->params, A, (float4 *)out_dev, c->counters.p, st), "shadow: launch");
+    DR_CUDA(launch_shadow_tile(c->scene, c->params, A, (float4 *)out_dev, c->counters.p, c->device, st),
+            "shadow: launch");
     return DR_OK;
 }
 
@@ -396,7 +397,8 @@ int dr_shadow_tile(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint32_t th
     if (rc != DR_OK) return rc;
     DR_CUDA(cudaMemsetAsync(c->call_counters.p, 0, sizeof(DevCounters), c->stream), "shadow: clear");
     DR_CUDA(cudaMemsetAsync(c->tile_sun.p, 0, n * sizeof(float4), c->stream), "shadow: clear");
-    DR_CUDA(launch_shadow_tile(c->scene, c->params, A, c->tile_sun.p, c->call_counters.p, c->stream), "shadow: launch");
+    DR_CUDA(launch_shadow_tile(c->scene, c->params, A, c->tile_sun.p, c->call_counters.p, c->device, c->stream),
+            "shadow: launch");
     DR_CUDA(cudaMemcpyAsync(out, c->tile_sun.p, n * sizeof(float4), cudaMemcpyDeviceToHost, c->stream),
             "shadow: copy out");
     return finish_call_counters(c, "dr_shadow_tile");

@@ -65,6 +65,25 @@ __device__ __forceinline__ float dlog(float x) {
     return fmaf(fe, kLn2Hi, fmaf(fe, kLn2Lo, atanh2));
 }
 
+// dlog of a uniform draw (normal, below 1): the same operations without the
+// tests for other arguments; the exponent becomes a float by its bits.
+__device__ __forceinline__ float dlog_unit(float x) {
+    const uint32_t u = __float_as_uint(x);
+    float m = __uint_as_float((u & 0x007fffffu) | 0x3f800000u);
+    const bool up = m > 1.41421356f;
+    m = up ? m * 0.5f : m;
+    const float fe = __uint_as_float(0x4b400000u + (u >> 23) - (up ? 126u : 127u)) - 12582912.0f;
+    const float s = (m - 1.0f) / (m + 1.0f);
+    const float s2 = s * s;
+    float p = 0.111111111f;
+    p = fmaf(p, s2, 0.142857143f);
+    p = fmaf(p, s2, 0.2f);
+    p = fmaf(p, s2, 0.333333333f);
+    const float t = s * s2;
+    const float atanh2 = fmaf(t * p, 2.0f, s * 2.0f);
+    return fmaf(fe, kLn2Hi, fmaf(fe, kLn2Lo, atanh2));
+}
+
 __device__ __forceinline__ float dexp(float x) {
     if (x != x) return x;
     if (x > 88.7f) return INFINITY;
@@ -149,9 +168,12 @@ struct Rng {
         uint32_t rot = (uint32_t)(old >> 59);
         return __funnelshift_r(xs, xs, rot);
     }
-    // (2k+1) 2^-24 on the open interval (0,1)
+    // (2k+1) 2^-24 on the open interval (0,1), k the upper 23 bits: k as the
+    // mantissa of 2^23 + k, then one exact fused step (an integer conversion has
+    // an eighth of the rate)
     __device__ __forceinline__ float uniform() {
-        return (float)(((next() >> 9) << 1) | 1u) * 5.96046448e-08f;
+        const float k = __uint_as_float(0x4b000000u | (next() >> 9)) - 8388608.0f;
+        return fmaf(k, 1.1920929e-07f, 5.96046448e-08f);
     }
 };
 
@@ -320,6 +342,26 @@ struct LocalStack {
     __device__ __forceinline__ bool full(int l) const { return l + 1 >= kMaxDepth - 1; }
 };
 
+// SlotStack: no arrays at all.  The child slots taken (T.slots) are the stack; a
+// pop descends from the root again for the node id as well as the interval.
+// For the rare rays that a kernel without a local frame sends through the octree.
+struct SlotStack {
+    const DevScene &S;
+    __device__ __forceinline__ void push(Trav &T, int l, uint32_t) const {
+        T.tns = (T.tns & ~(15ull << (4 * l))) | ((uint64_t)T.tn << (4 * l));
+    }
+    __device__ __forceinline__ bool pop(Trav &T, int l) const {
+        uint32_t node = 0;
+#pragma unroll 1
+        for (int k = 0; k < l; ++k) node = child_entry(S, node, ((uint32_t)(T.slots >> (3 * k)) & 7u) ^ T.a);
+        T.node = node;
+        T.tn = (uint32_t)(T.tns >> (4 * l)) & 15u;
+        return false;
+    }
+    __device__ __forceinline__ bool has_iv() const { return false; }
+    __device__ __forceinline__ bool full(int l) const { return l + 1 >= kMaxDepth - 1; }
+};
+
 template <class ST>
 __device__ __forceinline__ uint32_t trav_next_s(Trav &T, const DevScene &S, const ST &stk, uint32_t &leaf,
                                                 float &tra, float &trb, Count &cnt, uint32_t budget) {
@@ -384,6 +426,7 @@ __device__ __forceinline__ uint32_t trav_next_s(Trav &T, const DevScene &S, cons
             T.l = l;
             if (stk.pop(T, l)) continue;
             float t0[3] = {T.t0r[0], T.t0r[1], T.t0r[2]}, t1[3] = {T.t1r[0], T.t1r[1], T.t1r[2]};
+#pragma unroll 1
             for (int k = 0; k < l; ++k) {
                 const uint32_t s = (uint32_t)(T.slots >> (3 * k)) & 7u;
                 const float mx = 0.5f * (t0[0] + t1[0]), my = 0.5f * (t0[1] + t1[1]), mz = 0.5f * (t0[2] + t1[2]);
@@ -681,6 +724,7 @@ __device__ __noinline__ GridAxis grid_axis(float *col, uint32_t k, float ro, flo
     GridAxis g;
     g.cell = 0;
     g.h = hi;
+#pragma unroll 1
     for (int j = (int)levels - 1; j >= 0; --j) {
         const float mid = 0.5f * (lo + hi);
         const bool up = (uint32_t)j >= t ? ((cell >> j) & 1u) != 0u : mid < te;
@@ -815,7 +859,144 @@ __device__ __forceinline__ uint32_t grid_init(GridTrav &G, const DevScene &S, fl
     return 1u;
 }
 
-__device__ __forceinline__ uint32_t grid_leaf(const GridTrav &G, uint32_t idx, uint32_t w, float &tra, float &trb) {
+// OctreeNextNode's choice (src/KernelOctree.cpp:62-71) as the axis the ray
+// leaves its cell through: x, y or (neither) z, and the plane.
+struct GridExit {
+    bool x, y;
+    float t;
+    __device__ __forceinline__ uint32_t bit() const { return x ? 1u : (y ? 2u : 4u); }
+    __device__ __forceinline__ int axis() const { return x ? 0 : (y ? 1 : 2); }
+};
+__device__ __forceinline__ GridExit grid_exit(const GridTrav &G) {
+    GridExit e;
+    const bool xy = G.x[0] < G.x[1];
+    e.x = xy && G.x[0] < G.x[2];
+    e.y = !xy && G.x[1] < G.x[2];
+    e.t = e.x ? G.x[0] : (e.y ? G.x[1] : G.x[2]);
+    return e;
+}
+// Whether that exit leaves the 4^3 block.
+__device__ __forceinline__ bool grid_leaves_block(const GridTrav &G, const GridExit &e) {
+    const uint32_t nine = 9u * e.bit();
+    return (G.loc & kGridEmpty) || (G.loc & nine) == nine;
+}
+__device__ __forceinline__ void grid_set(GridTrav &G, const GridExit &e, float x, float h) {
+    G.x[0] = e.x ? x : G.x[0];
+    G.h[0] = e.x ? h : G.h[0];
+    G.x[1] = e.y ? x : G.x[1];
+    G.h[1] = e.y ? h : G.h[1];
+    const bool z = !(e.x || e.y);
+    G.x[2] = z ? x : G.x[2];
+    G.h[2] = z ? h : G.h[2];
+}
+
+// A step inside the block (grid_plain): to the upper cell of the same 2^3 block,
+// or to the next 2^3 block.  Returns true on a leaf.
+__device__ __forceinline__ bool grid_plain(const GridTrav &G, const GridExit &e) {
+    const uint32_t b = e.bit();
+    // not out of the block, and no tie where a 2^3 block is entered
+    return !grid_leaves_block(G, e) && ((G.loc & b) == 0u || G.tc < e.t);
+}
+template <int STRIDE>
+__device__ __forceinline__ bool grid_fine(GridTrav &G, const float *col, const GridExit &e, Count &cnt) {
+    const uint32_t b = e.bit();
+    const bool half = (G.loc & b) != 0u;  // a 2^3 block is entered
+    G.tc = e.t;
+    float nh = e.x ? G.h[0] : (e.y ? G.h[1] : G.h[2]);
+    if (half) nh = col[e.axis() * STRIDE];
+    const float nx = half ? 0.5f * (e.t + nh) : nh;
+    G.loc ^= half ? 9u * b : b;
+    grid_set(G, e, nx, nh);
+    uint32_t idx;
+    const uint32_t w = grid_cell_word(G, idx);
+    const uint32_t occ = (w >> (idx & 31u)) & 1u;
+    cnt.node_visits += (half ? (G.base >> (24u + (idx >> 3))) & 1u : 0u) + occ;
+    return occ != 0u;
+}
+
+// Any other step: into the next block, or into the next 2^3 block at a tie.  True
+// on a leaf; done past the root box (or when the segment's ties run out).
+template <int STRIDE>
+__device__ __forceinline__ bool grid_other(GridTrav &G, const DevScene &S, float *col, const float ro[3],
+                                           const float rd[3], const GridExit &e, Count &cnt, bool &done) {
+    const uint32_t lb = S.glevels - 2u, nbm = (1u << lb) - 1u, b = e.bit();
+    const int k = e.axis();
+    const bool tie = !(G.tc < e.t), out = grid_leaves_block(G, e);
+    float hi;
+    int tz = -1;  // levels 1 (the 2^3 block) .. 2 + tz are entered
+    if (out) {
+        const uint32_t s = (uint32_t)k * lb, f = (G.c >> s) & nbm;
+        done = f == nbm;
+        if (done) return false;
+        G.c += 1u << s;
+        tz = __ffs((int)(f + 1u)) - 1;
+        hi = col[(3 * (tz + 1) + k) * STRIDE];
+#pragma unroll 1
+        for (int j = tz;; --j) {
+            col[(3 * j + k) * STRIDE] = hi;
+            if (j == 0) break;
+            hi = 0.5f * (e.t + hi);
+        }
+        col[(3 * ((int)S.glevels - 1) + k) * STRIDE] = e.t;
+        G.loc &= ~(9u * b);
+    } else {
+        hi = col[k * STRIDE];
+        const float nx = 0.5f * (e.t + hi);
+        G.loc ^= 9u * b;
+        grid_set(G, e, nx, hi);
+    }
+    G.tc = e.t;
+    done = tie && !grid_resync<STRIDE>(G, S, col, ro, rd, b, 2u + (uint32_t)tz, e.t);
+    if (done) {
+        ++cnt.gave_up;
+        return false;
+    }
+    if (out) {
+        const uint4 g = __ldg(&S.gblock[G.c ^ G.am]);
+        G.mlo = g.x;
+        G.mhi = g.y;
+        G.base = g.z;
+        cnt.node_visits += (uint32_t)max(0, 2 + tz - (int)g.w);
+        const bool was_empty = (G.loc & kGridEmpty) != 0u;
+        if (!(g.z >> 24)) {
+            G.loc |= kGridEmpty;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) G.x[q] = col[q * STRIDE];
+            return false;
+        }
+        if (was_empty) {
+            // the cell that holds the crossing, on every axis
+            G.loc &= ~kGridEmpty;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                float l = col[(3 * ((int)S.glevels - 1) + q) * STRIDE], h = col[q * STRIDE];
+                float mid = 0.5f * (l + h);
+                bool up = mid < e.t;
+                l = up ? mid : l;
+                h = up ? h : mid;
+                G.loc = (G.loc & ~(9u << q)) | (up ? 8u << q : 0u);
+                G.h[q] = h;
+                mid = 0.5f * (l + h);
+                up = mid < e.t;
+                G.x[q] = up ? h : mid;
+                G.loc |= up ? 1u << q : 0u;
+            }
+        } else {
+            const float nh = 0.5f * (e.t + hi);
+            grid_set(G, e, 0.5f * (e.t + nh), nh);
+        }
+    }
+    uint32_t idx;
+    const uint32_t w = grid_cell_word(G, idx);
+    const uint32_t occ = (w >> (idx & 31u)) & 1u;
+    cnt.node_visits += ((G.base >> (24u + (idx >> 3))) & 1u) + occ;
+    return occ != 0u;
+}
+
+// The leaf in the current cell: its slot and interval.
+__device__ __forceinline__ uint32_t grid_leaf(const GridTrav &G, float &tra, float &trb) {
+    uint32_t idx;
+    const uint32_t w = grid_cell_word(G, idx);
     tra = G.tc;
     trb = std_min(std_min(G.x[0], G.x[1]), G.x[2]);
     return (G.base & 0xffffffu) + ((idx & 32u) ? __popc(G.mlo) : 0) + __popc(w & ((1u << (idx & 31u)) - 1u));
@@ -827,107 +1008,21 @@ template <int STRIDE>
 __device__ __forceinline__ uint32_t grid_next(GridTrav &G, const DevScene &S, float *col, const float ro[3],
                                               const float rd[3], uint32_t &leaf, float &tra, float &trb, Count &cnt,
                                               uint32_t budget) {
-    uint32_t idx;
-    if (G.loc & kGridCheck) {
-        G.loc &= ~kGridCheck;
-        const uint32_t w = grid_cell_word(G, idx);
-        leaf = grid_leaf(G, idx, w, tra, trb);
-        return kTravLeaf;
-    }
-    for (uint32_t it = 0; it != budget; ++it) {
-        // OctreeNextNode's choice (src/KernelOctree.cpp:62-71) as the exit axis
-        const bool xy = G.x[0] < G.x[1];
-        const bool bx = xy && G.x[0] < G.x[2];
-        const bool by = !xy && G.x[1] < G.x[2];
-        const float Xa = bx ? G.x[0] : (by ? G.x[1] : G.x[2]);
-        const uint32_t b = bx ? 1u : (by ? 2u : 4u);
-        const int k = bx ? 0 : (by ? 1 : 2);
-        const bool tie = !(G.tc < Xa);
-        G.tc = Xa;
-        bool half = true;  // a 2^3 block is entered
-        if (!(G.loc & kGridEmpty) && (G.loc & (9u * b)) != 9u * b) {
-            float nx, nh;
-            if (!(G.loc & b)) {  // the upper cell of the same 2^3 block
-                half = false;
-                nh = bx ? G.h[0] : (by ? G.h[1] : G.h[2]);
-                nx = nh;
-                G.loc |= b;
-            } else {  // the next 2^3 block of the same 4^3 block
-                nh = col[k * STRIDE];
-                nx = 0.5f * (Xa + nh);
-                G.loc ^= 9u * b;
-            }
-            if (bx) { G.x[0] = nx; G.h[0] = nh; }
-            else if (by) { G.x[1] = nx; G.h[1] = nh; }
-            else { G.x[2] = nx; G.h[2] = nh; }
-            if (half && tie && !grid_resync<STRIDE>(G, S, col, ro, rd, b, 1u, Xa)) {
-                ++cnt.gave_up;
-                return kTravDone;
-            }
-        } else {  // the next 4^3 block
-            const uint32_t lb = S.glevels - 2u, nbm = (1u << lb) - 1u;
-            const uint32_t s = (uint32_t)k * lb, f = (G.c >> s) & nbm;
-            if (f == nbm) return kTravDone;
-            G.c += 1u << s;
-            const int tz = __ffs((int)(f + 1u)) - 1;  // levels 2 .. 2 + tz are entered
-            float hi = col[(3 * (tz + 1) + k) * STRIDE];
-#pragma unroll 1
-            for (int j = tz;; --j) {
-                col[(3 * j + k) * STRIDE] = hi;
-                if (j == 0) break;
-                hi = 0.5f * (Xa + hi);
-            }
-            col[(3 * ((int)S.glevels - 1) + k) * STRIDE] = Xa;
-            const bool was_empty = (G.loc & kGridEmpty) != 0u;
-            G.loc &= ~(9u * b);
-            if (tie && !grid_resync<STRIDE>(G, S, col, ro, rd, b, 2u + (uint32_t)tz, Xa)) {
-                ++cnt.gave_up;
-                return kTravDone;
-            }
-            const uint4 e = __ldg(&S.gblock[G.c ^ G.am]);
-            G.mlo = e.x;
-            G.mhi = e.y;
-            G.base = e.z;
-            cnt.node_visits += (uint32_t)max(0, 2 + tz - (int)e.w);
-            if (!(e.z >> 24)) {
-                G.loc |= kGridEmpty;
-#pragma unroll
-                for (int q = 0; q < 3; ++q) G.x[q] = col[q * STRIDE];
-                continue;
-            }
-            const float nh = 0.5f * (Xa + hi), nx = 0.5f * (Xa + nh);
-            if (was_empty) {
-                // the cell of the other axes that holds the crossing
-                G.loc &= ~kGridEmpty;
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    float l = col[(3 * ((int)S.glevels - 1) + q) * STRIDE], h = col[q * STRIDE];
-                    float mid = 0.5f * (l + h);
-                    bool up = mid < Xa;
-                    l = up ? mid : l;
-                    h = up ? h : mid;
-                    G.loc = (G.loc & ~(9u << q)) | (up ? 8u << q : 0u);
-                    G.h[q] = h;
-                    mid = 0.5f * (l + h);
-                    up = mid < Xa;
-                    G.x[q] = up ? h : mid;
-                    G.loc |= up ? 1u << q : 0u;
-                }
-            } else {
-                if (bx) { G.x[0] = nx; G.h[0] = nh; }
-                else if (by) { G.x[1] = nx; G.h[1] = nh; }
-                else { G.x[2] = nx; G.h[2] = nh; }
-            }
+    bool found = (G.loc & kGridCheck) != 0u;
+    G.loc &= ~kGridCheck;
+    for (uint32_t it = 0; !found; ++it) {
+        if (it == budget) return kTravMore;
+        const GridExit e = grid_exit(G);
+        if (grid_plain(G, e)) {
+            found = grid_fine<STRIDE>(G, col, e, cnt);
+            continue;
         }
-        const uint32_t w = grid_cell_word(G, idx);
-        const uint32_t occ = (w >> (idx & 31u)) & 1u;
-        cnt.node_visits += (half ? (G.base >> (24u + (idx >> 3))) & 1u : 0u) + occ;
-        if (occ) {
-            leaf = grid_leaf(G, idx, w, tra, trb);
-            return kTravLeaf;
-        }
+        bool done;
+        found = grid_other<STRIDE>(G, S, col, ro, rd, e, cnt, done);
+        if (done) return kTravDone;
     }
-    return kTravMore;
+    leaf = grid_leaf(G, tra, trb);
+    return kTravLeaf;
 }
 
 // ---- free flights that need no logarithm ---------------------------------------
@@ -970,6 +1065,58 @@ __device__ __forceinline__ float sample_voxel_space(const float p[3], const floa
     const float v0 = lerp_ref(u0, u1, nl[1]);
     const float v1 = lerp_ref(u2, u3, nl[1]);
     return lerp_ref(v0, v1, nl[2]);
+}
+
+static __device__ __noinline__ float sample_voxel_far(float px, float py, float pz, const float *__restrict__ v, float4 ce) {
+    const float p[3] = {px, py, pz};
+    return sample_voxel_space(p, v, ce);
+}
+
+// The same lookup where every leaf has one half extent e, inv = 1 / e rounded
+// to nearest (DevScene::ginv; 0: leaves differ).  a / e as a correctly rounded
+// quotient from the correctly rounded reciprocal (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: one
+// product and one fused correction); floor, ceiling and the indices by adding
+// 1.5 * 2^23 and 2^23 instead of conversions, which have an eighth of the rate.
+// Positions this far outside the brick (2^20 cells) take the lookup above.
+__device__ __forceinline__ float sample_voxel_inv(const float p[3], const float *__restrict__ v, const float4 ce,
+                                                  float inv) {
+    const float cc[3] = {ce.x, ce.y, ce.z};
+    uint32_t ia[3], ib[3];
+    float nl[3];
+    bool far = inv == 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float a = (-0.5f * ((cc[k] - ce.w) - p[k])) * 7.0f;
+        const float q = a * inv;
+        const float ni = fmaf(fmaf(-ce.w, q, a), inv, q);
+        far = far || !(fabsf(ni) < 1048576.0f);
+        const float r = (ni + 12582912.0f) - 12582912.0f;  // nearest integer
+        const float fl = r > ni ? r - 1.0f : r;
+        const float nf = sse_max(fl, 0.0f);
+        nl[k] = ni - nf;
+        const float nc = fl < ni ? fl + 1.0f : fl;
+        ia[k] = __float_as_uint(sse_min(nf, 7.0f) + 8388608.0f) & 7u;
+        ib[k] = __float_as_uint(sse_max(sse_min(nc, 7.0f), 0.0f) + 8388608.0f) & 7u;
+    }
+    if (far) return sample_voxel_far(p[0], p[1], p[2], v, ce);
+    const uint32_t za = ia[2] * 64u, zb = ib[2] * 64u, ya = ia[1] * 8u, yb = ib[1] * 8u;
+    const float u0 = lerp_ref(__ldg(v + za + ya + ia[0]), __ldg(v + za + ya + ib[0]), nl[0]);
+    const float u1 = lerp_ref(__ldg(v + za + yb + ia[0]), __ldg(v + za + yb + ib[0]), nl[0]);
+    const float u2 = lerp_ref(__ldg(v + zb + ya + ia[0]), __ldg(v + zb + ya + ib[0]), nl[0]);
+    const float u3 = lerp_ref(__ldg(v + zb + yb + ia[0]), __ldg(v + zb + yb + ib[0]), nl[0]);
+    const float v0 = lerp_ref(u0, u1, nl[1]);
+    const float v1 = lerp_ref(u2, u3, nl[1]);
+    return lerp_ref(v0, v1, nl[2]);
+}
+
+// Whether rho / smax, rounded, lies below q: decided by the product when it is
+// clear of the rounding (2^-21 relative; each side is within 2^-23), else by the division.
+__device__ __forceinline__ bool ratio_below(float rho, float smax, float q) {
+    const float t = q * smax, slack = t * 4.76837158e-07f;
+    if (rho < t - slack) return true;
+    if (rho > t + slack) return false;
+    return rho / smax < q;
 }
 
 // Corner offsets (within the brick) and trilinear weights of the lookup above:
@@ -1036,6 +1183,7 @@ __device__ __forceinline__ float mie_scan_cdf(const MieSmem &M, float ub, uint32
 __device__ __forceinline__ float mie_theta_ref(const MieSmem &M, float u1) {
     const float ub = (float)M.n * u1;
     uint32_t lo = 0, hi = M.n - 1;
+#pragma unroll 1
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         float t;
@@ -1049,14 +1197,23 @@ __device__ __forceinline__ float mie_theta_ref(const MieSmem &M, float u1) {
 }
 
 // SamplingBasis, src/KernelSampler.cpp:145-154, and the direction composition
-__device__ __forceinline__ void compose_dir(const float iv[3], float st, float ct, float ph, float out[3]) {
+// (one copy per kernel: called for the phase and the sun sample of an event)
+static __device__ __noinline__ float3 compose_call(float ix, float iy, float iz, float st, float ct, float ph) {
+    const float iv[3] = {ix, iy, iz};
     const float len = sqrtf(iv[0] * iv[0] + 0.0f * 0.0f + iv[2] * iv[2]);
     const float b1[3] = {(0.0f - iv[2]) / len, 0.0f / len, iv[0] / len};
     const float b2[3] = {iv[1] * b1[2] - iv[2] * b1[1], iv[2] * b1[0] - iv[0] * b1[2], iv[0] * b1[1] - iv[1] * b1[0]};
-    float sph, cph;
+    float sph, cph, out[3];
     dsincos(ph, &sph, &cph);
 #pragma unroll
     for (int k = 0; k < 3; ++k) out[k] = ((b1[k] * st) * cph + (b2[k] * st) * sph) + iv[k] * ct;
+    return make_float3(out[0], out[1], out[2]);
+}
+__device__ __forceinline__ void compose_dir(const float iv[3], float st, float ct, float ph, float out[3]) {
+    const float3 d = compose_call(iv[0], iv[1], iv[2], st, ct, ph);
+    out[0] = d.x;
+    out[1] = d.y;
+    out[2] = d.z;
 }
 
 // ---- exact-mode sampler (DR_PHASE_MIE_EXACT) ------------------------------------
@@ -1110,20 +1267,25 @@ __device__ __forceinline__ void mie_exact_dir(const float4 *ex, uint32_t n, floa
     st = sse_max(S * cx + C * sx, 0.0f);
 }
 
+static __device__ __noinline__ float2 mie_exact_call(const float4 *ex, uint32_t n, float u1) {
+    float ct, st;
+    mie_exact_dir(ex, n, u1, ct, st);
+    return make_float2(ct, st);
+}
+
 __device__ __forceinline__ void mie_sample(const MieSmem &M, const float iv[3], float u1, float u2, float out[3]) {
+    float ct, st;
     if (M.ex) {
-        float ct, st;
-        mie_exact_dir(M.ex, M.n, u1, ct, st);
-        compose_dir(iv, st, ct, (2.0f * kPi) * u2, out);
-        return;
+        const float2 d = mie_exact_call(M.ex, M.n, u1);
+        ct = d.x;
+        st = d.y;
+    } else {
+        float s_, c_;
+        dsincos(mie_theta_ref(M, u1) * kPi, &s_, &c_);
+        ct = -c_;
+        st = sqrtf(sse_max(1.0f - ct * ct, 0.0f));
     }
-    const float th = mie_theta_ref(M, u1) * kPi;
-    const float ph = (2.0f * kPi) * u2;
-    float s_, c_;
-    dsincos(th, &s_, &c_);
-    const float ct = -c_;
-    const float st = sqrtf(sse_max(1.0f - ct * ct, 0.0f));
-    compose_dir(iv, st, ct, ph, out);
+    compose_dir(iv, st, ct, (2.0f * kPi) * u2, out);
 }
 
 // ---- phase function: HGPhase, src/KernelSampler.cpp:164-204 (DR_PHASE_HG) ----
@@ -1191,18 +1353,21 @@ __device__ __forceinline__ float3 sky_eval(const DevParams &P, const float rd[3]
     const float raym = gacs * gacs;
     const float zenh = sqrtf(thcs);
     const float izen = 1.0f / (thcs + 0.01f);  // c1 / (thcs + 0.01) as c1 * izen: one division for three channels
-    float out[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
+    float3 out = make_float3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {  // rolled: one copy of the exponentials and powers
         const float *c = P.sky_cfg[i];
         const float expm = dexp(c[4] * gmma);
         const float miem = (1.0f + raym) / dpow15((1.0f + c[8] * c[8]) - (2.0f * c[8]) * gacs);
         float ca = (1.0f + c[0] * dexp(c[1] * izen)) *
                    ((((c[2] + c[3] * expm) + c[5] * raym) + c[6] * miem) + c[7] * zenh);
         ca = ca * P.sky_rad[i];
-        out[i] = 1e-3f * dpow(ca, 2.2f);
+        const float v = 1e-3f * dpow(ca, 2.2f);
+        if (i == 0) out.x = v;
+        else if (i == 1) out.y = v;
+        else out.z = v;
     }
-    return make_float3(out[0], out[1], out[2]);
+    return out;
 }
 
 // atan2 of smmath.inl (src/smmath.inl:430-445): polynomial in min/max ratio,
@@ -1416,10 +1581,18 @@ struct NoVisit {
 
 // SDF: the scene may hold surface leaves (src/kernel.cpp:241-305); without it
 // every leaf is a fog leaf and the surface tests are not compiled in.
+template <class Visit, bool SDF, class ST>
+__device__ __forceinline__ uint32_t track_on(const DevScene &S, SegMedium med, const float ro[3], const float rd[3],
+                                             Rng &g, float depth, float &td_out, const ST &stk, Count &cnt,
+                                             const Visit &visit);
+
 template <class Visit, bool SDF = true>
 __device__ __forceinline__ uint32_t track_v(const DevScene &S, SegMedium med, const float ro[3], const float rd[3],
                                             Rng &g, float depth, float &td_out, uint32_t *nstack, Count &cnt,
-                                            const Visit &visit);
+                                            const Visit &visit) {
+    float tstack[kMaxDepth][6];
+    return track_on<Visit, SDF>(S, med, ro, rd, g, depth, td_out, LocalStack{nstack, tstack}, cnt, visit);
+}
 
 template <bool SDF = true>
 __device__ __forceinline__ uint32_t track(const DevScene &S, const DevParams &P, const float ro[3], const float rd[3],
@@ -1428,10 +1601,10 @@ __device__ __forceinline__ uint32_t track(const DevScene &S, const DevParams &P,
     return track_v<NoVisit, SDF>(S, seg_medium(P), ro, rd, g, depth, td_out, nstack, cnt, nv);
 }
 
-template <class Visit, bool SDF>
-__device__ __forceinline__ uint32_t track_v(const DevScene &S, SegMedium med, const float ro[3], const float rd[3],
-                                            Rng &g, float depth, float &td_out, uint32_t *nstack, Count &cnt,
-                                            const Visit &visit) {
+template <class Visit, bool SDF, class ST>
+__device__ __forceinline__ uint32_t track_on(const DevScene &S, SegMedium med, const float ro[3], const float rd[3],
+                                             Rng &g, float depth, float &td_out, const ST &stk, Count &cnt,
+                                             const Visit &visit) {
     const float sigma_e = med.sigma_e;
     Trav T;
     trav_init(T, S, ro, rd, cnt);
@@ -1440,8 +1613,7 @@ __device__ __forceinline__ uint32_t track_v(const DevScene &S, SegMedium med, co
     uint32_t leaf;
     float tra, trb;
     uint32_t budget = med.budget;
-    float tstack[kMaxDepth][6];
-    while (trav_next_k(T, S, nstack, leaf, tra, trb, cnt, 0xffffffffu, tstack) == kTravLeaf) {
+    while (trav_next_s(T, S, stk, leaf, tra, trb, cnt, 0xffffffffu) == kTravLeaf) {
         if (!(td < depth)) break;
         const float4 ce = __ldg(&S.leaf[2 * leaf]);
         const float4 meta = __ldg(&S.leaf[2 * leaf + 1]);

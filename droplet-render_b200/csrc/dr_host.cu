@@ -131,6 +131,11 @@ static void build_block_grid(const std::vector<TreeNode> &leaves, const std::vec
         out.gmaj[k] = meta.x;
     }
     out.glevels = levels;
+    // one half extent for all leaves, in a range whose quotients neither over- nor underflow
+    const float e = out.gleaf[0].w;
+    bool same = e > 1e-12f && e < 1e12f;
+    for (size_t k = 0; k < out.gleaf.size(); k += 2) same = same && out.gleaf[k].w == e;
+    out.ginv = same ? 1.0f / e : 0.0f;
 }
 
 int prepare_scene(const dr_scene_desc *s, HostScene &out) {
@@ -300,6 +305,7 @@ int upload_scene(const HostScene &h, SceneBufs &b, bool use_grid, cudaStream_t s
     S.gleaf = h.glevels ? b.gleaf.p : nullptr;
     S.gmaj = h.glevels ? b.gmaj.p : nullptr;
     S.glevels = h.glevels;
+    S.ginv = h.ginv;
     S.occ_nodes = nullptr;
     S.occ_tris = nullptr;
     S.occ_n_nodes = 0;

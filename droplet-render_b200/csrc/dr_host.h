@@ -69,6 +69,7 @@ struct HostScene {
     std::vector<float4> gleaf;     // leaf records by slot (DevScene::gleaf)
     std::vector<float> gmaj;       // majorants by slot (DevScene::gmaj)
     uint32_t glevels = 0;
+    float ginv = 0.0f;             // DevScene::ginv
     uint32_t n_nodes = 0, n_leaves = 0;
     float root_ce[4] = {0, 0, 0, 0};
     const float *bricks = nullptr;  // the caller's brick pool (n_leaves * 512 floats)

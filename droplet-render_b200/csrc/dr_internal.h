@@ -58,6 +58,7 @@ struct DevScene {
     const float4 *gleaf;
     const float *gmaj;  // majorant of each slot (gleaf[2 * slot + 1].x)
     uint32_t glevels;
+    float ginv;         // 1 / half extent when all leaves share it, else 0
     // Occluder BVH (null: no occluders).  Node i = occ_nodes[4i .. 4i+3]: left
     // box (min xyz, max x), (max yz, right min xy), (right min z, right max
     // xyz), then (left ref, right ref, left count, right count) as uint32

@@ -1527,8 +1527,9 @@ cudaError_t launch_render_tile(const DevScene &S, const DevParams &P, const Tile
 }
 
 cudaError_t launch_shadow_tile(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out, DevCounters *C,
-                               cudaStream_t st) {
+                               int device, cudaStream_t st) {
     if (A.n_paths == 0) return cudaSuccess;
+    if (S.glevels) return launch_shadow_paths(S, P, A, out, C, (S.occ_nodes && P.embree) || S.sdf_bricks, device, st);
     const uint64_t blocks = (A.n_paths + kRenderBlock - 1) / kRenderBlock;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
     shadow_tile_kernel<<<(unsigned)blocks, kRenderBlock, 0, st>>>(S, P, A, out, C);
@@ -1733,6 +1734,7 @@ cudaError_t launch_probe_sampler(const DevParams &P, const void *mie_pack, uint3
 cudaError_t launch_probe_transmittance(const DevScene &S, const DevParams &P, const float *ro, const float *rd,
                                        uint32_t n_rays, uint64_t nsamp, uint64_t seed, unsigned long long *escapes,
                                        cudaStream_t st) {
+    if (S.glevels) return launch_transmittance(S, P, ro, rd, n_rays, nsamp, seed, escapes, st);
     const uint64_t threads = ((nsamp + 63) / 64) * n_rays;
     const uint64_t blocks = (threads + 127) / 128;
     if (blocks == 0) return cudaSuccess;

@@ -11,7 +11,7 @@ constexpr int kPersistentBlock = 128;
 cudaError_t launch_render_tile(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                                float4 *sun_out, float4 *sky_out, DevCounters *C, cudaStream_t st);
 cudaError_t launch_shadow_tile(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out, DevCounters *C,
-                               cudaStream_t st);
+                               int device, cudaStream_t st);
 // Camera leaf list storage for one persistent launch: head[2 * cols * rows],
 // pool[cap] and its fill counter (head null: no lists).
 struct CamLists {
@@ -38,6 +38,12 @@ cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &
 cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
                                const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool feat, uint32_t glevels,
                                int device, cudaStream_t st);
+// The shadow pass and transmittance estimates on a scene with a block grid.
+cudaError_t launch_shadow_paths(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out,
+                                DevCounters *C, bool feat, int device, cudaStream_t st);
+cudaError_t launch_transmittance(const DevScene &S, const DevParams &P, const float *ro, const float *rd,
+                                 uint32_t n_rays, uint64_t nsamp, uint64_t seed, unsigned long long *escapes,
+                                 cudaStream_t st);
 uint32_t path_list_blocks(uint32_t cols, uint32_t rows);
 // Feature bits a frame needs (0: the plain kernels).
 uint32_t frame_features(const DevScene &S, const DevParams &P);

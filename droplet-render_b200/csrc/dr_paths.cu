@@ -15,8 +15,8 @@
 // rest is not.  One kernel for all three (render_persistent_kernel, which
 // serves the octrees without a block grid) was bound by instruction issue at 8
 // of 32 lanes per instruction: 38.5 ms for that frame at 64 samples, 51.9 ms for a
-// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 18.9 and 23.4 ms:
-// lists 0.26, camera 2.4, scatter 16 ms of the first, at 13 lanes per instruction.
+// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 18.3 and 19.2 ms:
+// lists 0.26, camera 2.4, scatter 15.5 ms of the first, at 13 lanes per instruction.
 //
 // Per path, the operations and random draws are those of path_sample(): a
 // path's result does not depend on the kernel that computed it.
@@ -37,11 +37,10 @@ constexpr int kListBlock = 128, kListTx = 16, kListTy = 8;  // camera lists: a b
 // contiguous range of the pool is taken and filled by a second traversal; a
 // pixel whose range does not fit gets x = ~0 and its samples traverse.
 // Rays with a zero direction component take the octree (node ids become slots).
-__device__ __noinline__ uint4 octree_list(const DevScene S, float ox, float oy, float oz, float dx, float dy, float dz,
+__device__ __noinline__ uint4 octree_list(const DevScene &S, float ox, float oy, float oz, float dx, float dy, float dz,
                                           uint4 *pool, uint32_t cap, unsigned int *used) {
     const float ro[3] = {ox, oy, oz}, rd[3] = {dx, dy, dz};
-    uint32_t nstack[kMaxDepth];
-    float tstack[kMaxDepth][6];
+    const SlotStack stk{S};
     Trav T;
     Count c;
     c.zero();
@@ -49,7 +48,7 @@ __device__ __noinline__ uint4 octree_list(const DevScene S, float ox, float oy, 
     uint4 h = make_uint4(0u, 0u, c.node_visits, 0u);
     uint32_t leaf, n = 0;
     float tra, trb;
-    while (trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack) == kTravLeaf) ++n;
+    while (trav_next_s(T, S, stk, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
     const unsigned int off = n ? atomicAdd(used, n) : 0u;
     if (n && (off > cap || n > cap - off)) {
         h.x = kNone;
@@ -60,12 +59,12 @@ __device__ __noinline__ uint4 octree_list(const DevScene S, float ox, float oy, 
     trav_init(T, S, ro, rd, c);
     c.zero();
     for (uint32_t k = 0; k < n; ++k) {
-        trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack);
+        trav_next_s(T, S, stk, leaf, tra, trb, c, kNone);
         pool[off + k] = make_uint4(__float_as_uint(__ldg(&S.leaf[2 * leaf + 1]).w), __float_as_uint(tra),
                                    __float_as_uint(trb), c.node_visits);
         c.zero();
     }
-    trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack);  // kTravDone
+    trav_next_s(T, S, stk, leaf, tra, trb, c, kNone);  // kTravDone
     h.w = c.node_visits;
     return h;
 }
@@ -130,8 +129,10 @@ __device__ __forceinline__ void list_pixel(const DevScene &S, const DevParams &P
     }
 }
 
-__global__ void __launch_bounds__(kListBlock) path_lists_kernel(DevScene S, DevParams P, TileArgs A, PathWork W,
-                                                                DevCounters *C) {
+__global__ void __launch_bounds__(kListBlock) path_lists_kernel(const __grid_constant__ DevScene S,
+                                                                const __grid_constant__ DevParams P,
+                                                                const __grid_constant__ TileArgs A,
+                                                                const __grid_constant__ PathWork W, DevCounters *C) {
     extern __shared__ __align__(16) unsigned char smem[];
     float *const col = reinterpret_cast<float *>(smem) + threadIdx.x;
     const uint32_t bx = (A.cols + kListTx - 1) / kListTx, by = blockIdx.x / bx;
@@ -213,7 +214,7 @@ __device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e
         }
     }
     const float u = first ? v : g.uniform();
-    const float sr = (first ? 0.0f : v) - dlog(u) / denom;
+    const float sr = (first ? 0.0f : v) - dlog_unit(u) / denom;
     v = sr;
     const float sc = s0 + sr;
     td = lo + sc;
@@ -236,12 +237,12 @@ __device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e
             }
         }
         if (look) {
-            rho = sample_voxel_space(rc, S.bricks + (size_t)fog * kBrick, ce);
+            rho = sample_voxel_inv(rc, S.bricks + (size_t)fog * kBrick, ce, S.ginv);
             ++cnt.density_lookups;
         }
     }
     const float q = g.uniform();
-    return rm && (rho / meta.x < q) && (dist > 0.0f) ? kNull : kReal;
+    return rm && ratio_below(rho, meta.x, q) && (dist > 0.0f) ? kNull : kReal;
 }
 
 // Whether a leaf may be passed by leaves_at_once: not with a surface brick
@@ -266,10 +267,9 @@ struct SlowSeg {
 };
 // A segment with a zero direction component, traced through the octree.
 template <uint32_t FEAT>
-__device__ __noinline__ SlowSeg slow_segment(const DevScene S, SegMedium med, float ox, float oy, float oz, float dx,
+__device__ __noinline__ SlowSeg slow_segment(const DevScene &S, SegMedium med, float ox, float oy, float oz, float dx,
                                              float dy, float dz, float depth, uint64_t state, uint64_t inc) {
     const float ro[3] = {ox, oy, oz}, rd[3] = {dx, dy, dz};
-    uint32_t nstack[kMaxDepth];
     const NoVisit nv;
     Count c;
     c.zero();
@@ -277,7 +277,7 @@ __device__ __noinline__ SlowSeg slow_segment(const DevScene S, SegMedium med, fl
     g.state = state;
     g.inc = inc;
     SlowSeg o;
-    o.res = track_v<NoVisit, (FEAT & kFeatSdf) != 0>(S, med, ro, rd, g, depth, o.td, nstack, c, nv);
+    o.res = track_on<NoVisit, (FEAT & kFeatSdf) != 0>(S, med, ro, rd, g, depth, o.td, SlotStack{S}, c, nv);
     o.visits = c.node_visits;
     o.lookups = c.density_lookups;
     o.gave_up = c.gave_up;
@@ -395,7 +395,10 @@ __device__ __forceinline__ void active_sample(const TileArgs &A, const uint32_t 
 // (W.limit = capacity - warps * kTicket), so the buffer never overflows and the
 // tickets taken are exactly those done: the next round goes on from there.
 template <uint32_t FEAT, bool BATCH>
-__global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(DevScene S0, DevParams P0, TileArgs A0, PathWork W,
+__global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __grid_constant__ DevScene S0,
+                                                                     const __grid_constant__ DevParams P0,
+                                                                     const __grid_constant__ TileArgs A0,
+                                                                     const __grid_constant__ PathWork W,
                                                                      float4 *sun0, float4 *sky0, DevCounters *C,
                                                                      BatchArgs B) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -494,6 +497,198 @@ __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(DevScene S0
     warp_sum_counts(cnt, C, paths);
 }
 
+// ---- shadow pass ------------------------------------------------------------------
+// RenderKernel::Shadow (src/kernel.cpp:569-607, see shadow_sample): the segments
+// of a pixel's samples start at one point and stay within the sun's cone, so
+// 32 samples side by side walk the grid together like camera samples.  Resident
+// warps loop over the samples: a warp's counters cost six additions to the same
+// words whatever it did, and with a warp per 32 samples those were the bound.
+template <uint32_t FEAT>
+__global__ void __launch_bounds__(kListBlock, 8) shadow_paths_kernel(const __grid_constant__ DevScene S,
+                                                                     const __grid_constant__ DevParams P,
+                                                                     const __grid_constant__ TileArgs A, float4 *out,
+                                                                     DevCounters *C) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float *const col = reinterpret_cast<float *>(smem) + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    Count cnt;
+    cnt.zero();
+    uint32_t paths = 0;
+    for (uint64_t q = (uint64_t)blockIdx.x * kListBlock + threadIdx.x; q - lane < A.n_paths;
+         q += (uint64_t)gridDim.x * kListBlock) {
+        uint32_t pix = kNone;
+        bool active = false;
+        float ro[3] = {0.f, 0.f, 0.f}, rd[3] = {0.f, 0.f, 0.f};
+        Rng g;
+        g.state = g.inc = 0;
+        if (q < A.n_paths) {
+            uint32_t s;
+            if (q <= 0xffffffffull) {
+                pix = fastdiv((uint32_t)q, A.spp_div);
+                s = (uint32_t)q - pix * A.spp;
+            } else {
+                const uint64_t l = q / A.spp;
+                pix = (uint32_t)l;
+                s = (uint32_t)(q - l * A.spp);
+            }
+            const uint32_t iy = fastdiv(pix, A.cols_div), ix = pix - iy * A.cols;
+            if (camera_ray(P, A.x0 + ix, A.y0 + iy, ro, rd)) {
+                ++paths;
+                const uint64_t fp = (uint64_t)(A.y0 + iy) * P.w + (A.x0 + ix);
+                const float depth = P.depth ? __ldg(&P.depth[fp]) : 3.402823466e+38f;
+                active = depth < P.clip_end;
+                g = rng_seed(A.seed, fp, A.sample_base + s);
+                const float u3 = g.uniform(), u4 = g.uniform();
+                for (int k = 0; k < 3; ++k) ro[k] = ro[k] + rd[k] * depth;
+                sun_sample(P, u3, u4, rd);
+            } else {
+                pix = kNone;  // outside the frame: nothing is written, as in the reference
+            }
+        }
+        if (active) ++cnt.vertices;
+        const CamSeg o = camera_segments<FEAT, false>(S, seg_medium(P), active, ro, rd, g, 3.402823466e+38f,
+                                                      make_uint4(0u, 0u, 0u, 0u), nullptr, col, cnt);
+        const bool esc = !active || o.res == kTrackEscaped;
+        const bool occ = (FEAT & kFeatOcc) && active && esc && P.embree && occluded(S, ro, rd);
+        const bool lit = pix != kNone && P.scattevs > 0u && esc && !occ && sun_hit(P, rd);
+        const bool one = pix != kNone && (P.scattevs > 0u || !esc) && !occ;
+        // a pixel's samples each add sun(lrd) / colour = colour / colour or 0 / colour,
+        // and 1 / 0 or 0 / 0 in w: summed by their numbers, once per pixel
+        const uint32_t peers = __match_any_sync(kFull, pix);
+        const uint32_t nl = __popc(__ballot_sync(kFull, lit) & peers), nw = __popc(__ballot_sync(kFull, one) & peers);
+        if (pix != kNone && lane == (uint32_t)__ffs((int)peers) - 1u) {
+            const uint32_t n = __popc(peers);
+            float v[3];
+            for (int k = 0; k < 3; ++k) {
+                const float c = P.sun_color[k];
+                v[k] = (nl ? (float)nl * __fdiv_rn(c, c) : 0.0f) + (n - nl ? (float)(n - nl) * __fdiv_rn(0.0f, c) : 0.0f);
+            }
+            const float w = (nw ? __fdiv_rn(1.0f, 0.0f) : 0.0f) + (n - nw ? __fdiv_rn(0.0f, 0.0f) : 0.0f);
+            const uint32_t iy = fastdiv(pix, A.cols_div);
+            atomicAdd(&out[(size_t)iy * A.tw + (pix - iy * A.cols)], make_float4(v[0], v[1], v[2], w));
+        }
+    }
+    warp_sum_counts(cnt, C, paths);
+}
+
+// ---- transmittance -----------------------------------------------------------------
+// Fraction of delta-tracked samples of a ray that escape.  A warp takes a ray
+// and `chunk` of its samples: it walks the ray once, keeping the leaves in
+// shared memory, and its lanes take samples from the chunk and run along that
+// list; most leaves then cost a draw and a comparison.  A ray with more than
+// kRayLeaves leaves (deep grids) is traversed per sample.  Nothing is
+// allocated, so the allocation-free entry point runs it too.
+constexpr uint32_t kRayLeaves = 96;
+constexpr uint32_t kRayRefill = 8;  // idle lanes that take new samples together
+
+__host__ __device__ constexpr size_t ray_smem(uint32_t levels) {
+    return (size_t)grid_words(levels) * 4 * kListBlock + (size_t)(kListBlock / 32) * kRayLeaves * 16;
+}
+
+template <uint32_t FEAT>
+__global__ void __launch_bounds__(kListBlock, 8) transmittance_kernel(const __grid_constant__ DevScene S,
+                                                                      SegMedium med, const float *ro_in,
+                                                                      const float *rd_in, uint32_t n_rays,
+                                                                      uint64_t nsamp, uint32_t chunk, uint64_t seed,
+                                                                      unsigned long long *escapes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint4 *const list = reinterpret_cast<uint4 *>(smem) + (threadIdx.x >> 5) * kRayLeaves;
+    float *const col = reinterpret_cast<float *>(smem + (size_t)(kListBlock / 32) * kRayLeaves * 16) + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint64_t chunks = (nsamp + chunk - 1) / chunk;
+    const uint64_t item = (uint64_t)blockIdx.x * (kListBlock / 32) + (threadIdx.x >> 5);
+    if (item >= chunks * n_rays) return;
+    const uint32_t r = (uint32_t)(item / chunks);
+    const uint64_t s0 = (item - (uint64_t)r * chunks) * chunk;
+    const uint32_t n = (uint32_t)(nsamp - s0 < chunk ? nsamp - s0 : chunk);
+    float ro[3], rd[3];
+    for (int k = 0; k < 3; ++k) {
+        ro[k] = __ldg(&ro_in[3 * (size_t)r + k]);
+        rd[k] = __ldg(&rd_in[3 * (size_t)r + k]);
+    }
+    Count cnt;
+    cnt.zero();
+    // the ray's leaves (every lane walks the same ray)
+    GridTrav G;
+    const uint32_t mode = grid_init<kListBlock>(G, S, col, ro, rd, cnt);
+    uint32_t leaves = 0, leaf;
+    float tra, trb;
+    if (mode == 1u) {
+        while (leaves <= kRayLeaves &&
+               grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, cnt, kNone) == kTravLeaf) {
+            if (lane == 0 && leaves < kRayLeaves)
+                list[leaves] = make_uint4(leaf, __float_as_uint(tra), __float_as_uint(trb),
+                                          __float_as_uint(med.sigma_e * __ldg(&S.gmaj[leaf])));
+            ++leaves;
+        }
+    }
+    __syncwarp();
+    uint32_t esc = 0, next = 0;
+    if (mode == 2u || leaves > kRayLeaves) {
+        for (uint32_t i = lane; i - lane < n; i += 32) {
+            const Rng g = rng_seed(seed, r, s0 + i);
+            const CamSeg o = camera_segments<FEAT, false>(S, med, i < n, ro, rd, g, 3.402823466e+38f,
+                                                          make_uint4(0u, 0u, 0u, 0u), nullptr, col, cnt);
+            if (i < n && o.res == kTrackEscaped) ++esc;
+        }
+    } else {
+        uint32_t st = kOut, k = 0, budget = 0;
+        float td = 0.0f, lo = 0.0f, v = 0.0f;
+        Rng g;
+        g.state = g.inc = 0;
+        for (;;) {
+            const uint32_t idle = __ballot_sync(kFull, st == kOut);
+            if (idle && next < n && ((uint32_t)__popc(idle) >= kRayRefill || idle == kFull)) {
+                const uint32_t i = next + __popc(idle & lt);
+                if (st == kOut && i < n) {
+                    g = rng_seed(seed, r, s0 + i);
+                    td = 0.0f;
+                    k = 0;
+                    budget = med.budget;
+                    st = kWalk;
+                }
+                next += __popc(idle);
+            } else if (idle == kFull) {
+                break;
+            }
+            if (st == kWalk) {
+                if (k == leaves) {
+                    ++esc;
+                    st = kOut;
+                } else {
+                    const uint4 e = list[k];
+                    v = g.uniform();
+                    if (leaves_at_once(v, __uint_as_float(e.w), __uint_as_float(e.y), __uint_as_float(e.z), td) &&
+                        fog_only<FEAT>(S, e.x)) {
+                        td = __uint_as_float(e.z);
+                        ++k;
+                    } else {
+                        lo = td;
+                        st = kHard;
+                    }
+                }
+            }
+            const bool hard = st == kHard || st == kHardAgain;
+            const uint32_t nl = __ballot_sync(kFull, hard);
+            if (nl && ((uint32_t)__popc(nl) >= kHardBatch || !__any_sync(kFull, st == kWalk)) && hard) {
+                const uint4 e = list[k];
+                const uint32_t f = leaf_flight<FEAT>(S, med.sigma_e, ro, rd, e.x, __uint_as_float(e.y),
+                                                     __uint_as_float(e.z), lo, st == kHard, v, td, g, cnt);
+                st = f == kLeft ? kWalk : kHardAgain;
+                if (f == kLeft) ++k;
+                if (f == kReal) {
+                    st = kOut;
+                } else if (f == kNull && --budget == 0) {
+                    ++esc;  // a segment that gives up counts as escaped
+                    st = kOut;
+                }
+            }
+        }
+    }
+    esc = __reduce_add_sync(kFull, esc);
+    if (lane == 0 && esc) atomicAdd(&escapes[r], (unsigned long long)esc);
+}
+
 // Between rounds: the tickets taken so far are done, the record buffer is empty.
 __global__ void next_round_kernel(PathCtl *ctl) {
     ctl->base = ctl->ticket;
@@ -517,8 +712,14 @@ __global__ void next_round_kernel(PathCtl *ctl) {
 // be computed in full; segment ends are processed when kEndBatch lanes have one.
 enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
 // Slots and residency were measured on the 512^3 frame: 64 slots at 4 blocks per
-// SM 19.7 ms, 56 at 5 20.8, 48 at 5 21.9, 48 at 6 (80 registers) 25.9; more warps
-// cost L1 (the slots are shared memory) and instruction cache.
+// SM (128 registers) 18.3 ms, 56 at 5 20.0, 52 at 5 20.9, 48 at 6 (80 registers)
+// 27.3: more warps cost registers, L1 (the slots are shared memory) and
+// instruction cache.  Code size counts: rolling the loops of the rare parts and
+// calling instead of inlining (111 to 83 KB of code) took the frame from 19.6 to
+// 18.3 ms and instruction stalls from 1.46 to 0.57 cycles per instruction.
+// No array of these kernels lives in local memory: with one (a stack for the
+// octree in slow_segment) beside spilled registers, a kernel counted a few node
+// visits too many now and then; the octree's stack here is its child slots.
 constexpr int kScatterBlock = 128;
 constexpr int kSlots = 64;
 constexpr uint32_t kEventBatch = kSlots - 32;  // events that make a shading pass
@@ -582,14 +783,13 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
     float *const slots = reinterpret_cast<float *>(area + (size_t)colwords * 4u * kScatterBlock +
                                                    (threadIdx.x >> 5) * scatter_warp_bytes<BATCH>());
     float *const skyq = slots + slot_words<BATCH>() * kSlots;
-    uint8_t *const ready = reinterpret_cast<uint8_t *>(skyq + skyq_words<BATCH>());
-    uint8_t *const event = ready + kSlots, *const freed = event + kSlots;
+    uint8_t *const lists = reinterpret_cast<uint8_t *>(skyq + skyq_words<BATCH>());
+#define ready(i) lists[i]
+#define event(i) lists[kSlots + (i)]
+#define freed(i) lists[2 * kSlots + (i)]
     uint32_t n_ready = 0, n_event = 0, n_free = kSlots, n_sky = 0;
-    for (uint32_t i = lane; i < (uint32_t)kSlots; i += 32) freed[i] = (uint8_t)i;
+    for (uint32_t i = lane; i < (uint32_t)kSlots; i += 32) freed(i) = (uint8_t)i;
     __syncwarp();
-    const uint32_t n_rec = W.ctl->records;
-    const uint64_t qbase = W.ctl->base * kTicket;
-    const uint64_t step = B.step ? *B.step : 0ull;
     bool more = true;
     Count cnt;
     cnt.zero();
@@ -683,8 +883,8 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                 }
             }
             const uint32_t em = __ballot_sync(kFull, to_event), fm = __ballot_sync(kFull, finish);
-            if (to_event) event[n_event + __popc(em & lt)] = (uint8_t)slot;
-            if (finish) freed[n_free + __popc(fm & lt)] = (uint8_t)slot;
+            if (to_event) event(n_event + __popc(em & lt)) = (uint8_t)slot;
+            if (finish) freed(n_free + __popc(fm & lt)) = (uint8_t)slot;
             n_event += __popc(em);
             n_free += __popc(fm);
             if (to_event || finish) st = kIdle;
@@ -692,7 +892,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
             const uint32_t im = __ballot_sync(kFull, st == kIdle);
             const uint32_t rank = __popc(im & lt);
             if (st == kIdle && rank < n_ready) {
-                slot = ready[n_ready - 1u - rank];
+                slot = ready(n_ready - 1u - rank);
                 for (int k = 0; k < 3; ++k) {
                     ro[k] = SLOT(wRo + k, slot);
                     rd[k] = SLOT(wRd + k, slot);
@@ -734,7 +934,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         if (n_event && (n_event >= kEventBatch || (!busy && !due))) {
             const uint32_t n = min(n_event, 32u);
             if (lane < n) {
-                const uint32_t s = event[n_event - n + lane];
+                const uint32_t s = event(n_event - n + lane);
                 const BatchView *V = BATCH ? &B.views[__float_as_uint(SLOT(BATCH ? wView : 0, s))] : nullptr;
                 const DevParams &P = BATCH ? V->P : P0;
                 Rng e;
@@ -751,20 +951,22 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                 const float3 p3 = path_phase_eval<FEAT>(P, M, dot3(lrd, d));
                 const float q1 = sun_hit(P, srd) ? P.sun_pdf : 0.0f;
                 const float f = P.albedo;
-                const float a1[3] = {p1.x, p1.y, p1.z}, a3[3] = {p3.x, p3.y, p3.z};
                 const float td = SLOT(wTd, s);
-                for (int k = 0; k < 3; ++k) {
+#pragma unroll 1
+                for (int k = 0; k < 3; ++k) {  // rolled, like the sky's channels: the instruction cache is the scarcer
+                    const float a1 = k == 0 ? p1.x : (k == 1 ? p1.y : p1.z), a3 = k == 0 ? p3.x : (k == 1 ? p3.y : p3.z);
+                    const float dk = k == 0 ? d[0] : (k == 1 ? d[1] : d[2]);
                     const float T = SLOT(wT + k, s);
-                    SLOT(wSw + k, s) = T * ((a3[k] / (a3[k] + p2)) * f);
-                    SLOT(wT + k, s) = T * ((a1[k] / (a1[k] + q1)) * f);
-                    SLOT(wRo + k, s) = SLOT(wRo + k, s) + d[k] * td;
-                    SLOT(wRd + k, s) = lrd[k];
-                    SLOT(wSrd + k, s) = srd[k];
+                    SLOT(wSw + k, s) = T * ((a3 / (a3 + p2)) * f);
+                    SLOT(wT + k, s) = T * ((a1 / (a1 + q1)) * f);
+                    SLOT(wRo + k, s) = SLOT(wRo + k, s) + dk * td;
+                    SLOT(wRd + k, s) = k == 0 ? lrd[0] : (k == 1 ? lrd[1] : lrd[2]);
+                    SLOT(wSrd + k, s) = k == 0 ? srd[0] : (k == 1 ? srd[1] : srd[2]);
                 }
                 SLOT(wState, s) = __uint_as_float((uint32_t)e.state);
                 SLOT(wState + 1, s) = __uint_as_float((uint32_t)(e.state >> 32));
                 SLOT(wEv, s) = __uint_as_float(__float_as_uint(SLOT(wEv, s)) + 1u);
-                ready[n_ready + lane] = (uint8_t)s;
+                ready(n_ready + lane) = (uint8_t)s;
                 ++scatters;
             }
             n_event -= n;
@@ -774,6 +976,10 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         }
         // ---- new paths
         if (more && n_free && (n_free >= kFetchBatch || !busy)) {
+            // (the round's constants are read here rather than kept: registers decide the residency)
+            const uint32_t n_rec = *(const volatile uint32_t *)&W.ctl->records;
+            const uint64_t qbase = *(const volatile unsigned long long *)&W.ctl->base * kTicket;
+            const uint64_t step = B.step ? *(const volatile unsigned long long *)B.step : 0ull;
             const uint32_t want = min(n_free, 32u);
             uint32_t at = 0;
             if (lane == 0) at = atomicAdd(&W.ctl->head, want);
@@ -781,7 +987,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
             const uint32_t n = at < n_rec ? min(want, n_rec - at) : 0u;
             if (n < want) more = false;
             if (lane < n) {
-                const uint32_t s = freed[n_free - 1u - lane];
+                const uint32_t s = freed(n_free - 1u - lane);
                 const uint4 r = __ldg(&W.records[at + lane]);
                 uint64_t q = qbase + (uint32_t)(r.w - (uint32_t)qbase);
                 uint32_t v = 0;
@@ -813,7 +1019,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                 SLOT(wTd, s) = __uint_as_float(r.z);
                 SLOT(wOff, s) = __uint_as_float(iy * A.tw + ix);
                 SLOT(wEv, s) = __uint_as_float(0u);
-                event[n_event + lane] = (uint8_t)s;
+                event(n_event + lane) = (uint8_t)s;
             }
             n_free -= n;
             n_event += n;
@@ -827,21 +1033,30 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
 #pragma unroll 1
         for (int it = 0; it < kBurst; ++it) {
+            bool found = false;
             if (st == kWalk) {
-                float tra = 0.0f, trb = 0.0f;
-                const uint32_t r = grid_next<kScatterBlock>(G, S, col, ro, rd, leaf, tra, trb, cnt, 1u);
-                if (r == kTravDone) {
-                    res = kTrackEscaped;
-                    st = kEnd;
-                } else if (r == kTravLeaf) {
-                    const float denom = P.sigma_e * __ldg(&S.gmaj[leaf]);
-                    v = g.uniform();
-                    if (leaves_at_once(v, denom, tra, trb, td) && fog_only<FEAT>(S, leaf)) {
-                        td = trb;
-                    } else {
-                        lo = td;
-                        st = kHard;
-                    }
+                const GridExit e = grid_exit(G);
+                if (G.loc & kGridCheck) {  // the first cell is a leaf
+                    G.loc &= ~kGridCheck;
+                    found = true;
+                } else if (grid_plain(G, e)) {
+                    found = grid_fine<kScatterBlock>(G, col, e, cnt);
+                } else {
+                    bool done;
+                    found = grid_other<kScatterBlock>(G, S, col, ro, rd, e, cnt, done);
+                    if (done) st = kEnd, res = kTrackEscaped;
+                }
+            }
+            if (found) {
+                float tra, trb;
+                leaf = grid_leaf(G, tra, trb);
+                const float denom = P.sigma_e * __ldg(&S.gmaj[leaf]);
+                v = g.uniform();
+                if (leaves_at_once(v, denom, tra, trb, td) && fog_only<FEAT>(S, leaf)) {
+                    td = trb;
+                } else {
+                    lo = td;
+                    st = kHard;
                 }
             }
             const bool hard = st == kHard || st == kHardAgain;
@@ -863,6 +1078,9 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         }
     }
 #undef SLOT
+#undef ready
+#undef event
+#undef freed
     if constexpr (FEAT == 0) {
         __syncwarp();
         if (lane < n_sky) path_sky_eval<BATCH>(P0, sky0, B, skyq, lane);
@@ -938,6 +1156,36 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_shadow_paths(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out,
+                                DevCounters *C, bool feat, int device, cudaStream_t st) {
+    int sms = 0;
+    const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    uint64_t blocks = (A.n_paths + kListBlock - 1) / kListBlock;
+    if (blocks == 0) return cudaSuccess;
+    if (blocks > (uint64_t)sms * 8) blocks = (uint64_t)sms * 8;
+    const auto fn = feat ? shadow_paths_kernel<kFeatAll> : shadow_paths_kernel<0>;
+    fn<<<(unsigned)blocks, kListBlock, (size_t)grid_words(S.glevels) * 4 * kListBlock, st>>>(S, P, A, out, C);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_transmittance(const DevScene &S, const DevParams &P, const float *ro, const float *rd,
+                                 uint32_t n_rays, uint64_t nsamp, uint64_t seed, unsigned long long *escapes,
+                                 cudaStream_t st) {
+    // samples per warp: enough warps to fill the GPU (about 16,000) before a walk of
+    // the ray is shared by more samples; at most 4,096
+    uint64_t chunk = nsamp * n_rays / 16384;
+    chunk = chunk < 64 ? 64 : chunk > 4096 ? 4096 : (chunk + 31) / 32 * 32;
+    const uint64_t items = (nsamp + chunk - 1) / chunk * n_rays;
+    const uint64_t blocks = (items + kListBlock / 32 - 1) / (kListBlock / 32);
+    if (blocks == 0) return cudaSuccess;
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    const auto fn = S.sdf_bricks ? transmittance_kernel<kFeatSdf> : transmittance_kernel<0>;
+    fn<<<(unsigned)blocks, kListBlock, ray_smem(S.glevels), st>>>(S, seg_medium(P), ro, rd, n_rays, nsamp,
+                                                                  (uint32_t)chunk, seed, escapes);
+    return cudaGetLastError();
 }
 
 bool paths_serve(const Tuning &tune, uint32_t glevels) { return tune.traversal != 1u && glevels != 0u; }

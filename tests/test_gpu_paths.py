@@ -88,3 +88,44 @@ def test_pixels_without_lists(renderer, pool):
         _check(_pair(renderer, c0_cfg(64, 64), (4, 6, 50, 52), 37))
     finally:
         renderer.set_camera_lists(0)
+
+
+def _rays(n, seed):
+    rng = np.random.default_rng(seed)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    ro = 0.5 + rng.uniform(-0.3, 0.3, (n, 3)) - rng.choice([0.0, 1.5], (n, 1)) * d
+    rd = d.astype(np.float32)
+    rd[0] = (0.0, 0.0, -1.0)  # a zero direction component: takes the octree
+    return ro.astype(np.float32), rd
+
+
+# samples around a warp's share of a ray (64 to 4,096)
+@pytest.mark.parametrize("n_rays,nsamp", [(1, 1), (3, 33), (700, 64), (5, 4097), (40, 20000)])
+def test_transmittance_counts(renderer, n_rays, nsamp):
+    """The escapes equal those the adjoint's replay counts (octree, one sample a thread), sample for sample."""
+    renderer.set_params(settings_from_cfg(c0_cfg(64, 64)))
+    ro, rd = _rays(n_rays, n_rays)
+    got = renderer.probe_transmittance(ro, rd, nsamp, seed=77)
+    _, ref = renderer.adjoint_transmittance(ro, rd, np.ones(n_rays), nsamp, 77, len(golden_octree()[1]))
+    assert np.array_equal(got, ref)
+
+
+def test_transmittance_of_long_leaf_lists():
+    """Rays with more leaves than a warp keeps (96) are traversed per sample."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import build_octree
+
+    i = np.arange(128)
+    org = np.stack([8 * i, 8 * i, 8 * i], 1).astype(np.int32)
+    oc = build_octree(org, np.full((128, 512), 0.02, np.float32), 1.0 / 1024, 12)
+    with Renderer(0) as r:
+        r.upload(oc)
+        r.set_params(settings_from_cfg(c0_cfg(64, 64)))
+        ro = np.array([[-0.2, -0.2001, -0.1999], [0.5, 0.5, 0.5]], np.float32)
+        rd = np.array([[1.0, 1.0001, 0.9999], [0.3, -0.2, 0.9]], np.float32)
+        rd /= np.linalg.norm(rd, axis=1, keepdims=True).astype(np.float32)
+        assert r.probe_leaf_sequence(ro, rd, 512)[3].max() > 96
+        got = r.probe_transmittance(ro, rd, 1000, seed=5)
+        _, ref = r.adjoint_transmittance(ro, rd, np.ones(2), 1000, 5, oc.n_leaves)
+        assert np.array_equal(got, ref) and got.min() < 1.0
