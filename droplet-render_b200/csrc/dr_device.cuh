@@ -924,11 +924,13 @@ __device__ __forceinline__ bool grid_other(GridTrav &G, const DevScene &S, float
     const bool tie = !(G.tc < e.t), out = grid_leaves_block(G, e);
     float hi;
     int tz = -1;  // levels 1 (the 2^3 block) .. 2 + tz are entered
+    uint4 g = make_uint4(0u, 0u, 0u, 0u);
     if (out) {
         const uint32_t s = (uint32_t)k * lb, f = (G.c >> s) & nbm;
         done = f == nbm;
         if (done) return false;
         G.c += 1u << s;
+        g = __ldg(&S.gblock[G.c ^ G.am]);  // first, so that the plane arithmetic covers its latency
         tz = __ffs((int)(f + 1u)) - 1;
         hi = col[(3 * (tz + 1) + k) * STRIDE];
 #pragma unroll 1
@@ -952,7 +954,7 @@ __device__ __forceinline__ bool grid_other(GridTrav &G, const DevScene &S, float
         return false;
     }
     if (out) {
-        const uint4 g = __ldg(&S.gblock[G.c ^ G.am]);
+        if (tie) g = __ldg(&S.gblock[G.c ^ G.am]);
         G.mlo = g.x;
         G.mhi = g.y;
         G.base = g.z;

@@ -206,7 +206,7 @@ struct PathCtl {
     uint32_t pool_used;         // leaf list entries taken
     uint32_t n_active;          // active pixels
 };
-constexpr uint32_t kRoundTickets = 1u << 24;  // tickets of one round: 2^31 samples, so 32 bits tell them apart
+constexpr uint32_t kRoundTickets = 1u << 24;  // tickets of one round: at most 2^31 samples, so 32 bits tell them apart
 
 // Storage of the path pipeline for one launch at a time.
 struct PathWork {
@@ -220,6 +220,7 @@ struct PathWork {
     uint4 *records;
     uint32_t cap;                    // records that fit
     uint32_t limit;                  // no new ticket above this count (set by the launcher)
+    uint32_t ticket;                 // camera samples per ticket (set by the launcher)
     // batches
     uint32_t *view_tickets;          // first ticket of each view, then their number
     uint32_t *view_active;           // active pixels of each view

@@ -27,8 +27,7 @@
 namespace dr {
 
 constexpr uint32_t kFull = 0xffffffffu;
-constexpr uint32_t kChunks = 4;             // groups of 32 camera samples per ticket
-constexpr uint32_t kTicket = 32 * kChunks;  // camera samples per ticket
+constexpr uint32_t kTicketMost = 128;  // camera samples per ticket (W.ticket: 128 or, in small launches, 32)
 constexpr int kListBlock = 128, kListTx = 16, kListTy = 8;  // camera lists: a block covers 16 x 8 pixels
 
 // ---- camera lists -------------------------------------------------------------
@@ -173,7 +172,7 @@ __global__ void view_tickets_kernel(BatchArgs B, PathWork W) {
     for (uint32_t v0 = 0; v0 < B.n_views; v0 += 32) {
         const uint32_t v = v0 + lane;
         uint32_t n = 0;
-        if (v < B.n_views) n = (uint32_t)(((uint64_t)W.view_active[v] * B.views[v].A.spp + kTicket - 1) / kTicket);
+        if (v < B.n_views) n = (uint32_t)(((uint64_t)W.view_active[v] * B.views[v].A.spp + W.ticket - 1) / W.ticket);
         uint32_t sum = n;
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t o = __shfl_up_sync(kFull, sum, d);
@@ -196,7 +195,7 @@ template <uint32_t FEAT>
 __device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e, const float ro[3], const float rd[3],
                                                 uint32_t slot, float tra, float trb, float lo, bool first, float &v,
                                                 float &td, Rng &g, Count &cnt) {
-    const float4 meta = __ldg(&S.gleaf[2 * slot + 1]);
+    const float4 meta = __ldg(&S.gleaf[2 * slot + 1]), ce = __ldg(&S.gleaf[2 * slot]);
     const float denom = sigma_e * meta.x;
     const float tr0 = tra - lo, tr1 = trb - lo;
     float s0 = tra > lo ? tr0 : __uint_as_float(__float_as_uint(tr0) & 1u);
@@ -208,7 +207,7 @@ __device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e
             s0 = 0.0f;
             if (tra > lo) {  // src/kernel.cpp:253-263
                 const float r0[3] = {ro[0] + rd[0] * tra, ro[1] + rd[1] * tra, ro[2] + rd[2] * tra};
-                if (sample_voxel_space(r0, sdf, __ldg(&S.gleaf[2 * slot])) > 0.0f) s0 = tr0;
+                if (sample_voxel_space(r0, sdf, ce) > 0.0f) s0 = tr0;
                 if (first) ++cnt.density_lookups;
             }
         }
@@ -225,7 +224,6 @@ __device__ __forceinline__ uint32_t leaf_flight(const DevScene &S, float sigma_e
     bool rm = sc > tr0;
     float rho = -1.0f, dist = 1.0f;
     if (rm) {
-        const float4 ce = __ldg(&S.gleaf[2 * slot]);
         const float rc[3] = {ro[0] + rd[0] * td, ro[1] + rd[1] * td, ro[2] + rd[2] * td};
         const uint32_t fog = __float_as_uint(meta.y);
         bool look = true;
@@ -390,9 +388,9 @@ __device__ __forceinline__ void active_sample(const TileArgs &A, const uint32_t 
     pix = __ldg(&active[a]);
 }
 
-// Camera samples are handed out in tickets of kTicket consecutive ones.  A warp
+// Camera samples are handed out in tickets of W.ticket consecutive ones.  A warp
 // takes a ticket only while the record buffer has room for every warp's
-// (W.limit = capacity - warps * kTicket), so the buffer never overflows and the
+// (W.limit = capacity - warps * W.ticket), so the buffer never overflows and the
 // tickets taken are exactly those done: the next round goes on from there.
 template <uint32_t FEAT, bool BATCH>
 __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __grid_constant__ DevScene S0,
@@ -414,7 +412,7 @@ __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __gri
         n_tickets = W.view_tickets[B.n_views];
     } else {
         total = (uint64_t)*W.n_active * A0.spp;
-        n_tickets = (uint32_t)((total + kTicket - 1) / kTicket);
+        n_tickets = (uint32_t)((total + W.ticket - 1) / W.ticket);
     }
     const unsigned long long base = W.ctl->base;
     for (;;) {
@@ -427,10 +425,10 @@ __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __gri
         t = __shfl_sync(kFull, t, 0);
         if (t >= n_tickets) break;
         uint32_t view = 0;
-        uint64_t q0 = t * kTicket;
+        uint64_t q0 = t * W.ticket;
         if constexpr (BATCH) {
             view = find_last(W.view_tickets, B.n_views, (uint32_t)t);
-            q0 = (t - W.view_tickets[view]) * kTicket;
+            q0 = (t - W.view_tickets[view]) * W.ticket;
             total = (uint64_t)W.view_active[view] * B.views[view].A.spp;
         }
         const BatchView *V = BATCH ? &B.views[view] : nullptr;
@@ -439,8 +437,8 @@ __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __gri
         const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
         const uint4 *head = BATCH ? A.cam_head : W.head;
         const uint32_t *active = BATCH ? W.active + W.pix_begins[view] : W.active;
-        for (uint32_t c = 0; c < kChunks; ++c) {
-            const uint64_t q = q0 + c * 32u + lane;
+        for (uint32_t c = 0; c < W.ticket; c += 32u) {
+            const uint64_t q = q0 + c + lane;
             if (q - lane >= total) break;
             const bool valid = q < total;
             uint32_t pix = kNone, s = 0;
@@ -490,7 +488,7 @@ __global__ void __launch_bounds__(kListBlock, 8) camera_paths_kernel(const __gri
                 at = __shfl_sync(kFull, at, 0) + __popc(gm & ((1u << lane) - 1u));
                 if (go)
                     W.records[at] = make_uint4((uint32_t)o.g.state, (uint32_t)(o.g.state >> 32), __float_as_uint(o.td),
-                                               (uint32_t)(t * kTicket + c * 32u + lane));
+                                               (uint32_t)(t * W.ticket + c + lane));
             }
         }
     }
@@ -712,7 +710,7 @@ __global__ void next_round_kernel(PathCtl *ctl) {
 // be computed in full; segment ends are processed when kEndBatch lanes have one.
 enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
 // Slots and residency were measured on the 512^3 frame: 64 slots at 4 blocks per
-// SM (128 registers) 18.3 ms, 56 at 5 20.0, 52 at 5 20.9, 48 at 6 (80 registers)
+// SM (128 registers) 17.8 ms, 56 at 5 20.0, 52 at 5 20.9, 48 at 6 (80 registers)
 // 27.3: more warps cost registers, L1 (the slots are shared memory) and
 // instruction cache.  Code size counts: rolling the loops of the rare parts and
 // calling instead of inlining (111 to 83 KB of code) took the frame from 19.6 to
@@ -722,10 +720,11 @@ enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
 // visits too many now and then; the octree's stack here is its child slots.
 constexpr int kScatterBlock = 128;
 constexpr int kSlots = 64;
-constexpr uint32_t kEventBatch = kSlots - 32;  // events that make a shading pass
-constexpr uint32_t kEndBatch = 10;             // lanes at a segment end (or idle with work ready) that make an end pass
-constexpr uint32_t kWaitBatch = 10;            // lanes that make a pass of full flights
+constexpr uint32_t kEventBatch = 28;           // events that make a shading pass
+constexpr uint32_t kEndBatch = 8;             // lanes at a segment end (or idle with work ready) that make an end pass
+constexpr uint32_t kWaitBatch = 6;            // lanes that make a pass of full flights
 constexpr uint32_t kFetchBatch = 16;           // free slots that make a fetch
+constexpr uint32_t kLeastShare = 4;            // paths a warp takes at least
 constexpr int kBurst = 3;                      // loop bodies between looks at the lists
 // slot words (word w of slot s at w * kSlots + s)
 enum : int { wState = 0, wInc = 2, wRo = 4, wRd = 7, wT = 10, wSun = 13, wSw = 16, wSrd = 19, wTd = 22, wOff = 23, wEv = 24,
@@ -791,6 +790,11 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
     for (uint32_t i = lane; i < (uint32_t)kSlots; i += 32) freed(i) = (uint8_t)i;
     __syncwarp();
     bool more = true;
+    // slots left empty where the records are too few to fill every warp's: a path's
+    // latency, not the lanes, is then what the launch waits for (a 64 x 64 tile at 16
+    // samples: scatter 189 -> 150 us; with it and the small tickets 0.39 -> 0.31 ms a call)
+    const uint32_t share = (W.ctl->records + gridDim.x * (kScatterBlock / 32) - 1) / (gridDim.x * (kScatterBlock / 32));
+    const uint32_t spare = share < (uint32_t)kSlots ? (uint32_t)kSlots - max(share, kLeastShare) : 0u;
     Count cnt;
     cnt.zero();
     uint32_t scatters = 0;
@@ -975,12 +979,13 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
             continue;
         }
         // ---- new paths
-        if (more && n_free && (n_free >= kFetchBatch || !busy)) {
+        const uint32_t room = n_free > spare ? n_free - spare : 0u;
+        if (more && room && (room >= kFetchBatch || !busy)) {
             // (the round's constants are read here rather than kept: registers decide the residency)
             const uint32_t n_rec = *(const volatile uint32_t *)&W.ctl->records;
-            const uint64_t qbase = *(const volatile unsigned long long *)&W.ctl->base * kTicket;
+            const uint64_t qbase = *(const volatile unsigned long long *)&W.ctl->base * W.ticket;
             const uint64_t step = B.step ? *(const volatile unsigned long long *)B.step : 0ull;
-            const uint32_t want = min(n_free, 32u);
+            const uint32_t want = min(room, 32u);
             uint32_t at = 0;
             if (lane == 0) at = atomicAdd(&W.ctl->head, want);
             at = __shfl_sync(kFull, at, 0);
@@ -992,8 +997,8 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                 uint64_t q = qbase + (uint32_t)(r.w - (uint32_t)qbase);
                 uint32_t v = 0;
                 if constexpr (BATCH) {
-                    v = find_last(W.view_tickets, B.n_views, (uint32_t)(q / kTicket));
-                    q -= (uint64_t)W.view_tickets[v] * kTicket;
+                    v = find_last(W.view_tickets, B.n_views, (uint32_t)(q / W.ticket));
+                    q -= (uint64_t)W.view_tickets[v] * W.ticket;
                     SLOT(wView, s) = __uint_as_float(v);
                 }
                 const BatchView *V = BATCH ? &B.views[v] : nullptr;
@@ -1101,8 +1106,8 @@ template <class F> static cudaError_t opt_in(F fn, size_t smem) {
                                 (int)smem);
 }
 
-static uint64_t rounds_of(uint64_t n_paths, uint64_t limit) {
-    const uint64_t span = (uint64_t)kRoundTickets * kTicket;
+static uint64_t rounds_of(uint64_t n_paths, uint64_t limit, uint32_t ticket) {
+    const uint64_t span = (uint64_t)kRoundTickets * ticket;
     return (n_paths + limit - 1) / limit + n_paths / span;
 }
 
@@ -1133,13 +1138,13 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sca, kScatterBlock, sca_smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const uint64_t cam_most = (n_paths + kTicket * 4 - 1) / (kTicket * 4), sca_most = (n_paths + 127) / 128;
+    const uint64_t cam_most = (n_paths + W.ticket * 4 - 1) / (W.ticket * 4), sca_most = (n_paths + 127) / 128;
     unsigned cam_blocks = (unsigned)(cam_most < (uint64_t)sms * 8 ? cam_most : (uint64_t)sms * 8);
     const unsigned sca_blocks =
         (unsigned)(sca_most < (uint64_t)sms * per_sm ? sca_most : (uint64_t)sms * (uint64_t)per_sm);
     // every warp of the camera kernel may add a ticket's samples after its last
     // look at the record count: half the buffer at most is kept for that
-    const uint64_t per_block = (uint64_t)(kListBlock / 32) * kTicket;
+    const uint64_t per_block = (uint64_t)(kListBlock / 32) * W.ticket;
     if (n_paths > W.cap) {
         if (W.cap < 2 * per_block) return cudaErrorInvalidValue;
         if (cam_blocks * per_block > W.cap / 2) cam_blocks = (unsigned)(W.cap / 2 / per_block);
@@ -1147,7 +1152,7 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
     } else {
         W.limit = W.cap;
     }
-    const uint64_t rounds = rounds_of(n_paths, W.limit);
+    const uint64_t rounds = rounds_of(n_paths, W.limit, W.ticket);
     for (uint64_t r = 0; r < rounds; ++r) {
         if (r) next_round_kernel<<<1, 1, 0, st>>>(W.ctl);
         cam<<<cam_blocks, kListBlock, cam_smem, st>>>(S, P, A, W, sun, sky, C, B);
@@ -1188,6 +1193,15 @@ cudaError_t launch_transmittance(const DevScene &S, const DevParams &P, const fl
     return cudaGetLastError();
 }
 
+// Samples per ticket: one group of 32 until every resident camera warp has
+// four tickets of 128 (the group's latency is what a small launch waits for),
+// then 128 (fewer draws on the ticket counter).
+static uint32_t ticket_samples(uint64_t n_paths, int device) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 1;
+    return n_paths < (uint64_t)sms * 8 * (kListBlock / 32) * kTicketMost * 4 ? 32u : kTicketMost;
+}
+
 bool paths_serve(const Tuning &tune, uint32_t glevels) { return tune.traversal != 1u && glevels != 0u; }
 
 uint32_t path_list_blocks(uint32_t cols, uint32_t rows) {
@@ -1195,10 +1209,12 @@ uint32_t path_list_blocks(uint32_t cols, uint32_t rows) {
 }
 
 cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
-                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &W, bool feat, int device,
+                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &storage, bool feat, int device,
                          cudaStream_t st, const unsigned long long *step) {
     const uint64_t n_paths = (uint64_t)A.cols * A.rows * A.spp;
     if (n_paths == 0) return cudaSuccess;
+    PathWork W = storage;
+    W.ticket = ticket_samples(n_paths, device);
     cudaError_t e = cudaMemsetAsync(W.ctl, 0, sizeof(PathCtl), st);
     if (e != cudaSuccess) return e;
     path_lists_kernel<<<path_list_blocks(A.cols, A.rows), kListBlock, (size_t)grid_words(S.glevels) * 4 * kListBlock,
@@ -1212,9 +1228,11 @@ cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &
 }
 
 cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                               const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool feat, uint32_t glevels,
-                               int device, cudaStream_t st) {
+                               const PathWork &storage, uint64_t n_paths, uint32_t n_blocks, bool feat,
+                               uint32_t glevels, int device, cudaStream_t st) {
     if (n_paths == 0) return cudaSuccess;
+    PathWork W = storage;
+    W.ticket = ticket_samples(n_paths, device);
     cudaError_t e = cudaMemsetAsync(W.ctl, 0, sizeof(PathCtl), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(W.view_active, 0, sizeof(uint32_t) * B.n_views, st);
     if (e != cudaSuccess) return e;

@@ -120,7 +120,7 @@ int main(int argc, char **argv) {
         float iv[kMaxDepth][6];
         trav_init(T, S, ro, rd, ca);
         GridTrav Gt;
-        float col[3 * kGridMaxLevels];
+        float col[grid_words(kGridMaxLevels)];
         const uint32_t mode = grid_init<1>(Gt, S, col, ro, rd, cb);
         if (mode == 2) {
             ++slow;
