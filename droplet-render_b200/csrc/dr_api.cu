@@ -100,16 +100,8 @@ int dr_destroy(dr_ctx *c) {
         c->env.release();
         c->occ_tris.release();
         c->band_work.release();
-        c->cam_head.release();
-        c->cam_pool.release();
-        c->band_cam_head.release();
-        c->band_cam_pool.release();
-        c->cam_used.release();
-        c->path_ctl.release();
-        c->path_active.release();
-        c->band_path_active.release();
-        c->path_rec_async.release();
-        c->path_rec_band.release();
+        c->lists.release();
+        c->band_lists.release();
         for (int k = 0; k < 2; ++k)
             if (c->band_stream[k]) cudaStreamSynchronize(c->band_stream[k]), cudaStreamDestroy(c->band_stream[k]);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream), cudaStreamDestroy(c->copy_stream);
@@ -211,16 +203,32 @@ static uint32_t pool_capacity(const dr_ctx *c, size_t pixels, uint32_t slot) {
     return (uint32_t)std::min((size_t)dr_ctx::kCamPool, std::max((size_t)1 << 18, pixels * (slot ? 8 : 32)));
 }
 
-// Storage of a persistent launch's camera leaf lists and path pipeline: slot 0
-// for the asynchronous render, 1 and 2 (one allocation) for the band streams.
-static bool reserve_lists(dr_ctx *c, uint32_t slot, size_t pixels, uint32_t rec_cap) {
-    const uint32_t pool = pool_capacity(c, pixels, slot);
+// Storage of a launch's camera leaf lists and path pipeline for up to `pixels`
+// pixels: slot 0 for the asynchronous render, 1 and 2 (one allocation, headers
+// and active pixels shared by rows) for the band streams.  Byte offsets.
+struct ListLayout {
+    uint32_t rec_cap, pool_cap;
+    size_t records, pool, head, active, ctl, used, bytes;
+};
+static ListLayout list_layout(const dr_ctx *c, uint32_t slot, size_t pixels) {
     const size_t two = slot ? 2 : 1;
-    return c->cam_used.reserve(3) == cudaSuccess && c->path_ctl.reserve(3) == cudaSuccess &&
-           (slot ? c->band_cam_head : c->cam_head).reserve(2 * pixels) == cudaSuccess &&
-           (slot ? c->band_path_active : c->path_active).reserve(pixels) == cudaSuccess &&
-           (slot ? c->path_rec_band : c->path_rec_async).reserve(two * rec_cap) == cudaSuccess &&
-           (slot ? c->band_cam_pool : c->cam_pool).reserve((size_t)two * pool) == cudaSuccess;
+    ListLayout l;
+    l.rec_cap = rec_capacity(pixels, slot);
+    l.pool_cap = pool_capacity(c, pixels, slot);
+    size_t at = 0;
+    auto part = [&at](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    l.records = part(two * l.rec_cap * sizeof(uint4));
+    l.pool = part(two * l.pool_cap * sizeof(uint4));
+    l.head = part(2 * pixels * sizeof(uint4));
+    l.active = part(pixels * sizeof(uint32_t));
+    l.ctl = part(two * sizeof(PathCtl));
+    l.used = part(two * sizeof(unsigned int));
+    l.bytes = at;
+    return l;
 }
 
 int dr_set_params(dr_ctx *c, const dr_render_params *p) {
@@ -253,9 +261,9 @@ int dr_set_params(dr_ctx *c, const dr_render_params *p) {
     // list and path pipeline storage for tiles up to the whole frame, so that
     // renders allocate nothing (without it they traverse per sample)
     const size_t frame = (size_t)p->w * p->h;
-    (void)reserve_lists(c, 0, frame, rec_capacity(frame, 0));
-    (void)reserve_lists(c, 1, frame, rec_capacity(frame, 1));
-    cudaGetLastError();  // a failure is not an error of the parameters
+    if (c->lists.reserve(list_layout(c, 0, frame).bytes) != cudaSuccess ||
+        c->band_lists.reserve(list_layout(c, 1, frame).bytes) != cudaSuccess)
+        cudaGetLastError();  // not an error of the parameters
     return DR_OK;
 }
 
@@ -327,21 +335,21 @@ static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t h
     CamLists L;
     // the storage follows the frame, or the tile when that is larger
     const size_t pixels = std::max(head_pixels, (size_t)c->params.w * c->params.h);
-    const uint32_t rec_cap = rec_capacity(pixels, slot);
-    if (!reserve_lists(c, slot, pixels, rec_cap)) {
+    const ListLayout l = list_layout(c, slot, pixels);
+    DevBuf<unsigned char> &buf = slot ? c->band_lists : c->lists;
+    if (buf.reserve(l.bytes) != cudaSuccess) {
         cudaGetLastError();  // not an error of the render
         return L;
     }
     const size_t second = slot == 2 ? 1 : 0;
-    const uint32_t pool = pool_capacity(c, pixels, slot);
-    L.head = (slot ? c->band_cam_head : c->cam_head).p + 2 * head_off;
-    L.pool = (slot ? c->band_cam_pool : c->cam_pool).p + second * pool;
-    L.cap = pool;
-    L.used = c->cam_used.p + slot;
-    L.ctl = c->path_ctl.p + slot;
-    L.active = (slot ? c->band_path_active : c->path_active).p + head_off;
-    L.records = (slot ? c->path_rec_band : c->path_rec_async).p + second * rec_cap;
-    L.rec_cap = rec_cap;
+    L.head = reinterpret_cast<uint4 *>(buf.p + l.head) + 2 * head_off;
+    L.pool = reinterpret_cast<uint4 *>(buf.p + l.pool) + second * l.pool_cap;
+    L.cap = l.pool_cap;
+    L.used = reinterpret_cast<unsigned int *>(buf.p + l.used) + second;
+    L.ctl = reinterpret_cast<PathCtl *>(buf.p + l.ctl) + second;
+    L.active = reinterpret_cast<uint32_t *>(buf.p + l.active) + head_off;
+    L.records = reinterpret_cast<uint4 *>(buf.p + l.records) + second * l.rec_cap;
+    L.rec_cap = l.rec_cap;
     return L;
 }
 

@@ -269,20 +269,15 @@ struct dr_ctx {
     cudaEvent_t band_done[kBands] = {};
     cudaEvent_t copy_done[kBands] = {};
     dr::DevBuf<dr::WorkQueue> band_work;
-    // camera leaf lists of the persistent kernel (TileArgs::cam_head): headers
-    // per pixel of a launch and a pool of kCamPool entries with a fill counter,
-    // for the asynchronous render (slot 0) and each band stream of the blocking
-    // render (slots 1, 2); allocated on first use
+    // camera leaf lists and path pipeline (TileArgs::cam_head, PathWork): headers and
+    // active pixels per pixel of a launch, a pool of list entries, a buffer of
+    // collided samples and control words, in one allocation for the asynchronous
+    // render (slot 0) and one for the two band streams of the blocking render
+    // (slots 1, 2); laid out by list_layout
     static constexpr uint32_t kCamPool = 1u << 23;
     uint32_t cam_cap = 0;      // entries per pool when set (dr_set_camera_lists; 0: no lists)
     bool cam_cap_set = false;  // else in proportion to the frame, up to kCamPool
-    dr::DevBuf<uint4> cam_head, cam_pool, band_cam_head, band_cam_pool;
-    dr::DevBuf<unsigned int> cam_used;
-    // path pipeline (PathWork): control words and active pixels like the lists,
-    // and a buffer of collided samples
-    dr::DevBuf<dr::PathCtl> path_ctl;
-    dr::DevBuf<uint32_t> path_active, band_path_active;
-    dr::DevBuf<uint4> path_rec_async, path_rec_band;
+    dr::DevBuf<unsigned char> lists, band_lists;
     float *pinned = nullptr;  // 2 * pinned_n float4: sun then sky
     size_t pinned_n = 0;
     dr::CopyPool copies;      // host threads for the staging -> caller copies
