@@ -96,12 +96,14 @@ int dr_destroy(dr_ctx *c) {
         c->grad_copies.release();
         c->albedo_slots.release();
         c->path_rec.release();
+        c->tape.release();
         c->occ_nodes.release();
         c->env.release();
         c->occ_tris.release();
         c->band_work.release();
         c->lists.release();
         c->band_lists.release();
+        c->adjoint_lists.release();
         for (int k = 0; k < 2; ++k)
             if (c->band_stream[k]) cudaStreamSynchronize(c->band_stream[k]), cudaStreamDestroy(c->band_stream[k]);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream), cudaStreamDestroy(c->copy_stream);
@@ -329,14 +331,17 @@ static int tile_args(const dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uin
 
 // The lists and pipeline storage of a launch: slot 0 for the asynchronous
 // render, 1 + (band & 1) for the blocking render's band streams (head_off: the
-// band's first pixel among the tile's headers).  A failed allocation leaves
+// band's first pixel among the tile's headers), kAdjointLists for the adjoint
+// (laid out as slot 0, its own: it may run on another stream than a render).  A failed allocation leaves
 // the launch without (its camera segments traverse per sample).
+constexpr uint32_t kAdjointLists = 3;
 static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t head_off) {
     CamLists L;
     // the storage follows the frame, or the tile when that is larger
     const size_t pixels = std::max(head_pixels, (size_t)c->params.w * c->params.h);
+    DevBuf<unsigned char> &buf = slot == kAdjointLists ? c->adjoint_lists : slot ? c->band_lists : c->lists;
+    if (slot == kAdjointLists) slot = 0;
     const ListLayout l = list_layout(c, slot, pixels);
-    DevBuf<unsigned char> &buf = slot ? c->band_lists : c->lists;
     if (buf.reserve(l.bytes) != cudaSuccess) {
         cudaGetLastError();  // not an error of the render
         return L;
@@ -809,6 +814,33 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
     if (!c->albedo_slots.p) {
         DR_CUDA(c->albedo_slots.reserve(adjoint_slots()), "adjoint: alloc slots");
         DR_CUDA(cudaMemset(c->albedo_slots.p, 0, sizeof(double) * adjoint_slots()), "adjoint: clear slots");
+    }
+    // on the path pipeline, in chunks of rows of at most 2^23 paths; the tape has room
+    // for 24 decisions a path up to 512 MB (a path that does not fit is replayed)
+    const uint64_t row_pair = 2 * (uint64_t)A.cols * spp;
+    if (c->scene.glevels && row_pair && row_pair <= (1ull << 23) && c->scene.n_leaves < (1u << 23)) {
+        const uint32_t rows = (uint32_t)std::min<uint64_t>(A.rows, 2 * ((1ull << 23) / row_pair));
+        std::vector<TileArgs> chunks;
+        uint64_t most = 0;
+        for (uint32_t r0 = 0; r0 < A.rows; r0 += rows) {
+            TileArgs R;
+            rc = make_tile_args(x0, y0 + r0, tw, std::min(rows, A.rows - r0), spp, seed, sample_base, 0u, R);
+            if (rc != DR_OK) return rc;
+            chunks.push_back(R);
+            most = std::max(most, R.n_paths);
+        }
+        const uint64_t entries = std::min<uint64_t>(1ull << 24, std::max<uint64_t>(1ull << 16, 24 * most));
+        const CamLists lists = cam_lists(c, kAdjointLists, (size_t)A.cols * A.rows, 0);
+        if (lists.ctl && c->path_rec.reserve(most) == cudaSuccess && c->tape.reserve(2 * entries) == cudaSuccess) {
+            DR_CUDA(launch_adjoint_tape(c->scene, c->params, chunks.data(), (uint32_t)chunks.size(), c->mie_pack.p,
+                                        (const float4 *)dsun_dev, (const float4 *)dsky_dev, grad_bricks_dev,
+                                        copies > 1 ? c->grad_copies.p : nullptr, copies, c->path_rec.p, c->tape.p,
+                                        (uint32_t)entries, grad_albedo_dev, c->albedo_slots.p, c->counters.p,
+                                        path_work(lists), c->device, st),
+                    "adjoint: launch");
+            return DR_OK;
+        }
+        cudaGetLastError();  // no room for the tape: two replays
     }
     // one 16-byte record per path of a chunk (at most 2^23 paths, 128 MB)
     const uint64_t chunk = std::min<uint64_t>(A.n_paths, 1ull << 23);

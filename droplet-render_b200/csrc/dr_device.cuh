@@ -1081,11 +1081,9 @@ static __device__ __noinline__ float sample_voxel_far(float px, float py, float 
 // product and one fused correction); floor, ceiling and the indices by adding
 // 1.5 * 2^23 and 2^23 instead of conversions, which have an eighth of the rate.
 // Positions this far outside the brick (2^20 cells) take the lookup above.
-__device__ __forceinline__ float sample_voxel_inv(const float p[3], const float *__restrict__ v, const float4 ce,
-                                                  float inv) {
+__device__ __forceinline__ bool voxel_cell_inv(const float p[3], const float4 ce, float inv, uint32_t ia[3],
+                                               uint32_t ib[3], float nl[3]) {
     const float cc[3] = {ce.x, ce.y, ce.z};
-    uint32_t ia[3], ib[3];
-    float nl[3];
     bool far = inv == 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -1101,7 +1099,14 @@ __device__ __forceinline__ float sample_voxel_inv(const float p[3], const float 
         ia[k] = __float_as_uint(sse_min(nf, 7.0f) + 8388608.0f) & 7u;
         ib[k] = __float_as_uint(sse_max(sse_min(nc, 7.0f), 0.0f) + 8388608.0f) & 7u;
     }
-    if (far) return sample_voxel_far(p[0], p[1], p[2], v, ce);
+    return !far;
+}
+
+__device__ __forceinline__ float sample_voxel_inv(const float p[3], const float *__restrict__ v, const float4 ce,
+                                                  float inv) {
+    uint32_t ia[3], ib[3];
+    float nl[3];
+    if (!voxel_cell_inv(p, ce, inv, ia, ib, nl)) return sample_voxel_far(p[0], p[1], p[2], v, ce);
     const uint32_t za = ia[2] * 64u, zb = ib[2] * 64u, ya = ia[1] * 8u, yb = ib[1] * 8u;
     const float u0 = lerp_ref(__ldg(v + za + ya + ia[0]), __ldg(v + za + ya + ib[0]), nl[0]);
     const float u1 = lerp_ref(__ldg(v + za + yb + ia[0]), __ldg(v + za + yb + ib[0]), nl[0]);
@@ -1124,12 +1129,11 @@ __device__ __forceinline__ bool ratio_below(float rho, float smax, float q) {
 // Corner offsets (within the brick) and trilinear weights of the lookup above:
 // rho = sum_k w[k] * v[idx[k]] (lerp_ref(a, b, t) = (1 - t) a + t b), the
 // derivative of rho with respect to each brick sample.
-__device__ __forceinline__ void voxel_weights(const float p[3], const float4 ce, uint32_t idx[8], float w[8]) {
+__device__ __forceinline__ void voxel_cell(const float p[3], const float4 ce, uint32_t ia[3], uint32_t ib[3],
+                                           float nl[3]) {
     const float nm1 = (float)kLvox - 1.0f;
     const float top = (float)(kLvox - 1);
     const float cc[3] = {ce.x, ce.y, ce.z};
-    uint32_t ia[3], ib[3];
-    float nl[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float ni = ((-0.5f * ((cc[k] - ce.w) - p[k])) * nm1) / ce.w;
@@ -1141,6 +1145,11 @@ __device__ __forceinline__ void voxel_weights(const float p[3], const float4 ce,
         ia[k] = (uint32_t)nf;
         ib[k] = (uint32_t)nc;
     }
+}
+__device__ __forceinline__ void voxel_weights(const float p[3], const float4 ce, uint32_t idx[8], float w[8]) {
+    uint32_t ia[3], ib[3];
+    float nl[3];
+    voxel_cell(p, ce, ia, ib, nl);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
         const uint32_t x = (c & 1) ? ib[0] : ia[0], y = (c & 2) ? ib[1] : ia[1], z = (c & 4) ? ib[2] : ia[2];

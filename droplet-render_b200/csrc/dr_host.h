@@ -254,6 +254,7 @@ struct dr_ctx {
     dr::DevBuf<float> grad_copies;    // adjoint: spread copies of the brick-pool gradient
     dr::DevBuf<double> albedo_slots;  // adjoint: partial sums of the albedo gradient (kept zeroed)
     dr::DevBuf<uint4> path_rec;       // adjoint: one record per path of a chunk (totals pass -> scatter pass)
+    dr::DevBuf<uint4> tape;           // adjoint: tracking decisions (AdjointArgs::tape)
     dr::DevBuf<float4> occ_nodes, occ_tris;  // occluder BVH (kept across scene uploads)
     uint32_t occ_n_nodes = 0;
     uint32_t n_leaf_nodes = 0;
@@ -273,11 +274,11 @@ struct dr_ctx {
     // active pixels per pixel of a launch, a pool of list entries, a buffer of
     // collided samples and control words, in one allocation for the asynchronous
     // render (slot 0) and one for the two band streams of the blocking render
-    // (slots 1, 2); laid out by list_layout
+    // (slots 1, 2); the adjoint has its own; laid out by list_layout
     static constexpr uint32_t kCamPool = 1u << 23;
     uint32_t cam_cap = 0;      // entries per pool when set (dr_set_camera_lists; 0: no lists)
     bool cam_cap_set = false;  // else in proportion to the frame, up to kCamPool
-    dr::DevBuf<unsigned char> lists, band_lists;
+    dr::DevBuf<unsigned char> lists, band_lists, adjoint_lists;
     float *pinned = nullptr;  // 2 * pinned_n float4: sun then sky
     size_t pinned_n = 0;
     dr::CopyPool copies;      // host threads for the staging -> caller copies

@@ -205,8 +205,37 @@ struct PathCtl {
     uint32_t head;              // the next record to scatter
     uint32_t pool_used;         // leaf list entries taken
     uint32_t n_active;          // active pixels
+    uint32_t tape_used;         // adjoint: tape entries handed out
+    uint32_t pad;
 };
 constexpr uint32_t kRoundTickets = 1u << 24;  // tickets of one round: at most 2^31 samples, so 32 bits tell them apart
+
+// What the adjoint's first pass keeps per path (16 bytes): the path's weight
+// dsun . C_sun + dsky . C_sky (NaN: left out), the bits of its lit shadow
+// segments (0-63), and kReplay when the tape does not hold all its decisions.
+struct alignas(16) PathRecord {
+    float w;
+    uint32_t esc_lo, esc_hi, pad;
+};
+constexpr uint32_t kReplay = 1;
+
+// Adjoint runs of the path pipeline: the image gradients (the tile's layout),
+// the path records (by pixel * spp + sample, preset to NaN) and the tape.  A
+// tape entry (two uint4) is one tracking decision: (path, brick sample of the
+// lower corner, flags, denominator), (trilinear fractions, segment value).
+// Flags: bits 0-2 the upper corner differs in x, y, z; bit 3 a shadow segment,
+// whose number is in bits 8-13.  Denominator: the density (a real collision) or
+// minus (majorant - density).  Segment value: a shadow segment's dsun . C, else
+// what the path had added before the segment.
+struct AdjointArgs {
+    const float4 *dsun, *dsky;
+    PathRecord *rec;
+    uint4 *tape;
+    uint32_t tape_cap;        // entries
+    uint32_t *tape_used;      // entries handed out (may exceed the capacity)
+    double *slots;            // albedo gradient, n_slots partial sums
+    uint32_t n_slots;
+};
 
 // Storage of the path pipeline for one launch at a time.
 struct PathWork {

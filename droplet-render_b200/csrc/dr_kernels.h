@@ -47,6 +47,20 @@ cudaError_t launch_transmittance(const DevScene &S, const DevParams &P, const fl
 uint32_t path_list_blocks(uint32_t cols, uint32_t rows);
 // Feature bits a frame needs (0: the plain kernels).
 uint32_t frame_features(const DevScene &S, const DevParams &P);
+// The pipeline's storage in a launch's lists.
+inline PathWork path_work(const CamLists &l) {
+    PathWork W{};
+    W.ctl = l.ctl;
+    W.pool_used = &l.ctl->pool_used;
+    W.n_active = &l.ctl->n_active;
+    W.head = l.head;
+    W.pool = l.pool;
+    W.pool_cap = l.cap;
+    W.active = l.active;
+    W.records = l.records;
+    W.cap = l.rec_cap;
+    return W;
+}
 // Tile render: the path pipeline where the scene has a block grid (and lists.ctl
 // its storage), else the persistent path kernel; Q->next must be 0 (the launcher clears it on st).
 // With a stack traversal and lists given, the camera rays' leaf lists are built
@@ -105,6 +119,18 @@ cudaError_t launch_adjoint_tile(const DevScene &S, const DevParams &P, const Til
                                 const float4 *dsun, const float4 *dsky, float *grad, float *copies_buf,
                                 uint32_t copies, void *records, uint64_t chunk, double *grad_albedo, double *slots,
                                 DevCounters *C, cudaStream_t st);
+// The same on the path pipeline, the decisions kept on a tape (AdjointArgs):
+// chunks are row ranges of the tile (at most 2^23 paths each, records as many),
+// tape holds tape_cap entries of 32 bytes.
+cudaError_t launch_adjoint_tape(const DevScene &S, const DevParams &P, const TileArgs *chunks, uint32_t n_chunks,
+                                const void *mie_pack, const float4 *dsun, const float4 *dsky, float *grad,
+                                float *copies_buf, uint32_t copies, void *records, uint4 *tape, uint32_t tape_cap,
+                                double *grad_albedo, double *slots, DevCounters *C, const PathWork &W, int device,
+                                cudaStream_t st);
+// Its first pass: path records, tape and albedo terms of one chunk.
+cudaError_t launch_paths_adjoint(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
+                                 DevCounters *C, const PathWork &W, const AdjointArgs &J, bool feat, int device,
+                                 cudaStream_t st);
 uint32_t adjoint_slots();
 // Reweighted replay of a tile (decisions from S's bricks, weights from pert):
 // adds the linearised loss to *loss through the zeroed slots.

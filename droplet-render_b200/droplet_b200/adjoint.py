@@ -2,9 +2,9 @@
 
 `render(bricks, albedo, views)` renders every view of one scene with the brick
 samples taken from a CUDA tensor and the single-scatter albedo from a scalar
-tensor; backward runs the GPU adjoint (dr_adjoint_tile_async), which replays
-each path from its random stream (no stored tape) and returns
-dL/d(brick samples) and dL/d(albedo).  The extinction sigma_t of every view is
+tensor; backward runs the GPU adjoint (dr_adjoint_tile_async), which traces
+each path from its random stream, scatters the weights of its tracking
+decisions and returns dL/d(brick samples) and dL/d(albedo).  The extinction sigma_t of every view is
 held fixed: sigma_s = albedo sigma_t, sigma_a = sigma_t - sigma_s.
 
 Images are means over the samples (tile sums / spp), shape (views, h, w, 4)

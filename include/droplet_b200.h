@@ -337,9 +337,12 @@ int dr_get_majorants(dr_ctx *ctx, float *out);
 /* Path-replay adjoint of dr_render_tile(_async) with the same arguments:
  * given dsun_dev / dsky_dev = dL/d(tile sums) (tw*th float4 each, rgb used),
  * ADDS dL/d(brick sample) into grad_bricks_dev (n_leaves * 512 floats) and
- * dL/d(albedo) into *grad_albedo_dev.  Each path is replayed from its own
- * random stream (no stored tape): unbiased for the expected image, with the
- * leaf majorants held fixed.  A path whose contribution is not finite is
+ * dL/d(albedo) into *grad_albedo_dev.  Each path is traced from its own
+ * random stream: unbiased for the expected image, with the leaf majorants held
+ * fixed.  Where the path pipeline serves (leaves at one depth, fewer than 2^23 of
+ * them, at most 2^23 paths in two rows) the decisions go to a tape of up to
+ * 512 MB kept by the context, and paths that do not fit are replayed; without the
+ * memory, and elsewhere, every path is traced twice.  A path whose contribution is not finite is
  * left out.  Enqueued on stream (NULL = context stream). */
 int dr_adjoint_tile_async(dr_ctx *ctx, uint32_t x0, uint32_t y0, uint32_t tw, uint32_t th, uint32_t spp,
                           uint64_t seed, uint64_t sample_base, const float *dsun_dev, const float *dsky_dev,
