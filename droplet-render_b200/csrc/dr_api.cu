@@ -815,11 +815,15 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
         DR_CUDA(c->albedo_slots.reserve(adjoint_slots()), "adjoint: alloc slots");
         DR_CUDA(cudaMemset(c->albedo_slots.p, 0, sizeof(double) * adjoint_slots()), "adjoint: clear slots");
     }
-    // on the path pipeline, in chunks of rows of at most 2^23 paths; the tape has room
-    // for 24 decisions a path up to 512 MB (a path that does not fit is replayed)
+    // on the path pipeline, in chunks of rows.  The tape has room for `per` decisions a
+    // path (a 128^3 cloud at 8 events makes 5, at sigma_t 40 and 16 events 9.5, at
+    // sigma_t 60 and 100 events 17) and 2^25 in all (1 GB); a path that does not fit is
+    // replayed, which costs more than the launches of a further chunk (384 x 384 at 28
+    // samples, sigma_t 40: two replays 43 ms, three chunks with the tape 18 ms)
+    const uint64_t per = 8 + std::min(c->params.scattevs, 24u), most_paths = (1ull << 25) / per;
     const uint64_t row_pair = 2 * (uint64_t)A.cols * spp;
-    if (c->scene.glevels && row_pair && row_pair <= (1ull << 23) && c->scene.n_leaves < (1u << 23)) {
-        const uint32_t rows = (uint32_t)std::min<uint64_t>(A.rows, 2 * ((1ull << 23) / row_pair));
+    if (c->scene.glevels && row_pair && row_pair <= most_paths && c->scene.n_leaves < (1u << 23)) {
+        const uint32_t rows = (uint32_t)std::min<uint64_t>(A.rows, 2 * (most_paths / row_pair));
         std::vector<TileArgs> chunks;
         uint64_t most = 0;
         for (uint32_t r0 = 0; r0 < A.rows; r0 += rows) {
@@ -829,7 +833,7 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
             chunks.push_back(R);
             most = std::max(most, R.n_paths);
         }
-        const uint64_t entries = std::min<uint64_t>(1ull << 24, std::max<uint64_t>(1ull << 16, 24 * most));
+        const uint64_t entries = std::max<uint64_t>(1ull << 16, per * most);
         const CamLists lists = cam_lists(c, kAdjointLists, (size_t)A.cols * A.rows, 0);
         if (lists.ctl && c->path_rec.reserve(most) == cudaSuccess && c->tape.reserve(2 * entries) == cudaSuccess) {
             DR_CUDA(launch_adjoint_tape(c->scene, c->params, chunks.data(), (uint32_t)chunks.size(), c->mie_pack.p,

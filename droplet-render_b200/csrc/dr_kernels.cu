@@ -1344,7 +1344,7 @@ __device__ __forceinline__ void add_pair(float *g, uint32_t x, bool two, bool wi
 // path's record, scattered to the eight brick samples of its lookup.  Bound by the
 // atomics: rows of two samples go out as one vector addition where they lie in an
 // aligned pair or quad (three of four rows: 5 rather than 8 additions on average).
-// 2 million paths, about 3 million decisions (100 MB of tape): 0.16 ms.  A grid of
+// 2 million paths, 10 million decisions (320 MB of tape): 0.16 ms.  A grid of
 // 16 blocks per SM strides over however many entries there are.
 __global__ void __launch_bounds__(256) tape_scatter_kernel(AdjointArgs J, float *grad, uint32_t copies, size_t stride,
                                                            bool wide) {

@@ -340,8 +340,8 @@ int dr_get_majorants(dr_ctx *ctx, float *out);
  * dL/d(albedo) into *grad_albedo_dev.  Each path is traced from its own
  * random stream: unbiased for the expected image, with the leaf majorants held
  * fixed.  Where the path pipeline serves (leaves at one depth, fewer than 2^23 of
- * them, at most 2^23 paths in two rows) the decisions go to a tape of up to
- * 512 MB kept by the context, and paths that do not fit are replayed; without the
+ * them, at most 2^20 paths in two rows) the decisions go to a tape of up to
+ * 1 GB kept by the context, and paths that do not fit are replayed; without the
  * memory, and elsewhere, every path is traced twice.  A path whose contribution is not finite is
  * left out.  Enqueued on stream (NULL = context stream). */
 int dr_adjoint_tile_async(dr_ctx *ctx, uint32_t x0, uint32_t y0, uint32_t tw, uint32_t th, uint32_t spp,

@@ -29,7 +29,7 @@ def _axis_cfg():
     return dict(c0_cfg(33, 33), viewi=viewi.ravel(), sun_dir=np.array([0.0, 1.0, 0.0], np.float32))
 
 
-# deep: more than 64 events a path, and about 10 times the tape's entries
+# deep: more than 64 events a path, and more decisions than the tape holds
 CASES = {
     "no events": (lambda: dict(c0_cfg(64, 64), scattevs=0), (8, 8, 48, 40), 8),
     "one event": (lambda: dict(c0_cfg(64, 64), scattevs=1), (5, 3, 49, 47), 5),
