@@ -1218,10 +1218,18 @@ def run_b200(args):
     cnt = r.counters()
     verts_local = cnt["vertices"]
     t_max, verts = ranks.slowest_and_total(t_local, float(verts_local), device="cuda")
-    # our kernels per timed frame: the camera leaf-list kernel and the
-    # persistent render kernel (stack traversals of the persistent kernel), else one
+    # our kernels per timed frame: with the path pipeline (the resident kernel's
+    # octree traversals) the leaf lists, then a camera and a scatter kernel per
+    # round and one between rounds; a round per filling of the buffer of collided
+    # samples (csrc/dr_paths.cu, launch_rounds), which this frame takes 128 a ticket.
+    # Else one kernel.
     tuned_now = r.get_tuning()
-    launches_per_step = 2 if (tuned_now[0] == 0 and tuned_now[3] != 1) else 1
+    launches_per_step = 1
+    if tuned_now[0] == 0 and tuned_now[3] != 1:
+        cap = min(1 << 25, max(1 << 20, 16 * W_IMG * H_IMG))
+        n_paths, sms = TW * TH * SPP, torch.cuda.get_device_properties(0).multi_processor_count
+        limit = cap if n_paths <= cap else cap - sms * 8 * 4 * 128
+        launches_per_step = 3 * ((n_paths + limit - 1) // limit)
     value = verts / t_max
 
     # end to end through the public blocking API with host buffers (params upload

@@ -3,17 +3,19 @@
 //
 // The reference renders one tile of one view per RenderKernel::Render call
 // (src/kernel.cpp:536-567).  A batch uploads every scene once, lays the paths
-// of all views out as one index space (view-major; inside a view, pixels in
-// the tuned order with consecutive samples), and captures
-//   memset(outputs, queues) -> camera leaf lists of every view
-//     -> persistent kernel over all views -> step counter += 1
-// as a graph.  With a split (dr_batch_set_split), each view of at least
-// min_paths paths gets a plain persistent kernel of its own instead (its
-// parameters in kernel arguments rather than per-lane records in global
-// memory); those kernels and the batched kernel over the remaining views are
-// independent branches between the lists and the step counter, on up to
-// kBranches capture streams, so a kernel's tail overlaps the next one's start.  Launch k of a batch renders samples [k spp, (k+1) spp) of every
-// view, the same streams dr_render_tile draws with sample_base = k spp.
+// of all views out as one index space (view-major; inside a view, pixels with
+// consecutive samples), and captures
+//   memset(outputs, control) -> leaf lists of every view -> tickets
+//     -> camera and scatter kernels over all views, in rounds -> step counter += 1
+// as a graph (csrc/dr_paths.cu), or, with a scene that has no block grid, the
+// persistent kernel over all views.  With a split (dr_batch_set_split), each view
+// of at least min_paths paths gets plain kernels of its own instead (its
+// parameters in kernel arguments rather than per-view records in global
+// memory); those and the batched kernels over the remaining views are
+// independent branches, on up to kBranches capture streams, so a kernel's tail
+// overlaps the next one's start.  Launch k of a batch renders samples
+// [k spp, (k+1) spp) of every view, the same streams dr_render_tile draws with
+// sample_base = k spp.
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -232,7 +234,7 @@ int build_graph(dr_batch *b) {
             Wv.records = W.records + (size_t)(1 + k % nbr) * W.cap;
             const DevScene &S = b->host_scenes[V.scene];
             e = launch_paths(S, V.P, V.A, b->mie_pack.p, V.sun, V.sky, b->ctx->counters.p, Wv,
-                             frame_features(S, V.P) != 0, b->ctx->device, b->branch[k % nbr], b->step.p);
+                             frame_features(S, V.P), b->ctx->device, b->branch[k % nbr], b->step.p);
             continue;
         }
         e = launch_batch_view(b->host_scenes[V.scene], V.P, V.A, b->mie_pack.p, V.sun, V.sky, b->ctx->counters.p,

@@ -141,9 +141,9 @@ struct TileArgs {
     // that escapes after scattering goes to the warp's queue of sky terms and is
     // evaluated 32 at a time (Hosek sky, no whole-path finiteness check).
     uint32_t defer_sky;
-    // Persistent kernel, stack traversals: the camera rays' leaf sequences,
-    // built once per launch by camera_list_kernel (every sample of a pixel
-    // shares its camera ray).  Pixel q = iy * cols + ix: cam_head[2q] = (first
+    // The camera rays' leaf sequences, built once per launch by camera_list_kernel
+    // (persistent kernel, octree traversal) or path_lists_batch_kernel (a batch on
+    // the path pipeline); every sample of a pixel shares its camera ray.  Pixel q = iy * cols + ix: cam_head[2q] = (first
     // entry in cam_pool, leaves, node visits of the root test, node visits
     // after the last leaf), or x = ~0 when the pixel's list did not fit (its
     // samples traverse); cam_head[2q + 1] = (the ray's direction bits, 1 if the

@@ -1652,7 +1652,7 @@ cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, cons
     size_t smem = mie_smem(P);
     const uint32_t feat = frame_features(S, P);
     if (paths_serve(tune, S.glevels) && lists.ctl) {
-        return launch_paths(S, P, A, mie_pack, sun_out, sky_out, C, path_work(lists), feat != 0, device, st);
+        return launch_paths(S, P, A, mie_pack, sun_out, sky_out, C, path_work(lists), feat, device, st);
     }
     // sky terms evaluated by full warps (Hosek sky only; a whole-path
     // finiteness check needs the path's sky sum in place)
@@ -1855,7 +1855,7 @@ cudaError_t launch_adjoint_tape(const DevScene &S, const DevParams &P, const Til
         const size_t off = (size_t)(A.y0 - chunks[0].y0) * A.tw;
         const AdjointArgs J{dsun + off, dsky + off, (PathRecord *)records, tape, tape_cap, &W.ctl->tape_used, slots, kSlots};
         e = cudaMemsetAsync(records, 0xff, sizeof(PathRecord) * A.n_paths, st);
-        if (e == cudaSuccess) e = launch_paths_adjoint(S, P, A, mie_pack, C, W, J, feat != 0, device, st);
+        if (e == cudaSuccess) e = launch_paths_adjoint(S, P, A, mie_pack, C, W, J, feat, device, st);
         if (e != cudaSuccess) break;
         tape_scatter_kernel<<<2368, 256, 0, st>>>(J, to, nc, stride, ((uintptr_t)to & 15u) == 0u);
         replay<<<(unsigned)((A.n_paths + kRenderBlock - 1) / kRenderBlock), kRenderBlock, smem, st>>>(

@@ -31,12 +31,12 @@ bool paths_serve(const Tuning &tune, uint32_t glevels);
 // The path pipeline of a tile.  feat: the frame needs the optional features.
 // step: a batch's launch counter (its view's samples start at A.sample_base + *step * spp), or null.
 cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
-                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &W, bool feat, int device,
+                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &W, uint32_t feat, int device,
                          cudaStream_t st, const unsigned long long *step = nullptr);
 // The path pipeline of every view of B (their TileArgs::cam_head set); n_paths:
 // their samples, n_blocks: the sum of their path_list_blocks.
 cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                               const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool feat, uint32_t glevels,
+                               const PathWork &W, uint64_t n_paths, uint32_t n_blocks, bool ext, uint32_t glevels,
                                int device, cudaStream_t st);
 // The shadow pass and transmittance estimates on a scene with a block grid.
 cudaError_t launch_shadow_paths(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out,
@@ -129,7 +129,7 @@ cudaError_t launch_adjoint_tape(const DevScene &S, const DevParams &P, const Til
                                 cudaStream_t st);
 // Its first pass: path records, tape and albedo terms of one chunk.
 cudaError_t launch_paths_adjoint(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
-                                 DevCounters *C, const PathWork &W, const AdjointArgs &J, bool feat, int device,
+                                 DevCounters *C, const PathWork &W, const AdjointArgs &J, uint32_t feat, int device,
                                  cudaStream_t st);
 uint32_t adjoint_slots();
 // Reweighted replay of a tile (decisions from S's bricks, weights from pert):

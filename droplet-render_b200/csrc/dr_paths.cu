@@ -834,33 +834,54 @@ enum : int { wPath = 25, wASun = 26, wEsc = 29 };
 template <bool BATCH, bool ADJ = false> __host__ __device__ constexpr int slot_words() {
     return ADJ ? 31 : (BATCH ? 26 : 25);
 }
-template <bool BATCH, bool ADJ = false> __host__ __device__ constexpr int skyq_words() {
-    return ADJ ? 0 : (BATCH ? 8 : 7) * 32;
+// The light queue's words an entry: the direction, a throughput, the output offset,
+// and with features the origin and kind; in a batch the view.
+template <uint32_t FEAT, bool BATCH, bool ADJ = false> __host__ __device__ constexpr int queue_words() {
+    return ADJ || (FEAT && !(FEAT & kFeatOcc)) ? 0 : (FEAT ? 11 : 7) + (BATCH ? 1 : 0);
 }
 // bytes per warp: slots, three lists of slot numbers, the sky queue
-template <bool BATCH, bool ADJ = false> __host__ __device__ constexpr size_t scatter_warp_bytes() {
-    return 4 * (size_t)(slot_words<BATCH, ADJ>() * kSlots + skyq_words<BATCH, ADJ>()) + 3 * (size_t)kSlots;
+template <uint32_t FEAT, bool BATCH, bool ADJ = false> __host__ __device__ constexpr size_t scatter_warp_bytes() {
+    return 4 * (size_t)(slot_words<BATCH, ADJ>() * kSlots + 32 * queue_words<FEAT, BATCH, ADJ>()) + 3 * (size_t)kSlots;
 }
 
 // The sky terms of escaped paths are evaluated by full warps: entry i of the
-// queue is (rd, T, output offset[, view]) in column i; T * sky(rd) is the value
-// the path would have added in place (its sky sum is 0 before the escape).
-template <bool BATCH>
-__device__ __noinline__ void path_sky_eval(const DevParams &P, float4 *sky_out, const BatchArgs &B, const float *q,
-                                              uint32_t i) {
+// queue is (rd, T, output offset, [ro, kind,] [view]) in column i; T * sky(rd) is
+// the value the path would have added in place (its sky sum is 0 before the
+// escape).  With occluders the light of lit shadow segments and escapes waits
+// there too (kShadowLight: T is the segment's sun term; kEscapeLight: sun and sky),
+// so that full warps test the rays: tested where 8 to 14 of a warp's segments end,
+// the dependent loads of the tree, which the path slots leave little L1 for, took
+// half the frame (640 x 360, 32 samples, 402 triangles: 1.57 -> 1.26 ms; 0.79 without
+// occluders).
+enum : uint32_t { kSkyLight = 0, kShadowLight = 1, kEscapeLight = 2 };
+template <uint32_t FEAT, bool BATCH>
+__device__ __noinline__ void path_light_eval(const DevScene &S0, const DevParams &P0, float4 *sun0, float4 *sky0,
+                                             const BatchArgs &B, const float *q, uint32_t i) {
+    const BatchView *V = nullptr;
+    if constexpr (BATCH) V = &B.views[__float_as_uint(q[32 * (queue_words<FEAT, BATCH>() - 1) + i])];
+    const DevParams &P = BATCH ? V->P : P0;
     const float rd[3] = {q[i], q[32 + i], q[64 + i]};
-    float3 sky;
-    float4 *out;
-    if constexpr (BATCH) {
-        const BatchView &V = B.views[__float_as_uint(q[224 + i])];
-        sky = escape_sky<0>(V.P, rd);
-        out = V.sky;
-    } else {
-        sky = escape_sky<0>(P, rd);
-        out = sky_out;
+    const float T[3] = {q[96 + i], q[128 + i], q[160 + i]};
+    const uint32_t off = __float_as_uint(q[192 + i]);
+    uint32_t kind = kSkyLight;
+    if constexpr (FEAT != 0) {
+        kind = __float_as_uint(q[320 + i]);
+        const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+        if (kind != kSkyLight) {
+            const float ro[3] = {q[224 + i], q[256 + i], q[288 + i]};
+            if (occluded(S, ro, rd)) return;
+            float c[3] = {T[0], T[1], T[2]};
+            if (kind == kEscapeLight) {
+                const bool hit = sun_hit(P, rd);
+                for (int k = 0; k < 3; ++k) c[k] = T[k] * (hit ? P.sun_color[k] : 0.0f);
+            }
+            if ((c[0] != 0.0f) | (c[1] != 0.0f) | (c[2] != 0.0f))
+                atomicAdd(&(BATCH ? V->sun : sun0)[off], make_float4(c[0], c[1], c[2], 0.0f));
+            if (kind == kShadowLight) return;
+        }
     }
-    atomicAdd(&out[__float_as_uint(q[192 + i])],
-              make_float4(q[96 + i] * sky.x, q[128 + i] * sky.y, q[160 + i] * sky.z, 0.0f));
+    const float3 e = escape_sky<FEAT>(P, rd);
+    atomicAdd(&(BATCH ? V->sky : sky0)[off], make_float4(T[0] * e.x, T[1] * e.y, T[2] * e.z, 0.0f));
 }
 
 __device__ __forceinline__ float dot_rgb(const float4 a, const float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
@@ -875,8 +896,8 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                                                                       const void *mie_pack, float4 *sun0, float4 *sky0,
                                                                       DevCounters *C, const __grid_constant__ BatchArgs B,
                                                                       uint32_t colwords,
-                                                                      uint32_t defer,
                                                                       const __grid_constant__ AdjointArgs J) {
+    constexpr bool kQueued = queue_words<FEAT, BATCH, ADJ>() != 0;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t mbar;
     if (W.ctl->records == 0u) return;  // a round without records: leave before staging
@@ -891,13 +912,13 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
     unsigned char *const area = smem + ((mb + 15u) & ~15u);
     float *const col = reinterpret_cast<float *>(area) + threadIdx.x;
     float *const slots = reinterpret_cast<float *>(area + (size_t)colwords * 4u * kScatterBlock +
-                                                   (threadIdx.x >> 5) * scatter_warp_bytes<BATCH, ADJ>());
-    float *const skyq = slots + slot_words<BATCH, ADJ>() * kSlots;
-    uint8_t *const lists = reinterpret_cast<uint8_t *>(skyq + skyq_words<BATCH, ADJ>());
+                                                   (threadIdx.x >> 5) * scatter_warp_bytes<FEAT, BATCH, ADJ>());
+    float *const queue = slots + slot_words<BATCH, ADJ>() * kSlots;
+    uint8_t *const lists = reinterpret_cast<uint8_t *>(queue + 32 * queue_words<FEAT, BATCH, ADJ>());
 #define ready(i) lists[i]
 #define event(i) lists[kSlots + (i)]
 #define freed(i) lists[2 * kSlots + (i)]
-    uint32_t n_ready = 0, n_event = 0, n_free = kSlots, n_sky = 0;
+    uint32_t n_ready = 0, n_event = 0, n_free = kSlots, n_queue = 0;
     for (uint32_t i = lane; i < (uint32_t)kSlots; i += 32) freed(i) = (uint8_t)i;
     __syncwarp();
     bool more = true;
@@ -927,15 +948,31 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         // ---- segment ends, and idle lanes with segments ready
         const uint32_t due = (uint32_t)__popc(endm) + min((uint32_t)__popc(idle), n_ready);
         if (due && (due >= kEndBatch || !busy)) {
-            bool init = false, finish = false, sky = false;
+            bool init = false, finish = false, queued = false;
+            uint32_t kind = kSkyLight;
             bool to_event = false;
-            float T[3] = {0.f, 0.f, 0.f};
+            float T[3] = {0.f, 0.f, 0.f}, qd[3] = {0.f, 0.f, 0.f};  // the queue entry (qd: rd may be the next segment's)
             const BatchView *V = BATCH ? &B.views[view] : nullptr;
             const DevParams &P = BATCH ? V->P : P0;
             const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+            // the queue takes light as it comes; whole-path sums are needed where a path
+            // that is not finite is left out, and for the adjoint.  With features but no
+            // occluders the light is cheaper in place (640 x 360, 32 samples, HG phase: no
+            // environment 0.72 ms a frame in place and 0.81 queued, a map 0.79 and 0.82; a
+            // kernel that has both ways takes 0.81 and 0.88)
+            const bool occ = (FEAT & kFeatOcc) && P.embree && S.occ_nodes;
+            const bool later = kQueued && !P.finite_paths;
             if (st == kEnd) {
                 if (shadow) {
-                    if (res == kTrackEscaped && !((FEAT & kFeatOcc) && P.embree && occluded(S, ro, rd))) {
+                    if (res == kTrackEscaped && occ && later) {
+                        queued = true;
+                        kind = kShadowLight;
+                        const bool hit = sun_hit(P, rd);
+                        for (int k = 0; k < 3; ++k) {
+                            T[k] = SLOT(wSw + k, slot) * (hit ? P.sun_color[k] : 0.0f);
+                            qd[k] = rd[k];
+                        }
+                    } else if (res == kTrackEscaped && !(occ && occluded(S, ro, rd))) {
                         const bool hit = sun_hit(P, rd);
                         for (int k = 0; k < 3; ++k) {
                             const float c = SLOT(wSw + k, slot) * (hit ? P.sun_color[k] : 0.0f);
@@ -968,20 +1005,25 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                 } else {
                     float4 sun = make_float4(SLOT(wSun, slot), SLOT(wSun + 1, slot), SLOT(wSun + 2, slot), 0.0f);
                     float4 skyv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (res == kTrackEscaped && !((FEAT & kFeatOcc) && P.embree && occluded(S, ro, rd))) {
-                        const bool hit = sun_hit(P, rd);
+                    const bool test = occ && later;  // by the queue
+                    if (res == kTrackEscaped && (test || !(occ && occluded(S, ro, rd)))) {
                         for (int k = 0; k < 3; ++k) T[k] = SLOT(wT + k, slot);
-                        sun.x = sun.x + T[0] * (hit ? P.sun_color[0] : 0.0f);
-                        sun.y = sun.y + T[1] * (hit ? P.sun_color[1] : 0.0f);
-                        sun.z = sun.z + T[2] * (hit ? P.sun_color[2] : 0.0f);
-                        const bool later = !ADJ && (BATCH ? V->A.defer_sky != 0u : defer != 0u);
-                        if constexpr (ADJ) {
-                            const float m = (float)__float_as_uint(SLOT(wEv, slot));
-                            for (int k = 0; k < 3; ++k)
-                                SLOT(wASun + k, slot) = SLOT(wASun + k, slot) + m * (T[k] * (hit ? P.sun_color[k] : 0.0f));
+                        if (!test) {
+                            const bool hit = sun_hit(P, rd);
+                            sun.x = sun.x + T[0] * (hit ? P.sun_color[0] : 0.0f);
+                            sun.y = sun.y + T[1] * (hit ? P.sun_color[1] : 0.0f);
+                            sun.z = sun.z + T[2] * (hit ? P.sun_color[2] : 0.0f);
+                            if constexpr (ADJ) {
+                                const float m = (float)__float_as_uint(SLOT(wEv, slot));
+                                for (int k = 0; k < 3; ++k)
+                                    SLOT(wASun + k, slot) = SLOT(wASun + k, slot) + m * (T[k] * (hit ? P.sun_color[k] : 0.0f));
+                            }
                         }
-                        if (FEAT == 0 && later) {
-                            sky = true;
+                        if (later) {
+                            queued = true;
+                            kind = test ? kEscapeLight : kSkyLight;
+                            if constexpr (FEAT != 0)
+                                for (int k = 0; k < 3; ++k) qd[k] = rd[k];
                         } else {
                             const float3 e = escape_sky<FEAT>(P, rd);
                             skyv.x = T[0] * e.x;
@@ -1018,27 +1060,29 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                     finish = true;
                 }
             }
-            if constexpr (FEAT == 0 && !ADJ) {  // the sky terms go to the warp's queue, evaluated 32 at a time
-                const uint32_t sm = __ballot_sync(kFull, sky);
-                if (sm) {
-                    const uint32_t pos = n_sky + __popc(sm & lt), total = n_sky + __popc(sm);
-                    const uint32_t off = sky ? __float_as_uint(SLOT(wOff, slot)) : 0u;
+            if constexpr (kQueued) {  // to the warp's queue, evaluated 32 at a time
+                const uint32_t qm = __ballot_sync(kFull, queued);
+                if (qm) {
+                    const uint32_t pos = n_queue + __popc(qm & lt), total = n_queue + __popc(qm);
+                    const uint32_t off = queued ? __float_as_uint(SLOT(wOff, slot)) : 0u;
                     for (uint32_t pass = 0; pass < 2; ++pass) {
                         const uint32_t p = pos - 32u * pass;
-                        if (sky && (pass ? pos >= 32u : pos < 32u)) {
+                        if (queued && (pass ? pos >= 32u : pos < 32u)) {
                             for (int k = 0; k < 3; ++k) {
-                                skyq[32 * k + p] = rd[k];
-                                skyq[96 + 32 * k + p] = T[k];
+                                queue[32 * k + p] = FEAT != 0 ? qd[k] : rd[k];
+                                queue[96 + 32 * k + p] = T[k];
+                                if constexpr (FEAT != 0) queue[224 + 32 * k + p] = ro[k];
                             }
-                            skyq[192 + p] = __uint_as_float(off);
-                            if constexpr (BATCH) skyq[224 + p] = __uint_as_float(view);
+                            queue[192 + p] = __uint_as_float(off);
+                            if constexpr (FEAT != 0) queue[320 + p] = __uint_as_float(kind);
+                            if constexpr (BATCH) queue[32 * (queue_words<FEAT, BATCH>() - 1) + p] = __uint_as_float(view);
                         }
                         __syncwarp();
                         if (pass == 1 || total < 32u) break;
-                        path_sky_eval<BATCH>(P0, sky0, B, skyq, lane);
+                        path_light_eval<FEAT, BATCH>(S0, P0, sun0, sky0, B, queue, lane);
                         __syncwarp();
                     }
-                    n_sky = total & 31u;
+                    n_queue = total & 31u;
                 }
             }
             const uint32_t em = __ballot_sync(kFull, to_event), fm = __ballot_sync(kFull, finish);
@@ -1267,10 +1311,9 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
         tape.mark(lane);
         return;
     }
-    if constexpr (FEAT == 0) {
-        __syncwarp();
-        if (lane < n_sky) path_sky_eval<BATCH>(P0, sky0, B, skyq, lane);
-    }
+    __syncwarp();
+    if constexpr (kQueued)
+        if (lane < n_queue) path_light_eval<FEAT, BATCH>(S0, P0, sun0, sky0, B, queue, lane);
     cnt.vertices = 2u * scatters;  // every event's shadow and continuation segments
     cnt.mie_evals = 3u * scatters;
     warp_sum_counts(cnt, C, 0u);
@@ -1295,7 +1338,7 @@ static uint64_t rounds_of(uint64_t n_paths, uint64_t limit, uint32_t ticket) {
 using CameraFn = void (*)(DevScene, DevParams, TileArgs, PathWork, float4 *, float4 *, DevCounters *, BatchArgs,
                           AdjointArgs);
 using ScatterFn = void (*)(DevScene, DevParams, TileArgs, PathWork, const void *, float4 *, float4 *, DevCounters *,
-                           BatchArgs, uint32_t, uint32_t, AdjointArgs);
+                           BatchArgs, uint32_t, AdjointArgs);
 
 constexpr int kScatterBlocks = 4;  // resident scatter blocks per SM the kernel is compiled for
 
@@ -1303,18 +1346,25 @@ constexpr int kScatterBlocks = 4;  // resident scatter blocks per SM the kernel 
 template <bool BATCH, bool ADJ>
 static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const TileArgs &A, const BatchArgs &B,
                                  PathWork W, const void *mie_pack, float4 *sun, float4 *sky, DevCounters *C,
-                                 bool feat, uint32_t glevels, uint64_t n_paths, uint32_t defer, int device,
+                                 uint32_t feat, uint32_t glevels, uint64_t n_paths, int device,
                                  cudaStream_t st, const AdjointArgs &J = {}) {
     int sms = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
     const CameraFn cam = feat ? camera_paths_kernel<kFeatAll, BATCH, ADJ> : camera_paths_kernel<0, BATCH, ADJ>;
-    const ScatterFn sca = feat ? scatter_kernel<kFeatAll, BATCH, kScatterBlocks, ADJ>
-                               : scatter_kernel<0, BATCH, kScatterBlocks, ADJ>;
+    // a batch's scenes have no occluders, and the adjoint has one kernel with features
+    constexpr uint32_t kOcc = BATCH ? kFeatAll & ~kFeatOcc : kFeatAll, kNoOcc = ADJ ? kFeatAll : kFeatAll & ~kFeatOcc;
+    const bool occ = (feat & kFeatOcc) != 0;
+    const ScatterFn sca = !feat ? scatter_kernel<0, BATCH, kScatterBlocks, ADJ>
+                          : occ ? scatter_kernel<kOcc, BATCH, kScatterBlocks, ADJ>
+                                : scatter_kernel<kNoOcc, BATCH, kScatterBlocks, ADJ>;
     const uint32_t words = grid_words(glevels);
     const size_t cam_smem = (size_t)words * 4 * kListBlock;
     const size_t sca_smem = ((table_bytes(P) + 15) & ~(size_t)15) + (size_t)words * 4 * kScatterBlock +
-                            scatter_warp_bytes<BATCH, ADJ>() * (kScatterBlock / 32);
+                            (!feat ? scatter_warp_bytes<0, BATCH, ADJ>()
+                             : occ ? scatter_warp_bytes<kOcc, BATCH, ADJ>()
+                                   : scatter_warp_bytes<kNoOcc, BATCH, ADJ>()) *
+                                (kScatterBlock / 32);
     e = opt_in(sca, sca_smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -1339,7 +1389,7 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
     for (uint64_t r = 0; r < rounds; ++r) {
         if (r) next_round_kernel<<<1, 1, 0, st>>>(W.ctl);
         cam<<<cam_blocks, kListBlock, cam_smem, st>>>(S, P, A, W, sun, sky, C, B, J);
-        sca<<<sca_blocks, kScatterBlock, sca_smem, st>>>(S, P, A, W, mie_pack, sun, sky, C, B, words, defer, J);
+        sca<<<sca_blocks, kScatterBlock, sca_smem, st>>>(S, P, A, W, mie_pack, sun, sky, C, B, words, J);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1392,7 +1442,7 @@ uint32_t path_list_blocks(uint32_t cols, uint32_t rows) {
 }
 
 cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
-                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &storage, bool feat, int device,
+                         float4 *sun, float4 *sky, DevCounters *C, const PathWork &storage, uint32_t feat, int device,
                          cudaStream_t st, const unsigned long long *step) {
     const uint64_t n_paths = (uint64_t)A.cols * A.rows * A.spp;
     if (n_paths == 0) return cudaSuccess;
@@ -1407,11 +1457,11 @@ cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &
     BatchArgs B{};
     B.step = step;
     return launch_rounds<false, false>(S, P, A, B, W, mie_pack, sun, sky, C, feat, S.glevels, n_paths,
-                                (!feat && !P.finite_paths) ? 1u : 0u, device, st);
+                                       device, st);
 }
 
 cudaError_t launch_paths_adjoint(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
-                                 DevCounters *C, const PathWork &storage, const AdjointArgs &J, bool feat, int device,
+                                 DevCounters *C, const PathWork &storage, const AdjointArgs &J, uint32_t feat, int device,
                                  cudaStream_t st) {
     if (A.n_paths == 0) return cudaSuccess;
     PathWork W = storage;
@@ -1423,11 +1473,11 @@ cudaError_t launch_paths_adjoint(const DevScene &S, const DevParams &P, const Ti
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_rounds<false, true>(S, P, A, BatchArgs{}, W, mie_pack, nullptr, nullptr, C, feat, S.glevels, A.n_paths,
-                                      0u, device, st, J);
+                                      device, st, J);
 }
 
 cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const void *mie_pack, DevCounters *C,
-                               const PathWork &storage, uint64_t n_paths, uint32_t n_blocks, bool feat,
+                               const PathWork &storage, uint64_t n_paths, uint32_t n_blocks, bool ext,
                                uint32_t glevels, int device, cudaStream_t st) {
     if (n_paths == 0) return cudaSuccess;
     PathWork W = storage;
@@ -1439,8 +1489,9 @@ cudaError_t launch_paths_batch(const BatchArgs &B, const DevParams &P0, const vo
     view_tickets_kernel<<<1, 32, 0, st>>>(B, W);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_rounds<true, false>(DevScene{}, P0, TileArgs{}, B, W, mie_pack, nullptr, nullptr, C, feat, glevels, n_paths,
-                               0u, device, st);
+    return launch_rounds<true, false>(DevScene{}, P0, TileArgs{}, B, W, mie_pack, nullptr, nullptr, C,
+                                      ext ? kFeatExt | kFeatSdf : 0u, glevels, n_paths,
+                                      device, st);
 }
 
 }  // namespace dr

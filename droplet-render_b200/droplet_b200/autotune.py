@@ -1,14 +1,16 @@
 """Launch-shape autotuner for the persistent path kernel (single frames and batches).
 
-The persistent kernel has seven knobs (`dr_tuning`):
+Octrees with their leaves at one depth (every scene the builder makes) render on
+the path pipeline, which has no launch shape: there the knobs below change nothing
+except for the cell walk and the kernel family, both slower.  Elsewhere the
+persistent kernel has seven knobs (`dr_tuning`):
 * the compiled variant, i.e. resident blocks per SM. 4/5/6/8 trade registers for
   occupancy; the smaller register budgets spill a little to L1-resident local memory.
 * the event batch: how many lanes of a warp must be waiting on a segment end before
   the warp shades them.
-* the traversal: octree descent with a node stack in local memory or in shared
-  memory (octrees that keep their leaves at one depth; otherwise the library uses
-  the local stack), or the cell walk over the leaf grid (faster where
-  leaves are dense along rays, slower through wide empty regions).
+* the traversal: octree descent (0 and 2 are the same here), or the cell walk over
+  the leaf grid (faster where leaves are dense along rays, slower through wide
+  empty regions).
 * the tile: pixels handed out row-major or square by square (ray coherence).
 * the work per loop iteration: how many octree nodes the stack traversal examines
   (0: up to the next leaf) and how many free-flight steps a lane takes before the
@@ -28,8 +30,7 @@ import time
 
 from . import _native as N
 
-# occupancy x event batch for both stacks: their best occupancies differ (the
-# shared-memory stack frees local memory, so more resident blocks pay)
+# occupancy x event batch
 STAGE1 = [(0, bps, batch, trav, 0, 0, 0) for trav in (0, 2) for bps in (4, 5, 6, 8) for batch in (8, 16, 24)]
 PER_PATH = (1, 0, 0, 0, 0, 0, 0)
 

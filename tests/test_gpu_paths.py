@@ -5,7 +5,7 @@ equal.  The per-path kernel is pinned to the CPU restatement elsewhere."""
 import numpy as np
 import pytest
 
-from conftest import c0_cfg, depth_texture, golden_octree, settings_from_cfg
+from conftest import c0_cfg, depth_texture, golden_octree, occluder_surfaces, settings_from_cfg
 from droplet_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
@@ -129,3 +129,17 @@ def test_transmittance_of_long_leaf_lists():
         got = r.probe_transmittance(ro, rd, 1000, seed=5)
         _, ref = r.adjoint_transmittance(ro, rd, np.ones(2), 1000, 5, oc.n_leaves)
         assert np.array_equal(got, ref) and got.min() < 1.0
+
+
+@pytest.mark.parametrize("flags", [{"embree": True}, {"embree": True, "finite_paths": True}, {"embree": False}])
+@pytest.mark.parametrize("tile,spp", [((30, 30, 2, 2), 1), ((9, 14, 17, 9), 33), ((2, 2, 60, 60), 40)])
+def test_occluder_light(flags, tile, spp):
+    """The light of lit shadow segments and escapes, tested against the occluders in
+    the warp's queue (embree), in place (finite_paths) or not at all."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    with Renderer(0) as r:
+        r.set_occluders(occluder_surfaces())
+        r.upload(Octree(*golden_octree()))
+        _check(_pair(r, dict(c0_cfg(64, 64), **flags), tile, spp))
