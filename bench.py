@@ -445,15 +445,14 @@ def profile_lines(name: str) -> dict:
 
 def profiled_l2():
     """L2 figures of the render kernel from the committed ncu summary
-    (profiles/render_persistent_kernel_c1.md, lines "l2_throughput_pct: X" and
+    (profiles/path_pipeline_c1.md, lines "l2_throughput_pct: X" and
     "lts_hit_rate: X")."""
-    p = os.path.join(ROOT, "profiles", "render_persistent_kernel_c1.md")
+    p = os.path.join(ROOT, "profiles", "path_pipeline_c1.md")
     out = {}
     try:
         with open(p) as f:
             for line in f:
-                for key in ("l2_throughput_pct", "lts_hit_rate", "alu_pipe_pct", "issue_active_pct",
-                            "lanes_per_instruction"):
+                for key in ("l2_throughput_pct", "lts_hit_rate", "issue_active_pct", "lanes_per_instruction"):
                     if line.startswith(key + ":"):
                         out[key] = float(line.split(":")[1])
     except Exception:
@@ -464,10 +463,10 @@ def profiled_l2():
 def profiled_traffic():
     """DRAM bytes of one full-frame render launch (dram__bytes_read.sum +
     dram__bytes_write.sum) from the committed ncu summary
-    (profiles/render_persistent_kernel_c1.md, lines "dram_bytes_per_frame: X",
+    (profiles/path_pipeline_c1.md, lines "dram_bytes_per_frame: X",
     "frame_tuning: ..." and "source_sha16: ..."), used only when it measured
     this build's sources."""
-    kv = profile_lines("render_persistent_kernel_c1.md")
+    kv = profile_lines("path_pipeline_c1.md")
     if "dram_bytes_per_frame" not in kv:
         return None
     return {"bytes": float(kv["dram_bytes_per_frame"]), "source_sha16": kv.get("source_sha16"),
@@ -1275,7 +1274,7 @@ def run_b200(args):
                 "peak_kind": peak_kind,
                 "traffic": traffic["bytes"] if usable else None,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one full-frame launch "
-                                  "(profiles/render_persistent_kernel_c1.md)"
+                                  "(profiles/path_pipeline_c1.md)"
                                   + (f"; captured at tuning {traffic['tuning']}, this run {tuned}" if usable else
                                      "; not used: " + ("no capture" if not traffic else "captured on other sources")),
                 "algorithmic_bytes_per_vertex": b_v,
@@ -1287,16 +1286,15 @@ def run_b200(args):
         roofline["l2"] = {"frac": l2.get("l2_throughput_pct", float("nan")) / 100.0,
                           "lts_hit_rate": l2.get("lts_hit_rate"),
                           "source": "ncu L2 throughput (% of peak) and lts__t_sector_hit_rate.pct on a 512^2 crop "
-                                    "launch (profiles/render_persistent_kernel_c1.md)"}
-        # the roof that binds: instruction issue on the ALU pipe (compares,
-        # selects and integer work of the octree traversal), same capture
-        if "alu_pipe_pct" in l2:
-            roofline["issue"] = {"alu_pipe_frac": l2["alu_pipe_pct"] / 100.0,
-                                 "issue_active_frac": l2.get("issue_active_pct", float("nan")) / 100.0,
+                                    "launch (profiles/path_pipeline_c1.md)"}
+        # what binds the scatter kernel: its warps' own latency (cycles that issue and
+        # lanes per instruction), same capture
+        if "issue_active_pct" in l2:
+            roofline["issue"] = {"issue_active_frac": l2["issue_active_pct"] / 100.0,
                                  "lanes_per_instruction": l2.get("lanes_per_instruction"),
-                                 "source": "ncu sm__inst_executed_pipe_alu, smsp__issue_active and "
+                                 "source": "ncu smsp__issue_active and "
                                            "smsp__thread_inst_executed_per_inst_executed on the same 512^2 crop "
-                                           "launch (profiles/render_persistent_kernel_c1.md)"}
+                                           "launch (profiles/path_pipeline_c1.md)"}
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
@@ -1318,7 +1316,7 @@ def run_b200(args):
     c0 = None
     if rank == 0 and world == 1 and not args.no_c0:
         c0 = measure_c0(r, pdf, cdf, cfgs, rads, steps=max(3, args.steps), warmup=max(3, args.warmup),
-                        cpu=not args.no_cpu)
+                        cpu=not args.no_cpu and bool(cpu and cpu.get("value")))  # the reference oracle needs oracle/_ref
         r.upload(Octree(nodes, bricks, mlevel))
         r.set_params(settings)
         log(f"c0: gpu {c0['gpu']['value'] / 1e9:.3f} G/s ({c0['gpu']['ms_per_frame']:.3f} ms/frame), "
