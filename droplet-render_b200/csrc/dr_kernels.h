@@ -26,7 +26,9 @@ struct CamLists {
     uint32_t rec_cap = 0;
 };
 // Whether the path pipeline (dr_paths.cu) serves launches with this tuning:
-// scenes with a block grid, unless the cell walk is asked for.
+// scenes with a block grid, unless the cell walk is asked for.  No size is left to
+// the persistent kernel: a 64 x 64 tile at 16 samples takes 0.31 ms against 0.38, a
+// 1920 x 1080 frame at 64 samples 16.3 against 37.5.
 bool paths_serve(const Tuning &tune, uint32_t glevels);
 // The path pipeline of a tile.  feat: the frame needs the optional features.
 // step: a batch's launch counter (its view's samples start at A.sample_base + *step * spp), or null.

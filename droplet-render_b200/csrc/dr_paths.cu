@@ -14,9 +14,9 @@
 // 119 M meet no leaf at all and about 5 M collide), those are coherent, and the
 // rest is not.  One kernel for all three (render_persistent_kernel, which
 // serves the octrees without a block grid) was bound by instruction issue at 8
-// of 32 lanes per instruction: 38.5 ms for that frame at 64 samples, 51.9 ms for a
-// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 18.3 and 19.2 ms:
-// lists 0.26, camera 2.4, scatter 15.5 ms of the first, at 13 lanes per instruction.
+// of 32 lanes per instruction: 37.5 ms for that frame at 64 samples, 55.3 ms for a
+// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 16.3 and 21.2 ms:
+// lists 0.26, camera 2.4, scatter 13.5 ms of the first, at 13 lanes per instruction.
 //
 // Per path, the operations and random draws are those of path_sample(): a
 // path's result does not depend on the kernel that computed it.
@@ -480,7 +480,8 @@ __device__ __forceinline__ void active_sample(const TileArgs &A, const uint32_t 
 // (W.limit = capacity - warps * W.ticket), so the buffer never overflows and the
 // tickets taken are exactly those done: the next round goes on from there.
 // ADJ: the adjoint's first pass (the samples of pixels without a gradient are
-// left out, nothing is counted or added to an image).
+// left out, nothing is counted or added to an image).  8 blocks per SM: 5 to 8 are
+// within 1% of each other (headline frame 17.7 to 17.9 ms, slab 17.4 to 17.6).
 template <uint32_t FEAT, bool BATCH, bool ADJ>
 __global__ void __launch_bounds__(kListBlock, ADJ ? 6 : 8) camera_paths_kernel(const __grid_constant__ DevScene S0,
                                                                      const __grid_constant__ DevParams P0,
@@ -599,6 +600,10 @@ __global__ void __launch_bounds__(kListBlock, ADJ ? 6 : 8) camera_paths_kernel(c
 // 32 samples side by side walk the grid together like camera samples.  Resident
 // warps loop over the samples: a warp's counters cost six additions to the same
 // words whatever it did, and with a warp per 32 samples those were the bound.
+// 960 x 540 at 16 samples: 0.76 ms, 0.98 with a thread per sample on the octree; bound
+// by the setup of the samples (48% of cycles issue).  Lanes that take a new sample
+// when theirs ends made it 1.41 to 1.55 ms (8 to 24 idle lanes at a time): the setup
+// then runs at those few lanes.
 template <uint32_t FEAT>
 __global__ void __launch_bounds__(kListBlock, 8) shadow_paths_kernel(const __grid_constant__ DevScene S,
                                                                      const __grid_constant__ DevParams P,
