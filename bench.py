@@ -1119,7 +1119,12 @@ def run_reference(args):
     cfg = frame_cfg(pdf, cdf, cfgs, rads)
     nodes, bricks, mlevel, occ = build_scene("oracle")
     threads = os.cpu_count() or 1
-    times = cpu_reference_times(nodes, bricks, cfg, threads, steps=max(1, args.steps), warmup=min(args.warmup, 1))
+    try:
+        times = cpu_reference_times(nodes, bricks, cfg, threads, steps=max(1, args.steps), warmup=min(args.warmup, 1))
+    except FileNotFoundError:
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref is not built (its sources are needed: "
+                                                              "make -C oracle ref)"}))
+        return 0
     verts = port_vertices(nodes, bricks, cfg, threads)
     dt = float(np.mean(times))
     value = verts / dt
