@@ -1550,12 +1550,18 @@ static size_t mie_smem(const DevParams &P) {
     return (size_t)P.mie_n * 20u + (P.phase_mode == 1u ? (2u * (size_t)P.mie_n + 1u) * 16u : 0u);
 }
 
-// Dynamic shared memory above the default 48 KB (phase tables of more than
-// about 2,400 entries) needs the kernel's opt-in, up to the 227 KB a block can have.
-template <class F> static cudaError_t allow_smem(F fn, size_t smem) {
+cudaError_t raise_smem(const void *fn, size_t smem) {
     if (smem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem);
+    static std::mutex m;
+    std::lock_guard<std::mutex> lk(m);
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, fn);
+    if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= smem) return e;
+    int device = 0, most = 0;
+    e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
 }
 
 // Feature bits a frame needs.

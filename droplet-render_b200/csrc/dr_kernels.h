@@ -8,6 +8,16 @@ namespace dr {
 constexpr int kRenderBlock = 128;
 constexpr int kPersistentBlock = 128;
 
+// Dynamic shared memory above the default 48 KB needs the kernel's opt-in on the
+// current device.  The limit belongs to the kernel, not to a context: threads
+// that set it to what each of their launches needs fail each other's launches.
+// So it is raised once, to all that a block can have (227 KB less the kernel's own),
+// and never lowered.
+cudaError_t raise_smem(const void *fn, size_t smem);
+template <class F> cudaError_t allow_smem(F fn, size_t smem) {
+    return raise_smem(reinterpret_cast<const void *>(fn), smem);
+}
+
 cudaError_t launch_render_tile(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,
                                float4 *sun_out, float4 *sky_out, DevCounters *C, cudaStream_t st);
 cudaError_t launch_shadow_tile(const DevScene &S, const DevParams &P, const TileArgs &A, float4 *out, DevCounters *C,

@@ -1329,12 +1329,6 @@ static size_t table_bytes(const DevParams &P) {
     return (size_t)P.mie_n * 20u + (P.phase_mode == 1u ? (2u * (size_t)P.mie_n + 1u) * 16u : 0u);
 }
 
-template <class F> static cudaError_t opt_in(F fn, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem);
-}
-
 static uint64_t rounds_of(uint64_t n_paths, uint64_t limit, uint32_t ticket) {
     const uint64_t span = (uint64_t)kRoundTickets * ticket;
     return (n_paths + limit - 1) / limit + n_paths / span;
@@ -1370,7 +1364,7 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
                              : occ ? scatter_warp_bytes<kOcc, BATCH, ADJ>()
                                    : scatter_warp_bytes<kNoOcc, BATCH, ADJ>()) *
                                 (kScatterBlock / 32);
-    e = opt_in(sca, sca_smem);
+    e = allow_smem(sca, sca_smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sca, kScatterBlock, sca_smem);
