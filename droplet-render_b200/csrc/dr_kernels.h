@@ -8,8 +8,8 @@ namespace dr {
 constexpr int kRenderBlock = 128;
 constexpr int kPersistentBlock = 128;
 
-// Dynamic shared memory above the default 48 KB needs the kernel's opt-in on the
-// current device.  The limit belongs to the kernel, not to a context: threads
+// Dynamic shared memory above the default of 48 KB less the kernel's own (a
+// barrier) needs the kernel's opt-in on the current device.  The limit belongs to the kernel, not to a context: threads
 // that set it to what each of their launches needs fail each other's launches.
 // So it is raised once, to all that a block can have (227 KB less the kernel's own),
 // and never lowered.

@@ -1,6 +1,9 @@
 """Dynamic shared memory of the path pipeline: what a launch needs depends on the
 phase tables and on the octree's depth, and the limit it runs under belongs to the
 kernel, for every context and thread of the process."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -32,7 +35,7 @@ def _scene(levels):
 
 def _cfg(**more):
     """A camera close enough that the cluster fills the frame."""
-    cfg = dict(c0_cfg(24, 24), sigma_s=600.0, sigma_a=6.0, scattevs=6, **more)
+    cfg = dict(c0_cfg(24, 24), **{"sigma_s": 600.0, "sigma_a": 6.0, "scattevs": 6, **more})
     viewi = np.array(cfg["viewi"], np.float32).reshape(4, 4)
     viewi[3, :3] = 0.5 + 0.25 * (viewi[3, :3] - 0.5)
     cfg["viewi"] = viewi.reshape(-1)
@@ -104,3 +107,41 @@ def test_split_batch_of_both_depths():
                 _close(b.read(v), _render(r))
         finally:
             b.close()
+
+
+# the pipeline's dynamic part at depth 5 is 11,520 + 7,680 + 29,952 = 49,152 bytes with 576 entries (plain) and
+# 8,960 + 7,680 + 32,512 = 49,152 with 448 (adjoint): exactly the default limit, which also holds the kernel's barrier
+@pytest.mark.parametrize("entries,adjoint", [(572, False), (576, False), (580, False), (444, True), (448, True)])
+def test_sizes_around_the_default_limit(entries, adjoint):
+    """In a process of its own: a limit raised before would hide the fault."""
+    subprocess.run([sys.executable, __file__, str(entries), str(int(adjoint))], check=True, timeout=300,
+                   cwd=os.path.dirname(__file__))
+
+
+def _at_the_limit(entries, adjoint):
+    import torch
+
+    from droplet_b200.renderer import Renderer
+
+    pdf, cdf = mie_table()
+    k = np.minimum(np.arange(entries) * len(pdf) // entries, len(pdf) - 1)
+    with Renderer(0) as r:
+        oc = _scene(5)
+        r.upload(oc)
+        r.set_params(settings_from_cfg(_cfg(mie_pdf=np.ascontiguousarray(pdf[k]), mie_cdf=np.ascontiguousarray(cdf[k]))))
+        if adjoint:
+            d = torch.ones((24, 24, 4), device="cuda")
+            g = torch.zeros((oc.n_leaves, 512), device="cuda")
+            a = torch.zeros(1, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            r.adjoint_tile_async(0, 0, 24, 24, 16, 3, 0, d.data_ptr(), d.data_ptr(), g.data_ptr(), a.data_ptr())
+            r.synchronize()
+            assert float(g.abs().sum()) > 0 and float(a) > 0
+            return
+        got = _render(r)
+        r.set_tuning(1)  # one thread per path
+        _close(got, _render(r))
+
+
+if __name__ == "__main__":
+    _at_the_limit(int(sys.argv[1]), bool(int(sys.argv[2])))
