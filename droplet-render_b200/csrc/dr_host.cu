@@ -148,6 +148,8 @@ int prepare_scene(const dr_scene_desc *s, HostScene &out) {
     if (is_leaf(0)) return need(false, DR_ERR_INVALID, "dr_upload_scene: the root must be an internal node");
     std::vector<uint32_t> &child = out.child;
     std::vector<float4> &leaf = out.leaf;
+    float no_slot;  // kNone bits: the block grid gives every leaf that the root reaches a slot
+    std::memcpy(&no_slot, &kNone, 4);
     child.assign((size_t)s->n_nodes * 8, 0u);
     leaf.assign((size_t)s->n_nodes * 2, make_float4(0.f, 0.f, 0.f, 0.f));
     for (uint32_t i = 0; i < s->n_nodes; ++i) {
@@ -166,7 +168,7 @@ int prepare_scene(const dr_scene_desc *s, HostScene &out) {
             std::memcpy(&sb, &o.volx[0], 4);
             leaf[2 * (size_t)i] = make_float4(o.ce[0], o.ce[1], o.ce[2], o.ce[3]);
             // src/kernel.cpp:245-251: an SDF leaf's majorant is 1, a fog leaf's qval[FOG]
-            leaf[2 * (size_t)i + 1] = make_float4(sdf ? 1.0f : o.qval[1], fb, sb, 0.0f);
+            leaf[2 * (size_t)i + 1] = make_float4(sdf ? 1.0f : o.qval[1], fb, sb, no_slot);
         } else {
             leaf[2 * (size_t)i] = make_float4(o.ce[0], o.ce[1], o.ce[2], o.ce[3]);
             leaf[2 * (size_t)i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);

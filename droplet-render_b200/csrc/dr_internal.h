@@ -26,7 +26,8 @@ constexpr uint32_t kStepBudget = 1u << 24;  // tracking steps per segment before
 //   leaf[2*id]   = (center.xyz, half extent)
 //   leaf[2*id+1] = (majorant, FOG brick index bits, SDF brick index bits, slot
 //                  bits); an index kNone = no such brick; SDF leaves have
-//                  majorant 1; slot: the leaf's place in gleaf (0 without a block grid)
+//                  majorant 1; slot: the leaf's place in gleaf (kNone without a block
+//                  grid, or when the root does not reach the leaf)
 struct DevScene {
     const uint4 *child;
     const float4 *leaf;

@@ -1468,7 +1468,8 @@ __global__ void adjoint_transmittance_kernel(DevScene S, DevParams P, const floa
 // (src/scene.cpp:889-904), times scale (>= 1: headroom that lets samples grow
 // while the majorant stays fixed); a leaf whose majorant was 0 (never
 // resampled) keeps 0.
-// gleaf, gmaj: the same by slot (null without a block grid).
+// gleaf, gmaj: the same by slot (null without a block grid); a leaf that the root
+// does not reach has none.
 __global__ void leaf_majorant_kernel(float4 *leaf, float4 *gleaf, float *gmaj, const uint32_t *leaf_nodes, uint32_t n_leafnodes,
                                      const float *bricks, float scale) {
     const uint32_t i = blockIdx.x;
@@ -1488,9 +1489,10 @@ __global__ void leaf_majorant_kernel(float4 *leaf, float4 *gleaf, float *gmaj, c
         wm[0] = fmaxf(m, wm[0]);
         if (meta.x != 0.0f) meta.x = fmaxf(wm[0], 0.01f) * scale;
         leaf[2 * (size_t)node + 1] = meta;
-        if (gleaf) {
-            gleaf[2 * (size_t)__float_as_uint(meta.w) + 1] = meta;
-            gmaj[__float_as_uint(meta.w)] = meta.x;
+        const uint32_t slot = __float_as_uint(meta.w);
+        if (gleaf && slot != kNone) {
+            gleaf[2 * (size_t)slot + 1] = meta;
+            gmaj[slot] = meta.x;
         }
     }
 }

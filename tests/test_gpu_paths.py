@@ -143,3 +143,33 @@ def test_occluder_light(flags, tile, spp):
         r.set_occluders(occluder_surfaces())
         r.upload(Octree(*golden_octree()))
         _check(_pair(r, dict(c0_cfg(64, 64), **flags), tile, spp))
+
+
+def test_majorants_with_unreachable_leaves():
+    """Leaf nodes that the root does not reach get majorants of their own from
+    dr_set_bricks_dev, and leave those of the leaves in the block grid alone: rays
+    through every leaf count the escapes of the octree's replay."""
+    import torch
+
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    nodes, bricks, mlevel = golden_octree()
+    leaves = np.flatnonzero(nodes["volx"][:, 1] != N.DR_NONE)
+    loose = np.repeat(nodes[leaves[:1]], 500)  # nodes without a parent, each with a denser brick
+    loose["volx"][:, 1] = len(bricks)
+    with Renderer(0) as r:
+        r.upload(Octree(np.concatenate([nodes, loose]), np.concatenate([bricks, np.full((1, 512), 7.0, np.float32)]),
+                        mlevel))
+        r.set_params(settings_from_cfg(c0_cfg(64, 64)))
+        b = torch.as_tensor(np.concatenate([0.5 * bricks, np.full((1, 512), 9.0, np.float32)]), device="cuda")
+        r.set_bricks_dev(b.data_ptr(), len(bricks) + 1, 1.0)
+        r.synchronize()
+        maj = r.majorants(len(nodes) + len(loose))
+        assert (maj[len(nodes):] == 9.0).all() and maj[:len(nodes)].max() < 9.0
+        d = np.random.default_rng(1).normal(size=(len(leaves), 3))
+        d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+        ro = nodes["ce"][leaves][:, :3] - 2.0 * d
+        got = r.probe_transmittance(ro, d, 256, seed=9)
+        _, ref = r.adjoint_transmittance(ro, d, np.ones(len(leaves)), 256, 9, len(bricks) + 1)
+        assert np.array_equal(got, ref) and got.min() < 1.0
