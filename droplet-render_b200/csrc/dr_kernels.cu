@@ -357,7 +357,7 @@ __device__ __forceinline__ void scatter_event(PathLane<WALK> &L, const DevScene 
     const float f = P.albedo;
     if (L.r == 0) L.sun.w = L.sky.w = first_alpha(P, L.esc);
     if (L.esc == kTrackEscaped) {
-        if (L.r > 0 && !((FEAT & kFeatOcc) && occluded(S, L.ro, L.rd))) {
+        if (L.r > 0 && !((FEAT & kFeatOcc) && P.embree && occluded(S, L.ro, L.rd))) {
             if (sun_hit(P, L.rd)) {
                 L.sun.x = L.sun.x + L.T[0] * P.sun_color[0];
                 L.sun.y = L.sun.y + L.T[1] * P.sun_color[1];
@@ -415,7 +415,7 @@ __device__ __forceinline__ void path_event(PathLane<WALK> &L, const DevScene &S,
                                         const TileArgs &A, float4 *sun_out, float4 *sky_out, Count &cnt,
                                         uint32_t &state, Trav *slow) {
     if (L.seg == kSegShadow) {
-        if (L.esc == kTrackEscaped && !((FEAT & kFeatOcc) && occluded(S, L.ro, L.rd))) {
+        if (L.esc == kTrackEscaped && !((FEAT & kFeatOcc) && P.embree && occluded(S, L.ro, L.rd))) {
             const bool hit = sun_hit(P, L.rd);
             const float s0 = hit ? P.sun_color[0] : 0.0f, s1 = hit ? P.sun_color[1] : 0.0f,
                         s2 = hit ? P.sun_color[2] : 0.0f;

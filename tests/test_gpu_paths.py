@@ -173,3 +173,25 @@ def test_majorants_with_unreachable_leaves():
         got = r.probe_transmittance(ro, d, 256, seed=9)
         _, ref = r.adjoint_transmittance(ro, d, np.ones(len(leaves)), 256, 9, len(bricks) + 1)
         assert np.array_equal(got, ref) and got.min() < 1.0
+
+
+@pytest.mark.parametrize("more", [dict(phase_mode=N.DR_PHASE_HG, hg_g=0.6), dict(env_mode=N.DR_ENV_NONE)])
+def test_occluders_without_the_flag(more):
+    """Occluders count with DR_KERNEL_EMBREE only, whatever other options choose the
+    kernel: pipeline, cell walk and one thread per path render the frame without any."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    cfg = dict(c0_cfg(64, 64), **more)
+    images = []
+    with Renderer(0) as r:
+        r.upload(Octree(*golden_octree()))
+        for occluders in ([], occluder_surfaces()):
+            r.set_occluders(occluders)
+            r.set_params(settings_from_cfg(cfg))
+            for kernel, traversal in ((0, 0), (0, 1), (1, 0)):
+                r.set_tuning(kernel, traversal=traversal)
+                images.append(r.render_tile(2, 2, 60, 60, 33, seed=11, sample_base=2))
+    for g in images[1:]:
+        for a, b in zip(g, images[0]):
+            assert np.allclose(a, b, rtol=2e-5, atol=1e-6 * np.abs(b).max() + 1e-30)
