@@ -228,7 +228,7 @@ static ListLayout list_layout(const dr_ctx *c, uint32_t slot, size_t pixels) {
     l.head = part(2 * pixels * sizeof(uint4));
     l.active = part(pixels * sizeof(uint32_t));
     l.ctl = part(two * sizeof(PathCtl));
-    l.used = part(two * sizeof(unsigned int));
+    l.used = part(two * sizeof(unsigned long long));
     l.bytes = at;
     return l;
 }
@@ -350,7 +350,7 @@ static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t h
     L.head = reinterpret_cast<uint4 *>(buf.p + l.head) + 2 * head_off;
     L.pool = reinterpret_cast<uint4 *>(buf.p + l.pool) + second * l.pool_cap;
     L.cap = l.pool_cap;
-    L.used = reinterpret_cast<unsigned int *>(buf.p + l.used) + second;
+    L.used = reinterpret_cast<unsigned long long *>(buf.p + l.used) + second;
     L.ctl = reinterpret_cast<PathCtl *>(buf.p + l.ctl) + second;
     L.active = reinterpret_cast<uint32_t *>(buf.p + l.active) + head_off;
     L.records = reinterpret_cast<uint4 *>(buf.p + l.records) + second * l.rec_cap;

@@ -54,7 +54,7 @@ struct dr_batch {
     cudaEvent_t fork = nullptr, join[kBranches] = {};
     // camera leaf lists (one header per pixel of every view, one entry pool)
     DevBuf<uint4> cam_head, cam_pool;
-    DevBuf<unsigned int> cam_used;
+    DevBuf<unsigned long long> cam_used;
     DevBuf<uint32_t> pix_begins;
     uint32_t n_pix = 0;
     // path pipeline (dr_paths.cu): control words, active pixels, per-view counts of
@@ -219,7 +219,7 @@ int build_graph(dr_batch *b) {
     DR_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "dr_batch: begin capture");
     cudaError_t e = cudaMemsetAsync(b->out.p, 0, sizeof(float4) * b->out_n, b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->work.p, 0, sizeof(WorkQueue) * b->work.n, b->stream);
-    if (e == cudaSuccess && paths) e = cudaMemsetAsync(b->cam_used.p, 0, sizeof(unsigned int), b->stream);
+    if (e == cudaSuccess && paths) e = cudaMemsetAsync(b->cam_used.p, 0, sizeof(*b->cam_used.p), b->stream);
     if (e == cudaSuccess && !paths) e = launch_batch_lists(B, bl, b->stream);
     if (e == cudaSuccess && nbr) e = cudaEventRecord(b->fork, b->stream);
     for (uint32_t k = 0; k < nbr && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(b->branch[k], b->fork, 0);

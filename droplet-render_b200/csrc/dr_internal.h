@@ -202,12 +202,11 @@ struct WorkQueue {
 struct PathCtl {
     unsigned long long ticket;  // next camera ticket
     unsigned long long base;    // the first ticket of this round
+    unsigned long long pool_used;  // leaf list entries asked for (may exceed the pool)
     uint32_t records;           // collided samples recorded in this round
     uint32_t head;              // the next record to scatter
-    uint32_t pool_used;         // leaf list entries taken
     uint32_t n_active;          // active pixels
     uint32_t tape_used;         // adjoint: tape entries handed out
-    uint32_t pad;
 };
 constexpr uint32_t kRoundTickets = 1u << 24;  // tickets of one round: at most 2^31 samples, so 32 bits tell them apart
 
@@ -241,7 +240,8 @@ struct AdjointArgs {
 // Storage of the path pipeline for one launch at a time.
 struct PathWork {
     PathCtl *ctl;
-    uint32_t *pool_used, *n_active;  // where the list kernel counts
+    unsigned long long *pool_used;   // where the list kernel counts
+    uint32_t *n_active;
     uint4 *head;                     // leaf list headers, 2 per pixel (TileArgs::cam_head)
     uint4 *pool;                     // leaf list entries: (slot, tra bits, trb bits, node visits since the previous leaf)
     uint32_t pool_cap;

@@ -751,7 +751,7 @@ __global__ void add_counters_kernel(DevCounters *dst, const DevCounters *src) {
 // fit gets x = ~0 and its samples traverse.  `ray`: the ray's direction bits
 // and whether the pixel has a ray (camera_ray's result).
 __device__ __forceinline__ uint4 camera_list(const DevScene &S, const DevParams &P, const TileArgs &A, uint32_t ix,
-                                             uint32_t iy, uint4 *pool, uint32_t cap, unsigned int *used, uint4 &ray) {
+                                             uint32_t iy, uint4 *pool, uint32_t cap, unsigned long long *used, uint4 &ray) {
     float ro[3], rd[3];
     uint4 h = make_uint4(0u, 0u, 0u, 0u);
     const bool ok = camera_ray(P, A.x0 + ix, A.y0 + iy, ro, rd);
@@ -767,12 +767,9 @@ __device__ __forceinline__ uint4 camera_list(const DevScene &S, const DevParams 
     uint32_t leaf, n = 0;
     float tra, trb;
     while (trav_next_k(T, S, nstack, leaf, tra, trb, c, 0xffffffffu, tstack) == kTravLeaf) ++n;
-    const unsigned int off = n ? atomicAdd(used, n) : 0u;
-    if (n && (off > cap || n > cap - off)) {
-        h.x = kNone;
-        return h;
-    }
+    const uint32_t off = n ? pool_range(used, n, cap) : 0u;
     h.x = off;
+    if (off == kNone) return h;
     h.y = n;
     trav_init(T, S, ro, rd, c);
     c.zero();
@@ -788,7 +785,7 @@ __device__ __forceinline__ uint4 camera_list(const DevScene &S, const DevParams 
 
 // The camera leaf lists of a single-tile launch (one thread per pixel).
 __global__ void __launch_bounds__(128) camera_list_kernel(DevScene S, DevParams P, TileArgs A, uint4 *head,
-                                                          uint4 *pool, uint32_t cap, unsigned int *used) {
+                                                          uint4 *pool, uint32_t cap, unsigned long long *used) {
     const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= A.cols * A.rows) return;
     const uint32_t iy = pix / A.cols, ix = pix - iy * A.cols;
@@ -802,7 +799,7 @@ __global__ void __launch_bounds__(128) camera_list_kernel(DevScene S, DevParams 
 // (the view's TileArgs::cam_head points at head + 2 pix_begins[v]).
 __global__ void __launch_bounds__(128) batch_camera_list_kernel(BatchArgs B, const uint32_t *pix_begins,
                                                                 uint32_t n_pix, uint4 *head, uint4 *pool,
-                                                                uint32_t cap, unsigned int *used) {
+                                                                uint32_t cap, unsigned long long *used) {
     const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= n_pix) return;
     uint32_t lo = 0, hi = B.n_views - 1;
@@ -1675,7 +1672,7 @@ cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, cons
     e = cudaMemsetAsync(Q, 0, sizeof(WorkQueue), st);
     if (e != cudaSuccess) return e;
     if (lists.head && lists.cap && tune.traversal != 1u) {  // the cell walk counts grid cells: it keeps its own traversal
-        e = cudaMemsetAsync(lists.used, 0, sizeof(unsigned int), st);
+        e = cudaMemsetAsync(lists.used, 0, sizeof(*lists.used), st);
         if (e != cudaSuccess) return e;
         const uint32_t npix = A.cols * A.rows;
         camera_list_kernel<<<(npix + 127) / 128, 128, 0, st>>>(S, P, A, lists.head, lists.pool, lists.cap,
@@ -1691,7 +1688,7 @@ cudaError_t launch_render_persistent(const DevScene &S, const DevParams &P, cons
 
 cudaError_t launch_batch_lists(const BatchArgs &B, const BatchLists &lists, cudaStream_t st) {
     if (!B.n_paths || !lists.lists.head || !lists.n_pix) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(lists.lists.used, 0, sizeof(unsigned int), st);
+    cudaError_t e = cudaMemsetAsync(lists.lists.used, 0, sizeof(*lists.lists.used), st);
     if (e != cudaSuccess) return e;
     batch_camera_list_kernel<<<(lists.n_pix + 127) / 128, 128, 0, st>>>(
         B, lists.pix_begins, lists.n_pix, lists.lists.head, lists.lists.pool, lists.lists.cap, lists.lists.used);

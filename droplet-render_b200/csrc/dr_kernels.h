@@ -28,7 +28,7 @@ struct CamLists {
     uint4 *head = nullptr;
     uint4 *pool = nullptr;
     uint32_t cap = 0;
-    unsigned int *used = nullptr;
+    unsigned long long *used = nullptr;
     // storage of the path pipeline (null: the persistent kernel runs)
     PathCtl *ctl = nullptr;
     uint32_t *active = nullptr;  // cols * rows

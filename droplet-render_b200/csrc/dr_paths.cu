@@ -37,7 +37,7 @@ constexpr int kListBlock = 128, kListTx = 16, kListTy = 8;  // camera lists: a b
 // pixel whose range does not fit gets x = ~0 and its samples traverse.
 // Rays with a zero direction component take the octree (node ids become slots).
 __device__ __noinline__ uint4 octree_list(const DevScene &S, float ox, float oy, float oz, float dx, float dy, float dz,
-                                          uint4 *pool, uint32_t cap, unsigned int *used) {
+                                          uint4 *pool, uint32_t cap, unsigned long long *used) {
     const float ro[3] = {ox, oy, oz}, rd[3] = {dx, dy, dz};
     const SlotStack stk{S};
     Trav T;
@@ -48,12 +48,9 @@ __device__ __noinline__ uint4 octree_list(const DevScene &S, float ox, float oy,
     uint32_t leaf, n = 0;
     float tra, trb;
     while (trav_next_s(T, S, stk, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
-    const unsigned int off = n ? atomicAdd(used, n) : 0u;
-    if (n && (off > cap || n > cap - off)) {
-        h.x = kNone;
-        return h;
-    }
+    const uint32_t off = n ? pool_range(used, n, cap) : 0u;
     h.x = off;
+    if (off == kNone) return h;
     h.y = n;
     trav_init(T, S, ro, rd, c);
     c.zero();
@@ -69,7 +66,7 @@ __device__ __noinline__ uint4 octree_list(const DevScene &S, float ox, float oy,
 }
 
 __device__ __forceinline__ uint4 grid_list(const DevScene &S, const float ro[3], const float rd[3], float *col,
-                                           uint4 *pool, uint32_t cap, unsigned int *used) {
+                                           uint4 *pool, uint32_t cap, unsigned long long *used) {
     GridTrav G;
     Count c;
     c.zero();
@@ -80,8 +77,8 @@ __device__ __forceinline__ uint4 grid_list(const DevScene &S, const float ro[3],
     float tra, trb;
     while (grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
     if (n == 0) return make_uint4(0u, 0u, 1u, c.node_visits - 1u);
-    const unsigned int off = atomicAdd(used, n);
-    if (off > cap || n > cap - off) return make_uint4(kNone, 0u, 0u, 0u);
+    const uint32_t off = pool_range(used, n, cap);
+    if (off == kNone) return make_uint4(kNone, 0u, 0u, 0u);
     c.zero();
     grid_init<kListBlock>(G, S, col, ro, rd, c);
     c.node_visits -= 1u;  // the root (h.z)

@@ -26,6 +26,7 @@ inline uint32_t __funnelshift_r(uint32_t lo, uint32_t hi, uint32_t s) {
     return s ? (lo >> s) | (hi << (32u - s)) : lo;
 }
 inline float __fdiv_rn(float a, float b) { return a / b; }
+inline unsigned long long atomicAdd(unsigned long long *p, unsigned long long v) { *p += v; return *p - v; }
 using std::isfinite;
 using std::max;
 using std::min;

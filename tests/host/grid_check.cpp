@@ -3,6 +3,7 @@
 // at a time, on random, lattice-aligned, tied and far-away rays.
 //   grid_check SCENE RAYS SEED    (SCENE: n_nodes, n_leaves, then the node records)
 //   grid_check flights N SEED     leaves_at_once against the flight in full
+//   grid_check pool N SEED        ranges of a leaf list pool while N lists ask for them
 #include "cuda_host_shim.h"
 #include "../../droplet-render_b200/csrc/dr_device.cuh"
 #include "../../include/droplet_b200.h"
@@ -47,8 +48,30 @@ static int flights(long long n, int seed) {
     return least < 1.0 - 1e-6 || bad || quick < left / 2;
 }
 
+static int pool(long long n, int seed) {
+    // lists of 1 to 2^20 entries: the ranges handed out lie in the pool one after the other, however many are asked for
+    std::mt19937_64 g(seed);
+    const uint32_t cap = (1u << 26) - 3;
+    unsigned long long used = 0;
+    uint64_t end = 0, bad = 0, asked = 0;
+    for (long long i = 0; i < n; ++i) {
+        const uint32_t k = 1u + (uint32_t)(g() >> (44 + g() % 20)), off = pool_range(&used, k, cap);
+        asked += k;
+        if (off == kNone) continue;
+        bad += off < end || (uint64_t)off + k > cap;
+        end = (uint64_t)off + k;
+    }
+    unsigned long long edge = cap - 5;  // exactly the rest, and one more
+    bad += pool_range(&edge, 6, cap) != kNone;
+    edge = cap - 5;
+    bad += pool_range(&edge, 5, cap) != cap - 5 || pool_range(&edge, 1, cap) != kNone;
+    std::printf("asked %llu end %llu bad %llu\n", (unsigned long long)asked, (unsigned long long)end, (unsigned long long)bad);
+    return bad || asked < 3ull << 32;
+}
+
 int main(int argc, char **argv) {
     if (argc != 4) return 2;
+    if (!std::strcmp(argv[1], "pool")) return pool(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "flights")) return flights(atoll(argv[2]), atoi(argv[3]));
     FILE *f = std::fopen(argv[1], "rb");
     uint32_t head[2];

@@ -59,3 +59,8 @@ def test_grid_traversal_equals_octree(check, name, levels):
 
 def test_first_flight_test_is_safe(check):
     check("flights", 20000000, 3)
+
+
+def test_leaf_list_pool_beyond_32_bits(check):
+    """Lists that do not fit are counted as well: the ranges stay apart when more than 2^32 entries are asked for."""
+    check("pool", 500000, 5)
