@@ -1007,9 +1007,11 @@ __device__ __forceinline__ uint32_t grid_leaf(const GridTrav &G, float &tra, flo
 // Takes n entries of a pool of cap for a leaf list: the first one, or kNone when
 // they do not fit.  Lists that do not fit are counted too, so the counter has 64
 // bits: the leaves of all a batch's pixels may pass 2^32.
+__device__ __forceinline__ uint32_t pool_place(unsigned long long first, uint32_t n, uint32_t cap) {
+    return first <= cap && n <= cap - first ? (uint32_t)first : kNone;
+}
 __device__ __forceinline__ uint32_t pool_range(unsigned long long *used, uint32_t n, uint32_t cap) {
-    const unsigned long long off = atomicAdd(used, (unsigned long long)n);
-    return off <= cap && n <= cap - off ? (uint32_t)off : kNone;
+    return pool_place(atomicAdd(used, (unsigned long long)n), n, cap);
 }
 
 // Up to `budget` steps towards the next leaf: kTravLeaf with its slot and

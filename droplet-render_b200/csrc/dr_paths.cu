@@ -65,19 +65,30 @@ __device__ __noinline__ uint4 octree_list(const DevScene &S, float ox, float oy,
     return h;
 }
 
-__device__ __forceinline__ uint4 grid_list(const DevScene &S, const float ro[3], const float rd[3], float *col,
+// The whole warp calls (ray: the lane has one); its lanes share one addition to the counter.
+__device__ __forceinline__ uint4 grid_list(const DevScene &S, bool ray, const float ro[3], const float rd[3], float *col,
                                            uint4 *pool, uint32_t cap, unsigned long long *used) {
     GridTrav G;
     Count c;
     c.zero();
-    const uint32_t mode = grid_init<kListBlock>(G, S, col, ro, rd, c);
-    if (mode == 2u) return octree_list(S, ro[0], ro[1], ro[2], rd[0], rd[1], rd[2], pool, cap, used);
-    if (mode == 0u) return make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t mode = ray ? grid_init<kListBlock>(G, S, col, ro, rd, c) : 0u;
     uint32_t leaf, n = 0;
     float tra, trb;
-    while (grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
+    if (mode == 1u)
+        while (grid_next<kListBlock>(G, S, col, ro, rd, leaf, tra, trb, c, kNone) == kTravLeaf) ++n;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t end = n;  // of the lane's entries among the warp's
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(kFull, end, d);
+        if (lane >= d) end += o;
+    }
+    unsigned long long first = 0;
+    if (lane == 31u && end) first = atomicAdd(used, (unsigned long long)end);
+    first = __shfl_sync(kFull, first, 31) + (end - n);
+    if (mode == 2u) return octree_list(S, ro[0], ro[1], ro[2], rd[0], rd[1], rd[2], pool, cap, used);
+    if (mode == 0u) return make_uint4(0u, 0u, 0u, 0u);
     if (n == 0) return make_uint4(0u, 0u, 1u, c.node_visits - 1u);
-    const uint32_t off = pool_range(used, n, cap);
+    const uint32_t off = pool_place(first, n, cap);
     if (off == kNone) return make_uint4(kNone, 0u, 0u, 0u);
     c.zero();
     grid_init<kListBlock>(G, S, col, ro, rd, c);
@@ -99,10 +110,10 @@ __device__ __forceinline__ void list_pixel(const DevScene &S, const DevParams &P
     uint4 h = make_uint4(0u, 0u, 0u, 0u);
     bool ray = false;
     const uint32_t pix = iy * A.cols + ix;
+    float ro[3], rd[3];
+    if (valid) ray = camera_ray(P, A.x0 + ix, A.y0 + iy, ro, rd);
+    h = grid_list(S, ray, ro, rd, col, W.pool, W.pool_cap, W.pool_used);
     if (valid) {
-        float ro[3], rd[3];
-        ray = camera_ray(P, A.x0 + ix, A.y0 + iy, ro, rd);
-        if (ray) h = grid_list(S, ro, rd, col, W.pool, W.pool_cap, W.pool_used);
         head[2 * (size_t)pix] = h;
         head[2 * (size_t)pix + 1] =
             make_uint4(__float_as_uint(rd[0]), __float_as_uint(rd[1]), __float_as_uint(rd[2]), ray ? 1u : 0u);
