@@ -150,6 +150,7 @@ int dr_upload_scene(dr_ctx *c, const dr_scene_desc *s) {
         c->scene.occ_nodes = c->occ_nodes.p;
         c->scene.occ_tris = c->occ_tris.p;
         c->scene.occ_n_nodes = c->occ_n_nodes;
+        c->scene.occ_stack = c->occ_stack;
     }
     std::vector<uint32_t> ln;
     for (uint32_t i = 0; i < h.n_nodes; ++i)  // leaves whose majorant comes from their fog brick
@@ -182,9 +183,11 @@ int dr_set_occluders(dr_ctx *c, const dr_surface *surfaces, uint32_t n_surfaces,
                 "dr_set_occluders: copy triangles");
     }
     c->occ_n_nodes = nn;
+    c->occ_stack = b.depth;
     c->scene.occ_nodes = nn ? c->occ_nodes.p : nullptr;
     c->scene.occ_tris = nn ? c->occ_tris.p : nullptr;
     c->scene.occ_n_nodes = nn;
+    c->scene.occ_stack = b.depth;
     return DR_OK;
 }
 

@@ -1543,18 +1543,11 @@ __device__ __forceinline__ bool occ_box(float x0, float y0, float z0, float x1, 
 
 // Any-hit traversal of the occluder BVH.  Every node is visited at most once,
 // so the loop ends within occ_n_nodes iterations; the stack holds at most one
-// entry per level of the (depth-capped) tree.  Not inlined: its stack then sits
-// in its own frame.  Inlined into the shadow-pass kernel, the kernel's local
-// frame came out smaller (384 B) than its node and interval stacks need at once
-// (448 B), and that kernel read out of bounds; every caller's frame now holds
-// all three stacks.
-static __device__ __noinline__ bool occluded_bvh(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
-                                          uint32_t n_nodes, float ox, float oy, float oz, float dx, float dy,
-                                          float dz) {
-    const float o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+// entry per level of the (depth-capped) tree.
+template <class ST>
+__device__ __forceinline__ bool occ_any_hit(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                            uint32_t n_nodes, const float o[3], const float d[3], ST &stack) {
     const float inv[3] = {1.0f / d[0], 1.0f / d[1], 1.0f / d[2]};
-    uint32_t stack[kOccMaxDepth + 2];
-    int sp = 0;
     uint32_t node = 0;
     for (uint32_t it = 0; it < n_nodes; ++it) {
         const float4 n0 = __ldg(&nodes[4 * (size_t)node]), n1 = __ldg(&nodes[4 * (size_t)node + 1]);
@@ -1573,18 +1566,41 @@ static __device__ __noinline__ bool occluded_bvh(const float4 *__restrict__ node
             hr = false;
         }
         if (hl && hr) {
-            if (sp < kOccMaxDepth + 2) stack[sp++] = n3.y;
+            stack.push(n3.y);
             node = n3.x;
         } else if (hl) {
             node = n3.x;
         } else if (hr) {
             node = n3.y;
         } else {
-            if (sp == 0) return false;
-            node = stack[--sp];
+            if (stack.empty()) return false;
+            node = stack.pop();
         }
     }
     return false;
+}
+
+struct OccLocalStack {
+    uint32_t e[kOccMaxDepth + 2];
+    int n;
+    __device__ __forceinline__ void push(uint32_t v) {
+        if (n < kOccMaxDepth + 2) e[n++] = v;
+    }
+    __device__ __forceinline__ bool empty() const { return n == 0; }
+    __device__ __forceinline__ uint32_t pop() { return e[--n]; }
+};
+
+// With the stack in a local frame of its own, so not inlined: inlined into the
+// octree's shadow-pass kernel, the kernel's local frame came out smaller (384 B)
+// than its node and interval stacks need at once (448 B), and that kernel read out
+// of bounds; every caller's frame now holds all three stacks.
+static __device__ __noinline__ bool occluded_bvh(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                          uint32_t n_nodes, float ox, float oy, float oz, float dx, float dy,
+                                          float dz) {
+    const float o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+    OccLocalStack stack;
+    stack.n = 0;
+    return occ_any_hit(nodes, tris, n_nodes, o, d, stack);
 }
 
 // Whether the ray (o, d) hits an occluder (false without occluders).

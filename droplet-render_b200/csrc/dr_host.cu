@@ -311,6 +311,7 @@ int upload_scene(const HostScene &h, SceneBufs &b, bool use_grid, cudaStream_t s
     S.occ_nodes = nullptr;
     S.occ_tris = nullptr;
     S.occ_n_nodes = 0;
+    S.occ_stack = 0;
     return DR_OK;
 }
 

@@ -122,6 +122,7 @@ struct OccBvh {
     std::vector<float> nodes;
     std::vector<float> tris;
     std::vector<uint32_t> source;
+    uint32_t depth = 0;  // levels of inner nodes below the root (DevScene::occ_stack)
 };
 int build_occluder_bvh(const dr_surface *s, uint32_t n, uint32_t mode, OccBvh &out);
 
@@ -256,7 +257,7 @@ struct dr_ctx {
     dr::DevBuf<uint4> path_rec;       // adjoint: one record per path of a chunk (totals pass -> scatter pass)
     dr::DevBuf<uint4> tape;           // adjoint: tracking decisions (AdjointArgs::tape)
     dr::DevBuf<float4> occ_nodes, occ_tris;  // occluder BVH (kept across scene uploads)
-    uint32_t occ_n_nodes = 0;
+    uint32_t occ_n_nodes = 0, occ_stack = 0;
     uint32_t n_leaf_nodes = 0;
     bool use_grid = true;
     dr::Tuning tuning{0u, 128u, 0u, 8u, 0u, 0u, 0u, 0u};

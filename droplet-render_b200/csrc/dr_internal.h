@@ -69,6 +69,7 @@ struct DevScene {
     const float4 *occ_nodes;
     const float4 *occ_tris;
     uint32_t occ_n_nodes;
+    uint32_t occ_stack;  // entries an any-hit traversal's stack needs: levels of inner nodes below the root
 };
 
 constexpr uint32_t kGridMaxLevels = 9;  // block grid: at most 128^3 blocks (32 MB)

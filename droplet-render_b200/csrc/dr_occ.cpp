@@ -49,6 +49,7 @@ struct Builder {
     std::vector<float> nodes;  // 16 floats per node
     std::vector<uint32_t> order;
     float pad = 0.0f;
+    uint32_t depth = 0;  // deepest inner node
 
     Box bounds(uint32_t b, uint32_t e) const {
         Box x;
@@ -110,6 +111,7 @@ struct Builder {
     // Node for [b, e) (at least two children's worth, or the whole set).
     uint32_t build(uint32_t b, uint32_t e, int depth) {
         const uint32_t id = (uint32_t)(nodes.size() / 16);
+        this->depth = std::max(this->depth, (uint32_t)depth);
         nodes.resize(nodes.size() + 16, 0.0f);
         uint32_t ref[2], count[2];
         Box box[2];
@@ -149,6 +151,7 @@ int build_occluder_bvh(const dr_surface *s, uint32_t n, uint32_t mode, OccBvh &o
     out.nodes.clear();
     out.tris.clear();
     out.source.clear();
+    out.depth = 0;
     if (n && !s) return need(false, DR_ERR_INVALID, "occluders: null surface list");
     if (mode != DR_OCCLUDE_ALL_SURFACES && mode != DR_OCCLUDE_HOLDOUT_ONLY)
         return need(false, DR_ERR_INVALID, "occluders: unknown mode");
@@ -190,6 +193,7 @@ int build_occluder_bvh(const dr_surface *s, uint32_t n, uint32_t mode, OccBvh &o
     }
     B.build(0, (uint32_t)nt, 0);
     out.nodes = std::move(B.nodes);
+    out.depth = B.depth;
     out.tris.resize(nt * 12);
     out.source.resize(nt);
     for (size_t i = 0; i < nt; ++i) {

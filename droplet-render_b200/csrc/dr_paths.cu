@@ -602,6 +602,51 @@ __global__ void __launch_bounds__(kListBlock, ADJ ? 6 : 8) camera_paths_kernel(c
     else warp_sum_counts(cnt, C, paths);
 }
 
+// ---- occluder test ------------------------------------------------------------------
+// occluded() with the stack in the lane's column of shared memory (S.occ_stack
+// words, STRIDE lanes apart), since these kernels keep no array in local memory.
+// The traversal is bound by instruction issue, hence the running 32-bit address, and
+// the test inlined: 640 x 360 at 32 samples and 402 triangles, HG phase and a map, takes
+// 1.525 ms (1.520 with the stack in local memory); with the test as a call 1.63, with
+// an index into a generic pointer 2% more, the last four entries in registers 4%.
+template <int STRIDE>
+struct OccSharedStack {
+    uint32_t p, base, end;
+    __device__ __forceinline__ OccSharedStack(const float *column, uint32_t entries) {
+        p = base = (uint32_t)__cvta_generic_to_shared(column);
+        end = base + entries * (4u * STRIDE);
+    }
+    __device__ __forceinline__ void push(uint32_t v) {
+        if (p == end) return;
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+        p += 4u * STRIDE;
+    }
+    __device__ __forceinline__ bool empty() const { return p == base; }
+    __device__ __forceinline__ uint32_t pop() {
+        uint32_t v;
+        p -= 4u * STRIDE;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+        return v;
+    }
+};
+template <int STRIDE>
+__device__ __forceinline__ bool occluded_col(const DevScene &S, const float o[3], const float d[3], const float *column) {
+    if (!S.occ_nodes) return false;
+    OccSharedStack<STRIDE> stack(column, S.occ_stack);
+    return occ_any_hit(S.occ_nodes, S.occ_tris, S.occ_n_nodes, o, d, stack);
+}
+
+// The same as a call, for the shadow kernel, which is short of registers: 960 x 540 at 16
+// samples beside the same triangles 1.43 ms, inlined 1.58 (stack in local memory 1.49).
+template <int STRIDE>
+__device__ __noinline__ bool occluded_call(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                           uint32_t n_nodes, uint32_t entries, float ox, float oy, float oz, float dx,
+                                           float dy, float dz, const float *column) {
+    const float o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+    OccSharedStack<STRIDE> stack(column, entries);
+    return occ_any_hit(nodes, tris, n_nodes, o, d, stack);
+}
+
 // ---- shadow pass ------------------------------------------------------------------
 // RenderKernel::Shadow (src/kernel.cpp:569-607, see shadow_sample): the segments
 // of a pixel's samples start at one point and stay within the sun's cone, so
@@ -659,7 +704,11 @@ __global__ void __launch_bounds__(kListBlock, 8) shadow_paths_kernel(const __gri
         const CamSeg o = camera_segments<FEAT, false>(none, 0u, S, seg_medium(P), active, ro, rd, g, 3.402823466e+38f,
                                                       make_uint4(0u, 0u, 0u, 0u), nullptr, col, cnt);
         const bool esc = !active || o.res == kTrackEscaped;
-        const bool occ = (FEAT & kFeatOcc) && active && esc && P.embree && occluded(S, ro, rd);
+        bool occ = false;  // (the segment is over: its column is the test's stack)
+        if constexpr ((FEAT & kFeatOcc) != 0)
+            occ = active && esc && P.embree && S.occ_nodes &&
+                  occluded_call<kListBlock>(S.occ_nodes, S.occ_tris, S.occ_n_nodes, S.occ_stack, ro[0], ro[1], ro[2], rd[0],
+                                            rd[1], rd[2], col);
         const bool lit = pix != kNone && P.scattevs > 0u && esc && !occ && sun_hit(P, rd);
         const bool one = pix != kNone && (P.scattevs > 0u || !esc) && !occ;
         // a pixel's samples each add sun(lrd) / colour = colour / colour or 0 / colour,
@@ -829,8 +878,9 @@ enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
 // calling instead of inlining (111 to 83 KB of code) took the frame from 19.6 to
 // 18.3 ms and instruction stalls from 1.46 to 0.57 cycles per instruction.
 // No array of these kernels lives in local memory: with one (a stack for the
-// octree in slow_segment) beside spilled registers, a kernel counted a few node
-// visits too many now and then; the octree's stack here is its child slots.
+// octree in slow_segment) beside spilled registers, the shadow kernel counted a few
+// node visits too many now and then, for a reason that was not found.  The octree's
+// stack here is its child slots, and the occluder test's a column of shared memory.
 constexpr int kScatterBlock = 128;
 constexpr int kSlots = 64;
 constexpr uint32_t kEventBatch = 28;           // events that make a shading pass
@@ -852,13 +902,23 @@ template <bool BATCH, bool ADJ = false> __host__ __device__ constexpr int slot_w
 template <uint32_t FEAT, bool BATCH, bool ADJ = false> __host__ __device__ constexpr int queue_words() {
     return ADJ || (FEAT && !(FEAT & kFeatOcc)) ? 0 : (FEAT ? 11 : 7) + (BATCH ? 1 : 0);
 }
-// bytes per warp: slots, three lists of slot numbers, the sky queue
-template <uint32_t FEAT, bool BATCH, bool ADJ = false> __host__ __device__ constexpr size_t scatter_warp_bytes() {
-    return 4 * (size_t)(slot_words<BATCH, ADJ>() * kSlots + 32 * queue_words<FEAT, BATCH, ADJ>()) + 3 * (size_t)kSlots;
+// An entry's words; those up to the direction are read again after the occluder
+// test, whose stack (occ_stack words) takes the place of the rest.
+template <uint32_t FEAT, bool ADJ = false> struct QueueAt {
+    static constexpr uint32_t T = FEAT ? 0 : 3, off = FEAT ? 3 : 6, kind = 4, rd = FEAT ? 5 : 0, ro = 8,
+                              stack = ADJ ? 0 : 5;
+};
+// bytes per warp: slots, three lists of slot numbers, the light queue
+template <uint32_t FEAT, bool BATCH, bool ADJ = false>
+__host__ __device__ constexpr size_t scatter_warp_bytes(uint32_t occ_stack) {
+    const uint32_t q = queue_words<FEAT, BATCH, ADJ>(), s = QueueAt<FEAT, ADJ>::stack + occ_stack;
+    return 4 * (size_t)(slot_words<BATCH, ADJ>() * kSlots + 32 * ((FEAT & kFeatOcc) && s > q ? s : q)) +
+           3 * (size_t)kSlots;
 }
 
 // The sky terms of escaped paths are evaluated by full warps: entry i of the
-// queue is (rd, T, output offset, [ro, kind,] [view]) in column i; T * sky(rd) is
+// queue is (rd, T, output offset, [view]) in column i, with features (T, output
+// offset, kind, rd, ro); T * sky(rd) is
 // the value the path would have added in place (its sky sum is 0 before the
 // escape).  With occluders the light of lit shadow segments and escapes waits
 // there too (kShadowLight: T is the segment's sun term; kEscapeLight: sun and sky),
@@ -867,22 +927,31 @@ template <uint32_t FEAT, bool BATCH, bool ADJ = false> __host__ __device__ const
 // half the frame (640 x 360, 32 samples, 402 triangles: 1.57 -> 1.26 ms; 0.79 without
 // occluders).
 enum : uint32_t { kSkyLight = 0, kShadowLight = 1, kEscapeLight = 2 };
+// The occluder test's stack lies in the lane's column of the warp's queue: over the
+// ray of the entry, which is in registers then, or, where rays are tested in place,
+// in a queue that holds nothing.  (Columns of its own, 6 KB a block there, halve the
+// L1 beside the slots: 1% more.)
 template <uint32_t FEAT, bool BATCH>
 __device__ __noinline__ void path_light_eval(const DevScene &S0, const DevParams &P0, float4 *sun0, float4 *sky0,
                                              const BatchArgs &B, const float *q, uint32_t i) {
     const BatchView *V = nullptr;
     if constexpr (BATCH) V = &B.views[__float_as_uint(q[32 * (queue_words<FEAT, BATCH>() - 1) + i])];
     const DevParams &P = BATCH ? V->P : P0;
-    const float rd[3] = {q[i], q[32 + i], q[64 + i]};
-    const float T[3] = {q[96 + i], q[128 + i], q[160 + i]};
-    const uint32_t off = __float_as_uint(q[192 + i]);
-    uint32_t kind = kSkyLight;
+    using Q = QueueAt<FEAT>;
+    const float rd[3] = {q[32 * Q::rd + i], q[32 * Q::rd + 32 + i], q[32 * Q::rd + 64 + i]};
     if constexpr (FEAT != 0) {
-        kind = __float_as_uint(q[320 + i]);
         const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
+        if (__float_as_uint(q[32 * Q::kind + i]) != kSkyLight) {
+            const float ro[3] = {q[32 * Q::ro + i], q[32 * Q::ro + 32 + i], q[32 * Q::ro + 64 + i]};
+            if constexpr ((FEAT & kFeatOcc) != 0)
+                if (occluded_col<32>(S, ro, rd, q + 32 * Q::stack + i)) return;
+        }
+    }
+    const float T[3] = {q[32 * Q::T + i], q[32 * Q::T + 32 + i], q[32 * Q::T + 64 + i]};
+    const uint32_t off = __float_as_uint(q[32 * Q::off + i]);
+    if constexpr (FEAT != 0) {
+        const uint32_t kind = __float_as_uint(q[32 * Q::kind + i]);
         if (kind != kSkyLight) {
-            const float ro[3] = {q[224 + i], q[256 + i], q[288 + i]};
-            if (occluded(S, ro, rd)) return;
             float c[3] = {T[0], T[1], T[2]};
             if (kind == kEscapeLight) {
                 const bool hit = sun_hit(P, rd);
@@ -925,9 +994,9 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
     unsigned char *const area = smem + ((mb + 15u) & ~15u);
     float *const col = reinterpret_cast<float *>(area) + threadIdx.x;
     float *const slots = reinterpret_cast<float *>(area + (size_t)colwords * 4u * kScatterBlock +
-                                                   (threadIdx.x >> 5) * scatter_warp_bytes<FEAT, BATCH, ADJ>());
-    float *const queue = slots + slot_words<BATCH, ADJ>() * kSlots;
-    uint8_t *const lists = reinterpret_cast<uint8_t *>(queue + 32 * queue_words<FEAT, BATCH, ADJ>());
+                                                   (threadIdx.x >> 5) * scatter_warp_bytes<FEAT, BATCH, ADJ>(S0.occ_stack));
+    uint8_t *const lists = reinterpret_cast<uint8_t *>(slots + slot_words<BATCH, ADJ>() * kSlots);
+    float *const queue = reinterpret_cast<float *>(lists + 3 * kSlots);
 #define ready(i) lists[i]
 #define event(i) lists[kSlots + (i)]
 #define freed(i) lists[2 * kSlots + (i)]
@@ -985,7 +1054,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                             T[k] = SLOT(wSw + k, slot) * (hit ? P.sun_color[k] : 0.0f);
                             qd[k] = rd[k];
                         }
-                    } else if (res == kTrackEscaped && !(occ && occluded(S, ro, rd))) {
+                    } else if (res == kTrackEscaped && !(occ && occluded_col<32>(S, ro, rd, queue + 32 * QueueAt<FEAT, ADJ>::stack + lane))) {
                         const bool hit = sun_hit(P, rd);
                         for (int k = 0; k < 3; ++k) {
                             const float c = SLOT(wSw + k, slot) * (hit ? P.sun_color[k] : 0.0f);
@@ -1019,7 +1088,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                     float4 sun = make_float4(SLOT(wSun, slot), SLOT(wSun + 1, slot), SLOT(wSun + 2, slot), 0.0f);
                     float4 skyv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     const bool test = occ && later;  // by the queue
-                    if (res == kTrackEscaped && (test || !(occ && occluded(S, ro, rd)))) {
+                    if (res == kTrackEscaped && (test || !(occ && occluded_col<32>(S, ro, rd, queue + 32 * QueueAt<FEAT, ADJ>::stack + lane)))) {
                         for (int k = 0; k < 3; ++k) T[k] = SLOT(wT + k, slot);
                         if (!test) {
                             const bool hit = sun_hit(P, rd);
@@ -1081,13 +1150,14 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
                     for (uint32_t pass = 0; pass < 2; ++pass) {
                         const uint32_t p = pos - 32u * pass;
                         if (queued && (pass ? pos >= 32u : pos < 32u)) {
+                            using Q = QueueAt<FEAT>;
                             for (int k = 0; k < 3; ++k) {
-                                queue[32 * k + p] = FEAT != 0 ? qd[k] : rd[k];
-                                queue[96 + 32 * k + p] = T[k];
-                                if constexpr (FEAT != 0) queue[224 + 32 * k + p] = ro[k];
+                                queue[32 * (Q::rd + k) + p] = FEAT != 0 ? qd[k] : rd[k];
+                                queue[32 * (Q::T + k) + p] = T[k];
+                                if constexpr (FEAT != 0) queue[32 * (Q::ro + k) + p] = ro[k];
                             }
-                            queue[192 + p] = __uint_as_float(off);
-                            if constexpr (FEAT != 0) queue[320 + p] = __uint_as_float(kind);
+                            queue[32 * Q::off + p] = __uint_as_float(off);
+                            if constexpr (FEAT != 0) queue[32 * Q::kind + p] = __uint_as_float(kind);
                             if constexpr (BATCH) queue[32 * (queue_words<FEAT, BATCH>() - 1) + p] = __uint_as_float(view);
                         }
                         __syncwarp();
@@ -1368,9 +1438,9 @@ static cudaError_t launch_rounds(const DevScene &S, const DevParams &P, const Ti
     const uint32_t words = grid_words(glevels);
     const size_t cam_smem = (size_t)words * 4 * kListBlock;
     const size_t sca_smem = ((table_bytes(P) + 15) & ~(size_t)15) + (size_t)words * 4 * kScatterBlock +
-                            (!feat ? scatter_warp_bytes<0, BATCH, ADJ>()
-                             : occ ? scatter_warp_bytes<kOcc, BATCH, ADJ>()
-                                   : scatter_warp_bytes<kNoOcc, BATCH, ADJ>()) *
+                            (!feat ? scatter_warp_bytes<0, BATCH, ADJ>(0u)
+                             : occ ? scatter_warp_bytes<kOcc, BATCH, ADJ>(S.occ_stack)
+                                   : scatter_warp_bytes<kNoOcc, BATCH, ADJ>(S.occ_stack)) *
                                 (kScatterBlock / 32);
     e = allow_smem(sca, sca_smem);
     if (e != cudaSuccess) return e;
@@ -1412,7 +1482,8 @@ cudaError_t launch_shadow_paths(const DevScene &S, const DevParams &P, const Til
     if (blocks == 0) return cudaSuccess;
     if (blocks > (uint64_t)sms * 8) blocks = (uint64_t)sms * 8;
     const auto fn = feat ? shadow_paths_kernel<kFeatAll> : shadow_paths_kernel<0>;
-    fn<<<(unsigned)blocks, kListBlock, (size_t)grid_words(S.glevels) * 4 * kListBlock, st>>>(S, P, A, out, C);
+    const uint32_t words = S.occ_stack > grid_words(S.glevels) ? S.occ_stack : grid_words(S.glevels);
+    fn<<<(unsigned)blocks, kListBlock, (size_t)words * 4 * kListBlock, st>>>(S, P, A, out, C);
     return cudaGetLastError();
 }
 

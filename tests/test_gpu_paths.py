@@ -195,3 +195,48 @@ def test_occluders_without_the_flag(more):
     for g in images[1:]:
         for a, b in zip(g, images[0]):
             assert np.allclose(a, b, rtol=2e-5, atol=1e-6 * np.abs(b).max() + 1e-30)
+
+
+def test_counters_repeat_with_occluders():
+    """Frames and shadow passes with occluders count the same in every launch."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    cfg = dict(c0_cfg(160, 120), depth=depth_texture(160, 120), embree=True, phase_mode=N.DR_PHASE_HG, hg_g=0.6)
+    with Renderer(0) as r:
+        r.set_occluders(occluder_surfaces())
+        r.upload(Octree(*golden_octree()))
+        r.set_params(settings_from_cfg(cfg))
+        counts = []
+        for _ in range(20):
+            r.reset_counters()
+            r.render_tile(0, 0, 160, 120, 48, seed=5, sample_base=0)
+            frame = r.counters()
+            r.reset_counters()
+            r.render_shadow_tile(0, 0, 160, 120, 48, seed=5, sample_base=0)
+            counts.append((frame, r.counters()))
+        assert all(c == counts[0] for c in counts)
+        r.set_tuning(1)  # one thread per path
+        r.reset_counters()
+        r.render_tile(0, 0, 160, 120, 48, seed=5, sample_base=0)
+        assert r.counters() == counts[0][0]
+
+
+def test_deep_occluder_tree():
+    """A fan of triangles whose boxes all overlap: a deep tree, and rays that go down both sides."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import Octree
+
+    n = 3000  # sizes over five decades make the surface-area splits uneven
+    rng = np.random.default_rng(8)
+    size = np.geomspace(1e-4, 0.5, n)[:, None, None]
+    v = (np.array([1.2, 1.0, 1.2]) + size * (1.0 + rng.normal(size=(n, 3, 3)))).reshape(-1, 3).astype(np.float32)
+    with Renderer(0) as r:
+        r.set_occluders([(v, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3), 2)])
+        r.upload(Octree(*golden_octree()))
+        got = _pair(r, dict(c0_cfg(64, 64), embree=True), (4, 4, 56, 56), 33)
+        _check(got)
+        r.set_occluders([])
+        r.set_tuning(1)
+        free = r.render_tile(4, 4, 56, 56, 33, seed=11, sample_base=2)
+        assert got[0][0][..., :3].sum() < 0.9 * free[0][..., :3].sum()
