@@ -162,7 +162,7 @@ int build_graph(dr_batch *b) {
             rest_paths += V.A.n_paths;
         }
     }
-    const bool paths = paths_serve(b->tuning, b->glevels) && b->path_rec.p;
+    const bool paths = paths_serve(b->tuning, b->glevels) && b->path_rec.p && batch_tickets_fit(b->n_paths);
     BatchArgs R = B;  // the batched kernel's views
     PathWork W{};     // and their pipeline
     uint32_t list_blocks = 0;

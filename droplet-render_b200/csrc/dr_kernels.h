@@ -40,6 +40,8 @@ struct CamLists {
 // the persistent kernel: a 64 x 64 tile at 16 samples takes 0.31 ms against 0.38, a
 // 1920 x 1080 frame at 64 samples 16.3 against 37.5.
 bool paths_serve(const Tuning &tune, uint32_t glevels);
+// Whether 32 bits number the tickets of a batch's views (view_tickets).
+bool batch_tickets_fit(uint64_t n_paths);
 // The path pipeline of a tile.  feat: the frame needs the optional features.
 // step: a batch's launch counter (its view's samples start at A.sample_base + *step * spp), or null.
 cudaError_t launch_paths(const DevScene &S, const DevParams &P, const TileArgs &A, const void *mie_pack,

@@ -506,13 +506,13 @@ __global__ void __launch_bounds__(kListBlock, ADJ ? 6 : 8) camera_paths_kernel(c
     auto tape = make_tape<ADJ>(J);
     uint32_t paths = 0;
     uint64_t total = 0;
-    uint32_t n_tickets;
+    uint64_t n_tickets;  // (a tile may have 2^32 and more)
     const uint64_t step = B.step ? *B.step : 0ull;
     if constexpr (BATCH) {
         n_tickets = W.view_tickets[B.n_views];
     } else {
         total = (uint64_t)*W.n_active * A0.spp;
-        n_tickets = (uint32_t)((total + W.ticket - 1) / W.ticket);
+        n_tickets = (total + W.ticket - 1) / W.ticket;
     }
     const unsigned long long base = W.ctl->base;
     for (;;) {
@@ -1512,6 +1512,8 @@ static uint32_t ticket_samples(uint64_t n_paths, int device) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 1;
     return n_paths < (uint64_t)sms * 8 * (kListBlock / 32) * kTicketMost * 4 ? 32u : kTicketMost;
 }
+
+bool batch_tickets_fit(uint64_t n_paths) { return n_paths / kTicketMost < 1ull << 31; }
 
 bool paths_serve(const Tuning &tune, uint32_t glevels) { return tune.traversal != 1u && glevels != 0u; }
 

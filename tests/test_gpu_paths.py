@@ -240,3 +240,31 @@ def test_deep_occluder_tree():
         r.set_tuning(1)
         free = r.render_tile(4, 4, 56, 56, 33, seed=11, sample_base=2)
         assert got[0][0][..., :3].sum() < 0.9 * free[0][..., :3].sum()
+
+
+def test_more_tickets_than_32_bits():
+    """2^39 + 4096 samples: 2^32 + 32 tickets, nearly all of them through the one leaf before the camera."""
+    import torch
+
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import build_octree
+
+    org = np.array([[0, 0, 0], [16, 16, 16], [32, 32, 32], [56, 56, 56]], np.int32)
+    oc = build_octree(org, np.full((4, 512), 0.01, np.float32), 1.0 / 64, 12)
+    spp = 2 ** 27 + 1
+    cfg = dict(c0_cfg(1920, 1080), sigma_s=1e-5, sigma_a=1e-7, scattevs=1)
+    eye = oc.nodes["ce"][np.flatnonzero(oc.nodes["volx"][:, 1] != N.DR_NONE)[1]][:3]
+    viewi = np.array(cfg["viewi"], np.float32).reshape(4, 4)
+    viewi[3, :3] = eye  # inside a leaf: every camera ray meets it
+    cfg["viewi"] = viewi.reshape(-1)
+    with Renderer(0) as r:
+        r.upload(oc)
+        r.set_params(settings_from_cfg(cfg))
+        sun, sky = (torch.zeros((64, 64, 4), device="cuda") for _ in range(2))
+        torch.cuda.synchronize()
+        r.reset_counters()
+        r.render_tile_async(930, 500, 64, 64, spp, 3, 0, sun.data_ptr(), sky.data_ptr())
+        r.synchronize()
+        c = r.counters()
+        assert c["paths"] == 4096 * spp
+        assert c["vertices"] >= 4096 * spp and c["gave_up"] == 0
