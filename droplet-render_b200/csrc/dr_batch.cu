@@ -62,7 +62,6 @@ struct dr_batch {
     DevBuf<PathCtl> path_ctl;
     DevBuf<uint32_t> path_active, view_active, view_tickets, rest_pix, rest_blocks;
     DevBuf<uint4> path_rec;
-    uint32_t rec_cap = 0;
     std::vector<BatchView> host_views;
     std::vector<size_t> out_off;  // float4 offset of view v's sun tile; its sky tile follows
     size_t out_n = 0;             // float4 count of all outputs
@@ -162,7 +161,20 @@ int build_graph(dr_batch *b) {
             rest_paths += V.A.n_paths;
         }
     }
-    const bool paths = paths_serve(b->tuning, b->glevels) && b->path_rec.p && batch_tickets_fit(b->n_paths);
+    // records of collided samples: up to 2^23 for the views rendered together and for
+    // each branch, fewer (more rounds) where the memory does not do
+    const uint32_t nbr = (uint32_t)std::min<size_t>(kBranches, own.size());
+    bool paths = paths_serve(b->tuning, b->glevels) && b->rest_blocks.p && batch_tickets_fit(b->n_paths);
+    uint64_t own_most = 0;
+    for (uint32_t v : own) own_most = std::max(own_most, b->host_views[v].A.n_paths);
+    uint32_t rec_rest = 0, rec_own = 0;
+    for (uint64_t most = 1ull << 23; paths; most >>= 1) {
+        rec_rest = (uint32_t)std::min(most, rest_paths);
+        rec_own = (uint32_t)std::min(most, own_most);
+        if (b->path_rec.reserve((size_t)rec_rest + (size_t)nbr * rec_own) == cudaSuccess) break;
+        cudaGetLastError();  // not an error of the batch: without any, the persistent kernels run
+        paths = most > 1ull << 16;
+    }
     BatchArgs R = B;  // the batched kernel's views
     PathWork W{};     // and their pipeline
     uint32_t list_blocks = 0;
@@ -174,7 +186,7 @@ int build_graph(dr_batch *b) {
         W.pool_cap = (uint32_t)b->cam_pool.n;
         W.active = b->path_active.p;
         W.records = b->path_rec.p;
-        W.cap = b->rec_cap;
+        W.cap = rec_rest;
         W.view_active = b->view_active.p;
         W.view_tickets = b->view_tickets.p;
         W.pix_begins = b->rest_pix.p;
@@ -215,7 +227,6 @@ int build_graph(dr_batch *b) {
         }
         if (!b->fork) DR_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "dr_batch: branch event");
     }
-    const uint32_t nbr = (uint32_t)std::min<size_t>(kBranches, own.size());
     DR_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "dr_batch: begin capture");
     cudaError_t e = cudaMemsetAsync(b->out.p, 0, sizeof(float4) * b->out_n, b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->work.p, 0, sizeof(WorkQueue) * b->work.n, b->stream);
@@ -231,7 +242,8 @@ int build_graph(dr_batch *b) {
             Wv.n_active = &Wv.ctl->n_active;
             Wv.head = b->cam_head.p + 2 * (size_t)pix_begins[own[k]];
             Wv.active = W.active + pix_begins[own[k]];
-            Wv.records = W.records + (size_t)(1 + k % nbr) * W.cap;
+            Wv.records = W.records + rec_rest + (size_t)(k % nbr) * rec_own;
+            Wv.cap = rec_own;
             const DevScene &S = b->host_scenes[V.scene];
             e = launch_paths(S, V.P, V.A, b->mie_pack.p, V.sun, V.sky, b->ctx->counters.p, Wv,
                              frame_features(S, V.P), b->ctx->device, b->branch[k % nbr], b->step.p);
@@ -414,16 +426,11 @@ int dr_batch_create(dr_ctx *c, const dr_scene_desc *scenes, uint32_t n_scenes, c
             b->cam_used.release();
             cudaGetLastError();  // not an error of the batch
         } else if (b->glevels) {
-            // the pipeline's storage: up to 2^23 records for the views rendered
-            // together and for each branch
-            uint64_t all = 0;
-            for (uint32_t v = 0; v < n_views; ++v) all += (uint64_t)hv[v].A.cols * hv[v].A.rows * hv[v].A.spp;
-            b->rec_cap = (uint32_t)std::min<uint64_t>(all, 1ull << 23);
+            // the pipeline's storage (build_graph adds the records)
             if (b->path_ctl.reserve(1 + kBranches) != cudaSuccess || b->path_active.reserve(n_pix) != cudaSuccess ||
                 b->view_active.reserve(n_views) != cudaSuccess || b->view_tickets.reserve(n_views + 1) != cudaSuccess ||
-                b->rest_pix.reserve(n_views) != cudaSuccess || b->rest_blocks.reserve(n_views) != cudaSuccess ||
-                b->path_rec.reserve((size_t)(1 + kBranches) * b->rec_cap) != cudaSuccess) {
-                b->path_rec.release();
+                b->rest_pix.reserve(n_views) != cudaSuccess || b->rest_blocks.reserve(n_views) != cudaSuccess) {
+                b->rest_blocks.release();
                 cudaGetLastError();  // not an error of the batch: the persistent kernels run
             }
         }

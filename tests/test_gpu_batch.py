@@ -131,3 +131,29 @@ def test_batch_rejects_mixed_phase_tables(batch_setup):
     c2["phase_mode"] = 1
     with pytest.raises(N.DrError):
         Batch(r, scenes, [BatchView(0, settings_from_cfg(c), 4), BatchView(0, settings_from_cfg(c2), 4)])
+
+
+def test_batch_memory_follows_its_branches():
+    """Four views rendered together (4.2 M paths): records for them, 67 MB, and none for
+    branches that the graph does not have (four times as much)."""
+    import torch
+
+    from droplet_b200.renderer import Batch, BatchView, Renderer
+    from droplet_b200.scene import Octree
+
+    from conftest import c0_cfg, golden_octree, settings_from_cfg
+
+    s = settings_from_cfg(c0_cfg(256, 256))
+    used = []
+    with Renderer(0) as r:
+        for _ in range(2):  # the first loads the kernels
+            free = torch.cuda.mem_get_info()[0]
+            b = Batch(r, [Octree(*golden_octree())], [BatchView(0, s, 16, k) for k in range(4)])
+            try:
+                b.set_split(0)
+                b.launch()
+                b.read(0)
+                used.append((free - torch.cuda.mem_get_info()[0]) / 1e6)
+            finally:
+                b.close()
+    assert used[1] < 150
