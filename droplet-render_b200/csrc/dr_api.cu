@@ -101,9 +101,7 @@ int dr_destroy(dr_ctx *c) {
         c->env.release();
         c->occ_tris.release();
         c->band_work.release();
-        c->lists.release();
-        c->band_lists.release();
-        c->adjoint_lists.release();
+        for (ListStore *s : {&c->lists, &c->band_lists, &c->adjoint_lists}) s->buf.release();
         for (int k = 0; k < 2; ++k)
             if (c->band_stream[k]) cudaStreamSynchronize(c->band_stream[k]), cudaStreamDestroy(c->band_stream[k]);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream), cudaStreamDestroy(c->copy_stream);
@@ -191,49 +189,13 @@ int dr_set_occluders(dr_ctx *c, const dr_surface *surfaces, uint32_t n_surfaces,
     return DR_OK;
 }
 
-// Records of collided samples kept for a render of up to `pixels` pixels (slot
-// 0: asynchronous, else one of the blocking render's two band streams, which
-// render an eighth of a large tile's rows at a time): 16 MB to 512 MB (128 MB a
-// band stream), in proportion to the pixels in between.  A render whose paths
-// may exceed it runs in rounds, and a round without work costs about 8 us.
-static uint32_t rec_capacity(size_t pixels, uint32_t slot) {
-    const size_t most = slot ? (size_t)1 << 23 : (size_t)1 << 25, want = pixels * (slot ? 4 : 16);
-    return (uint32_t)std::min(most, std::max((size_t)1 << 20, want));
-}
-
-// Leaf list entries of one pool: as dr_set_camera_lists says, else 32 a pixel (8 a
-// band stream) up to kCamPool.
-static uint32_t pool_capacity(const dr_ctx *c, size_t pixels, uint32_t slot) {
-    if (c->cam_cap_set) return c->cam_cap;
-    return (uint32_t)std::min((size_t)dr_ctx::kCamPool, std::max((size_t)1 << 18, pixels * (slot ? 8 : 32)));
-}
-
-// Storage of a launch's camera leaf lists and path pipeline for up to `pixels`
-// pixels: slot 0 for the asynchronous render, 1 and 2 (one allocation, headers
-// and active pixels shared by rows) for the band streams.  Byte offsets.
-struct ListLayout {
-    uint32_t rec_cap, pool_cap;
-    size_t records, pool, head, active, ctl, used, bytes;
-};
-static ListLayout list_layout(const dr_ctx *c, uint32_t slot, size_t pixels) {
-    const size_t two = slot ? 2 : 1;
-    ListLayout l;
-    l.rec_cap = rec_capacity(pixels, slot);
-    l.pool_cap = pool_capacity(c, pixels, slot);
-    size_t at = 0;
-    auto part = [&at](size_t bytes) {
-        const size_t o = at;
-        at += (bytes + 255) & ~(size_t)255;
-        return o;
-    };
-    l.records = part(two * l.rec_cap * sizeof(uint4));
-    l.pool = part(two * l.pool_cap * sizeof(uint4));
-    l.head = part(2 * pixels * sizeof(uint4));
-    l.active = part(pixels * sizeof(uint32_t));
-    l.ctl = part(two * sizeof(PathCtl));
-    l.used = part(two * sizeof(unsigned long long));
-    l.bytes = at;
-    return l;
+// Storage of the path pipeline and the camera lists for up to `pixels` pixels
+// (renders: the number side by side); smaller where the memory does not do.
+static bool reserve_lists(dr_ctx *c, ListStore &s, uint32_t renders, size_t pixels, size_t most_records = ~(size_t)0) {
+    const ListWant w{renders, pixels, c->cam_cap_set, c->cam_cap, most_records};
+    const bool ok = s.fit.fit(w, [&](size_t bytes) { return s.buf.reserve(bytes); });
+    cudaGetLastError();  // not an error of the call
+    return ok;
 }
 
 int dr_set_params(dr_ctx *c, const dr_render_params *p) {
@@ -266,9 +228,10 @@ int dr_set_params(dr_ctx *c, const dr_render_params *p) {
     // list and path pipeline storage for tiles up to the whole frame, so that
     // renders allocate nothing (without it they traverse per sample)
     const size_t frame = (size_t)p->w * p->h;
-    if (c->lists.reserve(list_layout(c, 0, frame).bytes) != cudaSuccess ||
-        c->band_lists.reserve(list_layout(c, 1, frame).bytes) != cudaSuccess)
-        cudaGetLastError();  // not an error of the parameters
+    for (ListStore *s : {&c->lists, &c->band_lists}) {
+        s->fit.retry();
+        reserve_lists(c, *s, s == &c->band_lists ? 2u : 1u, frame);
+    }
     return DR_OK;
 }
 
@@ -335,20 +298,19 @@ static int tile_args(const dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uin
 // The lists and pipeline storage of a launch: slot 0 for the asynchronous
 // render, 1 + (band & 1) for the blocking render's band streams (head_off: the
 // band's first pixel among the tile's headers), kAdjointLists for the adjoint
-// (laid out as slot 0, its own: it may run on another stream than a render).  A failed allocation leaves
-// the launch without (its camera segments traverse per sample).
+// (its own: it may run on another stream than a render; at most most_records
+// records).  Without any memory for it the launch goes without (its camera segments
+// traverse per sample).
 constexpr uint32_t kAdjointLists = 3;
-static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t head_off) {
+static CamLists cam_lists(dr_ctx *c, uint32_t slot, size_t head_pixels, size_t head_off,
+                          size_t most_records = ~(size_t)0) {
     CamLists L;
     // the storage follows the frame, or the tile when that is larger
     const size_t pixels = std::max(head_pixels, (size_t)c->params.w * c->params.h);
-    DevBuf<unsigned char> &buf = slot == kAdjointLists ? c->adjoint_lists : slot ? c->band_lists : c->lists;
-    if (slot == kAdjointLists) slot = 0;
-    const ListLayout l = list_layout(c, slot, pixels);
-    if (buf.reserve(l.bytes) != cudaSuccess) {
-        cudaGetLastError();  // not an error of the render
-        return L;
-    }
+    ListStore &store = slot == kAdjointLists ? c->adjoint_lists : slot ? c->band_lists : c->lists;
+    if (!reserve_lists(c, store, slot == 1u || slot == 2u ? 2u : 1u, pixels, most_records)) return L;
+    const ListLayout &l = store.fit.layout;
+    DevBuf<unsigned char> &buf = store.buf;
     const size_t second = slot == 2 ? 1 : 0;
     L.head = reinterpret_cast<uint4 *>(buf.p + l.head) + 2 * head_off;
     L.pool = reinterpret_cast<uint4 *>(buf.p + l.pool) + second * l.pool_cap;
@@ -813,7 +775,10 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
     // spread copies of the gradient: up to 16, within 256 MB
     const size_t gbytes = (size_t)c->scene.n_leaves * kBrick * sizeof(float);
     uint32_t copies = (uint32_t)std::min<size_t>(16, (256u << 20) / (gbytes ? gbytes : 1));
-    if (copies > 1 && c->grad_copies.reserve((size_t)copies * c->scene.n_leaves * kBrick) != cudaSuccess) copies = 1;
+    if (copies > 1 && c->grad_copies.reserve((size_t)copies * c->scene.n_leaves * kBrick) != cudaSuccess) {
+        copies = 1;
+        cudaGetLastError();  // not an error of the call (the launches below would report it)
+    }
     if (!c->albedo_slots.p) {
         DR_CUDA(c->albedo_slots.reserve(adjoint_slots()), "adjoint: alloc slots");
         DR_CUDA(cudaMemset(c->albedo_slots.p, 0, sizeof(double) * adjoint_slots()), "adjoint: clear slots");
@@ -823,9 +788,10 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
     // sigma_t 60 and 100 events 17) and 2^25 in all (1 GB); a path that does not fit is
     // replayed, which costs more than the launches of a further chunk (384 x 384 at 28
     // samples, sigma_t 40: two replays 43 ms, three chunks with the tape 18 ms)
-    const uint64_t per = 8 + std::min(c->params.scattevs, 24u), most_paths = (1ull << 25) / per;
-    const uint64_t row_pair = 2 * (uint64_t)A.cols * spp;
-    if (c->scene.glevels && row_pair && row_pair <= most_paths && c->scene.n_leaves < (1u << 23)) {
+    const uint64_t per = 8 + std::min(c->params.scattevs, 24u), row_pair = 2 * (uint64_t)A.cols * spp;
+    for (uint64_t tape = c->tape_most; c->scene.glevels && row_pair && c->scene.n_leaves < (1u << 23); tape >>= 1) {
+        const uint64_t most_paths = tape / per;
+        if (row_pair > most_paths) break;  // two replays
         const uint32_t rows = (uint32_t)std::min<uint64_t>(A.rows, 2 * (most_paths / row_pair));
         std::vector<TileArgs> chunks;
         uint64_t most = 0;
@@ -837,8 +803,11 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
             most = std::max(most, R.n_paths);
         }
         const uint64_t entries = std::max<uint64_t>(1ull << 16, per * most);
-        const CamLists lists = cam_lists(c, kAdjointLists, (size_t)A.cols * A.rows, 0);
-        if (lists.ctl && c->path_rec.reserve(most) == cudaSuccess && c->tape.reserve(2 * entries) == cudaSuccess) {
+        const CamLists lists = cam_lists(c, kAdjointLists, (size_t)A.cols * A.rows, 0, most);
+        if (!lists.ctl) break;
+        cudaError_t e = c->path_rec.reserve(most);
+        if (e == cudaSuccess) e = c->tape.reserve(2 * entries);
+        if (e == cudaSuccess) {
             DR_CUDA(launch_adjoint_tape(c->scene, c->params, chunks.data(), (uint32_t)chunks.size(), c->mie_pack.p,
                                         (const float4 *)dsun_dev, (const float4 *)dsky_dev, grad_bricks_dev,
                                         copies > 1 ? c->grad_copies.p : nullptr, copies, c->path_rec.p, c->tape.p,
@@ -847,7 +816,9 @@ int dr_adjoint_tile_async(dr_ctx *c, uint32_t x0, uint32_t y0, uint32_t tw, uint
                     "adjoint: launch");
             return DR_OK;
         }
-        cudaGetLastError();  // no room for the tape: two replays
+        cudaGetLastError();  // not an error of the call
+        if (e != cudaErrorMemoryAllocation) break;
+        c->tape_most = tape >> 1;  // more chunks with a smaller tape
     }
     // one 16-byte record per path of a chunk (at most 2^23 paths, 128 MB)
     const uint64_t chunk = std::min<uint64_t>(A.n_paths, 1ull << 23);

@@ -2,6 +2,7 @@
 // error reporting, device buffers, and the validation + conversion of scenes
 // and render settings into their device layouts.
 #pragma once
+#include <algorithm>
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
@@ -45,6 +46,91 @@ struct DevBuf {
         p = nullptr;
         n = 0;
     }
+};
+
+// Storage of the camera leaf lists and the path pipeline (TileArgs::cam_head,
+// PathWork) for `renders` launches side by side over up to `pixels` pixels in all:
+// headers and active pixels per pixel (shared out by rows), and for each launch a pool of list
+// entries, a buffer of collided samples and control words, in one allocation.
+constexpr uint32_t kCamPool = 1u << 23;
+struct ListWant {
+    uint32_t renders;     // 1, or 2 for the band streams of the blocking render
+    size_t pixels;
+    bool pool_set;        // dr_set_camera_lists: pool_entries, else in proportion to the pixels
+    uint32_t pool_entries;
+    size_t most_records;  // paths the launches have at most (the adjoint's chunks), or ~0
+    bool operator==(const ListWant &o) const {
+        return renders == o.renders && pixels == o.pixels && pool_set == o.pool_set && pool_entries == o.pool_entries &&
+               most_records == o.most_records;
+    }
+};
+struct ListLayout {
+    uint32_t rec_cap, pool_cap;
+    size_t records, pool, head, active, ctl, used, bytes;  // byte offsets, and their end
+};
+// shift: records and pool entries as many times halved (to no less than 2^16 and 2^14).
+inline ListLayout list_layout(const ListWant &w, uint32_t shift) {
+    ListLayout l;
+    // Records: 16 MB to 512 MB (128 MB a band stream, which renders an eighth of a
+    // large tile's rows at a time), in proportion to the pixels in between.  A render
+    // whose paths may exceed them runs in rounds, and a round without work costs about 8 us.
+    const bool two = w.renders == 2u;
+    const size_t most = two ? (size_t)1 << 23 : (size_t)1 << 25, least = (size_t)1 << 20;
+    size_t rec = std::min(most, std::max(least, w.pixels * (two ? 4 : 16)));
+    rec = std::min(rec, std::max(least, w.most_records));
+    l.rec_cap = (uint32_t)std::max(rec >> shift, std::min(rec, (size_t)1 << 16));
+    // list entries: 32 a pixel (8 a band stream) up to kCamPool
+    const size_t pool = w.pool_set ? w.pool_entries
+                                   : std::min((size_t)kCamPool, std::max((size_t)1 << 18, w.pixels * (two ? 8 : 32)));
+    l.pool_cap = (uint32_t)std::max(pool >> shift, std::min(pool, (size_t)1 << 14));
+    size_t at = 0;
+    auto part = [&at](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    l.records = part(w.renders * (size_t)l.rec_cap * sizeof(uint4));
+    l.pool = part(w.renders * (size_t)l.pool_cap * sizeof(uint4));
+    l.head = part(2 * w.pixels * sizeof(uint4));
+    l.active = part(w.pixels * sizeof(uint32_t));
+    l.ctl = part(w.renders * sizeof(PathCtl));
+    l.used = part(w.renders * sizeof(unsigned long long));
+    l.bytes = at;
+    return l;
+}
+// The largest of those layouts that the memory holds: with fewer records a render takes more
+// rounds, with a smaller pool more pixels traverse per sample, without any of it
+// the persistent kernel runs, which is half as fast.  The answer is kept until something
+// else is wanted; a lack of any memory until retry().  reserve returns a
+// cudaError_t; an error that is not about memory (a stream is being captured) says
+// nothing about the next call.
+struct ListFit {
+    ListWant want{};
+    ListLayout layout{};
+    bool known = false, ok = false;
+    void retry() { known = known && ok; }
+    template <class R> bool fit(const ListWant &w, R reserve) {
+        if (known && want == w) return ok;
+        want = w;
+        known = true;
+        ok = false;
+        size_t last = 0;
+        for (uint32_t shift = 0; shift < 32; ++shift) {
+            layout = list_layout(w, shift);
+            if (layout.bytes == last) break;  // the smallest
+            last = layout.bytes;
+            const cudaError_t e = reserve(layout.bytes);
+            ok = e == cudaSuccess;
+            if (ok) return true;
+            known = e == cudaErrorMemoryAllocation;
+            if (!known) return false;
+        }
+        return false;
+    }
+};
+struct ListStore {
+    DevBuf<unsigned char> buf;
+    ListFit fit;
 };
 
 struct DeviceGuard {
@@ -271,15 +357,12 @@ struct dr_ctx {
     cudaEvent_t band_done[kBands] = {};
     cudaEvent_t copy_done[kBands] = {};
     dr::DevBuf<dr::WorkQueue> band_work;
-    // camera leaf lists and path pipeline (TileArgs::cam_head, PathWork): headers and
-    // active pixels per pixel of a launch, a pool of list entries, a buffer of
-    // collided samples and control words, in one allocation for the asynchronous
-    // render (slot 0) and one for the two band streams of the blocking render
-    // (slots 1, 2); the adjoint has its own; laid out by list_layout
-    static constexpr uint32_t kCamPool = 1u << 23;
+    // camera leaf lists and path pipeline: the asynchronous render's storage, that of the
+    // blocking render's two band streams, and the adjoint's
     uint32_t cam_cap = 0;      // entries per pool when set (dr_set_camera_lists; 0: no lists)
     bool cam_cap_set = false;  // else in proportion to the frame, up to kCamPool
-    dr::DevBuf<unsigned char> lists, band_lists, adjoint_lists;
+    dr::ListStore lists, band_lists, adjoint_lists;
+    uint64_t tape_most = 1ull << 25;  // adjoint: tape entries (32 bytes) at most; halved while the memory does not do
     float *pinned = nullptr;  // 2 * pinned_n float4: sun then sky
     size_t pinned_n = 0;
     dr::CopyPool copies;      // host threads for the staging -> caller copies

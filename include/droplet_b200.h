@@ -181,7 +181,13 @@ int dr_set_occluders(dr_ctx *ctx, const dr_surface *surfaces, uint32_t n_surface
 int dr_build_occluder_bvh(const dr_surface *surfaces, uint32_t n_surfaces, uint32_t mode, float *nodes,
                           uint32_t *n_nodes, float *triangles, uint32_t *source, uint32_t *n_triangles);
 
-/* ---- render settings: RenderKernel::Initialize (src/kernel.cpp:497-534) ---- */
+/* ---- render settings: RenderKernel::Initialize (src/kernel.cpp:497-534) ----
+ * Also reserves the device memory that renders of the frame use beside the scene:
+ * for dr_render_tile_async about 740 MB at 1920 x 1080 (records of collided samples
+ * 16 bytes times 16 a pixel, 16 MB to 512 MB; leaf lists 16 bytes times 32 a pixel,
+ * up to 128 MB; 36 bytes a pixel), for dr_render_tile's two streams about 610 MB.
+ * Where that is not to be had, less is taken (more rounds, more pixels that
+ * traverse per sample), with the same results. */
 int dr_set_params(dr_ctx *ctx, const dr_render_params *params);
 
 /* Hosek-Wilkie state cook (src/ArHosekSkyModel.cpp:147-339) from the RGB
@@ -292,7 +298,10 @@ typedef struct {
 } dr_batch_view;
 /* Uploads every scene, copies every view's settings (and depth texture) and
  * captures the launch graph with the context's tuning (kernel forced to
- * DR_KERNEL_PERSISTENT).  Counters accumulate into the context's. */
+ * DR_KERNEL_PERSISTENT).  Counters accumulate into the context's.  Device memory
+ * beside the scenes: 32 bytes a pixel for the outputs, 36 for headers, up to 64 for leaf lists, and
+ * 128 MB of records for the views rendered together and for each of up to four
+ * branches (less for few samples, or where memory is short). */
 int dr_batch_create(dr_ctx *ctx, const dr_scene_desc *scenes, uint32_t n_scenes, const dr_batch_view *views,
                     uint32_t n_views, dr_batch **out);
 int dr_batch_destroy(dr_batch *batch);
@@ -341,7 +350,8 @@ int dr_get_majorants(dr_ctx *ctx, float *out);
  * random stream: unbiased for the expected image, with the leaf majorants held
  * fixed.  Where the path pipeline serves (leaves at one depth, fewer than 2^23 of
  * them, at most 2^20 paths in two rows) the decisions go to a tape of up to
- * 1 GB kept by the context, and paths that do not fit are replayed; without the
+ * 1 GB (less where memory is short: more chunks) kept by the context beside up to
+ * 300 MB of lists and records, and paths that do not fit are replayed; without the
  * memory, and elsewhere, every path is traced twice.  A path whose contribution is not finite is
  * left out.  Enqueued on stream (NULL = context stream). */
 int dr_adjoint_tile_async(dr_ctx *ctx, uint32_t x0, uint32_t y0, uint32_t tw, uint32_t th, uint32_t spp,

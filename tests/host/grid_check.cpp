@@ -4,6 +4,7 @@
 //   grid_check SCENE RAYS SEED    (SCENE: n_nodes, n_leaves, then the node records)
 //   grid_check flights N SEED     leaves_at_once against the flight in full
 //   grid_check pool N SEED        ranges of a leaf list pool while N lists ask for them
+//   grid_check storage N SEED     list and pipeline storage in N amounts of free memory
 #include "cuda_host_shim.h"
 #include "../../droplet-render_b200/csrc/dr_device.cuh"
 #include "../../include/droplet_b200.h"
@@ -69,8 +70,48 @@ static int pool(long long n, int seed) {
     return bad || asked < 3ull << 32;
 }
 
+static int storage(long long n, int seed) {
+    std::mt19937_64 g(seed);
+    long long bad = 0, fitted = 0, none = 0;
+    for (long long i = 0; i < n; ++i) {
+        const size_t pixels = (size_t)1 << (g() % 24);
+        ListWant w{1u + (uint32_t)(g() & 1), pixels + g() % pixels, (g() & 3) == 0, (uint32_t)(g() % (1u << 24)), ~(size_t)0};
+        if (g() & 1) w.most_records = g() % (1u << 23);
+        const size_t room = ((size_t)1 << 20) << (g() % 12);
+        int tries = 0;
+        auto reserve = [&](size_t bytes) { return ++tries, bytes <= room ? cudaSuccess : cudaErrorMemoryAllocation; };
+        ListFit f;
+        const bool ok = f.fit(w, reserve);
+        const ListLayout full = list_layout(w, 0), least = list_layout(w, 31), &l = f.layout;
+        bad += ok != (least.bytes <= room);  // some layout is found whenever the smallest fits
+        if (ok) {
+            ++fitted;
+            bad += l.bytes > room || (full.bytes <= room && l.bytes != full.bytes);
+            bad += l.rec_cap < std::min(full.rec_cap, 1u << 16) || l.pool_cap > full.pool_cap;
+            // the parts lie one after the other
+            bad += l.records + w.renders * (size_t)l.rec_cap * 16 > l.pool || l.pool + w.renders * (size_t)l.pool_cap * 16 > l.head ||
+                   l.head + w.pixels * 32 > l.active || l.active + w.pixels * 4 > l.ctl ||
+                   l.ctl + w.renders * sizeof(PathCtl) > l.used || l.used + w.renders * 8 > l.bytes;
+        }
+        none += !ok;
+        const int first = tries;  // the same wish asks for no memory again, also where there was none
+        bad += f.fit(w, reserve) != ok || tries != first;
+        f.retry();
+        bad += f.fit(w, reserve) != ok || (ok ? tries != first : tries == first);
+        ListFit other;  // any other error: nothing is kept, the next call asks again
+        bad += other.fit(w, [](size_t) { return cudaErrorStreamCaptureUnsupported; }) || other.fit(w, reserve) != ok;
+        w.pixels += 1000;  // another wish does
+        const int before = tries;
+        f.fit(w, reserve);
+        bad += tries == before;
+    }
+    std::printf("fitted %lld none %lld bad %lld\n", fitted, none, bad);
+    return bad || !fitted || !none;
+}
+
 int main(int argc, char **argv) {
     if (argc != 4) return 2;
+    if (!std::strcmp(argv[1], "storage")) return storage(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "pool")) return pool(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "flights")) return flights(atoll(argv[2]), atoi(argv[3]));
     FILE *f = std::fopen(argv[1], "rb");

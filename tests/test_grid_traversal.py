@@ -64,3 +64,8 @@ def test_first_flight_test_is_safe(check):
 def test_leaf_list_pool_beyond_32_bits(check):
     """Lists that do not fit are counted as well: the ranges stay apart when more than 2^32 entries are asked for."""
     check("pool", 500000, 5)
+
+
+def test_storage_takes_the_largest_size_that_fits(check):
+    """List and pipeline storage where memory is short: smaller, before the kernels without it; asked for once."""
+    check("storage", 200000, 11)
