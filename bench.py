@@ -41,8 +41,7 @@ GOLDEN = os.path.join(ROOT, "tests", "golden")
 W_IMG, H_IMG, SPP = 1920, 1080, 64
 METRIC = "path-vertices/s (plain renderer, single large cumulus 512^3, 1920x1080, 64 spp)"
 CPU_CROP = 384  # reference / cpu_baseline sample: centre crop at full spp (about 10 s of 16 cores)
-TRAVERSALS = {0: "octree stack traversal (local memory)", 1: "leaf-grid cell walk",
-              2: "octree stack traversal (shared memory)"}
+TRAVERSALS = {0: "octree stack traversal", 1: "leaf-grid cell walk", 2: "octree stack traversal"}
 PHASE_SAMPLER = ("the reference's Mie sampler (src/KernelSampler.cpp:258-273: interpolated scan of the red CDF), "
                  "reproduced for image parity; it fails a chi-square test against its own table (the last two "
                  "theta bins are never drawn); DR_PHASE_MIE_EXACT is the sampler that passes")
@@ -874,8 +873,7 @@ def build_large(pdf, cdf, cfgs, rads):
 
 def profile_large(crop: int, launches: int = 3, spp: int = 256):
     """Capture case for ncu: the config-4 scene, an crop x crop centre crop of
-    its 3840x2160 frame at 256 spp, the launch shape the bench renders the full
-    frame with (the shared-memory stack traversal, [0, 8, 24, 2, 0, 3, 2]),
+    its 3840x2160 frame at 256 spp, the path pipeline,
     `launches` launches; prints one line of counters."""
     import torch
 

@@ -1,24 +1,24 @@
 """Launch-shape autotuner for the persistent path kernel (single frames and batches).
 
 Octrees with their leaves at one depth (every scene the builder makes) render on
-the path pipeline, which has no launch shape: there the knobs below change nothing
-except for the cell walk and the kernel family, both slower.  Elsewhere the
-persistent kernel has seven knobs (`dr_tuning`):
+the path pipeline, which has no launch shape: there only the pipeline itself (for
+batches with the residencies that decide which views get kernels of their own), the
+cell walk and one thread per path are timed.  Elsewhere the persistent kernel has
+seven knobs (`dr_tuning`):
 * the compiled variant, i.e. resident blocks per SM. 4/5/6/8 trade registers for
   occupancy; the smaller register budgets spill a little to L1-resident local memory.
 * the event batch: how many lanes of a warp must be waiting on a segment end before
   the warp shades them.
-* the traversal: octree descent (0 and 2 are the same here), or the cell walk over
-  the leaf grid (faster where leaves are dense along rays, slower through wide
-  empty regions).
+* the traversal: octree descent (0; 2 is the same), or the cell walk over the leaf
+  grid (faster where leaves are dense along rays, slower through wide empty regions).
 * the tile: pixels handed out row-major or square by square (ray coherence).
 * the work per loop iteration: how many octree nodes the stack traversal examines
   (0: up to the next leaf) and how many free-flight steps a lane takes before the
   warp moves on; balancing them keeps traversing and tracking lanes busy alike.
 * the kernel family (persistent, or one thread per path; single frames only).
 
-`tune` searches in two stages: occupancy x event batch (for both octree stacks)
-first, then traversal x tile around the best; each candidate is timed with CUDA events on a dedicated stream.
+`tune` searches in two stages: occupancy x event batch first, then traversal x
+tile around the best; each candidate is timed with CUDA events on a dedicated stream.
 Results are cached per (GPU name, workload key) in a small JSON file, so a later run
 with the same key skips the search.
 """
@@ -31,17 +31,21 @@ import time
 from . import _native as N
 
 # occupancy x event batch
-STAGE1 = [(0, bps, batch, trav, 0, 0, 0) for trav in (0, 2) for bps in (4, 5, 6, 8) for batch in (8, 16, 24)]
+STAGE1 = [(0, bps, batch, 0, 0, 0, 0) for bps in (4, 5, 6, 8) for batch in (8, 16, 24)]
 PER_PATH = (1, 0, 0, 0, 0, 0, 0)
+# the path pipeline: no knob of a single frame; of a batch the blocks per SM (DR_BATCH_SPLIT_AUTO counts lanes)
+PIPELINE = [(0, 0, 0, 0, 0, 0, 0)]
+PIPELINE_BATCH = [(0, bps, 0, 0, 0, 0, 0) for bps in (0, 4, 6)]
+WALK = [(0, bps, 16, 1, 0, 0, 0) for bps in (4, 8)]
 
 
 def stage2(best):
     """Around the best occupancy and event batch: traversal x tile, neighbouring
     event batches, and the work per loop iteration (visits x steps)."""
     k, bps, batch = best[:3]
-    out = [(k, bps, batch, trav, tile, 0, 0) for trav in (0, 1, 2) for tile in (0, 8, 16)]
+    out = [(k, bps, batch, trav, tile, 0, 0) for trav in (0, 1) for tile in (0, 8, 16)]
     out += [(k, bps, b2, 0, 0, 0, 0) for b2 in (12, 20, 28, 32) if b2 != batch]
-    out += [(k, bps, batch, trav, 0, v, st) for trav in (0, 2) for v in (2, 3, 4, 8) for st in (1, 2, 4)]
+    out += [(k, bps, batch, 0, 0, v, st) for v in (2, 3, 4, 8) for st in (1, 2, 4)]
     return out
 
 
@@ -98,7 +102,8 @@ def time_batch(batch, repeats: int, stream) -> float:
 
 def search(target, timer, per_path: bool = True):
     """Two-stage search over target.set_tuning(*candidate), then the three fastest
-    timed again; returns (best, table)."""
+    timed again; returns (best, table).  A target on the path pipeline
+    (target.pipeline) has only the few shapes that differ there."""
     table = []
     seen = set()
 
@@ -110,10 +115,13 @@ def search(target, timer, per_path: bool = True):
             target.set_tuning(*c)
             table.append((list(c), timer()))
 
-    run(STAGE1 + ([PER_PATH] if per_path else []))
-    best = tuple(min(table, key=lambda r: r[1])[0])
-    if best[0] == 0:
-        run(stage2(best))
+    if getattr(target, "pipeline", False):
+        run((PIPELINE + WALK + [PER_PATH]) if per_path else PIPELINE_BATCH + WALK)
+    else:
+        run(STAGE1 + ([PER_PATH] if per_path else []))
+        best = tuple(min(table, key=lambda r: r[1])[0])
+        if best[0] == 0:
+            run(stage2(best))
     table.sort(key=lambda r: r[1])
     # the leaders are often within a percent of each other: time the three
     # fastest again, interleaved (clock drift falls on all alike), and keep the

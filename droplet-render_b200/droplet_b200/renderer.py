@@ -138,12 +138,24 @@ def stream_handle(torch_stream) -> int:
     return int(torch_stream.cuda_stream) or CUDA_STREAM_LEGACY
 
 
+def one_depth(nodes) -> bool:
+    """Whether an octree keeps its leaves at one depth of 2 to 9 (fewer than 2^24 of
+    them): the scenes of the path pipeline.  For the launch-shape search only; the
+    library decides by the tree itself."""
+    half = nodes["ce"][nodes["volx"].min(axis=1) != N.DR_NONE][:, 3]
+    if not len(half) or len(half) >= 1 << 24:
+        return False
+    ratio = nodes["ce"][0, 3] / half
+    return bool((np.abs(ratio - ratio[0]) < 1e-3 * ratio[0]).all() and 3.5 < ratio[0] < 600.0)
+
+
 class Renderer:
     def __init__(self, device: int = 0):
         self._ctx = C.c_void_p()
         N.check(N.lib().dr_create(int(device), C.byref(self._ctx)))
         self.device = device
         self.sample_base = 0
+        self.pipeline = False  # the scene renders on the path pipeline
 
     @property
     def handle(self) -> C.c_void_p:
@@ -175,6 +187,7 @@ class Renderer:
             sdf = np.ascontiguousarray(sdf, np.float32).reshape(-1, 512)
             d.sdf_bricks, d.n_sdf_leaves = sdf.ctypes.data, len(sdf)
         N.check(N.lib().dr_upload_scene(self._ctx, C.byref(d)))
+        self.pipeline = one_depth(nodes)
 
     def set_occluders(self, surfaces, mode: int = OCCLUDE_ALL_SURFACES):
         """Occluder meshes (SceneOcclusion): surfaces = [(vertices (n, 3), indices
@@ -415,6 +428,7 @@ class Batch:
         self._h = C.c_void_p()
         self.renderer = renderer
         N.check(N.lib().dr_batch_create(renderer.handle, descs, len(scenes), bv, len(views), C.byref(self._h)))
+        self.pipeline = all(one_depth(oc.nodes) for oc in scenes)
 
     def close(self):
         if self._h:

@@ -58,3 +58,34 @@ def test_final_stage_keeps_the_fastest_on_the_full_workload():
     assert best == (0, 8, 24, 2, 0, 3, 1) and target.tuning == best
     assert times == [((0, 5, 16, 2, 0, 4, 2), 468.0), ((0, 8, 24, 2, 0, 3, 1), 448.0)]
     assert all(n == 1 for n in target.calls.values())
+
+
+def test_pipeline_scenes_time_only_shapes_that_differ():
+    """Scenes on the path pipeline have no launch shape: no knob's duplicates are timed."""
+    for per_path, shapes in ((True, autotune.PIPELINE + autotune.WALK + [autotune.PER_PATH]),
+                             (False, autotune.PIPELINE_BATCH + autotune.WALK)):
+        target = FakeTarget()
+        target.pipeline = True
+
+        def timer():
+            target.calls[target.tuning] = target.calls.get(target.tuning, 0) + 1
+            return 50.0 + (target.tuning != shapes[0])
+
+        best, table = autotune.search(target, timer, per_path)
+        assert best == shapes[0]
+        assert sorted(target.calls) == sorted(shapes) and len(table) == len(shapes)
+    assert all(c[3] != 2 for c in autotune.STAGE1 + autotune.stage2((0, 8, 24, 0, 0, 0, 0)))
+
+
+def test_one_depth_of_scenes():
+    import numpy as np
+
+    from conftest import golden_octree
+    from droplet_b200 import _native as N
+    from droplet_b200.renderer import one_depth
+
+    nodes = golden_octree()[0].copy()
+    assert one_depth(nodes)
+    leaf = np.flatnonzero(nodes["volx"].min(axis=1) != N.DR_NONE)[3]
+    nodes["ce"][leaf, 3] *= 2  # a leaf one level up
+    assert not one_depth(nodes)
