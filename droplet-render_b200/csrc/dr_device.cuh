@@ -1091,6 +1091,7 @@ static __device__ __noinline__ float sample_voxel_far(float px, float py, float 
 // product and one fused correction); floor, ceiling and the indices by adding
 // 1.5 * 2^23 and 2^23 instead of conversions, which have an eighth of the rate.
 // Positions this far outside the brick (2^20 cells) take the lookup above.
+// (A fraction of zero may be +0 where the quotient gives -0; the density is the same.)
 __device__ __forceinline__ bool voxel_cell_inv(const float p[3], const float4 ce, float inv, uint32_t ia[3],
                                                uint32_t ib[3], float nl[3]) {
     const float cc[3] = {ce.x, ce.y, ce.z};

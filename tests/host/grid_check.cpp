@@ -4,6 +4,7 @@
 //   grid_check SCENE RAYS SEED    (SCENE: n_nodes, n_leaves, then the node records)
 //   grid_check flights N SEED     leaves_at_once against the flight in full
 //   grid_check pool N SEED        ranges of a leaf list pool while N lists ask for them
+//   grid_check exact N SEED       draws, logarithms, lookups and collision tests against the plain operations
 //   grid_check storage N SEED     list and pipeline storage in N amounts of free memory
 #include "cuda_host_shim.h"
 #include "../../droplet-render_b200/csrc/dr_device.cuh"
@@ -70,6 +71,59 @@ static int pool(long long n, int seed) {
     return bad || asked < 3ull << 32;
 }
 
+static int exact(long long n, int seed) {
+    auto bits = [](float f) { return __float_as_uint(f); };
+    long long bad[4] = {}, near = 0, close = 0;
+    for (uint32_t k = 0; k < (1u << 23); ++k) {  // every value of Rng::uniform
+        const float u = (float)(2 * k + 1) * 5.96046448e-08f;
+        bad[0] += bits(dlog_unit(u)) != bits(dlog(u));
+    }
+    std::mt19937_64 g(seed);
+    std::uniform_real_distribution<double> U(0, 1);
+    static float brick[512];
+    Rng a;
+    a.state = g();
+    a.inc = g() | 1;
+    for (long long i = 0; i < n; ++i) {
+        Rng b = a;
+        const uint32_t w = b.next();
+        bad[1] += bits(a.uniform()) != bits((float)(((w >> 9) << 1) | 1u) * 5.96046448e-08f) || a.state != b.state;
+        // rho / smax < q, also within a few ulp of the tie, and with values that are not finite
+        const float smax = (g() & 1023) ? (float)std::pow(10, -8 + 16 * U(g)) : (g() & 1) ? 0.0f : INFINITY;
+        const float q = (float)(2 * (g() >> 41) + 1) * 5.96046448e-08f;
+        float rho = (float)(smax * U(g) * ((g() & 15) ? 1.0 : -1.0));
+        if (g() & 1) {
+            rho = q * smax;
+            for (int d = (int)(g() % 17) - 8; d; d += d < 0 ? 1 : -1) rho = std::nextafterf(rho, d < 0 ? -1e30f : 1e30f);
+        }
+        if ((g() & 4095) == 0) rho = NAN;
+        bad[2] += ratio_below(rho, smax, q) != (rho / smax < q);
+        near += rho / smax == q;
+        // the lookup's cell and fractions: inside the brick, on its lattice, at its faces and far away
+        const float e = (float)std::pow(10, -6 + 8 * U(g)), inv = 1.0f / e;
+        float c[3], p[3];
+        for (int k = 0; k < 3; ++k) {
+            c[k] = (float)((g() & 3) ? e * (double)(g() % 1000) : (2 * U(g) - 1) * 100 * e);
+            const double x = (g() & 3) == 0 ? (double)(g() % 15) / 7 - 1 : (g() & 7) ? 2 * U(g) - 1 : 6 * U(g) - 3;
+            p[k] = (float)(c[k] + x * e * ((g() & 255) ? 1.0 : std::pow(10, 9 * U(g))));
+            for (int d = (int)(g() % 5) - 2; d; d += d < 0 ? 1 : -1) p[k] = std::nextafterf(p[k], d < 0 ? -1e30f : 1e30f);
+        }
+        uint32_t ia[3], ib[3], ja[3], jb[3];
+        float na[3], nb[3];
+        const float4 ce = make_float4(c[0], c[1], c[2], e);
+        if (!voxel_cell_inv(p, ce, inv, ia, ib, na)) continue;  // far: takes the plain lookup
+        ++close;
+        voxel_cell(p, ce, ja, jb, nb);
+        // (a fraction of zero may differ in its sign: the density looked up does not)
+        for (int k = 0; k < 3; ++k) bad[3] += ia[k] != ja[k] || ib[k] != jb[k] || na[k] != nb[k];
+        if (i % 64 == 0)
+            for (float &v : brick) v = (g() & 3) ? (float)U(g) : 0.0f;
+        bad[3] += bits(sample_voxel_inv(p, brick, ce, inv)) != bits(sample_voxel_space(p, brick, ce));
+    }
+    std::printf("ties %lld close %lld bad %lld %lld %lld %lld\n", near, close, bad[0], bad[1], bad[2], bad[3]);
+    return bad[0] || bad[1] || bad[2] || bad[3] || near < n / 100 || close < n / 2;
+}
+
 static int storage(long long n, int seed) {
     std::mt19937_64 g(seed);
     long long bad = 0, fitted = 0, none = 0;
@@ -111,6 +165,7 @@ static int storage(long long n, int seed) {
 
 int main(int argc, char **argv) {
     if (argc != 4) return 2;
+    if (!std::strcmp(argv[1], "exact")) return exact(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "storage")) return storage(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "pool")) return pool(atoll(argv[2]), atoi(argv[3]));
     if (!std::strcmp(argv[1], "flights")) return flights(atoll(argv[2]), atoi(argv[3]));

@@ -69,3 +69,9 @@ def test_leaf_list_pool_beyond_32_bits(check):
 def test_storage_takes_the_largest_size_that_fits(check):
     """List and pipeline storage where memory is short: smaller, before the kernels without it; asked for once."""
     check("storage", 200000, 11)
+
+
+def test_cheaper_operations_give_the_same_bits(check):
+    """Uniform draws, their logarithm, the brick lookup and the collision test without
+    conversions and divisions, against the operations they replace."""
+    check("exact", 20000000, 13)
