@@ -1084,24 +1084,46 @@ static __device__ __noinline__ float sample_voxel_far(float px, float py, float 
     return sample_voxel_space(p, v, ce);
 }
 
+// The largest (NaN if one is) and the smallest of three numbers, an instruction each.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    float m;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+#else
+    return a != a || b != b || c != c ? NAN : fmaxf(fmaxf(a, b), c);
+#endif
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    float m;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+#else
+    return fminf(fminf(a, b), c);
+#endif
+}
+
 // The same lookup where every leaf has one half extent e, inv = 1 / e rounded
 // to nearest (DevScene::ginv; 0: leaves differ).  a / e as a correctly rounded
 // quotient from the correctly rounded reciprocal (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990: one
 // product and one fused correction); floor, ceiling and the indices by adding
 // 1.5 * 2^23 and 2^23 instead of conversions, which have an eighth of the rate.
-// Positions this far outside the brick (2^20 cells) take the lookup above.
-// (A fraction of zero may be +0 where the quotient gives -0; the density is the same.)
+// Positions this far outside the brick (2^20 cells) take the lookup above, and those
+// within 2^-60 cells of its lower faces, where the correction could underflow (or lose
+// the sign of a zero).  Both bounds together, because each comparison of an axis of
+// its own costs 0.4% of a large frame.
 __device__ __forceinline__ bool voxel_cell_inv(const float p[3], const float4 ce, float inv, uint32_t ia[3],
                                                uint32_t ib[3], float nl[3]) {
     const float cc[3] = {ce.x, ce.y, ce.z};
-    bool far = inv == 0.0f;
+    float size[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float a = (-0.5f * ((cc[k] - ce.w) - p[k])) * 7.0f;
         const float q = a * inv;
         const float ni = fmaf(fmaf(-ce.w, q, a), inv, q);
-        far = far || !(fabsf(ni) < 1048576.0f);
+        size[k] = fabsf(ni);
         const float r = (ni + 12582912.0f) - 12582912.0f;  // nearest integer
         const float fl = r > ni ? r - 1.0f : r;
         const float nf = sse_max(fl, 0.0f);
@@ -1110,7 +1132,8 @@ __device__ __forceinline__ bool voxel_cell_inv(const float p[3], const float4 ce
         ia[k] = __float_as_uint(sse_min(nf, 7.0f) + 8388608.0f) & 7u;
         ib[k] = __float_as_uint(sse_max(sse_min(nc, 7.0f), 0.0f) + 8388608.0f) & 7u;
     }
-    return !far;
+    return inv != 0.0f && max3_nan(size[0], size[1], size[2]) < 1048576.0f &&
+           min3(size[0], size[1], size[2]) > 8.67361738e-19f;
 }
 
 __device__ __forceinline__ float sample_voxel_inv(const float p[3], const float *__restrict__ v, const float4 ce,

@@ -114,8 +114,7 @@ static int exact(long long n, int seed) {
         if (!voxel_cell_inv(p, ce, inv, ia, ib, na)) continue;  // far: takes the plain lookup
         ++close;
         voxel_cell(p, ce, ja, jb, nb);
-        // (a fraction of zero may differ in its sign: the density looked up does not)
-        for (int k = 0; k < 3; ++k) bad[3] += ia[k] != ja[k] || ib[k] != jb[k] || na[k] != nb[k];
+        for (int k = 0; k < 3; ++k) bad[3] += ia[k] != ja[k] || ib[k] != jb[k] || bits(na[k]) != bits(nb[k]);
         if (i % 64 == 0)
             for (float &v : brick) v = (g() & 3) ? (float)U(g) : 0.0f;
         bad[3] += bits(sample_voxel_inv(p, brick, ce, inv)) != bits(sample_voxel_space(p, brick, ce));
