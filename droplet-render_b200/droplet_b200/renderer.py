@@ -155,11 +155,16 @@ class Renderer:
         N.check(N.lib().dr_create(int(device), C.byref(self._ctx)))
         self.device = device
         self.sample_base = 0
-        self.pipeline = False  # the scene renders on the path pipeline
+        self._nodes = None  # of the uploaded scene
 
     @property
     def handle(self) -> C.c_void_p:
         return self._ctx
+
+    @property
+    def pipeline(self) -> bool:
+        """Whether the uploaded scene renders on the path pipeline."""
+        return self._nodes is not None and one_depth(self._nodes)
 
     def close(self):
         if self._ctx:
@@ -187,7 +192,7 @@ class Renderer:
             sdf = np.ascontiguousarray(sdf, np.float32).reshape(-1, 512)
             d.sdf_bricks, d.n_sdf_leaves = sdf.ctypes.data, len(sdf)
         N.check(N.lib().dr_upload_scene(self._ctx, C.byref(d)))
-        self.pipeline = one_depth(nodes)
+        self._nodes = nodes
 
     def set_occluders(self, surfaces, mode: int = OCCLUDE_ALL_SURFACES):
         """Occluder meshes (SceneOcclusion): surfaces = [(vertices (n, 3), indices
@@ -428,7 +433,12 @@ class Batch:
         self._h = C.c_void_p()
         self.renderer = renderer
         N.check(N.lib().dr_batch_create(renderer.handle, descs, len(scenes), bv, len(views), C.byref(self._h)))
-        self.pipeline = all(one_depth(oc.nodes) for oc in scenes)
+        self._nodes = [oc.nodes for oc in scenes]
+
+    @property
+    def pipeline(self) -> bool:
+        """Whether the batch renders on the path pipeline."""
+        return all(one_depth(n) for n in self._nodes)
 
     def close(self):
         if self._h:
