@@ -9,8 +9,9 @@ constexpr int kRenderBlock = 128;
 constexpr int kPersistentBlock = 128;
 
 // Dynamic shared memory above the default of 48 KB less the kernel's own (a
-// barrier) needs the kernel's opt-in on the current device.  The limit belongs to the kernel, not to a context: threads
-// that set it to what each of their launches needs fail each other's launches.
+// barrier) needs the kernel's opt-in on the current device.  The limit belongs to the
+// kernel, not to a context: threads that set it to what each of their launches needs
+// fail each other's launches.
 // So it is raised once, to all that a block can have (227 KB less the kernel's own),
 // and never lowered.
 cudaError_t raise_smem(const void *fn, size_t smem);
@@ -37,8 +38,8 @@ struct CamLists {
 };
 // Whether the path pipeline (dr_paths.cu) serves launches with this tuning:
 // scenes with a block grid, unless the cell walk is asked for.  No size is left to
-// the persistent kernel: a 64 x 64 tile at 16 samples takes 0.31 ms against 0.38, a
-// 1920 x 1080 frame at 64 samples 16.3 against 37.5.
+// the persistent kernel: a 64 x 64 tile at 16 samples takes 0.33 ms against 0.38, a
+// 1920 x 1080 frame at 64 samples 17.6 against 39.4.
 bool paths_serve(const Tuning &tune, uint32_t glevels);
 // Whether 32 bits number the tickets of a batch's views (view_tickets).
 bool batch_tickets_fit(uint64_t n_paths);

@@ -14,9 +14,12 @@
 // 119 M meet no leaf at all and about 5 M collide), those are coherent, and the
 // rest is not.  One kernel for all three (render_persistent_kernel, which
 // serves the octrees without a block grid) was bound by instruction issue at 8
-// of 32 lanes per instruction: 37.5 ms for that frame at 64 samples, 55.3 ms for a
-// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 16.3 and 21.2 ms:
-// lists 0.26, camera 2.4, scatter 13.5 ms of the first, at 13 lanes per instruction.
+// of 32 lanes per instruction: 39.4 ms for that frame at 64 samples, 63.4 ms for a
+// 1024^3 sparse slab at 1920 x 1080 x 256.  The pipeline takes 17.6 and 24.9 ms, the
+// scatter kernel at 12.5 lanes per instruction.  (Times here are those of the timing
+// cases in perf/cases.py, single passes by CUDA events, the mean of three seeds; the
+// camera and the noise differ by seed, and with them these frames by up to 9%.  The benchmark's
+// frame, another camera again, takes 16.2 ms: lists 0.21, camera 2.34, scatter 13.7.)
 //
 // Per path, the operations and random draws are those of path_sample(): a
 // path's result does not depend on the kernel that computed it.
@@ -489,7 +492,7 @@ __device__ __forceinline__ void active_sample(const TileArgs &A, const uint32_t 
 // tickets taken are exactly those done: the next round goes on from there.
 // ADJ: the adjoint's first pass (the samples of pixels without a gradient are
 // left out, nothing is counted or added to an image).  8 blocks per SM: 5 to 8 are
-// within 1% of each other (headline frame 17.7 to 17.9 ms, slab 17.4 to 17.6).
+// within 1% of each other (512^3 frame 17.65 ms, with 5 or 6 17.80; slab 24.9 and 25.1).
 template <uint32_t FEAT, bool BATCH, bool ADJ>
 __global__ void __launch_bounds__(kListBlock, ADJ ? 6 : 8) camera_paths_kernel(const __grid_constant__ DevScene S0,
                                                                      const __grid_constant__ DevParams P0,
@@ -653,10 +656,10 @@ __device__ __noinline__ bool occluded_call(const float4 *__restrict__ nodes, con
 // 32 samples side by side walk the grid together like camera samples.  Resident
 // warps loop over the samples: a warp's counters cost six additions to the same
 // words whatever it did, and with a warp per 32 samples those were the bound.
-// 960 x 540 at 16 samples: 0.76 ms, 0.98 with a thread per sample on the octree; bound
+// 960 x 540 at 16 samples: 0.72 ms, 0.96 with a thread per sample on the octree; bound
 // by the setup of the samples (48% of cycles issue).  Lanes that take a new sample
-// when theirs ends made it 1.41 to 1.55 ms (8 to 24 idle lanes at a time): the setup
-// then runs at those few lanes.
+// when theirs ends made it 1.7 to 1.9 times as long (8 to 24 idle lanes at a time):
+// the setup then runs at those few lanes.
 template <uint32_t FEAT>
 __global__ void __launch_bounds__(kListBlock, 8) shadow_paths_kernel(const __grid_constant__ DevScene S,
                                                                      const __grid_constant__ DevParams P,
@@ -871,12 +874,12 @@ __global__ void next_round_kernel(PathCtl *ctl) {
 // finds, for the lanes on their way and, when enough of them wait, the flights to
 // be computed in full; segment ends are processed when kEndBatch lanes have one.
 enum : uint32_t { kEnd = 3, kIdle = 4 };  // and kWalk, kHard, kHardAgain
-// Slots and residency were measured on the 512^3 frame: 64 slots at 4 blocks per
-// SM (128 registers) 17.8 ms, 56 at 5 20.0, 52 at 5 20.9, 48 at 6 (80 registers)
-// 27.3: more warps cost registers, L1 (the slots are shared memory) and
-// instruction cache.  Code size counts: rolling the loops of the rare parts and
-// calling instead of inlining (111 to 83 KB of code) took the frame from 19.6 to
-// 18.3 ms and instruction stalls from 1.46 to 0.57 cycles per instruction.
+// Slots and residency, on the 512^3 frame and the slab: 64 slots at 4 blocks per SM (128
+// registers) 17.65 and 24.9 ms, 56 at 5 21.0 and 28.5, 48 at 6 (80 registers) 28.3 and
+// 39.5: more warps cost registers, L1 (the slots are shared memory) and instruction
+// cache.  Code size counts: rolling the loops of the rare parts and calling instead of
+// inlining (111 to 83 KB of code) took 7% off the frame and instruction stalls from
+// 1.46 to 0.57 cycles per instruction.
 // No array of these kernels lives in local memory: with one (a stack for the
 // octree in slow_segment) beside spilled registers, the shadow kernel counted a few
 // node visits too many now and then, for a reason that was not found.  The octree's
@@ -924,8 +927,8 @@ __host__ __device__ constexpr size_t scatter_warp_bytes(uint32_t occ_stack) {
 // there too (kShadowLight: T is the segment's sun term; kEscapeLight: sun and sky),
 // so that full warps test the rays: tested where 8 to 14 of a warp's segments end,
 // the dependent loads of the tree, which the path slots leave little L1 for, took
-// half the frame (640 x 360, 32 samples, 402 triangles: 1.57 -> 1.26 ms; 0.79 without
-// occluders).
+// half the frame (640 x 360, 32 samples, 402 triangles, one seed: 1.57 -> 1.26 ms;
+// 0.79 without occluders).
 enum : uint32_t { kSkyLight = 0, kShadowLight = 1, kEscapeLight = 2 };
 // The occluder test's stack lies in the lane's column of the warp's queue: over the
 // ray of the entry, which is in registers then, or, where rays are tested in place,
@@ -1039,7 +1042,7 @@ __global__ void __launch_bounds__(kScatterBlock, MINB) scatter_kernel(const __gr
             const DevScene &S = BATCH ? B.scenes[V->scene] : S0;
             // the queue takes light as it comes; whole-path sums are needed where a path
             // that is not finite is left out, and for the adjoint.  With features but no
-            // occluders the light is cheaper in place (640 x 360, 32 samples, HG phase: no
+            // occluders the light is cheaper in place (640 x 360, 32 samples, HG phase, one seed: no
             // environment 0.72 ms a frame in place and 0.81 queued, a map 0.79 and 0.82; a
             // kernel that has both ways takes 0.81 and 0.88)
             const bool occ = (FEAT & kFeatOcc) && P.embree && S.occ_nodes;

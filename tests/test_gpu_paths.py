@@ -268,3 +268,28 @@ def test_more_tickets_than_32_bits():
         c = r.counters()
         assert c["paths"] == 4096 * spp
         assert c["vertices"] >= 4096 * spp and c["gave_up"] == 0
+
+
+@pytest.mark.parametrize("levels,leaves", [(4, 300), (7, 3000), (9, 6000)])
+def test_deep_sparse_octrees(levels, leaves):
+    """Scattered leaves in deep octrees: empty nodes of every size between them, so that
+    rays cross the upper levels of the grid.  Frames, shadow segments and every counter."""
+    from droplet_b200.renderer import Renderer
+    from droplet_b200.scene import build_octree
+
+    rng = np.random.default_rng(levels)
+    n = 15 * 2 ** (levels - 3)  # blocks a side: the root's 2^levels cells hold them at 7 voxels a block
+    cells = rng.choice(n ** 3, leaves, replace=False)
+    near = n // 2 + rng.integers(-3, 4, (leaves // 3, 3))  # a third of them close together
+    org = np.unique(np.concatenate([np.stack(np.unravel_index(cells, (n, n, n)), 1), near,
+                                    [[0, 0, 0], [n - 1] * 3]]), axis=0).astype(np.int32) * 8
+    oc = build_octree(org, rng.uniform(0.1, 1.0, (len(org), 512)).astype(np.float32), 1.0 / (8 * n), 12)
+    cfg = dict(c0_cfg(96, 80), sigma_s=40.0 * 2 ** levels, sigma_a=2.0, scattevs=12)
+    with Renderer(0) as r:
+        r.upload(oc)
+        got = _pair(r, cfg, (0, 0, 96, 80), 24)
+        assert got[0][2]["mie_evals"] > 1000
+        _check(got)
+        ro, rd = _rays(200, levels)
+        _, ref = r.adjoint_transmittance(ro, rd, np.ones(200), 500, 3, oc.n_leaves)
+        assert np.array_equal(r.probe_transmittance(ro, rd, 500, seed=3), ref) and ref.min() < 1.0
